@@ -27,12 +27,6 @@ int fail(int code, const char* msg) {
   return code;
 }
 
-// Serialises CUDA-graph construction and destruction across the handles of the process.
-std::mutex& graph_build_mutex() {
-  static std::mutex mu;
-  return mu;
-}
-
 int cuda_fail(cudaError_t e, const char* where) {
   g_err = std::string(where) + ": " + cudaGetErrorString(e);
   return GC_ERR_CUDA;
@@ -158,12 +152,9 @@ struct Pool {
   size_t pin_bytes = 0;
   int32_t* h_count = nullptr;  // pinned
   int32_t* h_ctl = nullptr;    // pinned copy of the control words
-  unsigned long long* lab_slot = nullptr;     // device: output buffer of the in-graph labels
-  unsigned long long* h_labslot = nullptr;    // pinned: its source word (inside h_count's slot)
-  uint8_t* lab_slot_val = nullptr;            // what lab_slot holds
   bool use_graph = true;
   ImageAcc* h_acc = nullptr;   // pinned
-  int grid_dis = 0, grid_warps = 0, sms = 1;
+  int grid_dis = 0, grid_warps = 0, grid_solve = 0, sms = 1;
   unsigned long long* dsum = nullptr;     // device: sum of |dI|^2 (gc_upload_rgba)
   int32_t* ntab = nullptr;                // device: n-link thresholds (gc_upload_rgba)
   bool uploaded = false, solved = false, edited = false, collect = false;
@@ -175,9 +166,11 @@ struct Pool {
   char* d_sel = nullptr;
   char* h_sel = nullptr;
   size_t sel_bytes = 0;
+  int sel_tiles = 0;                        // tiles of the current selection
   std::vector<int32_t> sel_key, sel_last;   // a selection; the one last copied to the device
   int32_t* trace_words = nullptr;   // device: trace on/off and entry count (P.trace_ctl when on)
-  bool graph_warm = false;          // the last graph solve ran the warm variant
+  bool one_launch = false;          // the last solve ran as one launch (k_solve)
+  bool lists_stale = false;         // worklists or barrier words may be left over
   gc_stats stats{};
   // profiling: event pairs around every launch, tiles processed per kernel kind
   bool prof = false;
@@ -248,7 +241,6 @@ struct Pool {
       cudaEventDestroy(done_ev);
       done_ev = nullptr;
     }
-    release_graphs();
     if (stage) cudaFree(stage);   // host-upload staging, allocated on first use
     if (arena && own_arena) cudaFree(arena);
     pinned_give(pin, pin_bytes);
@@ -262,7 +254,6 @@ struct Pool {
     tl = list = counts = stage = pts = nullptr;
     acc = nullptr; lstage = nullptr; h_count = nullptr; h_ctl = nullptr; h_acc = nullptr;
     dsum = nullptr; ntab = nullptr; d_sel = nullptr; h_sel = nullptr;
-    lab_slot = nullptr; h_labslot = nullptr; lab_slot_val = nullptr;
     trace_words = nullptr;
   }
 
@@ -299,6 +290,7 @@ struct Pool {
     c.take(&ktiles, GC_NKERN);
     c.take(&P.trace, 2 * GC_TRACE_MAX);
     c.take(&P.trace_ctl, 2);
+    c.take(&P.bar, BAR_N);
     // look-back slots: the scan uses one per 4096 items, the list rebuild one per 1024 tiles
     const int chunks = scan_chunks(nt) > nt / 1024 + 1 ? scan_chunks(nt) : nt / 1024 + 1;
     c.take(&scan.st.status, chunks);
@@ -307,7 +299,6 @@ struct Pool {
     c.take(&pts, 2 * 1024);
     c.take(&dsum, 1);
     c.take(&ntab, GC_NLINK_LEVELS);
-    c.take(&lab_slot, 1);
     if (imgs.size() == 1) c.take(&lstage, (size_t)imgs[0].W * imgs[0].H);
   }
 
@@ -410,10 +401,9 @@ struct Pool {
     pin = pinned_take(pin_bytes);
     if (!pin) { release(); return fail(GC_ERR_OOM, "pinned host allocation failed"); }
     h_count = static_cast<int32_t*>(pin);
-    h_labslot = reinterpret_cast<unsigned long long*>(static_cast<char*>(pin) + 128);
     h_ctl = reinterpret_cast<int32_t*>(static_cast<char*>(pin) + 256);
     h_acc = reinterpret_cast<ImageAcc*>(static_cast<char*>(pin) + 512);
-    {   // the kernel that ends a graph solve writes the results here itself (no copy node)
+    {   // k_solve writes the results here itself (no copy)
       void* dptr = nullptr;
       if (cudaHostGetDevicePointer(&dptr, h_ctl, 0) == cudaSuccess && dptr)
         P.host_out = static_cast<int32_t*>(dptr);
@@ -442,6 +432,7 @@ struct Pool {
     CK(cudaStreamSynchronize(cudaStreamLegacy));
     grid_dis = occupancy_discharge(device);
     grid_warps = occupancy_warps(device);
+    grid_solve = occupancy_solve(device);
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     return GC_OK;
   }
@@ -504,14 +495,15 @@ struct Pool {
   // Writes the selection of a solve (the listed images, in order) to the pinned mirror and
   // queues its copy to the device.  An image is fresh (mode 1: trivial labelling, no flood
   // before its first pulses) right after its upload, else it continues from its previous
-  // flow (mode 2); initial_relabel makes every image mode 2.  *any_warm: some image is mode 2.
+  // flow (mode 2); initial_relabel makes every image mode 2.  *any_warm / *any_fresh: some
+  // image is mode 2 / 1.
   // Repeated solves of the same images (every solve of a one-image handle) find the
   // selection already on the device and skip both copies.
-  int set_selection(const int* idx, int n, bool* any_warm, cudaStream_t s) {
+  int set_selection(const int* idx, int n, bool* any_warm, cudaStream_t s, bool* any_fresh = nullptr) {
     // n, selected tiles, then per range: first tile, tiles, first selected index, image, mode
     sel_key.assign(2 + 5 * (size_t)n, 0);
     long long start = 0;
-    bool warm = false;
+    bool warm = false, fresh = false;
     for (int k = 0; k < n; ++k) {
       const int i = idx[k];
       const ImageDesc& im = imgs[i];
@@ -523,12 +515,15 @@ struct Pool {
       e[3] = i;
       e[4] = (opts.initial_relabel || img_solved[i] || img_edited[i]) ? 2 : 1;
       warm |= e[4] == 2;
+      fresh |= e[4] == 1;
       start += tiles;
     }
     if (start > nt) return fail(GC_ERR_INTERNAL, "selection larger than the pool");
     sel_key[0] = n;
     sel_key[1] = (int)start;
     *any_warm = warm;
+    if (any_fresh) *any_fresh = fresh;
+    sel_tiles = (int)start;
     if (sel_key == sel_last) return GC_OK;
     // the previous copy out of the pinned mirror finished with the previous (synchronous) solve
     int32_t* cnt = reinterpret_cast<int32_t*>(h_sel);
@@ -559,7 +554,7 @@ struct Pool {
   // handle when captured into a graph (0: host-driven rounds)
   int global_relabel(cudaStream_t s, int first = 1) {
     RK(timed(K_MASKS, s, [&] { return launch_masks(P, grid_warps, s); }));
-    RK(timed(K_BFS_FIRST, s, [&] { return launch_bfs_round(P, first, 0, grid_warps, s); }));
+    RK(timed(K_BFS_FIRST, s, [&] { return launch_bfs_round(P, first, grid_warps, s); }));
     return frontier_rounds(s, /*flood=*/false);
   }
 
@@ -569,8 +564,8 @@ struct Pool {
     int batch = 4;
     while (true) {
       for (int k = 0; k < batch; ++k) {
-        if (flood) RK(timed(K_FLOOD, s, [&] { return launch_flood_round(P, 0, abort_hit, 0, acc, grid_warps, s); }));
-        else RK(timed(K_BFS, s, [&] { return launch_bfs_round(P, 0, 0, grid_warps, s); }));
+        if (flood) RK(timed(K_FLOOD, s, [&] { return launch_flood_round(P, 0, abort_hit, acc, grid_warps, s); }));
+        else RK(timed(K_BFS, s, [&] { return launch_bfs_round(P, 0, grid_warps, s); }));
       }
       RK(read_ctl(s));
       if (h_ctl[CTL_ERR] == 1) return fail(GC_ERR_NOT_CONVERGED, "BFS round cap reached");
@@ -638,16 +633,27 @@ struct Pool {
     }
     CK(cudaSetDevice(device));
     stats = gc_stats{};
-    bool warm = false;
-    RK(set_selection(idx, n, &warm, s));
+    bool warm = false, fresh = false;
+    RK(set_selection(idx, n, &warm, s, &fresh));
     const bool host = prof || collect || !use_graph;
-    int r = host ? solve_host(s, warm) : solve_graph(s, warm, after, lmode, lbuf);
+    one_launch = !host;
+    list_valid = false;   // the next manual push starts from a new list
+    // left by manual steps or a failed solve: worklist flags, barrier words
+    if (lists_stale) {
+      CK(cudaMemsetAsync(P.inq[0], 0, sizeof(int32_t) * nt, s));
+      CK(cudaMemsetAsync(P.inq[1], 0, sizeof(int32_t) * nt, s));
+      CK(cudaMemsetAsync(P.bar, 0, sizeof(unsigned long long) * BAR_N, s));
+    }
+    lists_stale = true;   // until this solve succeeds
+    int r = host ? solve_host(s, warm) : solve_launch(s, warm, fresh, n, after, lmode, lbuf);
     if (r) return r;
     if (host && after) {   // the host-driven solve has finished: queue the work and wait
       RK((*after)(s));
       CK(cudaStreamSynchronize(s));
     }
     RK(finish_check(s, idx, n, /*err_in_ctl=*/true));
+    one_launch = false;
+    lists_stale = host;   // the host-driven loop leaves worklist flags set
     for (int k = 0; k < n; ++k) {
       img_solved[idx[k]] = 1;
       img_edited[idx[k]] = 0;
@@ -670,11 +676,11 @@ struct Pool {
     int n = 0;
     if (warm) {
       RK(flood_phase(s, /*mode=*/3));   // its first round rebuilds the masks of edited tiles
-      RK(timed(K_COMPACT, s, [&] { return launch_flood_check(P, 1, 0, 0, s); }));
+      RK(timed(K_COMPACT, s, [&] { return launch_flood_check(P, 1, s); }));
       RK(read_ctl(s));
       if (h_ctl[CTL_LEFT] > 0) RK(bfs_phase(s));
     }
-    RK(timed(K_COMPACT, s, [&] { return launch_active_list(P, scan.st, list, counts, 0, 0, 2, 0, acc, 2 * sms, s); }));
+    RK(timed(K_COMPACT, s, [&] { return launch_active_list(P, scan.st, list, counts, 0, 0, 2, acc, 2 * sms, s); }));
     RK(read_count(s, &n));
     for (int cycle = 0; n > 0; ++cycle) {
       if (cycle >= opts.max_cycles) return fail(GC_ERR_NOT_CONVERGED, "cycle cap reached before the cut was final");
@@ -689,12 +695,12 @@ struct Pool {
         stats.pulses++;
       }
       RK(flood_phase(s, /*mode=*/2));   // its first round rebuilds the masks of changed tiles
-      RK(timed(K_COMPACT, s, [&] { return launch_flood_check(P, 0, 0, 0, s); }));
+      RK(timed(K_COMPACT, s, [&] { return launch_flood_check(P, 0, s); }));
       RK(read_ctl(s));
       n = 0;
       if (h_ctl[CTL_LEFT] > 0) {
         RK(bfs_phase(s));
-        RK(timed(K_COMPACT, s, [&] { return launch_active_list(P, scan.st, list, counts, 1, 1, 1, 0, acc, 2 * sms, s); }));
+        RK(timed(K_COMPACT, s, [&] { return launch_active_list(P, scan.st, list, counts, 1, 1, 1, acc, 2 * sms, s); }));
         RK(read_count(s, &n));
       }
     }
@@ -706,270 +712,44 @@ struct Pool {
 
   // global relabel of the live images: first round, then frontier rounds until none is left
   int bfs_phase(cudaStream_t s) {
-    RK(timed(K_BFS_FIRST, s, [&] { return launch_bfs_round(P, 2, 0, grid_warps, s); }));
+    RK(timed(K_BFS_FIRST, s, [&] { return launch_bfs_round(P, 2, grid_warps, s); }));
     return frontier_rounds(s, /*flood=*/false);
   }
 
   // flood of every image (mode 1) or of the live images (mode 2), to its end
   int flood_phase(cudaStream_t s, int mode) {
-    RK(timed(K_FLOOD_FIRST, s, [&] { return launch_flood_round(P, mode, 1, 0, acc, grid_warps, s); }));
+    RK(timed(K_FLOOD_FIRST, s, [&] { return launch_flood_round(P, mode, 1, acc, grid_warps, s); }));
     return frontier_rounds(s, /*flood=*/true, /*abort_hit=*/1);
   }
 
-  // ---- CUDA graph solve: the whole solve is one graph launch.  The loops are WHILE nodes
-  // whose conditions are set on the device (frontier rounds by their last CTA, cycles by
-  // k_ctl_cycle), so the host waits once, at the end.
-  cudaStream_t cap_stream = nullptr;
-  cudaGraphExec_t gexec[2] = {nullptr, nullptr};   // [relabel_first]
-  cudaGraph_t graph[2] = {nullptr, nullptr};
-  // Solve graphs that end with the labels of a pool's one image (gc_solve_labels), [warm]
-  // [packed]: the labels start right after the solve's last kernel instead of after the
-  // graph has left its loop nodes and ended.  Their kernels read the output buffer from a
-  // device word (lab_slot), which is set from the pinned h_labslot when the caller's buffer
-  // changes, so the graphs stay as built.
-  cudaGraphExec_t lexec[2][2] = {};
-  cudaGraph_t lgraph[2][2] = {};
-  int bl_mode = 0;   // during a build: the labels the graph ends with (0 none, 1 bytes, 2 packed)
-
-  template <class F>
-  int capture(cudaGraph_t g, std::vector<cudaGraphNode_t>& leaves, F&& fn) {
-    CK(cudaStreamBeginCaptureToGraph(cap_stream, g, leaves.empty() ? nullptr : leaves.data(),
-                                     nullptr, leaves.size(), cudaStreamCaptureModeThreadLocal));
-    const int r = fn(cap_stream);
-    cudaStreamCaptureStatus st;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t nd = 0;
-    const cudaError_t e1 = cudaStreamGetCaptureInfo(cap_stream, &st, nullptr, nullptr, &deps, &nd);
-    std::vector<cudaGraphNode_t> nl(deps, deps + (e1 == cudaSuccess ? nd : 0));
-    cudaGraph_t out = nullptr;
-    const cudaError_t e2 = cudaStreamEndCapture(cap_stream, &out);
-    if (r) return r;
-    if (e1) return cuda_fail(e1, "cudaStreamGetCaptureInfo");
-    if (e2) return cuda_fail(e2, "cudaStreamEndCapture");
-    if (!nl.empty()) leaves = nl;
-    return GC_OK;
-  }
-
-  int add_cond(cudaGraph_t g, std::vector<cudaGraphNode_t>& leaves,
-               cudaGraphConditionalHandle h, cudaGraphConditionalNodeType type, cudaGraph_t* body) {
-    cudaGraphNodeParams p{};
-    p.type = cudaGraphNodeTypeConditional;
-    p.conditional.handle = h;
-    p.conditional.type = type;
-    p.conditional.size = 1;
-    cudaGraphNode_t node;
-    CK(cudaGraphAddNode(&node, g, leaves.empty() ? nullptr : leaves.data(), leaves.size(), &p));
-    *body = p.conditional.phGraph_out[0];
-    leaves.assign(1, node);
-    return GC_OK;
-  }
-  int add_while(cudaGraph_t g, std::vector<cudaGraphNode_t>& leaves,
-                cudaGraphConditionalHandle h, cudaGraph_t* body) {
-    return add_cond(g, leaves, h, cudaGraphCondTypeWhile, body);
-  }
-  int add_if(cudaGraph_t g, std::vector<cudaGraphNode_t>& leaves,
-             cudaGraphConditionalHandle h, cudaGraph_t* body) {
-    return add_cond(g, leaves, h, cudaGraphCondTypeIf, body);
-  }
-
-  // The kernels read a conditional handle of value 0 as "not launched from a graph" (the
-  // host-driven loop passes 0).  The runtime does not promise that 0 is never a valid handle,
-  // so a handle that comes out as 0 is left unused in the graph and another one is created.
-  int cond_handle(cudaGraphConditionalHandle* h, cudaGraph_t g) {
-    for (int tries = 0; tries < 4; ++tries) {
-      CK(cudaGraphConditionalHandleCreate(h, g, 0, 0));
-      if (*h != 0) return GC_OK;
-    }
-    return fail(GC_ERR_INTERNAL, "cudaGraphConditionalHandleCreate gave only handle 0");
-  }
-
-  // A labels node of the pool's one image, into the buffer held in lab_slot.  first: the
-  // node after the first cycle's flood (it writes only when that cycle ended the solve).
-  int capture_labels(cudaGraph_t g, std::vector<cudaGraphNode_t>& L, int first) {
-    return capture(g, L, [&](cudaStream_t cs) {
-      return bl_mode == 2 ? launch_labels_packed(P, imgs[0], nullptr, cs, first, lab_slot, 4 * sms)
-                          : launch_labels_out(P, imgs[0], nullptr, cs, first, lab_slot, 4 * sms);
-    });
-  }
-
-  // Appends to g: flood first round (mode) + WHILE(frontier rounds) + the check, then
-  // IF(images left) { global relabel [+ the next cycle's active list (bump = count_cycle =
-  // 1)] }.  all: the warm prologue's flood (the solve does not end at its check; the first
-  // active list that follows decides).  first_cycle: the first cycle of a fresh solve, which
-  // runs ahead of the solve loop: the loop and its handle sit inside the IF body, after the
-  // list, so a solve that ends after one cycle never enters or leaves a loop node (each
-  // conditional node a solve passes costs several microseconds of device time).
-  int graph_cycle_tail(cudaGraph_t g, std::vector<cudaGraphNode_t>& L, int mode, int all,
-                       int bump, cudaGraphConditionalHandle hmain, bool first_cycle = false) {
-    cudaGraphConditionalHandle hf, hbfs, hb;
-    RK(cond_handle(&hf, g));
-    RK(cond_handle(&hbfs, g));
-    // the round that ends the flood runs the flood check (retires the solved images, sets
-    // the IF condition below and, when none is left, ends the solve loop and publishes)
-    const cudaGraphConditionalHandle hm = all ? 0 : hmain;
-    const int publish = all ? 0 : 1;
-    RK(capture(g, L, [&](cudaStream_t cs) {
-      return launch_flood_round(P, mode, 1, hf, acc, grid_warps, cs, all, hbfs, hm, publish);
-    }));
-    cudaGraph_t bf;
-    RK(add_while(g, L, hf, &bf));
-    {
-      std::vector<cudaGraphNode_t> Lf;
-      RK(capture(bf, Lf, [&](cudaStream_t cs) {
-        return launch_flood_round(P, 0, 1, hf, acc, grid_warps, cs, all, hbfs, hm, publish);
-      }));
-    }
-    // a graph that ends with the labels: they follow the first cycle's flood on a branch of
-    // their own (writing only when its check ended the solve), beside the IF node
-    std::vector<cudaGraphNode_t> Lq = L;
-    if (first_cycle && bl_mode) RK(capture_labels(g, Lq, 1));
-    cudaGraph_t bi;
-    RK(add_if(g, L, hbfs, &bi));
-    if (first_cycle && bl_mode) L.push_back(Lq[0]);   // what follows waits for both
-    std::vector<cudaGraphNode_t> Li;
-    RK(cond_handle(&hb, bi));
-    RK(capture(bi, Li, [&](cudaStream_t cs) { return launch_bfs_round(P, 2, hb, grid_warps, cs); }));
-    cudaGraph_t bb;
-    RK(add_while(bi, Li, hb, &bb));
-    {
-      std::vector<cudaGraphNode_t> Lb;
-      RK(capture(bb, Lb, [&](cudaStream_t cs) { return launch_bfs_round(P, 0, hb, grid_warps, cs); }));
-    }
-    if (!bump) return GC_OK;   // the first list of a solve follows the IF node
-    cudaGraphConditionalHandle hl = hmain;
-    if (first_cycle) RK(cond_handle(&hl, bi));   // the solve loop's handle, in the IF body
-    RK(capture(bi, Li, [&](cudaStream_t cs) {
-      return launch_active_list(P, scan.st, list, counts, 1, 1, 1, hl, acc, 2 * sms, cs);
-    }));
-    if (!first_cycle) return GC_OK;
-    RK(add_solve_loop(bi, Li, hl));
-    // the labels of a solve that went on past its first cycle, after its loop
-    return bl_mode ? capture_labels(bi, Li, 0) : GC_OK;
-  }
-
-  // WHILE(hloop) { pulses x discharge, then the cycle's flood, check and relabel, and the
-  // next active list, which sets hloop }
-  int add_solve_loop(cudaGraph_t g, std::vector<cudaGraphNode_t>& L,
-                     cudaGraphConditionalHandle hloop) {
-    cudaGraph_t bm;
-    RK(add_while(g, L, hloop, &bm));
-    std::vector<cudaGraphNode_t> Lm;
-    RK(capture(bm, Lm, [&](cudaStream_t cs) { return launch_pulses(cs); }));
-    return graph_cycle_tail(bm, Lm, /*mode=*/2, /*all=*/0, /*bump=*/1, hloop);
-  }
-
-  int launch_pulses(cudaStream_t s) {
-    for (int p = 0; p < opts.pulses_per_relabel; ++p)
-      RK(launch_discharge(P, opts.discharge_iters, grid_dis, s));
-    return GC_OK;
-  }
-
-  // Builds the solve graph of a variant into *gout / *eout; with bl_mode set, the graph
-  // ends with the labels of the pool's one image.
-  int build_graph(int variant, cudaGraph_t* gout, cudaGraphExec_t* eout) {
-    // One graph construction at a time in the process (building, instantiating and
-    // destroying graphs with nested conditional nodes from several threads at once was the
-    // suspected trigger of an intermittent fault under concurrent serving).
-    std::lock_guard<std::mutex> lock(graph_build_mutex());
-    if (!cap_stream) CK(cudaStreamCreateWithFlags(&cap_stream, cudaStreamNonBlocking));
-    cudaGraph_t g;
-    CK(cudaGraphCreate(&g, 0));
-    *gout = g;
-    std::vector<cudaGraphNode_t> L;
-    if (!variant) {
-      // fresh images only: the prologue and the first active list (one CTA for a small
-      // pool), then the first cycle unrolled, with the solve loop inside its IF node.  The
-      // list sets no condition: an empty one leaves nothing for the pulses, the flood finds
-      // no live image and its check ends the solve.
-      if (nt <= begin_list_max_tiles()) {
-        RK(capture(g, L, [&](cudaStream_t cs) {
-          return launch_begin_list(P, opts.max_bfs_rounds, opts.max_cycles, acc, list, counts, 0, cs);
-        }));
-      } else {
-        RK(capture(g, L, [&](cudaStream_t cs) {
-          RK(launch_ctl_begin(P, opts.max_bfs_rounds, opts.max_cycles, acc, cs));
-          return launch_active_list(P, scan.st, list, counts, 0, 0, 2, 0, acc, 2 * sms, cs);
-        }));
-      }
-      RK(capture(g, L, [&](cudaStream_t cs) { return launch_pulses(cs); }));
-      RK(graph_cycle_tail(g, L, /*mode=*/2, /*all=*/0, /*bump=*/1, 0, /*first_cycle=*/true));
-    } else {
-      cudaGraphConditionalHandle hmain;
-      RK(cond_handle(&hmain, g));
-      RK(capture(g, L, [&](cudaStream_t cs) { return launch_ctl_begin(P, opts.max_bfs_rounds, opts.max_cycles, acc, cs); }));
-      // images that continue from a previous flow: flood them; relabel the ones not solved
-      RK(graph_cycle_tail(g, L, /*mode=*/3, /*all=*/1, /*bump=*/0, hmain));
-      RK(capture(g, L, [&](cudaStream_t cs) {   // the first active list (fresh and live images)
-        return launch_active_list(P, scan.st, list, counts, 0, 0, 2, hmain, acc, 2 * sms, cs);
-      }));
-      RK(add_solve_loop(g, L, hmain));
-    }
-    if (bl_mode && variant) RK(capture_labels(g, L, 0));   // (fresh: inside the IF node)
-    if (!P.host_out) {   // else the kernel that ends the solve wrote them already
-      RK(capture(g, L, [&](cudaStream_t cs) {
-        // control words and per-image sums are adjacent on both sides: one copy
-        CK(cudaMemcpyAsync(h_ctl, P.ctl, sizeof(int32_t) * CTL_N + sizeof(ImageAcc) * imgs.size(),
-                           cudaMemcpyDeviceToHost, cs));
-        return GC_OK;
-      }));
-    }
-    CK(cudaGraphInstantiate(eout, g, 0));
-    // upload the executable graph here, under the construction lock, rather than implicitly
-    // at its first launch next to other threads' graph work
-    CK(cudaGraphUpload(*eout, cap_stream));
-    CK(cudaStreamSynchronize(cap_stream));
-    return GC_OK;
-  }
-
-
-  // variant 1: some selected image continues from a previous flow (the graph floods first).
-  // lmode 1 / 2: the graph that ends with the labels (bytes / packed) of the pool's one
-  // image, into lbuf.
-  int solve_graph(cudaStream_t s, bool warm, const After* after = nullptr, int lmode = 0,
-                  uint8_t* lbuf = nullptr) {
-    const int v = warm ? 1 : 0;
-    cudaGraphExec_t* ex = lmode ? &lexec[v][lmode - 1] : &gexec[v];
-    cudaGraph_t* gr = lmode ? &lgraph[v][lmode - 1] : &graph[v];
-    if (!*ex) {
-      bl_mode = lmode;
-      const int r = build_graph(v, gr, ex);
-      bl_mode = 0;
-      if (r) {
-        if (*ex) { cudaGraphExecDestroy(*ex); *ex = nullptr; }
-        if (*gr) { cudaGraphDestroy(*gr); *gr = nullptr; }
-        return r;
-      }
-    }
-    if (lmode && lab_slot_val != lbuf) {   // the labels kernels read their buffer from here
-      *h_labslot = (unsigned long long)(uintptr_t)lbuf;
-      CK(cudaMemcpyAsync(lab_slot, h_labslot, sizeof(unsigned long long), cudaMemcpyHostToDevice, s));
-      lab_slot_val = lbuf;
-    }
+  // The whole solve as one cooperative launch (k_solve).  lmode 1 / 2: it ends with the labels
+  // (bytes / packed) of the pool's one image, into lbuf.  As many CTAs as the device holds,
+  // but no more than selected tiles: a barrier among few CTAs is cheaper, and each tile still
+  // has a CTA of its own.
+  int solve_launch(cudaStream_t s, bool warm, bool fresh, int ranges, const After* after,
+                   int lmode, uint8_t* lbuf) {
+    SolveArgs a{};
+    a.acc = acc;
+    a.ranges = ranges;
+    a.tiles = sel_tiles;
+    a.warm = warm;
+    a.fresh = fresh;
+    a.iters = opts.discharge_iters;
+    a.pulses = opts.pulses_per_relabel;
+    a.max_rounds = opts.max_bfs_rounds;
+    a.max_cycles = opts.max_cycles;
+    a.lmode = lmode;
+    a.labels = lbuf;
+    a.im = imgs[0];
     P.ktiles = nullptr;
-    graph_warm = warm;
-    CK(cudaGraphLaunch(*ex, s));
+    const int grid = grid_solve < sel_tiles ? grid_solve : sel_tiles;
+    if (launch_solve(P, a, grid > 0 ? grid : 1, s)) return fail(GC_ERR_CUDA, "solve launch failed");
+    if (!P.host_out)   // control words and per-image sums are adjacent on both sides: one copy
+      CK(cudaMemcpyAsync(h_ctl, P.ctl, sizeof(int32_t) * CTL_N + sizeof(ImageAcc) * imgs.size(),
+                         cudaMemcpyDeviceToHost, s));
     if (after) RK((*after)(s));
     CK(cudaStreamSynchronize(s));
-    stats.launches = -1;  // inside the graph; see gc_stats
     return GC_OK;
-  }
-
-  void release_graphs() {
-    std::lock_guard<std::mutex> lock(graph_build_mutex());
-    for (int v = 0; v < 2; ++v) {
-      if (gexec[v]) cudaGraphExecDestroy(gexec[v]);
-      if (graph[v]) cudaGraphDestroy(graph[v]);
-      gexec[v] = nullptr;
-      graph[v] = nullptr;
-      for (int m = 0; m < 2; ++m) {
-        if (lexec[v][m]) cudaGraphExecDestroy(lexec[v][m]);
-        if (lgraph[v][m]) cudaGraphDestroy(lgraph[v][m]);
-        lexec[v][m] = nullptr;
-        lgraph[v][m] = nullptr;
-      }
-    }
-    if (cap_stream) cudaStreamDestroy(cap_stream);
-    cap_stream = nullptr;
   }
 
   // errors and results common to both paths (h_acc / h_ctl are filled and synchronised).
@@ -984,6 +764,7 @@ struct Pool {
     }
     if (h_ctl[CTL_ERR] == 1) return fail(GC_ERR_NOT_CONVERGED, "BFS round cap reached");
     if (h_ctl[CTL_ERR] == 2) return fail(GC_ERR_NOT_CONVERGED, "cycle cap reached before the cut was final");
+    if (h_ctl[CTL_ERR] == 5) return fail(GC_ERR_INTERNAL, "a bounded grid-barrier wait gave up");
     if (h_ctl[CTL_ERR] == 3) return fail(GC_ERR_INTERNAL, "a bounded wait for a tile copy gave up");
     if (h_ctl[CTL_ERR] == 4) {
       char msg[96];
@@ -995,13 +776,12 @@ struct Pool {
       if (h_acc[idx ? idx[k] : k].bad_caps) return fail(GC_ERR_INVALID, "negative capacity in the upload");
     stats.bfs_rounds = h_ctl[CTL_BFS_TOTAL];
     stats.flood_rounds = h_ctl[CTL_FLOOD_TOTAL];
-    if (stats.launches < 0) {  // graph solve: count the kernel nodes that ran
+    if (one_launch) {
+      // the solve's steps: the prologue (with the fresh images' first list), the pulses and
+      // every BFS / flood round
       stats.cycles = h_ctl[CTL_CYCLES];
       stats.pulses = stats.cycles * opts.pulses_per_relabel;
-      // the prologue (k_begin_list also builds the first active list), the active lists,
-      // the pulses and every BFS / flood round (the flood check runs inside the last round)
-      const bool begin_list = !graph_warm && nt <= begin_list_max_tiles();
-      stats.launches = (begin_list ? 0 : 1) + h_ctl[CTL_NACT] + stats.pulses +
+      stats.launches = (h_ctl[CTL_NACT] ? 0 : 1) + h_ctl[CTL_NACT] + stats.pulses +
                        stats.bfs_rounds + stats.flood_rounds;
     }
     for (int k = 0; k < (idx ? n : (int)imgs.size()); ++k) {
@@ -1018,11 +798,12 @@ struct Pool {
     if (!uploaded) return fail(GC_ERR_STATE, "push before upload");
     if (!list_valid) {
       RK(compact(P.tact, nullptr, s));
-      RK(launch_ctl_cycle(P, counts, 0, 0, s));
+      RK(launch_ctl_cycle(P, s));
       list_valid = true;
     }
     solved = false;
     bfs_fresh = false;
+    lists_stale = true;
     img_solved.assign(imgs.size(), 0);
     img_edited.assign(imgs.size(), 1);   // the next solve starts by flooding
     return launch_discharge(P, opts.discharge_iters, grid_dis, s);
@@ -1035,7 +816,7 @@ struct Pool {
     img_solved.assign(imgs.size(), 0);
     img_edited.assign(imgs.size(), 1);
     RK(launch_edge_relabel_build(P, list, counts, scan.st, s));
-    return launch_ctl_cycle(P, counts, 0, 0, s);
+    return launch_ctl_cycle(P, s);
   }
   int step_start_bfs(cudaStream_t s) {
     if (!uploaded) return fail(GC_ERR_STATE, "startBfs before upload");
@@ -1044,7 +825,7 @@ struct Pool {
     RK(launch_ctl_begin(P, opts.max_bfs_rounds, opts.max_cycles, acc, s));
     RK(global_relabel(s));
     RK(compact(P.tact, nullptr, s));
-    RK(launch_ctl_cycle(P, counts, 0, 0, s));
+    RK(launch_ctl_cycle(P, s));
     list_valid = true;
     bfs_fresh = true;
     return GC_OK;
@@ -1056,7 +837,7 @@ struct Pool {
     *done = n == 0;
     if (*done) {
       RK(launch_acc_reset(acc, (int)imgs.size(), s));
-      RK(launch_flood_round(P, 1, 0, 0, acc, grid_warps, s));
+      RK(launch_flood_round(P, 1, 0, acc, grid_warps, s));
       RK(frontier_rounds(s, /*flood=*/true));
       CK(cudaMemcpyAsync(h_acc, acc, sizeof(ImageAcc) * imgs.size(), cudaMemcpyDeviceToHost, s));
       RK(read_ctl(s));
@@ -1089,13 +870,8 @@ struct Pool {
     CK(cudaMemcpyAsync(trace_words, w, 2 * sizeof(int32_t), cudaMemcpyHostToDevice, s));
     CK(cudaStreamSynchronize(s));
     // the kernels take the trace words as an argument (null when off, so an untraced solve
-    // pays no load for it): switching rebuilds the solve graphs at their next use
-    int32_t* want = on ? trace_words : nullptr;
-    if (P.trace_ctl != want) {
-      if (done_ev) CK(cudaEventSynchronize(done_ev));   // no solve graph of ours in flight
-      P.trace_ctl = want;
-      release_graphs();
-    }
+    // pays no load for it)
+    P.trace_ctl = on ? trace_words : nullptr;
     return GC_OK;
   }
 
@@ -1125,7 +901,7 @@ struct Pool {
     if (n < 1 || !idx || !outs) return fail(GC_ERR_INVALID, "bad argument");
     for (int k = 0; k < n; ++k)
       if (!outs[k]) return fail(GC_ERR_INVALID, "null label buffer");
-    // a pool of one image solved by graph: the solve graph itself ends with the labels
+    // a pool of one image: the solve's launch ends with the labels
     if (n == 1 && imgs.size() == 1 && idx[0] == 0 && use_graph && !prof && !collect)
       return solve_images(idx, n, s, nullptr, packed ? 2 : 1, outs[0]);
     const After after = [&](cudaStream_t cs) {

@@ -65,14 +65,20 @@ struct PoolView {
   // null while tracing is off, so the kernels skip the mark without a memory access.
   unsigned long long* trace;
   int32_t* trace_ctl;
-  // pinned host memory (as the device sees it) that the kernel ending a graph solve writes
-  // the control words and the per-image sums to; null: the graph copies them instead
+  // pinned host memory (as the device sees it) that k_solve writes the control words and the
+  // per-image sums to; null: the host copies them instead
   int32_t* host_out;
+  unsigned long long* bar;  // [BAR_N] grid barrier of k_solve: arrivals (+ abort flag), exits
 };
 
-// Device-side loop control words.  The last CTA of every frontier round advances the round
-// parity and decides whether another round follows; in a CUDA graph it also sets the
-// condition of the enclosing WHILE node, so no host round trip is needed per round.
+// Grid barrier words: arrivals of the running k_solve (bit 63: abort) and CTAs that left it,
+// in separate 128-byte lines.  The last CTA to leave clears both for the next launch.
+enum BarSlot { BAR_ARRIVE = 0, BAR_EXIT = 16, BAR_N = 32 };
+constexpr unsigned long long GC_BAR_ABORT = 1ull << 63;
+
+// Device-side loop control words.  In the host-driven loops the last CTA of every frontier
+// round advances the round parity; k_solve keeps its loop state in registers and uses the
+// rotating counters (CTL_Q0.., CTL_F0.., CTL_H0..) and the totals.
 enum CtlSlot {
   CTL_RND = 0,        // frontier round number (its parity selects the mark buffer)
   CTL_DONE = 1,       // CTAs finished in the current round
@@ -81,7 +87,8 @@ enum CtlSlot {
   CTL_BFS_TOTAL = 4,  // BFS rounds of the solve
   CTL_FLOOD_TOTAL = 5,
   CTL_CYCLES = 6,     // global-relabel cycles of the solve
-  CTL_ERR = 7,        // 1: round cap, 2: cycle cap, 3: copy wait gave up, 4: self-check
+  CTL_ERR = 7,        // 1: round cap, 2: cycle cap, 3: copy wait gave up, 4: self-check,
+                      // 5: grid-barrier wait gave up
   CTL_MAXROUNDS = 8,
   CTL_MAXCYCLES = 9,
   CTL_PULSE = 10,     // discharge launches since the last list rebuild (parity = worklist)
@@ -95,6 +102,11 @@ enum CtlSlot {
   CTL_NACT = 16,      // active-list rebuilds run (k_active_list launches)
   CTL_LEFT = 17,      // images still running after the last flood check
   CTL_SCANERR = 18,   // the scan state's error word, as the last active list saw it
+  // k_solve's counters, three of each: a step reads one (filled by the step before), adds to
+  // the next and clears the third, so one grid barrier per step orders all three uses
+  CTL_Q0 = 20,        // worklist lengths
+  CTL_F0 = 24,        // frontier lengths
+  CTL_H0 = 28,        // images whose flood reached a sink
   CTL_N = 64          // the control words fill 256 bytes; the per-image sums follow them
 };
 
@@ -122,10 +134,11 @@ struct SelCursor {
 };
 
 // A self-check found a worklist value outside the pool: keep the first one, flag the solve
-// (the loops stop at the next check and the host returns GC_ERR_INTERNAL).
+// (it stops at its next check or barrier and the host returns GC_ERR_INTERNAL).
 __device__ __forceinline__ void record_bad(const PoolView& P, int where, int value) {
   if (atomicCAS(&P.ctl[CTL_BADWHERE], 0, where) == 0) P.ctl[CTL_BAD] = value;
   atomicCAS(&P.ctl[CTL_ERR], 0, 4);
+  atomicOr(P.bar + BAR_ARRIVE, GC_BAR_ABORT);   // a running k_solve ends at its next barrier
 }
 
 __device__ __forceinline__ unsigned long long global_ns() {

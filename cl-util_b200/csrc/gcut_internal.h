@@ -77,49 +77,42 @@ int launch_dsum(const uint32_t* rgba, int W, int H, unsigned long long* sum, int
 int launch_discharge(const PoolView& P, int iters, int grid, cudaStream_t s);
 int launch_edge_relabel_build(const PoolView& P, int32_t* list, int32_t* count,
                               const ScanState& st, cudaStream_t s);
-// h: condition of the enclosing WHILE node of a CUDA graph (0 outside graphs).
 // first: 0 frontier round, 1 first round over every tile, 2 first round over the tiles of
 // images that still had active tiles at the previous check.
-int launch_bfs_round(const PoolView& P, int first, cudaGraphConditionalHandle h, int grid,
-                     cudaStream_t s);
-// mode: 0 frontier round, 1 first round over every tile, 2 first round over the tiles of the
-// images live in this cycle; abort_hit: frontier rounds skip images that reached a sink
-// check >= 0: the round that ends the flood also runs the flood check (its `all`), with the
-// IF / WHILE handles of launch_flood_check; publish: a check that finds no image left writes
-// the results to the handle's pinned host block (the graph solve ends there)
-int launch_flood_round(const PoolView& P, int mode, int abort_hit, cudaGraphConditionalHandle h,
-                       ImageAcc* acc, int grid, cudaStream_t s, int check = -1,
-                       cudaGraphConditionalHandle hbfs = 0, cudaGraphConditionalHandle hmain = 0,
-                       int publish = 0);
+int launch_bfs_round(const PoolView& P, int first, int grid, cudaStream_t s);
+// mode: 0 frontier round; first rounds over the selected tiles: 1 all, 2 those of the images
+// live in this cycle, 3 those of the images that continue from a previous flow; abort_hit:
+// frontier rounds skip images that reached a sink
+int launch_flood_round(const PoolView& P, int mode, int abort_hit, ImageAcc* acc, int grid,
+                       cudaStream_t s);
 // retires the images whose flood reached no sink; all: every image takes part
-int launch_flood_check(const PoolView& P, int all, cudaGraphConditionalHandle hbfs,
-                       cudaGraphConditionalHandle hmain, cudaStream_t s);
+int launch_flood_check(const PoolView& P, int all, cudaStream_t s);
 int launch_ctl_begin(const PoolView& P, int max_rounds, int max_cycles, ImageAcc* acc,
                      cudaStream_t s);
 // over the solve's selected tiles; filter 1: only tiles of the images a flood check kept
 // (img_live == the cycle stamp), 2: those and the tiles of freshly uploaded images; grid:
 // most CTAs (a few per SM), which loop over the selection's chunks
 int launch_active_list(const PoolView& P, const ScanState& st, int32_t* list, int32_t* count,
-                       int bump, int count_cycle, int filter, cudaGraphConditionalHandle h,
-                       ImageAcc* acc, int grid, cudaStream_t s);
-// launch_ctl_begin followed by the first launch_active_list (filter 2, no flood before it) in
-// one single-CTA launch, for pools of at most begin_list_max_tiles() tiles
-int begin_list_max_tiles();
-int launch_begin_list(const PoolView& P, int max_rounds, int max_cycles, ImageAcc* acc,
-                      int32_t* list, int32_t* count, cudaGraphConditionalHandle h, cudaStream_t s);
+                       int bump, int count_cycle, int filter, ImageAcc* acc, int grid,
+                       cudaStream_t s);
+// The whole solve as one cooperative launch of `grid` CTAs (at most occupancy_solve()).
+struct SolveArgs {
+  ImageAcc* acc;
+  int ranges, tiles;        // the selection's size (its ranges are in P.sel)
+  int warm, fresh;          // some selected image continues from a flow / is freshly uploaded
+  int iters, pulses;        // sweeps per discharge, discharges per cycle
+  int max_rounds, max_cycles;
+  int lmode;                // 0 no labels; image im's labels: 1 a byte per pixel, 2 packed
+  uint8_t* labels;
+  ImageDesc im;
+};
+int launch_solve(const PoolView& P, const SolveArgs& a, int grid, cudaStream_t s);
 int launch_acc_reset(ImageAcc* acc, int n, cudaStream_t s);
-int launch_ctl_cycle(const PoolView& P, const int32_t* count, int count_cycle,
-                     cudaGraphConditionalHandle h, cudaStream_t s);
+int launch_ctl_cycle(const PoolView& P, cudaStream_t s);
 // neighbour ids and image index of the tiles of image img (a session-pool slot)
 int launch_image_tiles(const PoolView& P, const ImageDesc& im, int img, cudaStream_t s);
-// Inside a solve graph that ends with the labels: first = 1 for the launch after the first
-// cycle's flood (it writes only when that cycle ended the solve); slot: the device word that
-// holds the output buffer (out is then ignored); grid_cap > 0 caps the CTAs.
-int launch_labels_out(const PoolView& P, const ImageDesc& im, uint8_t* out, cudaStream_t s,
-                      int first = 0, const unsigned long long* slot = nullptr, int grid_cap = 0);
-int launch_labels_packed(const PoolView& P, const ImageDesc& im, uint8_t* out, cudaStream_t s,
-                         int first = 0, const unsigned long long* slot = nullptr,
-                         int grid_cap = 0);
+int launch_labels_out(const PoolView& P, const ImageDesc& im, uint8_t* out, cudaStream_t s);
+int launch_labels_packed(const PoolView& P, const ImageDesc& im, uint8_t* out, cudaStream_t s);
 int launch_state_out(const PoolView& P, const ImageDesc& im, const int32_t* plane,
                      int32_t* out, cudaStream_t s);
 int launch_edit(const PoolView& P, const ImageDesc& im, int img, const int32_t* idx,
@@ -143,5 +136,6 @@ int launch_view_colorize(const int32_t* values, int values_w, int values_h, int 
                          const uint32_t* base, uint32_t* out, cudaStream_t s);
 int occupancy_discharge(int device);
 int occupancy_warps(int device);
+int occupancy_solve(int device);
 
 }  // namespace gcut

@@ -382,9 +382,10 @@ k_masks(PoolView P) {
 // neighbour's height under the same bound.  Flow leaving the tile is added to the
 // neighbour's excess and reverse residual with atomics at the end of the tile.
 //
-// Active tiles form a worklist: the launch reads queue[c] (c = pulse parity, device-side)
-// and appends, deduplicated by inq[c ^ 1], every tile that is still active or received flow
-// to queue[c ^ 1]; the last CTA advances the parity.  One launch per pulse, no compaction.
+// Active tiles form a worklist: a pulse reads queue[c] (c = pulse parity) and appends,
+// deduplicated by inq[c ^ 1], every tile that is still active or received flow to
+// queue[c ^ 1].  No compaction between pulses; the last pulse before a relabel appends
+// nothing in k_solve, since the relabel rebuilds the list.
 // ------------------------------------------------------------------------------------
 struct DisSmem {
   int32_t hs[GC_TILE_PX];   // heights
@@ -401,13 +402,18 @@ struct DisSmem {
   int32_t xu[GC_TILE], xd[GC_TILE], xl[GC_TILE], xr[GC_TILE];
 };
 
-__device__ __forceinline__ void worklist_add(const PoolView& P, int nxt, int t) {
-  if (*((volatile int32_t*)&P.inq[nxt][t]) != 0) return;   // common case: already queued
-  if (atomicExch(&P.inq[nxt][t], 1) == 0) {
-    const int pos = atomicAdd(&P.qcount[nxt], 1);
-    if (pos < P.nt) P.queue[nxt][pos] = t;   // inq deduplicates, so pos < nt always holds
-    else record_bad(P, 1, pos);
-  }
+// A worklist of tiles: list, length, and the per-tile flag that keeps a tile in it once.
+struct Worklist { int32_t *list, *count, *in; };
+
+__device__ __forceinline__ void worklist_append(const PoolView& P, const Worklist& w, int t) {
+  const int pos = atomicAdd(w.count, 1);
+  if (pos < P.nt) w.list[pos] = t;   // each tile at most once, so pos < nt always holds
+  else record_bad(P, 1, pos);
+}
+
+__device__ __forceinline__ void worklist_add(const PoolView& P, const Worklist& w, int t) {
+  if (*((volatile int32_t*)&w.in[t]) != 0) return;   // common case: already queued
+  if (atomicExch(&w.in[t], 1) == 0) worklist_append(P, w, t);
 }
 
 __device__ __forceinline__ int4 lds4(const int32_t* p) { return *reinterpret_cast<const int4*>(p); }
@@ -474,24 +480,17 @@ __device__ __forceinline__ void dis_prefetch(const PoolView& P, int t, int32_t* 
     bulk_g2s(buf + k * GC_TILE_PX, dis_plane(P, k) + (long long)t * GC_TILE_PX, GC_TILE_PX * 4, mbar);
 }
 
-__global__ void __launch_bounds__(DIS_THREADS, 4)
-k_discharge(PoolView P, int iters) {
-  trace_mark(P, TR_DISCHARGE);
-  extern __shared__ __align__(128) int32_t dsm[];
-  int32_t* const buf = dsm;                                    // [6][1024] staging
-  DisSmem& S = *reinterpret_cast<DisSmem*>(dsm + DIS_PLANES * GC_TILE_PX);
-  __shared__ uint64_t mbar;
-  __shared__ int s_cur, s_n, s_sent;
+// Discharges the n tiles of list `in` with the CTAs 0 .. nb-1 (this is CTA `bid`); the tiles
+// active afterwards or sent flow go to list `out` (none: out.list null).  buf, S and mbar are
+// the CTA's staging buffer, exchange arrays and (initialised) mbarrier; `phase` its parity,
+// kept from call to call.  Every thread of the CTA calls it.
+__device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, int bid, int nb_ctas,
+                                                const Worklist& in, int n, const Worklist& out,
+                                                int32_t* buf, DisSmem& S, uint64_t* mbar,
+                                                unsigned& phase) {
+  __shared__ int s_sent;
   const int tid = threadIdx.x;
   const int r = tid >> 3, q = tid & 7, c0 = q * 4;
-  if (tid == 0) {
-    s_cur = *((volatile int32_t*)&P.ctl[CTL_PULSE]) & 1;
-    s_n = *((volatile int32_t*)&P.qcount[s_cur]);
-    mbar_init(&mbar, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  const int cur = s_cur, nxt = cur ^ 1;
   // Bookkeeping log: each finished tile leaves (tile, neighbours, flags) here, and the CTA's
   // threads settle up to DIS_LOG tiles at once (its list entry, and the list entries and
   // dirty flags of the neighbours it sent flow to), so the dependent L2 round trips of that
@@ -510,25 +509,23 @@ k_discharge(PoolView P, int iters) {
         P.touched[target] = 1;
         mark_dirty(P, target);   // its masks are rebuilt by the next flood's first round
         if (k == 0) P.act_int[tt] = (f >> 5) & 1;
-        if (k != 0 || ((f >> 4) & 1)) worklist_add(P, nxt, target);
+        if (out.list && (k != 0 || ((f >> 4) & 1))) worklist_add(P, out, target);
         if (k == 0 && P.ktiles) atomicAdd(&P.ktiles[K_DISCHARGE], 1ull);
       }
     }
   };
-  int n = s_n;
   if (n < 0 || n > P.nt) {   // self-check: a list never holds more than every tile once
-    if (tid == 0 && blockIdx.x == 0) record_bad(P, 2, n);
+    if (tid == 0 && bid == 0) record_bad(P, 2, n);
     n = 0;
   }
   // list entry li: every position below the checked count was written with a tile id of
   // the pool (by worklist_add or the compaction) before this launch
-  auto entry = [&](int li) { return P.queue[cur][li]; };
+  auto entry = [&](int li) { return in.list[li]; };
   const bool erow = (r == 0) || (r == 31);
   const int pix = r * GC_TILE + c0;
-  unsigned phase = 0;
-  bool failed = false, pending = false;
-  if (tid == 0 && (int)blockIdx.x < n) dis_prefetch(P, entry(blockIdx.x), buf, &mbar);
-  for (int li = blockIdx.x; li < n; li += gridDim.x) {
+  bool failed = false;
+  if (tid == 0 && bid < n) dis_prefetch(P, entry(bid), buf, mbar);
+  for (int li = bid; li < n; li += nb_ctas) {
     const int t = entry(li);
     const int4 nb = P.nbr[t];
     if (tid < 32) S.hu[tid] = nb.x >= 0 ? P.hgt[(long long)nb.x * GC_TILE_PX + 31 * GC_TILE + tid] : GC_HINF;
@@ -539,9 +536,9 @@ k_discharge(PoolView P, int iters) {
     else if (tid < 192) S.xd[tid - 160] = 0;
     else if (tid < 224) S.xl[tid - 192] = 0;
     else S.xr[tid - 224] = 0;
-    if (tid == 0) { P.inq[cur][t] = 0; s_sent = 0; }
-    const bool ok = mbar_wait(&mbar, phase);
-    if (__syncthreads_or(!ok)) { failed = true; pending = true; break; }  // block-uniform
+    if (tid == 0) { in.in[t] = 0; s_sent = 0; }
+    const bool ok = mbar_wait(mbar, phase);
+    if (__syncthreads_or(!ok)) { failed = true; break; }  // block-uniform
     phase ^= 1u;
     int e[4], h[4], cu[4], cd[4], cl[4], cr[4];
     {
@@ -574,7 +571,7 @@ k_discharge(PoolView P, int iters) {
     sts4(S.hs + pix, h[0], h[1], h[2], h[3]);
     __syncthreads();   // every thread has its values in registers: the buffer is free
     // prefetch this CTA's next tile into the buffer while this one is worked on
-    if (tid == 0 && li + (int)gridDim.x < n) dis_prefetch(P, entry(li + gridDim.x), buf, &mbar);
+    if (tid == 0 && li + nb_ctas < n) dis_prefetch(P, entry(li + nb_ctas), buf, mbar);
 
     for (int it = 0; it < iters; ++it) {
       // neighbour heights (fixed during the push phase)
@@ -796,13 +793,36 @@ k_discharge(PoolView P, int iters) {
     // a bulk copy did not complete in time: record it, let our copy drain, stop
     if (tid == 0) {
       atomicExch(&P.ctl[CTL_ERR], 3);
-      if (pending) mbar_wait(&mbar, phase, 5 * GC_COPY_WAIT_NS);
+      atomicOr(P.bar + BAR_ARRIVE, GC_BAR_ABORT);
+      mbar_wait(mbar, phase, 5 * GC_COPY_WAIT_NS);
     }
     __syncthreads();
   }
+}
+
+// One pulse of the host-driven loop or of a manual push: the worklist of the pulse parity.
+__global__ void __launch_bounds__(DIS_THREADS, 4)
+k_discharge(PoolView P, int iters) {
+  trace_mark(P, TR_DISCHARGE);
+  extern __shared__ __align__(128) int32_t dsm[];
+  DisSmem& S = *reinterpret_cast<DisSmem*>(dsm + DIS_PLANES * GC_TILE_PX);
+  __shared__ uint64_t mbar;
+  __shared__ int s_cur, s_n;
+  if (threadIdx.x == 0) {
+    s_cur = *((volatile int32_t*)&P.ctl[CTL_PULSE]) & 1;
+    s_n = *((volatile int32_t*)&P.qcount[s_cur]);
+    mbar_init(&mbar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  const int cur = s_cur, nxt = cur ^ 1;
+  const Worklist in{P.queue[cur], P.qcount + cur, P.inq[cur]};
+  const Worklist out{P.queue[nxt], P.qcount + nxt, P.inq[nxt]};
+  unsigned phase = 0;
+  discharge_phase(P, iters, blockIdx.x, gridDim.x, in, s_n, out, dsm, S, &mbar, phase);
   // last CTA: the queue just read is consumed; the next launch reads the other one
   __syncthreads();
-  if (tid == 0) {
+  if (threadIdx.x == 0) {
     __threadfence();
     const int d = atomicAdd(&P.ctl[CTL_DDONE], 1);
     if (d == (int)gridDim.x - 1) {
@@ -991,10 +1011,9 @@ __device__ __forceinline__ uint32_t tile_bfs_seeded(int* row, uint32_t sink, uin
 // tiles (grid-stride over the selection); round r > 0 processes the list fq[r & 1] built by
 // round r - 1.  A tile whose boundary
 // values changed queues its neighbours in fq[(r + 1) & 1], deduplicated by mark[(r + 1) & 1];
-// the round that processes a tile clears its mark.  Only the CTAs the list needs take part
-// (at least one, so every launched round is finalised), and the last of them consumes the
-// list, advances the round number (device memory, ctl[CTL_RND]) and, inside a CUDA graph,
-// sets the WHILE condition: another round runs only when the next list is not empty.
+// the round that processes a tile clears its mark.  In the host-driven loops only the CTAs
+// the list needs take part (at least one, so every launched round is finalised), and the last
+// of them consumes the list and advances the round number (device memory, ctl[CTL_RND]).
 __device__ __forceinline__ int frontier_round_number(const PoolView& P, int first) {
   return first ? 0 : *((volatile int32_t*)&P.ctl[CTL_RND]);
 }
@@ -1029,18 +1048,17 @@ __device__ __forceinline__ void frontier_work(const PoolView& P, int first, int 
 
 // Queue tile t for the next round (once).  Within a round the next round's marks only go
 // from 0 to 1, so a set mark read with a plain load needs no atomic.
-__device__ __forceinline__ void frontier_push(const PoolView& P, int out, int t) {
-  if (*((volatile int32_t*)&P.mark[out][t]) != 0) return;
-  if (atomicExch(&P.mark[out][t], 1) == 0) {
-    const int pos = atomicAdd(&P.fcount[out], 1);
-    if (pos < P.nt) P.fq[out][pos] = t;   // the mark deduplicates, so pos < nt always holds
+__device__ __forceinline__ void frontier_push(const PoolView& P, const Worklist& out, int t) {
+  if (*((volatile int32_t*)&out.in[t]) != 0) return;
+  if (atomicExch(&out.in[t], 1) == 0) {
+    const int pos = atomicAdd(out.count, 1);
+    if (pos < P.nt) out.list[pos] = t;   // the mark deduplicates, so pos < nt always holds
     else record_bad(P, 5, pos);
   }
 }
 
 __device__ __forceinline__ void frontier_round_end(const PoolView& P, int first, int in,
-                                                   int total_slot, int participants,
-                                                   cudaGraphConditionalHandle h) {
+                                                   int total_slot, int participants) {
   __syncthreads();
   if (threadIdx.x != 0) return;
   __threadfence();
@@ -1058,13 +1076,9 @@ __device__ __forceinline__ void frontier_round_end(const PoolView& P, int first,
   ctl[CTL_ROUNDS] = rounds;
   ctl[total_slot] = ctl[total_slot] + 1;
   ctl[CTL_DONE] = 0;
-  bool more = next > 0 && ctl[CTL_ERR] < 3;   // a copy or self-check error ends the loop
-  if (more && rounds >= ctl[CTL_MAXROUNDS]) {
-    ctl[CTL_ERR] = 1;
-    more = false;
-  }
+  const bool more = next > 0 && ctl[CTL_ERR] < 3;   // a copy or self-check error ends the loop
+  if (more && rounds >= ctl[CTL_MAXROUNDS]) ctl[CTL_ERR] = 1;
   __threadfence();
-  if (h) cudaGraphSetConditional(h, more ? 1u : 0u);
 }
 
 // Solve prologue: reset the control words and the image stamps; the images of the
@@ -1096,22 +1110,19 @@ __global__ void k_ctl_begin(PoolView P, int max_rounds, int max_cycles, ImageAcc
   }
 }
 
-// The solve's results written straight into pinned host memory by the kernel that ends a
-// graph solve, so the graph needs no copy node after its loops: the control words, then the
-// sums of the solve's images at their places in the host mirror (the other images' sums have
-// not changed since their own solves).  Threads 0 .. nthreads-1 take part.  The host reads
-// the block only after synchronising with the solve's stream, which makes every write of the
-// finished kernels visible to it, so no system-scope fence is needed here (one cost about
-// 1 % of a 2048^2 step: the labels that follow waited for it).
-__device__ __forceinline__ void publish_results(const PoolView& P, const ImageAcc* acc,
-                                                int nthreads) {
+// The solve's results written straight into pinned host memory by k_solve, so no copy follows
+// it: the control words, then the sums of the solve's images at their places in the host
+// mirror (the other images' sums have not changed since their own solves).  One CTA calls it.
+// The host reads the block only after synchronising with the solve's stream, which makes
+// every write of the finished kernel visible to it, so no system-scope fence is needed.
+__device__ __forceinline__ void publish_results(const PoolView& P, const ImageAcc* acc) {
   if (!P.host_out) return;
   constexpr int AW = (int)(sizeof(ImageAcc) / sizeof(int32_t));
   int nr = *((volatile int32_t*)&P.nsel[0]);
   nr = nr < 0 ? 0 : nr > P.nimg ? P.nimg : nr;
   const volatile int32_t* c = P.ctl;
   const volatile int32_t* a = reinterpret_cast<const volatile int32_t*>(acc);
-  for (int i = threadIdx.x; i < CTL_N + AW * nr; i += nthreads) {
+  for (int i = threadIdx.x; i < CTL_N + AW * nr; i += blockDim.x) {
     if (i < CTL_N) {
       P.host_out[i] = c[i];
     } else {
@@ -1152,7 +1163,7 @@ __device__ __forceinline__ void stamp_image(const PoolView& P, ImageAcc* acc, in
 
 __global__ void __launch_bounds__(ACT_THREADS)
 k_active_list(PoolView P, ScanState st, int32_t* list, int32_t* count, int bump,
-              int count_cycle, int filter, cudaGraphConditionalHandle h, ImageAcc* acc) {
+              int count_cycle, int filter, ImageAcc* acc) {
   trace_mark(P, TR_ACTIVE_LIST);
   __shared__ int32_t sm[32];
   __shared__ int32_t s_chunk, s_excl, s_cur, s_n, s_nr;
@@ -1261,145 +1272,88 @@ k_active_list(PoolView P, ScanState st, int32_t* list, int32_t* count, int bump,
   // a look-back that gave up (here or in an earlier list of this solve) reaches the host
   // with the control words
   ctl[CTL_SCANERR] = ctl[CTL_SCANERR] | *((volatile int32_t*)st.err);
-  bool more = nact > 0 && ctl[CTL_ERR] < 3;
-  if (more && cycles >= ctl[CTL_MAXCYCLES]) {
-    ctl[CTL_ERR] = 2;
-    more = false;
-  }
+  if (nact > 0 && ctl[CTL_ERR] < 3 && cycles >= ctl[CTL_MAXCYCLES]) ctl[CTL_ERR] = 2;
   __threadfence();
-  if (h) cudaGraphSetConditional(h, more ? 1u : 0u);
-  if (h && !more) publish_results(P, acc, 1);   // the graph solve ends here
 }
 
-// k_ctl_begin and the first active-tile list of a solve of fresh images only (no flood
-// precedes that list), in one CTA for pools of at most BL_MAX tiles: the reset, a barrier,
-// then the list with a block-wide scan instead of a look-back, and the list's cycle check.
-// One launch instead of two, and none of the multi-CTA list's tickets and waits.
-constexpr int BL_THREADS = 1024;
-constexpr int BL_ITEMS = 4;
-constexpr int BL_MAX = BL_THREADS * BL_ITEMS;
-
-__global__ void __launch_bounds__(BL_THREADS)
-k_begin_list(PoolView P, int max_rounds, int max_cycles, ImageAcc* acc, int32_t* list,
-             int32_t* count, cudaGraphConditionalHandle h) {
-  trace_mark(P, TR_BEGIN);
-  __shared__ int32_t sm[32];
-  const int tid = threadIdx.x, lane = tid & 31;
-  for (int i = tid; i < CTL_N; i += BL_THREADS) P.ctl[i] = 0;
-  for (int i = tid; i < P.nimg; i += BL_THREADS) {
-    P.img_live[i] = 0;
-    P.img_hit[i] = 0;
-    P.img_mode[i] = 0;
-  }
-  __syncthreads();
-  int nr = *((volatile int32_t*)&P.nsel[0]), n = *((volatile int32_t*)&P.nsel[1]);
-  if (n < 0 || n > P.nt || n > BL_MAX || nr < 0 || nr > P.nimg) {   // self-check
-    if (tid == 0) record_bad(P, 9, n);
-    n = nr = 0;
-  }
-  for (int k = tid; k < nr; k += BL_THREADS) {
-    const int img = P.sel[k].w;
-    if ((unsigned)img >= (unsigned)P.nimg) continue;
-    P.img_mode[img] = P.sel_mode[k];
-    acc[img].sumpos_e = 0;   // the floods of this solve accumulate it
-  }
-  if (tid == 0) {
-    P.ctl[CTL_MAXROUNDS] = max_rounds;
-    P.ctl[CTL_MAXCYCLES] = max_cycles;
-    P.rcnt[0] = 0;
-    P.rcnt[1] = 0;
-    P.fcount[0] = 0;
-    P.fcount[1] = 0;
-    trace_record(P, TR_ACTIVE_LIST);
-  }
-  __syncthreads();   // the modes above are visible to every thread
-  // the list: active tiles of the fresh images (cycle stamp 1)
-  const int stamp = 1;
-  const int base = tid * BL_ITEMS;
-  SelCursor cursor(P, nr, base < n ? base : 0);
-  int32_t v[BL_ITEMS], tl[BL_ITEMS], im[BL_ITEMS];
-#pragma unroll
-  for (int k = 0; k < BL_ITEMS; ++k) {
-    tl[k] = -1;
-    im[k] = -1;
-    if (base + k < n) {
-      tl[k] = cursor.tile(base + k);
-      im[k] = cursor.image();
-    }
-    v[k] = 0;
-    if ((unsigned)tl[k] < (unsigned)P.nt && (unsigned)im[k] < (unsigned)P.nimg)
-      v[k] = P.tact[tl[k]] != 0 && P.img_mode[im[k]] == 1;
-    else if (tl[k] >= 0)
-      record_bad(P, 4, (unsigned)im[k] < (unsigned)P.nimg ? tl[k] : im[k]);
-  }
-  int32_t tsum = 0, first = -1;
-#pragma unroll
-  for (int k = BL_ITEMS - 1; k >= 0; --k) {
-    tsum += v[k];
-    if (v[k]) first = im[k];
-  }
-  int32_t agg;
-  int32_t run = block_exclusive_scan(tsum, sm, &agg);
-  const unsigned peers = __match_any_sync(0xffffffffu, first);
-  if (first >= 0 && __ffs(peers) - 1 == lane) stamp_image(P, acc, first, stamp);
-  int last = first;
-#pragma unroll
-  for (int k = 0; k < BL_ITEMS; ++k) {
-    if (v[k]) {
-      if ((unsigned)run < (unsigned)P.nt) list[run] = tl[k];
-      if (im[k] != last) {
-        stamp_image(P, acc, im[k], stamp);
-        last = im[k];
-      }
-      ++run;
-    }
-  }
-  if (tid != 0) return;
-  // the cycle check of k_active_list (count_cycle 0: no cycle has run yet)
-  *count = agg;
-  volatile int32_t* ctl = P.ctl;
-  ctl[CTL_PULSE] = 0;   // the list sits in queue[0]
-  ctl[CTL_DDONE] = 0;
-  P.qcount[1] = 0;
-  ctl[CTL_NACT] = 1;
-  bool more = agg > 0 && ctl[CTL_ERR] < 3;
-  if (more && ctl[CTL_MAXCYCLES] <= 0) {
-    ctl[CTL_ERR] = 2;
-    more = false;
-  }
-  __threadfence();
-  if (h) cudaGraphSetConditional(h, more ? 1u : 0u);
-  if (h && !more) publish_results(P, acc, 1);   // the graph solve ends here
-}
-
-// After the active-tile compaction: another cycle runs while tiles are active and the cycle
-// cap is not reached (`count_cycle` counts this check as a finished cycle).
-__global__ void k_ctl_cycle(PoolView P, const int32_t* count, int count_cycle,
-                            cudaGraphConditionalHandle h) {
+// After the active-tile compaction of a manual step: the list becomes the first worklist.
+__global__ void k_ctl_cycle(PoolView P) {
   if (threadIdx.x != 0) return;
   volatile int32_t* ctl = P.ctl;
   ctl[CTL_PULSE] = 0;   // the compacted list sits in queue[0]
   ctl[CTL_DDONE] = 0;
   P.qcount[1] = 0;
-  int cycles = ctl[CTL_CYCLES] + (count_cycle ? 1 : 0);
-  ctl[CTL_CYCLES] = cycles;
-  bool more = *((volatile const int32_t*)count) > 0 && ctl[CTL_ERR] < 3;
-  if (more && cycles >= ctl[CTL_MAXCYCLES]) {
-    ctl[CTL_ERR] = 2;
-    more = false;
-  }
   __threadfence();
-  if (h) cudaGraphSetConditional(h, more ? 1u : 0u);
+}
+
+// One tile of a global relabel, by one warp: the in-tile BFS seeded by the tile's sink pixels
+// and (frontier rounds) the halo distances, the heights written back, and the neighbours whose
+// edge distances dropped queued.  T: the warp's 32 x 33 words of shared memory.  Returns
+// whether the tile holds an active pixel.
+__device__ __forceinline__ int bfs_tile(const PoolView& P, int t, int lane, int first, int32_t* T,
+                                        const Worklist& out) {
+  const int4 nb = P.nbr[t];
+  const long long base = (long long)t * GC_TILE_PX;
+  // the masks are current: the flood that precedes every global relabel of a solve (or
+  // k_masks, before gc_start_bfs) rebuilt every tile that changed since they were written
+  const uint32_t* mc = P.mcan + (long long)t * 128;
+  const uint32_t canU = mc[lane], canD = mc[32 + lane], canL = mc[64 + lane], canR = mc[96 + lane];
+  const uint32_t sink = P.msink[(long long)t * 32 + lane];
+  // seeds from the neighbour tiles' heights (frontier rounds only): an edge pixel with a
+  // residual edge into the neighbour starts at the neighbour's height + 1
+  int top = GC_HINF, bot = GC_HINF, sl = GC_HINF, sr = GC_HINF;
+  if (!first) {
+    const uint32_t cu0 = __shfl_sync(0xffffffffu, canU, 0);
+    const uint32_t cd31 = __shfl_sync(0xffffffffu, canD, 31);
+    const int vu = nb.x >= 0 ? P.hgt[(long long)nb.x * GC_TILE_PX + 31 * GC_TILE + lane] : GC_HINF;
+    const int vd = nb.y >= 0 ? P.hgt[(long long)nb.y * GC_TILE_PX + lane] : GC_HINF;
+    const int vl = nb.z >= 0 ? P.hgt[(long long)nb.z * GC_TILE_PX + lane * GC_TILE + 31] : GC_HINF;
+    const int vr = nb.w >= 0 ? P.hgt[(long long)nb.w * GC_TILE_PX + lane * GC_TILE] : GC_HINF;
+    if (((cu0 >> lane) & 1u) && vu < GC_HINF) top = vu + 1;
+    if (((cd31 >> lane) & 1u) && vd < GC_HINF) bot = vd + 1;
+    if ((canL & 1u) && vl < GC_HINF) sl = vl + 1;
+    if ((canR >> 31) && vr < GC_HINF) sr = vr + 1;
+  }
+  const uint32_t fin = tile_bfs_seeded(T + lane * 33, sink, canU, canD, canL, canR, lane, top,
+                                       bot, sl, sr);
+  __syncwarp();
+  int chU = 0, chD = 0, chL = 0, chR = 0;
+  for (int rr = 0; rr < 32; ++rr) {
+    const int nv = T[rr * 33 + lane];
+    int* p = P.hgt + base + rr * GC_TILE + lane;
+    if (first) {
+      *p = nv;
+      const int fv = nv < GC_HINF;
+      chU |= (rr == 0) & fv; chD |= (rr == 31) & fv; chL |= (lane == 0) & fv; chR |= (lane == 31) & fv;
+    } else {
+      const int ov = *p;
+      if (nv != ov) *p = nv;
+      const int dec = nv < ov;
+      chU |= (rr == 0) & dec; chD |= (rr == 31) & dec; chL |= (lane == 0) & dec; chR |= (lane == 31) & dec;
+    }
+  }
+  __syncwarp();
+  chU = __any_sync(0xffffffffu, chU); chD = __any_sync(0xffffffffu, chD);
+  chL = __any_sync(0xffffffffu, chL); chR = __any_sync(0xffffffffu, chR);
+  const uint32_t pos = P.mexc[(long long)t * 32 + lane];
+  const int act = __any_sync(0xffffffffu, (pos & fin) != 0);
+  // the neighbours to queue, one lane each (their atomics run in parallel)
+  if (lane < 4) {
+    const int go = lane == 0 ? chU : lane == 1 ? chD : lane == 2 ? chL : chR;
+    const int nt = lane == 0 ? nb.x : lane == 1 ? nb.y : lane == 2 ? nb.z : nb.w;
+    if (go && nt >= 0) frontier_push(P, out, nt);
+  }
+  return act;
 }
 
 __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
-k_bfs_round(PoolView P, int first, cudaGraphConditionalHandle h) {
+k_bfs_round(PoolView P, int first) {
   trace_mark(P, first ? TR_BFS_FIRST : TR_BFS);
   __shared__ int32_t tr[WARPS_PER_CTA][32 * 33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int in = frontier_round_number(P, first) & 1, out = in ^ 1;
+  const int in = frontier_round_number(P, first) & 1;
+  const Worklist out{P.fq[in ^ 1], P.fcount + (in ^ 1), P.mark[in ^ 1]};
   int32_t* const markin = P.mark[in];
-  int32_t* T = tr[warp];
   int done = 0;
   // first == 2: a global relabel inside the solve loop skips images whose cut was final at
   // the previous check (no active tile); their state no longer changes
@@ -1428,79 +1382,23 @@ k_bfs_round(PoolView P, int first, cudaGraphConditionalHandle h) {
       }
     }
     ++done;
-    const int4 nb = P.nbr[t];
-    const long long base = (long long)t * GC_TILE_PX;
-    // the masks are current: the flood that precedes every global relabel of a solve (or
-    // k_masks, before gc_start_bfs) rebuilt every tile that changed since they were written
-    const uint32_t* mc = P.mcan + (long long)t * 128;
-    const uint32_t canU = mc[lane], canD = mc[32 + lane], canL = mc[64 + lane], canR = mc[96 + lane];
-    const uint32_t sink = P.msink[(long long)t * 32 + lane];
-    // seeds from the neighbour tiles' heights (frontier rounds only): an edge pixel with a
-    // residual edge into the neighbour starts at the neighbour's height + 1
-    int top = GC_HINF, bot = GC_HINF, sl = GC_HINF, sr = GC_HINF;
-    if (!first) {
-      const uint32_t cu0 = __shfl_sync(0xffffffffu, canU, 0);
-      const uint32_t cd31 = __shfl_sync(0xffffffffu, canD, 31);
-      const int vu = nb.x >= 0 ? P.hgt[(long long)nb.x * GC_TILE_PX + 31 * GC_TILE + lane] : GC_HINF;
-      const int vd = nb.y >= 0 ? P.hgt[(long long)nb.y * GC_TILE_PX + lane] : GC_HINF;
-      const int vl = nb.z >= 0 ? P.hgt[(long long)nb.z * GC_TILE_PX + lane * GC_TILE + 31] : GC_HINF;
-      const int vr = nb.w >= 0 ? P.hgt[(long long)nb.w * GC_TILE_PX + lane * GC_TILE] : GC_HINF;
-      if (((cu0 >> lane) & 1u) && vu < GC_HINF) top = vu + 1;
-      if (((cd31 >> lane) & 1u) && vd < GC_HINF) bot = vd + 1;
-      if ((canL & 1u) && vl < GC_HINF) sl = vl + 1;
-      if ((canR >> 31) && vr < GC_HINF) sr = vr + 1;
-    }
-    const uint32_t fin = tile_bfs_seeded(T + lane * 33, sink, canU, canD, canL, canR, lane, top,
-                                         bot, sl, sr);
-    __syncwarp();
-    int chU = 0, chD = 0, chL = 0, chR = 0;
-    for (int rr = 0; rr < 32; ++rr) {
-      const int nv = T[rr * 33 + lane];
-      int* p = P.hgt + base + rr * GC_TILE + lane;
-      if (first) {
-        *p = nv;
-        const int fv = nv < GC_HINF;
-        chU |= (rr == 0) & fv; chD |= (rr == 31) & fv; chL |= (lane == 0) & fv; chR |= (lane == 31) & fv;
-      } else {
-        const int ov = *p;
-        if (nv != ov) *p = nv;
-        const int dec = nv < ov;
-        chU |= (rr == 0) & dec; chD |= (rr == 31) & dec; chL |= (lane == 0) & dec; chR |= (lane == 31) & dec;
-      }
-    }
-    __syncwarp();
-    chU = __any_sync(0xffffffffu, chU); chD = __any_sync(0xffffffffu, chD);
-    chL = __any_sync(0xffffffffu, chL); chR = __any_sync(0xffffffffu, chR);
-    const uint32_t pos = P.mexc[(long long)t * 32 + lane];
-    const int act = __any_sync(0xffffffffu, (pos & fin) != 0);
+    const int act = bfs_tile(P, t, lane, first, tr[warp], out);
     if (lane == 0) P.tact[t] = act;
-    // the neighbours to queue, one lane each (their atomics run in parallel)
-    if (lane < 4) {
-      const int go = lane == 0 ? chU : lane == 1 ? chD : lane == 2 ? chL : chR;
-      const int nt = lane == 0 ? nb.x : lane == 1 ? nb.y : lane == 2 ? nb.z : nb.w;
-      if (go && nt >= 0) frontier_push(P, out, nt);
-    }
   }
   if (lane == 0 && done) {
     atomicAdd(&P.rcnt[in], done);
     if (P.ktiles) atomicAdd(&P.ktiles[first ? K_BFS_FIRST : K_BFS], (unsigned long long)done);
   }
-  frontier_round_end(P, first, in, CTL_BFS_TOTAL, parts, h);
+  frontier_round_end(P, first, in, CTL_BFS_TOTAL, parts);
 }
 
-// After a flood: an image whose flood reached no sink pixel is solved (its flood is the
-// canonical cut, its sums are final) and leaves the live set; the others go on to a global
-// relabel.  all != 0: the images that continue from a previous flow (img_mode == 2; the
-// first check of a solve); else the images live in this cycle.  Sets the condition of the
-// IF node around the relabel (hbfs) and, when no image is left, ends the solve loop (hmain,
-// 0 outside the loop) and, with `publish`, writes the results to the host (the graph solve
-// ends here); the last cycle of a solve is counted here.  Every thread of one CTA calls it: k_flood_check,
-// or the last CTA of the flood's last round, which reads what the round's other CTAs wrote
-// (their fence before the round's count orders it), hence the volatile loads.
-__device__ void flood_check_cta(const PoolView& P, int all, cudaGraphConditionalHandle hbfs,
-                                cudaGraphConditionalHandle hmain, int publish,
-                                const ImageAcc* acc) {
-  __shared__ int s_left, s_n;
+// After a flood of the host-driven loop: an image whose flood reached no sink pixel is solved
+// (its flood is the canonical cut, its sums are final) and leaves the live set; the others go
+// on to a global relabel.  all != 0: the images that continue from a previous flow
+// (img_mode == 2; the first check of a solve); else the images live in this cycle.  The last
+// cycle of a solve is counted here.  One CTA.
+__global__ void k_flood_check(PoolView P, int all) {
+  __shared__ int s_left;
   if (threadIdx.x == 0) {
     s_left = 0;
     trace_record(P, TR_CHECK);
@@ -1522,61 +1420,13 @@ __device__ void flood_check_cta(const PoolView& P, int all, cudaGraphConditional
   }
   if (left) atomicAdd(&s_left, left);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int n = s_left;
-    if (ctl[CTL_ERR] != 0) n = 0;   // a cap or a self-check ends the loops
-    ctl[CTL_LEFT] = n;
-    ctl[CTL_NCHECK] = ctl[CTL_NCHECK] + 1;
-    if (n == 0 && !all) ctl[CTL_CYCLES] = ctl[CTL_CYCLES] + 1;
-    __threadfence();
-    if (hbfs) cudaGraphSetConditional(hbfs, n > 0 ? 1u : 0u);
-    if (hmain && n == 0) cudaGraphSetConditional(hmain, 0u);
-    if (n == 0) trace_record(P, TR_END);
-    s_n = n;
-  }
-  __syncthreads();
-  if (s_n == 0 && publish) publish_results(P, acc, blockDim.x);   // the graph solve ends here
-}
-
-// End of a flood round: frontier_round_end's bookkeeping by the round's last CTA; when the
-// flood is over (no frontier left, or a cap), that CTA runs the flood check too (check >= 0
-// is its `all`), so the solve graph needs no separate check launch.  Every thread calls it.
-__device__ __forceinline__ void flood_round_end(const PoolView& P, int first, int in, int parts,
-                                                cudaGraphConditionalHandle h, int check,
-                                                cudaGraphConditionalHandle hbfs,
-                                                cudaGraphConditionalHandle hmain, int publish,
-                                                const ImageAcc* acc) {
-  __shared__ int s_last, s_more;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    s_last = atomicAdd(&P.ctl[CTL_DONE], 1) == parts - 1;
-    if (s_last) {
-      __threadfence();
-      volatile int32_t* ctl = P.ctl;
-      const int out = in ^ 1;
-      P.rcnt[in] = 0;
-      const int next = *((volatile int32_t*)&P.fcount[out]);
-      P.fcount[in] = 0;   // this round's list is consumed
-      ctl[CTL_LASTCNT] = next;
-      ctl[CTL_RND] = first ? 1 : ctl[CTL_RND] + 1;
-      const int rounds = first ? 1 : ctl[CTL_ROUNDS] + 1;
-      ctl[CTL_ROUNDS] = rounds;
-      ctl[CTL_FLOOD_TOTAL] = ctl[CTL_FLOOD_TOTAL] + 1;
-      ctl[CTL_DONE] = 0;
-      bool more = next > 0 && ctl[CTL_ERR] < 3;   // a copy or self-check error ends the loop
-      if (more && rounds >= ctl[CTL_MAXROUNDS]) {
-        ctl[CTL_ERR] = 1;
-        more = false;
-      }
-      __threadfence();
-      if (h) cudaGraphSetConditional(h, more ? 1u : 0u);
-      s_more = more;
-    }
-  }
-  __syncthreads();
-  if (!s_last || check < 0 || s_more) return;
-  flood_check_cta(P, check, hbfs, hmain, publish, acc);
+  if (threadIdx.x != 0) return;
+  int n = s_left;
+  if (ctl[CTL_ERR] != 0) n = 0;   // a cap or a self-check ends the loops
+  ctl[CTL_LEFT] = n;
+  ctl[CTL_NCHECK] = ctl[CTL_NCHECK] + 1;
+  if (n == 0 && !all) ctl[CTL_CYCLES] = ctl[CTL_CYCLES] + 1;
+  if (n == 0) trace_record(P, TR_END);
 }
 
 // ------------------------------------------------------------------------------------
@@ -1586,22 +1436,124 @@ __device__ __forceinline__ void flood_round_end(const PoolView& P, int first, in
 // The flood also decides termination: an excess pixel can reach a sink pixel exactly when
 // the flood from the excess pixels reaches one, so an image whose flood reaches no sink
 // pixel is solved (its flood is the canonical cut) and one whose flood does needs another
-// global relabel and push cycle.  Every round stamps img_hit[img] with the cycle stamp
-// (ctl[CTL_CYCLES] + 1) when a tile's reached set meets its sink pixels.
-//
-// mode: 0 frontier round; first rounds over the selected tiles: 1 all of them, 2 those of the
-// images live in this cycle (img_live == stamp), 3 those of the images that continue from a
-// previous flow (img_mode == 2).  abort_hit: frontier rounds skip the tiles of images already
-// stamped (their flood is redone in a later cycle).
+// global relabel and push cycle.  Every round stamps img_hit[img] with the flood's stamp
+// when a tile's reached set meets its sink pixels.
 // ------------------------------------------------------------------------------------
+// Sum of max(excess, 0) of the tiles a warp has flooded, added to an image's word when the
+// image changes (flood_sum_flush adds the rest, once per image and CTA).
+struct FloodSum {
+  int img = -1;
+  unsigned long long sum = 0;
+  __device__ __forceinline__ void add(ImageAcc* acc, int i, long long v) {
+    if (i != img) {
+      if (sum) atomicAdd(&acc[img].sumpos_e, sum);
+      img = i;
+      sum = 0;
+    }
+    sum += (unsigned long long)v;
+  }
+};
+
+// One tile of a flood round, by one warp.  hits: counts the images whose sink-reached stamp
+// this flood sets (null: not counted).
+__device__ __forceinline__ void flood_tile(const PoolView& P, int t, int lane, int first, int img,
+                                           int stamp, int32_t* hits, const Worklist& out,
+                                           ImageAcc* acc, FloodSum& fs) {
+  const int4 nb = P.nbr[t];
+  uint32_t canU, canD, canL, canR, sink, R, R0;
+  long long ps = 0;
+  if (first && P.mdirty[t] != 0) {
+    // the tile changed since its masks were written (a discharge or an edit): rebuild them
+    // here, before anything reads them (every tile of an image this round covers is done
+    // in this round, so the frontier rounds and the global relabel after it see them)
+    const RowMasks m = warp_rebuild_masks(P, t, lane, &ps);
+    canU = m.up; canD = m.down; canL = m.left; canR = m.right;
+    sink = m.sink;
+    R = m.exc;
+  } else {
+    const uint32_t* mc = P.mcan + (long long)t * 128;
+    canU = mc[lane]; canD = mc[32 + lane]; canL = mc[64 + lane]; canR = mc[96 + lane];
+    sink = P.msink[(long long)t * 32 + lane];
+    if (first) {
+      R = P.mexc[(long long)t * 32 + lane];
+      ps = P.tpos[t];
+    }
+  }
+  if (first) {
+    R0 = 0;
+    if (lane == 0 && ps) fs.add(acc, img, ps);   // taken with the tile's masks
+  } else {
+    R = R0 = P.mreach[(long long)t * 32 + lane];
+    if (lane == 0 && nb.x >= 0)
+      R |= P.mreach[(long long)nb.x * 32 + 31] & P.mcan[(long long)nb.x * 128 + 32 + 31];
+    if (lane == 31 && nb.y >= 0)
+      R |= P.mreach[(long long)nb.y * 32] & P.mcan[(long long)nb.y * 128 + 0];
+    if (nb.z >= 0 && ((P.mreach[(long long)nb.z * 32 + lane] & P.mcan[(long long)nb.z * 128 + 96 + lane]) >> 31))
+      R |= 1u;
+    if (nb.w >= 0 && ((P.mreach[(long long)nb.w * 32 + lane] & P.mcan[(long long)nb.w * 128 + 64 + lane]) & 1u))
+      R |= 0x80000000u;
+  }
+  for (int guard = 0; guard < GC_TILE_PX + 1; ++guard) {
+    uint32_t dn = __shfl_up_sync(0xffffffffu, R & canD, 1);   // row r-1 flows down into r
+    uint32_t up = __shfl_down_sync(0xffffffffu, R & canU, 1); // row r+1 flows up into r
+    if (lane == 0) dn = 0;
+    if (lane == 31) up = 0;
+    const uint32_t N = R | ((R & canR) << 1) | ((R & canL) >> 1) | dn | up;
+    if (!__any_sync(0xffffffffu, N != R)) break;
+    R = N;
+  }
+  P.mreach[(long long)t * 32 + lane] = R;
+  if (__any_sync(0xffffffffu, (R & sink) != 0) && lane == 0 &&
+      *((volatile int32_t*)&P.img_hit[img]) != stamp) {
+    if (!hits) P.img_hit[img] = stamp;
+    else if (atomicExch(&P.img_hit[img], stamp) != stamp) atomicAdd(hits, 1);
+  }
+  const uint32_t nw = first ? R : (R & ~R0);
+  const int sU = __any_sync(0xffffffffu, lane == 0 && (nw & canU));
+  const int sD = __any_sync(0xffffffffu, lane == 31 && (nw & canD));
+  const int sL = __any_sync(0xffffffffu, (nw & canL & 1u) != 0);
+  const int sR = __any_sync(0xffffffffu, ((nw & canR) >> 31) != 0);
+  if (lane < 4) {   // the neighbours to queue, one lane each
+    const int go = lane == 0 ? sU : lane == 1 ? sD : lane == 2 ? sL : sR;
+    const int nt = lane == 0 ? nb.x : lane == 1 ? nb.y : lane == 2 ? nb.z : nb.w;
+    if (go && nt >= 0) frontier_push(P, out, nt);
+  }
+}
+
+// The CTA's warps add their sums, once per image.  Every thread of the CTA calls it.
+template <int WARPS>
+__device__ __forceinline__ void flood_sum_flush(ImageAcc* acc, const FloodSum& fs) {
+  __shared__ int s_img[WARPS];
+  __shared__ unsigned long long s_sum[WARPS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0) {
+    s_img[warp] = fs.sum ? fs.img : -1;
+    s_sum[warp] = fs.sum;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int a = 0; a < WARPS; ++a) {
+      if (s_img[a] < 0) continue;
+      unsigned long long v = s_sum[a];
+      for (int b = a + 1; b < WARPS; ++b)
+        if (s_img[b] == s_img[a]) { v += s_sum[b]; s_img[b] = -1; }
+      atomicAdd(&acc[s_img[a]].sumpos_e, v);
+    }
+  }
+}
+
+// A flood round of the host-driven loop.  mode: 0 frontier round; first rounds over the
+// selected tiles: 1 all of them, 2 those of the images live in this cycle (img_live ==
+// stamp), 3 those of the images that continue from a previous flow (img_mode == 2).
+// abort_hit: frontier rounds skip the tiles of images already stamped (their flood is redone
+// in a later cycle).
 __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
-k_flood_round(PoolView P, int mode, int abort_hit, cudaGraphConditionalHandle h, ImageAcc* acc,
-              int check, cudaGraphConditionalHandle hbfs, cudaGraphConditionalHandle hmain,
-              int publish) {
+k_flood_round(PoolView P, int mode, int abort_hit, ImageAcc* acc) {
   trace_mark(P, mode ? TR_FLOOD_FIRST : TR_FLOOD);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int first = mode != 0;
-  const int in = frontier_round_number(P, first) & 1, out = in ^ 1;
+  const int in = frontier_round_number(P, first) & 1;
+  const Worklist out{P.fq[in ^ 1], P.fcount + (in ^ 1), P.mark[in ^ 1]};
   const int stamp = *((volatile int32_t*)&P.ctl[CTL_CYCLES]) + 1;
   int32_t* const markin = P.mark[in];
   int done = 0;
@@ -1610,8 +1562,7 @@ k_flood_round(PoolView P, int mode, int abort_hit, cudaGraphConditionalHandle h,
   if ((int)blockIdx.x >= parts) return;
   const int i0 = blockIdx.x * WARPS_PER_CTA + warp;
   SelCursor cursor(P, first ? nr : 0, i0);
-  int wimg = -1;                 // first round: the image whose tile sums this warp holds
-  unsigned long long wsum = 0;
+  FloodSum fs;
   for (int i = i0; i < n; i += parts * WARPS_PER_CTA) {
     const int t = first ? cursor.tile(i) : P.fq[in][i];
     if (!first && lane == 0) markin[t] = 0;
@@ -1624,103 +1575,14 @@ k_flood_round(PoolView P, int mode, int abort_hit, cudaGraphConditionalHandle h,
     if (mode == 3 && P.img_mode[img] != 2) continue;
     if (mode == 0 && abort_hit && *((volatile int32_t*)&P.img_hit[img]) == stamp) continue;
     ++done;
-    const int4 nb = P.nbr[t];
-    uint32_t canU, canD, canL, canR, sink, R, R0;
-    long long ps = 0;
-    if (first && P.mdirty[t] != 0) {
-      // the tile changed since its masks were written (a discharge or an edit): rebuild them
-      // here, before anything reads them (every tile of an image this round covers is done
-      // in this round, so the frontier rounds and the global relabel after it see them)
-      const RowMasks m = warp_rebuild_masks(P, t, lane, &ps);
-      canU = m.up; canD = m.down; canL = m.left; canR = m.right;
-      sink = m.sink;
-      R = m.exc;
-    } else {
-      const uint32_t* mc = P.mcan + (long long)t * 128;
-      canU = mc[lane]; canD = mc[32 + lane]; canL = mc[64 + lane]; canR = mc[96 + lane];
-      sink = P.msink[(long long)t * 32 + lane];
-      if (first) {
-        R = P.mexc[(long long)t * 32 + lane];
-        ps = P.tpos[t];
-      }
-    }
-    if (first) {
-      R0 = 0;
-      // Σ max(excess, 0) of the tile, taken with its masks; summed per warp and per CTA
-      // before the add to the image's word
-      if (lane == 0 && ps) {
-        if (img != wimg) {
-          if (wsum) atomicAdd(&acc[wimg].sumpos_e, wsum);
-          wimg = img;
-          wsum = 0;
-        }
-        wsum += (unsigned long long)ps;
-      }
-    } else {
-      R = R0 = P.mreach[(long long)t * 32 + lane];
-      if (lane == 0 && nb.x >= 0)
-        R |= P.mreach[(long long)nb.x * 32 + 31] & P.mcan[(long long)nb.x * 128 + 32 + 31];
-      if (lane == 31 && nb.y >= 0)
-        R |= P.mreach[(long long)nb.y * 32] & P.mcan[(long long)nb.y * 128 + 0];
-      if (nb.z >= 0 && ((P.mreach[(long long)nb.z * 32 + lane] & P.mcan[(long long)nb.z * 128 + 96 + lane]) >> 31))
-        R |= 1u;
-      if (nb.w >= 0 && ((P.mreach[(long long)nb.w * 32 + lane] & P.mcan[(long long)nb.w * 128 + 64 + lane]) & 1u))
-        R |= 0x80000000u;
-    }
-    for (int guard = 0; guard < GC_TILE_PX + 1; ++guard) {
-      uint32_t dn = __shfl_up_sync(0xffffffffu, R & canD, 1);   // row r-1 flows down into r
-      uint32_t up = __shfl_down_sync(0xffffffffu, R & canU, 1); // row r+1 flows up into r
-      if (lane == 0) dn = 0;
-      if (lane == 31) up = 0;
-      const uint32_t N = R | ((R & canR) << 1) | ((R & canL) >> 1) | dn | up;
-      if (!__any_sync(0xffffffffu, N != R)) break;
-      R = N;
-    }
-    P.mreach[(long long)t * 32 + lane] = R;
-    if (__any_sync(0xffffffffu, (R & sink) != 0) && lane == 0 &&
-        *((volatile int32_t*)&P.img_hit[img]) != stamp)
-      P.img_hit[img] = stamp;
-    const uint32_t nw = first ? R : (R & ~R0);
-    const int sU = __any_sync(0xffffffffu, lane == 0 && (nw & canU));
-    const int sD = __any_sync(0xffffffffu, lane == 31 && (nw & canD));
-    const int sL = __any_sync(0xffffffffu, (nw & canL & 1u) != 0);
-    const int sR = __any_sync(0xffffffffu, ((nw & canR) >> 31) != 0);
-    if (lane < 4) {   // the neighbours to queue, one lane each
-      const int go = lane == 0 ? sU : lane == 1 ? sD : lane == 2 ? sL : sR;
-      const int nt = lane == 0 ? nb.x : lane == 1 ? nb.y : lane == 2 ? nb.z : nb.w;
-      if (go && nt >= 0) frontier_push(P, out, nt);
-    }
+    flood_tile(P, t, lane, first, img, stamp, nullptr, out, acc, fs);
   }
   if (lane == 0 && done) {
     atomicAdd(&P.rcnt[in], done);
     if (P.ktiles) atomicAdd(&P.ktiles[first ? K_FLOOD_FIRST : K_FLOOD], (unsigned long long)done);
   }
-  if (first) {   // the CTA's warps that summed the same image add once
-    __shared__ int s_img[WARPS_PER_CTA];
-    __shared__ unsigned long long s_sum[WARPS_PER_CTA];
-    if (lane == 0) {
-      s_img[warp] = wsum ? wimg : -1;
-      s_sum[warp] = wsum;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int a = 0; a < WARPS_PER_CTA; ++a) {
-        if (s_img[a] < 0) continue;
-        unsigned long long v = s_sum[a];
-        for (int b = a + 1; b < WARPS_PER_CTA; ++b)
-          if (s_img[b] == s_img[a]) { v += s_sum[b]; s_img[b] = -1; }
-        atomicAdd(&acc[s_img[a]].sumpos_e, v);
-      }
-    }
-  }
-  flood_round_end(P, first, in, parts, h, check, hbfs, hmain, publish, acc);
-}
-
-// After a flood (host-driven loops; the solve graph runs the check at the end of its last
-// flood round instead): see flood_check_cta.  One CTA.
-__global__ void k_flood_check(PoolView P, int all, cudaGraphConditionalHandle hbfs,
-                              cudaGraphConditionalHandle hmain) {
-  flood_check_cta(P, all, hbfs, hmain, 0, nullptr);
+  if (first) flood_sum_flush<WARPS_PER_CTA>(acc, fs);
+  frontier_round_end(P, first, in, CTL_FLOOD_TOTAL, parts);
 }
 
 // Neighbour tile ids and image index of one image's tiles (row-major from im.tile0), for an
@@ -1734,29 +1596,13 @@ __global__ void k_image_tiles(PoolView P, ImageDesc im, int img) {
   P.img_of[t] = img;
 }
 
-// The labels kernels inside a solve graph that ends with the labels of its one image:
-// `first`: the launch that follows the first cycle's flood writes only when that cycle's
-// check left no image (the solve ended there; otherwise the launch at the end of the relabel
-// IF node writes them).  `slot`: the output buffer is read from this device word, which the
-// host sets when the caller's buffer changes, so the graph never changes.  Every thread
-// reads words that earlier launches (or copies) wrote.
-__device__ __forceinline__ bool labels_skip(const PoolView& P, int first) {
-  return first && *((volatile int32_t*)&P.ctl[CTL_LEFT]) != 0;
-}
-__device__ __forceinline__ uint8_t* labels_dest(uint8_t* out, const unsigned long long* slot) {
-  return slot ? reinterpret_cast<uint8_t*>(*((const volatile unsigned long long*)slot)) : out;
-}
-
-// Labels of one image, row-major, padding excluded.  One thread writes the 32 pixels of
-// one tile row (one mask word); consecutive threads take consecutive tiles of an image row.
-__global__ void k_labels_out(PoolView P, ImageDesc im, uint8_t* __restrict__ out_arg, int first,
-                             const unsigned long long* slot) {
-  if (labels_skip(P, first)) return;
-  trace_mark(P, TR_LABELS);
-  uint8_t* const out = labels_dest(out_arg, slot);
+// Labels of one image, row-major, padding excluded: threads i0, i0 + stride, ... each write the
+// 32 pixels of a tile row (one mask word); consecutive threads take consecutive tiles of an
+// image row.
+__device__ __forceinline__ void write_labels(const PoolView& P, const ImageDesc& im, uint8_t* out,
+                                             long long i0, long long stride) {
   const long long n = (long long)im.H * im.tw;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
+  for (long long i = i0; i < n; i += stride) {
     const int y = (int)(i / im.tw), tx = (int)(i % im.tw);
     const int t = im.tile0 + (y >> 5) * im.tw + tx;
     const uint32_t m = P.mreach[(long long)t * 32 + (y & 31)];
@@ -1778,15 +1624,11 @@ __global__ void k_labels_out(PoolView P, ImageDesc im, uint8_t* __restrict__ out
 // Bit-packed labels: thread (y, tx) writes the up to four bytes of tile column tx in row y
 // (row stride (W + 7) / 8 bytes, little bit order).  Pixels of a ragged tile beyond the
 // image have no capacities and no excess, so their reach bits are 0.
-__global__ void k_labels_packed(PoolView P, ImageDesc im, uint8_t* __restrict__ out_arg,
-                                int first, const unsigned long long* slot) {
-  if (labels_skip(P, first)) return;
-  trace_mark(P, TR_LABELS);
-  uint8_t* const out = labels_dest(out_arg, slot);
+__device__ __forceinline__ void write_labels_packed(const PoolView& P, const ImageDesc& im,
+                                                    uint8_t* out, long long i0, long long step) {
   const long long n = (long long)im.H * im.tw;
   const int stride = (im.W + 7) >> 3;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
+  for (long long i = i0; i < n; i += step) {
     const int y = (int)(i / im.tw), tx = (int)(i % im.tw);
     const int t = im.tile0 + (y >> 5) * im.tw + tx;
     const uint32_t m = P.mreach[(long long)t * 32 + (y & 31)];
@@ -1797,6 +1639,290 @@ __global__ void k_labels_packed(PoolView P, ImageDesc im, uint8_t* __restrict__ 
     } else {
       for (int k = 0; k < nb; ++k) row[k] = (uint8_t)(m >> (8 * k));
     }
+  }
+}
+
+__global__ void k_labels_out(PoolView P, ImageDesc im, uint8_t* out) {
+  trace_mark(P, TR_LABELS);
+  write_labels(P, im, out, (long long)blockIdx.x * blockDim.x + threadIdx.x,
+               (long long)gridDim.x * blockDim.x);
+}
+__global__ void k_labels_packed(PoolView P, ImageDesc im, uint8_t* out) {
+  trace_mark(P, TR_LABELS);
+  write_labels_packed(P, im, out, (long long)blockIdx.x * blockDim.x + threadIdx.x,
+                      (long long)gridDim.x * blockDim.x);
+}
+
+// ------------------------------------------------------------------------------------
+// The whole solve as one cooperative launch: every CTA runs the same steps (pulses, flood
+// rounds, relabel rounds), with a grid barrier after each, and the loop decisions are taken
+// by every CTA from the counters it reads behind the barrier.
+//
+// A barrier costs 1-2 us.  The CUDA graph this replaces (the same steps as kernel nodes under
+// WHILE and IF nodes) paid a kernel's launch and drain per step and 5-11 us per conditional
+// node passed.
+// ------------------------------------------------------------------------------------
+// A barrier wait gives up after this long (a step of the largest pool takes well under a
+// second): it raises the abort flag, and every CTA leaves at its next barrier.
+constexpr unsigned long long GC_BARRIER_WAIT_NS = 5000000000ull;
+
+__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// Grid barrier: every CTA's writes before it are visible to every CTA after it, the bulk
+// copies (async proxy) that follow it included.  Then thread 0 reads the words *w0 and *w1 for
+// the whole CTA: counters that no CTA writes before the barrier after this one.  Returns false
+// (the same in every thread) when the solve was aborted.  `s` : 4 words of shared memory.
+__device__ __forceinline__ bool grid_sync(const PoolView& P, unsigned long long& target,
+                                          volatile int32_t* s, const int32_t* w0,
+                                          const int32_t* w1, int& v0, int& v1) {
+  asm volatile("fence.proxy.async;" ::: "memory");   // this thread's writes, before later copies
+  __syncthreads();
+  target += gridDim.x;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(P.bar + BAR_ARRIVE, 1ull);
+    bool ok = false;
+    unsigned long long t0 = 0;
+    for (unsigned i = 1; i < (1u << 31); ++i) {
+      const unsigned long long v = ld_acquire(P.bar + BAR_ARRIVE);
+      if (v & GC_BAR_ABORT) break;
+      if (v >= target) { ok = true; break; }
+      if ((i & 1023u) == 0) {
+        const unsigned long long now = global_ns();
+        if (t0 == 0) t0 = now;
+        else if (now - t0 > GC_BARRIER_WAIT_NS) {
+          atomicCAS(&P.ctl[CTL_ERR], 0, 5);
+          __threadfence();
+          atomicOr(P.bar + BAR_ARRIVE, GC_BAR_ABORT);
+          break;
+        }
+      }
+    }
+    __threadfence();
+    asm volatile("fence.proxy.async;" ::: "memory");
+    s[0] = ok;
+    s[1] = ok ? *((const volatile int32_t*)w0) : 0;
+    s[2] = ok ? *((const volatile int32_t*)w1) : 0;
+  }
+  __syncthreads();
+  v0 = s[1];
+  v1 = s[2];
+  return s[0] != 0;
+}
+
+// The solve over the selection (see Pool::solve_images): images that continue from a previous
+// flow (mode 2) are flooded first, and those whose flood reaches a sink pixel get a global
+// relabel; freshly uploaded ones (mode 1) start from the trivial labelling.  Then cycles of
+// {pulses of discharge, flood, relabel of the images whose flood reached a sink}, until no
+// flood does: each image's last flood is its canonical cut.  A flood's stamp is its number
+// in the solve; an image whose flood reached a sink carries that stamp in img_hit, which
+// selects it for the relabel and for the next flood.
+//
+// 4 CTAs of 256 threads per SM (k_discharge's shape: registers and shared memory bound it);
+// the relabel's staging shares the discharge's shared memory.
+constexpr int SOLVE_WARPS = DIS_THREADS / 32;
+constexpr size_t SOLVE_BFS_SMEM = (size_t)SOLVE_WARPS * 32 * 33 * sizeof(int32_t);
+constexpr size_t SOLVE_DYN_SMEM = DIS_DYN_SMEM > SOLVE_BFS_SMEM ? DIS_DYN_SMEM : SOLVE_BFS_SMEM;
+
+__global__ void __launch_bounds__(DIS_THREADS, 4)
+k_solve(PoolView P, SolveArgs A) {
+  extern __shared__ __align__(128) int32_t dsm[];
+  __shared__ uint64_t mbar;
+  __shared__ int32_t s_bc[4];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int bid = blockIdx.x, nb = gridDim.x;
+  unsigned long long target = 0;
+  unsigned phase = 0;     // of mbar
+  int qk = 0, fk = 0;     // steps of the worklist and of the frontier (counter slots mod 3)
+  int stamp = 0, cycles = 0, err = 0;
+  int nrounds_f = 0, nrounds_b = 0;
+  int v0, v1;
+  // ---- prologue: control words, image modes and flow sums
+  trace_mark(P, TR_BEGIN);
+  if (tid == 0) {
+    mbar_init(&mbar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  const int nr = A.ranges, n_sel = A.tiles;
+  if (bid == 0) {
+    for (int i = tid; i < CTL_N; i += DIS_THREADS) P.ctl[i] = 0;
+    for (int i = tid; i < P.nimg; i += DIS_THREADS) {
+      P.img_hit[i] = 0;
+      P.img_mode[i] = 0;
+    }
+    __syncthreads();
+    for (int k = tid; k < nr; k += DIS_THREADS) {
+      const int img = P.sel[k].w;
+      if ((unsigned)img >= (unsigned)P.nimg) { record_bad(P, 4, img); continue; }
+      P.img_mode[img] = P.sel_mode[k];
+      A.acc[img].sumpos_e = 0;   // the floods of this solve accumulate it
+    }
+  }
+  bool alive = grid_sync(P, target, s_bc, &P.ctl[CTL_ERR], &P.ctl[CTL_ERR], v0, v1);
+
+  for (int cyc = 0; alive; ++cyc) {
+    // cyc 0 is the part before the first pulses: the warm images' flood and relabel, and the
+    // fresh images' first list
+    if (cyc > 0) {
+      // ---- pulses: step qk reads counter qk, adds to qk + 1, clears qk + 2 (all mod 3)
+      for (int p = 0; p < A.pulses && alive; ++p) {
+        trace_mark(P, TR_DISCHARGE);
+        const Worklist in{P.queue[qk & 1], nullptr, P.inq[qk & 1]};
+        Worklist out{P.queue[(qk + 1) & 1], &P.ctl[CTL_Q0 + (qk + 1) % 3], P.inq[(qk + 1) & 1]};
+        if (p == A.pulses - 1) out.list = nullptr;   // the relabel makes the next list
+        if (bid == 0 && tid == 0) P.ctl[CTL_Q0 + (qk + 2) % 3] = 0;
+        discharge_phase(P, A.iters, bid, nb, in, v0, out, dsm,
+                        *reinterpret_cast<DisSmem*>(dsm + DIS_PLANES * GC_TILE_PX), &mbar, phase);
+        ++qk;
+        alive = grid_sync(P, target, s_bc, &P.ctl[CTL_Q0 + qk % 3], &P.ctl[CTL_ERR], v0, v1);
+      }
+      if (!alive) break;
+    }
+    int left = 0;
+    if (cyc > 0 || A.warm) {
+      // ---- flood, first round over the selection, then frontier rounds
+      const int prev = stamp++;
+      int32_t* const hits = &P.ctl[CTL_H0 + stamp % 3];
+      if (bid == 0 && tid == 0) P.ctl[CTL_H0 + (stamp + 1) % 3] = 0;
+      int n = n_sel, rounds = 0;
+      FloodSum fs;
+      for (bool first = true;; first = false) {
+        trace_mark(P, first ? TR_FLOOD_FIRST : TR_FLOOD);
+        const Worklist out{P.fq[(fk + 1) & 1], &P.ctl[CTL_F0 + (fk + 1) % 3], P.mark[(fk + 1) & 1]};
+        if (bid == 0 && tid == 0) P.ctl[CTL_F0 + (fk + 2) % 3] = 0;
+        const int i0 = warp * nb + bid;
+        SelCursor cursor(P, first ? nr : 0, i0 < n ? i0 : 0);
+        for (int i = i0; i < n; i += SOLVE_WARPS * nb) {
+          const int t = first ? cursor.tile(i) : P.fq[fk & 1][i];
+          if (!first && lane == 0) P.mark[fk & 1][t] = 0;
+          const int img = first ? cursor.image() : P.img_of[t];
+          if ((unsigned)img >= (unsigned)P.nimg || (unsigned)t >= (unsigned)P.nt) {   // self-check
+            if (lane == 0) record_bad(P, 4, img);
+            continue;
+          }
+          const int hit = *((volatile int32_t*)&P.img_hit[img]);
+          if (first) {
+            const int mode = P.img_mode[img];
+            const bool part = cyc == 0 ? mode == 2
+                                       : (hit == stamp || (prev > 0 && hit == prev) || (cyc == 1 && mode == 1));
+            if (!part) continue;
+          } else if (hit == stamp) {
+            continue;   // not solved: its flood is redone in a later cycle
+          }
+          flood_tile(P, t, lane, first, img, stamp, hits, out, A.acc, fs);
+        }
+        if (first) {
+          flood_sum_flush<SOLVE_WARPS>(A.acc, fs);
+          fs = FloodSum{};
+        }
+        ++fk;
+        ++rounds;
+        alive = grid_sync(P, target, s_bc, &P.ctl[CTL_F0 + fk % 3], hits, v0, v1);
+        n = v0;
+        if (!alive || n == 0) break;
+        if (n < 0 || n > P.nt) { alive = false; break; }   // (never: frontier_push counts a tile once)
+        if (rounds >= A.max_rounds) { err = 1; break; }
+      }
+      nrounds_f += rounds;
+      left = v1;   // images whose flood reached a sink
+      if (cyc > 0) ++cycles;
+      if (bid == 0 && tid == 0) trace_record(P, TR_CHECK);
+      if (!alive || err) break;
+      if (left == 0 && !(cyc == 0 && A.fresh)) break;   // solved
+      if (left > 0) {
+        // ---- global relabel of the images not solved; it lists their active tiles
+        if (bid == 0)   // their sums start afresh with their next flood
+          for (int i = tid; i < P.nimg; i += DIS_THREADS)
+            if (P.img_hit[i] == stamp) A.acc[i].sumpos_e = 0;
+        const Worklist act_out{P.queue[qk & 1], &P.ctl[CTL_Q0 + qk % 3], nullptr};
+        n = n_sel;
+        rounds = 0;
+        for (bool first = true;; first = false) {
+          trace_mark(P, first ? TR_BFS_FIRST : TR_BFS);
+          const Worklist out{P.fq[(fk + 1) & 1], &P.ctl[CTL_F0 + (fk + 1) % 3], P.mark[(fk + 1) & 1]};
+          if (bid == 0 && tid == 0) P.ctl[CTL_F0 + (fk + 2) % 3] = 0;
+          const int i0 = warp * nb + bid;
+          SelCursor cursor(P, first ? nr : 0, i0 < n ? i0 : 0);
+          for (int i = i0; i < n; i += SOLVE_WARPS * nb) {
+            const int t = first ? cursor.tile(i) : P.fq[fk & 1][i];
+            if (first && P.img_hit[cursor.image()] != stamp) continue;
+            if (!first && lane == 0) P.mark[fk & 1][t] = 0;
+            const int act = bfs_tile(P, t, lane, first, dsm + warp * (32 * 33), out);
+            if (lane == 0) {
+              // a tile becomes active once (its reached set only grows): list it then
+              if (act && (first || P.tact[t] == 0)) worklist_append(P, act_out, t);
+              if (first || act) P.tact[t] = act;
+            }
+          }
+          ++fk;
+          ++rounds;
+          alive = grid_sync(P, target, s_bc, &P.ctl[CTL_F0 + fk % 3], &P.ctl[CTL_Q0 + qk % 3], v0, v1);
+          n = v0;
+          if (!alive || n == 0) break;
+          if (n < 0 || n > P.nt) { alive = false; break; }
+          if (rounds >= A.max_rounds) { err = 1; break; }
+        }
+        nrounds_b += rounds;
+        if (!alive || err) break;
+      }
+    }
+    if (cyc == 0 && A.fresh) {
+      // ---- the fresh images' first list: tiles with positive excess
+      trace_mark(P, TR_ACTIVE_LIST);
+      const Worklist act_out{P.queue[qk & 1], &P.ctl[CTL_Q0 + qk % 3], nullptr};
+      const int i0 = bid * DIS_THREADS + tid;
+      SelCursor cursor(P, nr, i0 < n_sel ? i0 : 0);
+      for (int b = bid * DIS_THREADS; b < n_sel; b += nb * DIS_THREADS) {   // CTA-uniform
+        int t = -1;
+        if (b + tid < n_sel) {
+          t = cursor.tile(b + tid);
+          if (P.img_mode[cursor.image()] != 1 || P.tact[t] == 0) t = -1;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, t >= 0);
+        if (m == 0) continue;
+        int pos = 0;
+        if (lane == 0) pos = atomicAdd(act_out.count, __popc(m));
+        pos = __shfl_sync(0xffffffffu, pos, 0) + __popc(m & ((1u << lane) - 1u));
+        if (t >= 0) {
+          if (pos < P.nt) act_out.list[pos] = t;
+          else record_bad(P, 1, pos);
+        }
+      }
+      alive = grid_sync(P, target, s_bc, &P.ctl[CTL_Q0 + qk % 3], &P.ctl[CTL_Q0 + qk % 3], v0, v1);
+    }
+    v0 = v1;   // the worklist's length
+    if (!alive || v0 == 0) break;
+    if (cycles >= A.max_cycles) { err = 2; break; }
+  }
+
+  // ---- results: control words and sums to the host, labels of a one-image handle
+  if (bid == 0) {
+    if (tid == 0) {
+      volatile int32_t* ctl = P.ctl;
+      if (err || !alive) atomicCAS(&P.ctl[CTL_ERR], 0, err ? err : 5);
+      ctl[CTL_BFS_TOTAL] = nrounds_b;
+      ctl[CTL_FLOOD_TOTAL] = nrounds_f;
+      ctl[CTL_CYCLES] = cycles;
+      ctl[CTL_NACT] = A.fresh ? 1 : 0;
+      trace_record(P, TR_END);
+    }
+    __syncthreads();
+    publish_results(P, A.acc);
+  }
+  if (A.lmode && alive && !err) {
+    trace_mark(P, TR_LABELS);
+    const long long i0 = (long long)bid * DIS_THREADS + tid, step = (long long)nb * DIS_THREADS;
+    if (A.lmode == 2) write_labels_packed(P, A.im, A.labels, i0, step);
+    else write_labels(P, A.im, A.labels, i0, step);
+  }
+  // the last CTA to leave clears the barrier for the next launch
+  if (tid == 0 && atomicAdd(P.bar + BAR_EXIT, 1ull) == (unsigned long long)nb - 1) {
+    P.bar[BAR_EXIT] = 0;
+    P.bar[BAR_ARRIVE] = 0;
   }
 }
 
@@ -2013,25 +2139,30 @@ int launch_edge_relabel_build(const PoolView& P, int32_t* list, int32_t* count,
   return ok();
 }
 
-int launch_bfs_round(const PoolView& P, int first, cudaGraphConditionalHandle h, int grid,
-                     cudaStream_t s) {
-  k_bfs_round<<<grid, WARPS_PER_CTA * 32, 0, s>>>(P, first, h);
+int launch_bfs_round(const PoolView& P, int first, int grid, cudaStream_t s) {
+  k_bfs_round<<<grid, WARPS_PER_CTA * 32, 0, s>>>(P, first);
   return ok();
 }
 
-int launch_flood_round(const PoolView& P, int mode, int abort_hit, cudaGraphConditionalHandle h,
-                       ImageAcc* acc, int grid, cudaStream_t s, int check,
-                       cudaGraphConditionalHandle hbfs, cudaGraphConditionalHandle hmain,
-                       int publish) {
-  k_flood_round<<<grid, WARPS_PER_CTA * 32, 0, s>>>(P, mode, abort_hit, h, acc, check, hbfs, hmain,
-                                                    publish);
+int launch_flood_round(const PoolView& P, int mode, int abort_hit, ImageAcc* acc, int grid,
+                       cudaStream_t s) {
+  k_flood_round<<<grid, WARPS_PER_CTA * 32, 0, s>>>(P, mode, abort_hit, acc);
   return ok();
 }
 
-int launch_flood_check(const PoolView& P, int all, cudaGraphConditionalHandle hbfs,
-                       cudaGraphConditionalHandle hmain, cudaStream_t s) {
-  k_flood_check<<<1, 256, 0, s>>>(P, all, hbfs, hmain);
+int launch_flood_check(const PoolView& P, int all, cudaStream_t s) {
+  k_flood_check<<<1, 256, 0, s>>>(P, all);
   return ok();
+}
+
+int launch_solve(const PoolView& P, const SolveArgs& a, int grid, cudaStream_t s) {
+  PoolView p = P;
+  SolveArgs args = a;
+  void* params[] = {&p, &args};
+  const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_solve, dim3(grid), dim3(DIS_THREADS),
+                                                    params, SOLVE_DYN_SMEM, s);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e == cudaSuccess ? GC_OK : GC_ERR_CUDA;
 }
 
 __global__ void k_acc_reset(ImageAcc* acc, int n) {
@@ -2051,28 +2182,18 @@ int launch_ctl_begin(const PoolView& P, int max_rounds, int max_cycles, ImageAcc
 }
 
 int launch_active_list(const PoolView& P, const ScanState& st, int32_t* list, int32_t* count,
-                       int bump, int count_cycle, int filter, cudaGraphConditionalHandle h,
-                       ImageAcc* acc, int grid, cudaStream_t s) {
+                       int bump, int count_cycle, int filter, ImageAcc* acc, int grid,
+                       cudaStream_t s) {
   const int nch = (P.nt + ACT_CHUNK - 1) / ACT_CHUNK;   // enough for any selection
   if (nch > st.max_chunks) return GC_ERR_INVALID;
   grid = grid < nch ? grid : nch;
   k_active_list<<<grid > 0 ? grid : 1, ACT_THREADS, 0, s>>>(P, st, list, count, bump, count_cycle,
-                                                            filter, h, acc);
+                                                            filter, acc);
   return ok();
 }
 
-int begin_list_max_tiles() { return BL_MAX; }
-
-int launch_begin_list(const PoolView& P, int max_rounds, int max_cycles, ImageAcc* acc,
-                      int32_t* list, int32_t* count, cudaGraphConditionalHandle h, cudaStream_t s) {
-  if (P.nt > BL_MAX) return GC_ERR_INVALID;
-  k_begin_list<<<1, BL_THREADS, 0, s>>>(P, max_rounds, max_cycles, acc, list, count, h);
-  return ok();
-}
-
-int launch_ctl_cycle(const PoolView& P, const int32_t* count, int count_cycle,
-                     cudaGraphConditionalHandle h, cudaStream_t s) {
-  k_ctl_cycle<<<1, 32, 0, s>>>(P, count, count_cycle, h);
+int launch_ctl_cycle(const PoolView& P, cudaStream_t s) {
+  k_ctl_cycle<<<1, 32, 0, s>>>(P);
   return ok();
 }
 
@@ -2083,22 +2204,19 @@ int launch_image_tiles(const PoolView& P, const ImageDesc& im, int img, cudaStre
   return ok();
 }
 
-// one thread per tile row of the image; grid_cap > 0 caps the CTAs (they stride over rows)
-static unsigned labels_grid(const ImageDesc& im, int grid_cap) {
-  const long long need = ((long long)im.H * im.tw + 255) / 256;
-  const long long g = grid_cap > 0 && need > grid_cap ? grid_cap : need;
+// one thread per tile row of the image
+static unsigned labels_grid(const ImageDesc& im) {
+  const long long g = ((long long)im.H * im.tw + 255) / 256;
   return (unsigned)(g < 1 ? 1 : g);
 }
 
-int launch_labels_out(const PoolView& P, const ImageDesc& im, uint8_t* out, cudaStream_t s,
-                      int first, const unsigned long long* slot, int grid_cap) {
-  k_labels_out<<<labels_grid(im, grid_cap), 256, 0, s>>>(P, im, out, first, slot);
+int launch_labels_out(const PoolView& P, const ImageDesc& im, uint8_t* out, cudaStream_t s) {
+  k_labels_out<<<labels_grid(im), 256, 0, s>>>(P, im, out);
   return ok();
 }
 
-int launch_labels_packed(const PoolView& P, const ImageDesc& im, uint8_t* out, cudaStream_t s,
-                         int first, const unsigned long long* slot, int grid_cap) {
-  k_labels_packed<<<labels_grid(im, grid_cap), 256, 0, s>>>(P, im, out, first, slot);
+int launch_labels_packed(const PoolView& P, const ImageDesc& im, uint8_t* out, cudaStream_t s) {
+  k_labels_packed<<<labels_grid(im), 256, 0, s>>>(P, im, out);
   return ok();
 }
 
@@ -2163,7 +2281,7 @@ int launch_brush(const PoolView& P, const ImageDesc& im, int img, const int32_t*
 }
 
 // Loads every kernel of the library on the current device.  With lazy module loading (the
-// CUDA default) a kernel is loaded at its first launch or graph instantiation; doing it
+// CUDA default) a kernel is loaded at its first launch; doing it
 // here, once per device under a lock, keeps that loading away from threads that solve on
 // several streams at once.
 void preload_kernels() {
@@ -2179,8 +2297,8 @@ void preload_kernels() {
       (const void*)k_nlink_table,
       (const void*)k_masks, (const void*)k_discharge, (const void*)k_edge_relabel_build,
       (const void*)k_bfs_round, (const void*)k_flood_round, (const void*)k_ctl_begin,
-      (const void*)k_active_list, (const void*)k_begin_list, (const void*)k_ctl_cycle,
-      (const void*)k_flood_check,
+      (const void*)k_active_list, (const void*)k_ctl_cycle, (const void*)k_flood_check,
+      (const void*)k_solve,
       (const void*)k_image_tiles,
       (const void*)k_acc_reset, (const void*)k_labels_out, (const void*)k_labels_packed,
       (const void*)k_state_out, (const void*)k_edit, (const void*)k_stroke,
@@ -2194,8 +2312,8 @@ void preload_kernels() {
 namespace {
 // Launch geometry per device, set up once: the dynamic shared memory opt-in of k_discharge
 // changes the function's state, so it is not repeated while other threads launch or
-// instantiate graphs that contain the kernel.
-struct Geometry { int dis = 0, warps = 0; };
+// launch it.
+struct Geometry { int dis = 0, warps = 0, solve = 0; };
 std::mutex g_geom_mu;
 std::unordered_map<int, Geometry> g_geom;
 
@@ -2204,13 +2322,16 @@ Geometry device_geometry(int device) {
   auto it = g_geom.find(device);
   if (it != g_geom.end()) return it->second;
   preload_kernels();
-  int per_dis = 0, per_bfs = 0, sms = 0;
+  int per_dis = 0, per_bfs = 0, per_solve = 0, sms = 0;
+  cudaFuncSetAttribute(k_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOLVE_DYN_SMEM);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_solve, k_solve, DIS_THREADS, SOLVE_DYN_SMEM);
   cudaFuncSetAttribute(k_discharge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DIS_DYN_SMEM);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_dis, k_discharge, DIS_THREADS, DIS_DYN_SMEM);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_bfs, k_bfs_round, WARPS_PER_CTA * 32, 0);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   sms = sms > 0 ? sms : 1;
-  Geometry g{(per_dis > 0 ? per_dis : 1) * sms, (per_bfs > 0 ? per_bfs : 1) * sms};
+  Geometry g{(per_dis > 0 ? per_dis : 1) * sms, (per_bfs > 0 ? per_bfs : 1) * sms,
+             (per_solve > 0 ? per_solve : 1) * sms};
   g_geom.emplace(device, g);
   return g;
 }
@@ -2218,5 +2339,6 @@ Geometry device_geometry(int device) {
 
 int occupancy_discharge(int device) { return device_geometry(device).dis; }
 int occupancy_warps(int device) { return device_geometry(device).warps; }
+int occupancy_solve(int device) { return device_geometry(device).solve; }
 
 }  // namespace gcut
