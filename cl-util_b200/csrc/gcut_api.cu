@@ -267,7 +267,7 @@ struct Pool {
     c.take(&P.msink, (size_t)nt * 32);
     c.take(&P.mexc, (size_t)nt * 32);
     c.take(&P.mreach, (size_t)nt * 32);
-    int32_t** small[] = {&P.touched, &P.act_int, &P.mark[0], &P.mark[1], &P.tact, &P.img_of,
+    int32_t** small[] = {&P.touched, &P.act_int, &P.mark[0], &P.mark[1], &P.tact, &P.tflag, &P.img_of,
                          &P.queue[0], &P.queue[1], &P.inq[0], &P.inq[1], &P.mdirty};
     for (auto** p : small) c.take(p, nt);
     c.take(&P.qcount, 2);
@@ -554,18 +554,18 @@ struct Pool {
   // handle when captured into a graph (0: host-driven rounds)
   int global_relabel(cudaStream_t s, int first = 1) {
     RK(timed(K_MASKS, s, [&] { return launch_masks(P, grid_warps, s); }));
-    RK(timed(K_BFS_FIRST, s, [&] { return launch_bfs_round(P, first, grid_warps, s); }));
-    return frontier_rounds(s, /*flood=*/false);
+    RK(timed(K_BFS_FIRST, s, [&] { return launch_bfs_round(P, first, GC_HINF, 0, grid_warps, s); }));
+    return frontier_rounds(s, /*flood=*/false, GC_HINF);
   }
 
   // host-driven rounds over the marked tiles until a round finds none; the host reads
   // the control words once per batch of rounds
-  int frontier_rounds(cudaStream_t s, bool flood, int abort_hit = 0) {
+  int frontier_rounds(cudaStream_t s, bool flood, int cap, int abort_hit = 0, int stamp = 0) {
     int batch = 4;
     while (true) {
       for (int k = 0; k < batch; ++k) {
-        if (flood) RK(timed(K_FLOOD, s, [&] { return launch_flood_round(P, 0, abort_hit, acc, grid_warps, s); }));
-        else RK(timed(K_BFS, s, [&] { return launch_bfs_round(P, 0, grid_warps, s); }));
+        if (flood) RK(timed(K_FLOOD, s, [&] { return launch_flood_round(P, 0, abort_hit, stamp, acc, grid_warps, s); }));
+        else RK(timed(K_BFS, s, [&] { return launch_bfs_round(P, 0, cap, 0, grid_warps, s); }));
       }
       RK(read_ctl(s));
       if (h_ctl[CTL_ERR] == 1) return fail(GC_ERR_NOT_CONVERGED, "BFS round cap reached");
@@ -645,7 +645,7 @@ struct Pool {
       CK(cudaMemsetAsync(P.bar, 0, sizeof(unsigned long long) * BAR_N, s));
     }
     lists_stale = true;   // until this solve succeeds
-    int r = host ? solve_host(s, warm) : solve_launch(s, warm, fresh, n, after, lmode, lbuf);
+    int r = host ? solve_host(s, warm, fresh) : solve_launch(s, warm, fresh, n, after, lmode, lbuf);
     if (r) return r;
     if (host && after) {   // the host-driven solve has finished: queue the work and wait
       RK((*after)(s));
@@ -670,19 +670,34 @@ struct Pool {
   // its termination check, and for the images that are not solved a global relabel and the
   // next active-tile list.  The last flood of every image is its canonical cut, so no
   // separate flood phase follows.
-  int solve_host(cudaStream_t s, bool warm) {
+  int solve_host(cudaStream_t s, bool warm, bool fresh) {
     RK(prof_begin(s));
-    RK(launch_ctl_begin(P, opts.max_bfs_rounds, opts.max_cycles, acc, s));
-    int n = 0;
-    if (warm) {
-      RK(flood_phase(s, /*mode=*/3));   // its first round rebuilds the masks of edited tiles
-      RK(timed(K_COMPACT, s, [&] { return launch_flood_check(P, 1, s); }));
+    RK(launch_ctl_begin(P, opts.max_bfs_rounds, acc, s));
+    int n = 0, cap = kFirstCap, hlim = GC_HINF, stamp = 1;
+    auto list_active = [&](int first) {
+      RK(timed(K_COMPACT, s, [&] { return launch_active_list(P, scan.st, list, counts, stamp + 1, first, 2 * sms, s); }));
+      return read_count(s, &n);
+    };
+    // a flood with its check; then, for the images left, capped relabels until excess lies
+    // within the cap, and their active list
+    auto flood_and_relabel = [&](int mode) {
+      RK(flood_phase(s, mode, stamp));   // its first round rebuilds the masks of changed tiles
+      RK(timed(K_COMPACT, s, [&] { return launch_flood_check(P, mode == 3, stamp, acc, s); }));
       RK(read_ctl(s));
-      if (h_ctl[CTL_LEFT] > 0) RK(bfs_phase(s));
-    }
-    RK(timed(K_COMPACT, s, [&] { return launch_active_list(P, scan.st, list, counts, 0, 0, 2, acc, 2 * sms, s); }));
-    RK(read_count(s, &n));
-    for (int cycle = 0; n > 0; ++cycle) {
+      n = 0;
+      while (h_ctl[CTL_LEFT] > 0) {
+        RK(bfs_phase(s, cap, stamp + 1));
+        RK(list_active(0));
+        hlim = cap < GC_HINF ? cap + 1 : GC_HINF;
+        const bool last = cap >= GC_HINF;
+        cap = next_cap(cap);
+        if (n > 0 || last) break;
+      }
+      return GC_OK;
+    };
+    if (warm) RK(flood_and_relabel(3));
+    if (fresh) RK(list_active(1));   // with the warm images' active tiles
+    for (int cycle = 0; n > 0 || (cycle == 0 && fresh); ++cycle) {
       if (cycle >= opts.max_cycles) return fail(GC_ERR_NOT_CONVERGED, "cycle cap reached before the cut was final");
       stats.cycles++;
       for (int p = 0; p < opts.pulses_per_relabel; ++p) {
@@ -691,18 +706,11 @@ struct Pool {
           CK(cudaMemcpy(h_count, P.qcount, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost));
           stats.tiles_discharged += h_count[h_ctl[CTL_PULSE] & 1];
         }
-        RK(timed(K_DISCHARGE, s, [&] { return launch_discharge(P, opts.discharge_iters, grid_dis, s); }));
+        RK(timed(K_DISCHARGE, s, [&] { return launch_discharge(P, opts.discharge_iters, hlim, grid_dis, s); }));
         stats.pulses++;
       }
-      RK(flood_phase(s, /*mode=*/2));   // its first round rebuilds the masks of changed tiles
-      RK(timed(K_COMPACT, s, [&] { return launch_flood_check(P, 0, s); }));
-      RK(read_ctl(s));
-      n = 0;
-      if (h_ctl[CTL_LEFT] > 0) {
-        RK(bfs_phase(s));
-        RK(timed(K_COMPACT, s, [&] { return launch_active_list(P, scan.st, list, counts, 1, 1, 1, acc, 2 * sms, s); }));
-        RK(read_count(s, &n));
-      }
+      ++stamp;
+      RK(flood_and_relabel(2));
     }
     CK(cudaMemcpyAsync(h_acc, acc, sizeof(ImageAcc) * imgs.size(), cudaMemcpyDeviceToHost, s));
     RK(read_ctl(s));
@@ -710,16 +718,18 @@ struct Pool {
     return GC_OK;
   }
 
-  // global relabel of the live images: first round, then frontier rounds until none is left
-  int bfs_phase(cudaStream_t s) {
-    RK(timed(K_BFS_FIRST, s, [&] { return launch_bfs_round(P, 2, grid_warps, s); }));
-    return frontier_rounds(s, /*flood=*/false);
+  // global relabel, up to distance cap, of the images live at stamp `live`: first round, then
+  // frontier rounds until none is left
+  int bfs_phase(cudaStream_t s, int cap, int live) {
+    RK(timed(K_BFS_FIRST, s, [&] { return launch_bfs_round(P, 2, cap, live, grid_warps, s); }));
+    return frontier_rounds(s, /*flood=*/false, cap);
   }
 
-  // flood of every image (mode 1) or of the live images (mode 2), to its end
-  int flood_phase(cudaStream_t s, int mode) {
-    RK(timed(K_FLOOD_FIRST, s, [&] { return launch_flood_round(P, mode, 1, acc, grid_warps, s); }));
-    return frontier_rounds(s, /*flood=*/true, /*abort_hit=*/1);
+  // flood of the images live at `stamp` (mode 2) or of those that continue from a previous
+  // flow (mode 3), to its end
+  int flood_phase(cudaStream_t s, int mode, int stamp) {
+    RK(timed(K_FLOOD_FIRST, s, [&] { return launch_flood_round(P, mode, 1, stamp, acc, grid_warps, s); }));
+    return frontier_rounds(s, /*flood=*/true, 0, /*abort_hit=*/1, stamp);
   }
 
   // The whole solve as one cooperative launch (k_solve).  lmode 1 / 2: it ends with the labels
@@ -738,6 +748,7 @@ struct Pool {
     a.pulses = opts.pulses_per_relabel;
     a.max_rounds = opts.max_bfs_rounds;
     a.max_cycles = opts.max_cycles;
+    a.cap = kFirstCap;
     a.lmode = lmode;
     a.labels = lbuf;
     a.im = imgs[0];
@@ -806,7 +817,7 @@ struct Pool {
     lists_stale = true;
     img_solved.assign(imgs.size(), 0);
     img_edited.assign(imgs.size(), 1);   // the next solve starts by flooding
-    return launch_discharge(P, opts.discharge_iters, grid_dis, s);
+    return launch_discharge(P, opts.discharge_iters, GC_HINF, grid_dis, s);
   }
   int step_relabel(cudaStream_t s) {
     if (!uploaded) return fail(GC_ERR_STATE, "relabel before upload");
@@ -822,7 +833,7 @@ struct Pool {
     if (!uploaded) return fail(GC_ERR_STATE, "startBfs before upload");
     bool warm;
     RK(select_all(&warm, s));
-    RK(launch_ctl_begin(P, opts.max_bfs_rounds, opts.max_cycles, acc, s));
+    RK(launch_ctl_begin(P, opts.max_bfs_rounds, acc, s));
     RK(global_relabel(s));
     RK(compact(P.tact, nullptr, s));
     RK(launch_ctl_cycle(P, s));
@@ -837,8 +848,8 @@ struct Pool {
     *done = n == 0;
     if (*done) {
       RK(launch_acc_reset(acc, (int)imgs.size(), s));
-      RK(launch_flood_round(P, 1, 0, acc, grid_warps, s));
-      RK(frontier_rounds(s, /*flood=*/true));
+      RK(launch_flood_round(P, 1, 0, 1, acc, grid_warps, s));
+      RK(frontier_rounds(s, /*flood=*/true, 0, 0, 1));
       CK(cudaMemcpyAsync(h_acc, acc, sizeof(ImageAcc) * imgs.size(), cudaMemcpyDeviceToHost, s));
       RK(read_ctl(s));
       RK(finish_check(s));

@@ -46,6 +46,7 @@ struct PoolView {
   int32_t* fq[2];         // [nt] frontier lists of the BFS / flood rounds (dedup by mark[k])
   int32_t* fcount;        // [2] frontier list lengths
   int32_t* tact;          // [nt] tile has an active pixel (excess > 0, height < HINF)
+  int32_t* tflag;         // [nt] where the uploaded tile has excess and sinks (TileFlag)
   int32_t* img_of;        // [nt] image index of the tile
   int32_t* mdirty;        // [nt] the tile's planes changed after its masks were written
   long long* tpos;        // [nt] sum of max(excess, 0) over the tile (with the masks)
@@ -70,6 +71,12 @@ struct PoolView {
   int32_t* host_out;
   unsigned long long* bar;  // [BAR_N] grid barrier of k_solve: arrivals (+ abort flag), exits
 };
+
+// PoolView::tflag: positive excess / sink pixels anywhere in the uploaded tile and on its
+// sides; TF_BAD: a negative capacity.
+enum TileFlag { TF_POS = 1, TF_SINK = 2, TF_POS_UP = 4, TF_POS_DOWN = 8, TF_POS_LEFT = 16,
+                TF_POS_RIGHT = 32, TF_SINK_UP = 64, TF_SINK_DOWN = 128, TF_SINK_LEFT = 256,
+                TF_SINK_RIGHT = 512, TF_BAD = 1024 };
 
 // Grid barrier words: arrivals of the running k_solve (bit 63: abort) and CTAs that left it,
 // in separate 128-byte lines.  The last CTA to leave clears both for the next launch.

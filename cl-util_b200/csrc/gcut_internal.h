@@ -74,27 +74,31 @@ int launch_nlink_table(const unsigned long long* sum, long long npairs, int32_t*
                        cudaStream_t s);
 int launch_dsum(const uint32_t* rgba, int W, int H, unsigned long long* sum, int sms,
                 cudaStream_t s);
-int launch_discharge(const PoolView& P, int iters, int grid, cudaStream_t s);
+// hlim: pixels below this height are active
+int launch_discharge(const PoolView& P, int iters, int hlim, int grid, cudaStream_t s);
 int launch_edge_relabel_build(const PoolView& P, int32_t* list, int32_t* count,
                               const ScanState& st, cudaStream_t s);
-// first: 0 frontier round, 1 first round over every tile, 2 first round over the tiles of
-// images that still had active tiles at the previous check.
-int launch_bfs_round(const PoolView& P, int first, int grid, cudaStream_t s);
+// first: 0 frontier round, 1 first round over the selected tiles, 2 over those of the images
+// live at stamp `live`; distances beyond `cap` stay GC_HINF.
+int launch_bfs_round(const PoolView& P, int first, int cap, int live, int grid, cudaStream_t s);
 // mode: 0 frontier round; first rounds over the selected tiles: 1 all, 2 those of the images
-// live in this cycle, 3 those of the images that continue from a previous flow; abort_hit:
-// frontier rounds skip images that reached a sink
-int launch_flood_round(const PoolView& P, int mode, int abort_hit, ImageAcc* acc, int grid,
-                       cudaStream_t s);
-// retires the images whose flood reached no sink; all: every image takes part
-int launch_flood_check(const PoolView& P, int all, cudaStream_t s);
-int launch_ctl_begin(const PoolView& P, int max_rounds, int max_cycles, ImageAcc* acc,
-                     cudaStream_t s);
-// over the solve's selected tiles; filter 1: only tiles of the images a flood check kept
-// (img_live == the cycle stamp), 2: those and the tiles of freshly uploaded images; grid:
-// most CTAs (a few per SM), which loop over the selection's chunks
+// live at `stamp`, 3 those of the images that continue from a previous flow; abort_hit:
+// frontier rounds skip images that reached a sink (they carry `stamp` in img_hit)
+int launch_flood_round(const PoolView& P, int mode, int abort_hit, int stamp, ImageAcc* acc,
+                       int grid, cudaStream_t s);
+// retires the images whose flood reached no sink; all: every image that continues from a flow
+int launch_flood_check(const PoolView& P, int all, int stamp, ImageAcc* acc, cudaStream_t s);
+int launch_ctl_begin(const PoolView& P, int max_rounds, ImageAcc* acc, cudaStream_t s);
+// active tiles of the selected images live at stamp `live`; fresh: freshly uploaded images
+// take part by fresh_tile_active; grid: most CTAs, which loop over the selection's chunks
 int launch_active_list(const PoolView& P, const ScanState& st, int32_t* list, int32_t* count,
-                       int bump, int count_cycle, int filter, ImageAcc* acc, int grid,
-                       cudaStream_t s);
+                       int live, int fresh, int grid, cudaStream_t s);
+// The relabel's distance cap: its first value in a solve, and the next after `cap`.
+constexpr int kFirstCap = 16;
+constexpr int kLastCap = 1 << 12;   // above it: exact distances
+__device__ __host__ __forceinline__ int next_cap(int cap) {
+  return cap >= kLastCap ? GC_HINF : cap * 4;
+}
 // The whole solve as one cooperative launch of `grid` CTAs (at most occupancy_solve()).
 struct SolveArgs {
   ImageAcc* acc;
@@ -102,6 +106,7 @@ struct SolveArgs {
   int warm, fresh;          // some selected image continues from a flow / is freshly uploaded
   int iters, pulses;        // sweeps per discharge, discharges per cycle
   int max_rounds, max_cycles;
+  int cap;                  // distance cap of the first relabel
   int lmode;                // 0 no labels; image im's labels: 1 a byte per pixel, 2 packed
   uint8_t* labels;
   ImageDesc im;

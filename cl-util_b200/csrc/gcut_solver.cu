@@ -285,7 +285,7 @@ k_upload(PoolView P, ImageDesc im, int img, Source src, int32_t* __restrict__ tl
   const int y = ty * GC_TILE + r;
   int e[4], h[4], cu[4], cd[4], cl[4], cr[4];
   long long pos = 0;
-  int bad = 0, anypos = 0;
+  int bad = 0;
   const int xb = tx * GC_TILE + c0;
   if (src.vec && y < im.H && xb + 3 < im.W) {
     src.pixel4(im, xb, y, e, cu, cd, cl, cr);
@@ -302,8 +302,14 @@ k_upload(PoolView P, ImageDesc im, int img, Source src, int32_t* __restrict__ tl
     bad |= (cu[j] | cd[j] | cl[j] | cr[j]) < 0;
     h[j] = e[j] < 0 ? 0 : 1;
     pos += e[j] > 0 ? e[j] : 0;
-    anypos |= e[j] > 0;
   }
+  const bool p4 = e[0] > 0 || e[1] > 0 || e[2] > 0 || e[3] > 0;
+  const bool s4 = e[0] < 0 || e[1] < 0 || e[2] < 0 || e[3] < 0;
+  unsigned tf = (p4 ? TF_POS | (r == 0 ? TF_POS_UP : 0) | (r == 31 ? TF_POS_DOWN : 0) : 0) |
+                (s4 ? TF_SINK | (r == 0 ? TF_SINK_UP : 0) | (r == 31 ? TF_SINK_DOWN : 0) : 0) |
+                (c0 == 0 ? (e[0] > 0 ? TF_POS_LEFT : 0) | (e[0] < 0 ? TF_SINK_LEFT : 0) : 0) |
+                (c0 == 28 ? (e[3] > 0 ? TF_POS_RIGHT : 0) | (e[3] < 0 ? TF_SINK_RIGHT : 0) : 0) |
+                (bad ? TF_BAD : 0);
   const long long off = (long long)t * GC_TILE_PX + r * GC_TILE + c0;
   *(int4*)(P.exc + off) = make_int4(e[0], e[1], e[2], e[3]);
   *(int4*)(tl + off) = make_int4(e[0], e[1], e[2], e[3]);
@@ -315,19 +321,28 @@ k_upload(PoolView P, ImageDesc im, int img, Source src, int32_t* __restrict__ tl
   write_tile_masks(P, t, e, cu, cd, cl, cr);
   if (threadIdx.x < 32) P.mreach[(long long)t * 32 + threadIdx.x] = 0u;   // no flood yet
   __shared__ long long wpos[DIS_THREADS / 32];
+  __shared__ unsigned wflag[DIS_THREADS / 32];
 #pragma unroll
   for (int o = 16; o; o >>= 1) pos += __shfl_xor_sync(0xffffffffu, pos, o);
-  if ((threadIdx.x & 31) == 0) wpos[threadIdx.x >> 5] = pos;
-  bad = __syncthreads_or(bad);
-  anypos = __syncthreads_or(anypos);
+  tf = __reduce_or_sync(0xffffffffu, tf);
+  if ((threadIdx.x & 31) == 0) {
+    wpos[threadIdx.x >> 5] = pos;
+    wflag[threadIdx.x >> 5] = tf;
+  }
+  __syncthreads();
   if (threadIdx.x == 0) {
     long long tp = 0;
-    for (int k = 0; k < DIS_THREADS / 32; ++k) tp += wpos[k];
+    tf = 0;
+    for (int k = 0; k < DIS_THREADS / 32; ++k) {
+      tp += wpos[k];
+      tf |= wflag[k];
+    }
     P.tpos[t] = tp;
     // one add per tile: the adds of all of an image's tiles go to one address
     if (tp) atomicAdd(&acc[img].sumpos_t, (unsigned long long)tp);
-    if (bad) atomicAdd(&acc[img].bad_caps, 1);
-    P.tact[t] = anypos;
+    if (tf & TF_BAD) atomicAdd(&acc[img].bad_caps, 1);
+    P.tflag[t] = (int32_t)tf;
+    P.tact[t] = (tf & TF_POS) != 0;
     P.touched[t] = 0;
     P.act_int[t] = 0;
     P.mark[0][t] = 0;
@@ -337,6 +352,23 @@ k_upload(PoolView P, ImageDesc im, int img, Source src, int32_t* __restrict__ tl
     P.img_of[t] = img;
     P.mdirty[t] = 0;     // the masks above are current
   }
+}
+
+// Whether a freshly uploaded tile belongs in the first list of a solve: it holds excess, and a
+// sink lies in the tile or just across one of its sides.  Under the trivial labelling (0 at
+// sinks, 1 elsewhere) the first sweep of any other tile pushes nothing, and its excess is too
+// far from a sink to deliver any within the first cycle; if it can reach one, the relabel
+// after the cycle's flood lists its tile with exact distances.  On six 1024^2 synthetic grids
+// the rule lists 146 to 661 tiles of the 654 to 927 that hold excess (median 270 of 792).
+__device__ __forceinline__ bool fresh_tile_active(const PoolView& P, int t) {
+  const int f = P.tflag[t];
+  if (!(f & TF_POS)) return false;
+  if (f & TF_SINK) return true;
+  const int4 nb = P.nbr[t];
+  return ((f & TF_POS_UP) && nb.x >= 0 && (P.tflag[nb.x] & TF_SINK_DOWN)) ||
+         ((f & TF_POS_DOWN) && nb.y >= 0 && (P.tflag[nb.y] & TF_SINK_UP)) ||
+         ((f & TF_POS_LEFT) && nb.z >= 0 && (P.tflag[nb.z] & TF_SINK_RIGHT)) ||
+         ((f & TF_POS_RIGHT) && nb.w >= 0 && (P.tflag[nb.w] & TF_SINK_LEFT));
 }
 
 // Mask rebuild of the selected tiles whose planes changed since their masks were written
@@ -480,11 +512,16 @@ __device__ __forceinline__ void dis_prefetch(const PoolView& P, int t, int32_t* 
     bulk_g2s(buf + k * GC_TILE_PX, dis_plane(P, k) + (long long)t * GC_TILE_PX, GC_TILE_PX * 4, mbar);
 }
 
+// hlim: pixels with a smaller height are active (GC_HINF: all that can reach a sink; smaller
+// after a relabel capped at distance hlim - 1, whose heights from hlim on only mean "at least
+// hlim").  A pixel that rises to hlim stays there, inactive until the next relabel.
+//
 // Discharges the n tiles of list `in` with the CTAs 0 .. nb-1 (this is CTA `bid`); the tiles
 // active afterwards or sent flow go to list `out` (none: out.list null).  buf, S and mbar are
 // the CTA's staging buffer, exchange arrays and (initialised) mbarrier; `phase` its parity,
 // kept from call to call.  Every thread of the CTA calls it.
-__device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, int bid, int nb_ctas,
+__device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, int hlim, int bid,
+                                                int nb_ctas,
                                                 const Worklist& in, int n, const Worklist& out,
                                                 int32_t* buf, DisSmem& S, uint64_t* mbar,
                                                 unsigned& phase) {
@@ -566,7 +603,7 @@ __device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, in
     for (int j = 0; j < 4; ++j) {
       const int c = c0 + j;
       const bool edge = erow || c == 0 || c == 31;
-      hcap[j] = edge ? (h[j] >= GC_HINF - 2 ? GC_HINF : h[j] + 2) : GC_HINF;
+      hcap[j] = edge ? imin(h[j] + 2, hlim) : hlim;
     }
     sts4(S.hs + pix, h[0], h[1], h[2], h[3]);
     __syncthreads();   // every thread has its values in registers: the buffer is free
@@ -593,13 +630,13 @@ __device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, in
       unsigned rem = 0;
 #pragma unroll
       for (int j = 0; j < 4; ++j) ou[j] = od[j] = ol[j] = orr[j] = 0;
-      const bool any_act = (e[0] > 0 && h[0] < GC_HINF) || (e[1] > 0 && h[1] < GC_HINF) ||
-                           (e[2] > 0 && h[2] < GC_HINF) || (e[3] > 0 && h[3] < GC_HINF);
+      const bool any_act = (e[0] > 0 && h[0] < hlim) || (e[1] > 0 && h[1] < hlim) ||
+                           (e[2] > 0 && h[2] < hlim) || (e[3] > 0 && h[3] < hlim);
       if (__any_sync(0xffffffffu, any_act)) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           int ej = e[j];
-          if (ej > 0 && h[j] < GC_HINF) {
+          if (ej > 0 && h[j] < hlim) {
             const int hm1 = h[j] - 1;
             if (cd[j] > 0 && hnd[j] == hm1) { const int f = imin(ej, cd[j]); ej -= f; cd[j] -= f; od[j] = f; }
             if (ej > 0 && cu[j] > 0 && hnu[j] == hm1) { const int f = imin(ej, cu[j]); ej -= f; cu[j] -= f; ou[j] = f; }
@@ -664,7 +701,7 @@ __device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, in
               if (cu[j] > 0) m = imin(m, hnu[j] + 1);
               if (cr[j] > 0) m = imin(m, hnr[j] + 1);
               if (cl[j] > 0) m = imin(m, hnl[j] + 1);
-              nh[j] = imin(imin(m, GC_HINF), hcap[j]);
+              nh[j] = imin(m, hcap[j]);
               changed |= nh[j] != h[j];
             }
           }
@@ -769,7 +806,7 @@ __device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, in
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int c = c0 + j;
-      const int a = e[j] > 0 && h[j] < GC_HINF;
+      const int a = e[j] > 0 && h[j] < hlim;
       act |= a;
       act_int |= a && !erow && c > 0 && c < 31;
     }
@@ -802,7 +839,7 @@ __device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, in
 
 // One pulse of the host-driven loop or of a manual push: the worklist of the pulse parity.
 __global__ void __launch_bounds__(DIS_THREADS, 4)
-k_discharge(PoolView P, int iters) {
+k_discharge(PoolView P, int iters, int hlim) {
   trace_mark(P, TR_DISCHARGE);
   extern __shared__ __align__(128) int32_t dsm[];
   DisSmem& S = *reinterpret_cast<DisSmem*>(dsm + DIS_PLANES * GC_TILE_PX);
@@ -819,7 +856,7 @@ k_discharge(PoolView P, int iters) {
   const Worklist in{P.queue[cur], P.qcount + cur, P.inq[cur]};
   const Worklist out{P.queue[nxt], P.qcount + nxt, P.inq[nxt]};
   unsigned phase = 0;
-  discharge_phase(P, iters, blockIdx.x, gridDim.x, in, s_n, out, dsm, S, &mbar, phase);
+  discharge_phase(P, iters, hlim, blockIdx.x, gridDim.x, in, s_n, out, dsm, S, &mbar, phase);
   // last CTA: the queue just read is consumed; the next launch reads the other one
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -966,18 +1003,20 @@ __device__ __forceinline__ int warp_min(int v) {
 // in the top row (`top`) and the bottom row (`bot`); lane r holds the seeds of row r at column
 // 0 (`sl`) and 31 (`sr`); GC_HINF where there is none.  Level L visits the unvisited pixels
 // that are seeds of value L or neighbours, over residual edges, of level L - 1; an empty level
-// jumps to the smallest unvisited seed.  Lane r writes the distances of row r into `row`
-// (GC_HINF where unreached) and gets the mask of reached pixels.
+// jumps to the smallest unvisited seed.  Levels above `cap` stay unreached.  Lane r writes the
+// distances of row r into `row` (GC_HINF where unreached) and gets the mask of reached pixels.
 __device__ __forceinline__ uint32_t tile_bfs_seeded(int* row, uint32_t sink, uint32_t canU,
                                                     uint32_t canD, uint32_t canL, uint32_t canR,
-                                                    int lane, int top, int bot, int sl, int sr) {
+                                                    int lane, int top, int bot, int sl, int sr,
+                                                    int cap) {
   const unsigned FULL = 0xffffffffu;
 #pragma unroll
   for (int c = 0; c < 32; ++c) row[c] = GC_HINF;
   uint32_t vis = 0, F = 0;
+  const int last = imin(cap, GC_HINF - 1);
   int L = __any_sync(FULL, sink != 0) ? 0 : warp_min(imin(imin(top, bot), imin(sl, sr)));
   // every step visits a pixel or jumps to an unvisited seed: at most 1024 + 128 steps
-  for (int step = 0; step < 2 * GC_TILE_PX && L < GC_HINF; ++step) {
+  for (int step = 0; step < 2 * GC_TILE_PX && L <= last; ++step) {
     uint32_t Fu = __shfl_up_sync(FULL, F, 1);
     uint32_t Fd = __shfl_down_sync(FULL, F, 1);
     if (lane == 0) Fu = 0;
@@ -1084,7 +1123,10 @@ __device__ __forceinline__ void frontier_round_end(const PoolView& P, int first,
 // Solve prologue: reset the control words and the image stamps; the images of the
 // selection take their mode for this solve and restart their flow sums (the others keep
 // their results).  One CTA.
-__global__ void k_ctl_begin(PoolView P, int max_rounds, int max_cycles, ImageAcc* acc) {
+// Stamps of the host-driven loop: the floods are numbered, 1 the flood before the first
+// pulses (only warm images), 2 + c the flood of cycle c; an image is live at the stamp of the
+// next flood it takes part in.
+__global__ void k_ctl_begin(PoolView P, int max_rounds, ImageAcc* acc) {
   trace_mark(P, TR_BEGIN);
   for (int i = threadIdx.x; i < CTL_N; i += blockDim.x) P.ctl[i] = 0;
   for (int i = threadIdx.x; i < P.nimg; i += blockDim.x) {
@@ -1098,11 +1140,11 @@ __global__ void k_ctl_begin(PoolView P, int max_rounds, int max_cycles, ImageAcc
     const int img = P.sel[k].w;
     if ((unsigned)img >= (unsigned)P.nimg) continue;
     P.img_mode[img] = P.sel_mode[k];
+    if (P.sel_mode[k] == 1) P.img_live[img] = 2;
     acc[img].sumpos_e = 0;   // the floods of this solve accumulate it
   }
   if (threadIdx.x == 0) {
     P.ctl[CTL_MAXROUNDS] = max_rounds;
-    P.ctl[CTL_MAXCYCLES] = max_cycles;
     P.rcnt[0] = 0;
     P.rcnt[1] = 0;
     P.fcount[0] = 0;
@@ -1132,46 +1174,28 @@ __device__ __forceinline__ void publish_results(const PoolView& P, const ImageAc
   }
 }
 
-// The active-tile list after a global relabel, in one launch: a single-pass scan (chunks by
-// arrival ticket, decoupled look-back) of the activity flags of the selected tiles writes the
-// ids of the active tiles in order and stamps their images live for the next cycle (stamp =
-// cycles + 1 + bump); the last CTA to finish closes the scan and applies the cycle check:
-// another cycle runs while tiles are active and the cycle cap is not reached (`count_cycle`
-// counts this check as a finished cycle).  Replaces a compaction and a separate stamping
-// launch.  filter: 1 only tiles of the images a flood check kept (img_live == the cycle
-// stamp; a solved image keeps the activity flags of its last relabel), 2 those and the tiles
-// of freshly uploaded images (the first list of a solve).
+// The active-tile list of the host-driven loop, in one launch: a single-pass scan (chunks by
+// arrival ticket, decoupled look-back) of the activity flags of the selected tiles whose
+// image is live at stamp `live` writes the ids of the active tiles in order.  fresh: the
+// first list of a solve, in which freshly uploaded images follow fresh_tile_active.
 //
 // The grid is a fixed number of CTAs (a few per SM) that take chunk tickets in a loop until
 // the selection's chunks run out, so a pool of millions of tiles costs no more launch work
-// than one image, and a 2048^2 image (4096 tiles) spreads over four CTAs.  Every ticket
-// holder is already running, so a look-back only ever waits for a running CTA.  The image
-// of each item comes from the selection (one range per image), and an image's live stamp,
-// flood sum and sink-reached stamp are written once per warp that holds one of its active
-// tiles rather than once per tile: thousands of stores to one address serialise in L2.
+// than one image.  Every ticket holder is already running, so a look-back only ever waits for
+// a running CTA.
 constexpr int ACT_THREADS = 256;
 constexpr int ACT_ITEMS = 4;
 constexpr int ACT_CHUNK = ACT_THREADS * ACT_ITEMS;
 
-__device__ __forceinline__ void stamp_image(const PoolView& P, ImageAcc* acc, int img, int stamp) {
-  P.img_live[img] = stamp;
-  // the image's next flood starts afresh: its sum and its sink-reached stamp (the first
-  // cycle of a warm solve reuses the stamp of the flood before it)
-  acc[img].sumpos_e = 0;
-  P.img_hit[img] = 0;
-}
-
 __global__ void __launch_bounds__(ACT_THREADS)
-k_active_list(PoolView P, ScanState st, int32_t* list, int32_t* count, int bump,
-              int count_cycle, int filter, ImageAcc* acc) {
+k_active_list(PoolView P, ScanState st, int32_t* list, int32_t* count, int live, int fresh) {
   trace_mark(P, TR_ACTIVE_LIST);
   __shared__ int32_t sm[32];
-  __shared__ int32_t s_chunk, s_excl, s_cur, s_n, s_nr;
+  __shared__ int32_t s_chunk, s_excl, s_n, s_nr;
   __shared__ uint32_t s_tag;
   if (threadIdx.x == 0) {
     s_chunk = atomicAdd(st.ticket, 1);
     s_tag = *((volatile uint32_t*)st.seq);
-    s_cur = *((volatile int32_t*)&P.ctl[CTL_CYCLES]) + 1;
     int n = *((volatile int32_t*)&P.nsel[1]), nr = *((volatile int32_t*)&P.nsel[0]);
     if (n < 0 || n > P.nt || nr < 0 || nr > P.nimg) {   // self-check
       record_bad(P, 9, n);
@@ -1181,41 +1205,27 @@ k_active_list(PoolView P, ScanState st, int32_t* list, int32_t* count, int bump,
     s_nr = nr;
   }
   __syncthreads();
-  const int cur = s_cur, stamp = cur + bump;
   const int n = s_n;
   const int nchunks = (n + ACT_CHUNK - 1) / ACT_CHUNK;
-  const int lane = threadIdx.x & 31;
   for (int chunk = s_chunk; chunk < nchunks;) {
     const int base = chunk * ACT_CHUNK + threadIdx.x * ACT_ITEMS;
     SelCursor cursor(P, s_nr, base < n ? base : 0);
-    int32_t v[ACT_ITEMS], tl[ACT_ITEMS], im[ACT_ITEMS];
+    int32_t v[ACT_ITEMS], tl[ACT_ITEMS];
+    int32_t tsum = 0;
 #pragma unroll
     for (int k = 0; k < ACT_ITEMS; ++k) {
       tl[k] = -1;
-      im[k] = -1;
-      if (base + k < n) {
-        tl[k] = cursor.tile(base + k);
-        im[k] = cursor.image();
-      }
       v[k] = 0;
-      if ((unsigned)tl[k] < (unsigned)P.nt && (unsigned)im[k] < (unsigned)P.nimg)
-        v[k] = P.tact[tl[k]] != 0;
-      else if (tl[k] >= 0)
-        record_bad(P, 4, (unsigned)im[k] < (unsigned)P.nimg ? tl[k] : im[k]);
-    }
-    if (filter) {
-#pragma unroll
-      for (int k = 0; k < ACT_ITEMS; ++k) {
-        if (!v[k]) continue;
-        const int il = *((volatile int32_t*)&P.img_live[im[k]]);
-        v[k] = il == cur || il == stamp || (filter == 2 && P.img_mode[im[k]] == 1);
+      if (base + k >= n) continue;
+      tl[k] = cursor.tile(base + k);
+      const int im = cursor.image();
+      if ((unsigned)tl[k] >= (unsigned)P.nt || (unsigned)im >= (unsigned)P.nimg) {
+        record_bad(P, 4, (unsigned)im < (unsigned)P.nimg ? tl[k] : im);
+        continue;
       }
-    }
-    int32_t tsum = 0, first = -1;
-#pragma unroll
-    for (int k = ACT_ITEMS - 1; k >= 0; --k) {
+      if (P.img_live[im] != live) continue;
+      v[k] = fresh && P.img_mode[im] == 1 ? fresh_tile_active(P, tl[k]) : P.tact[tl[k]] != 0;
       tsum += v[k];
-      if (v[k]) first = im[k];
     }
     int32_t agg;
     const int32_t tex = block_exclusive_scan(tsum, sm, &agg);
@@ -1224,23 +1234,13 @@ k_active_list(PoolView P, ScanState st, int32_t* list, int32_t* count, int bump,
       if (threadIdx.x == 0) s_excl = ex;
     }
     __syncthreads();
-    // one lane per distinct first image in the warp stamps it; the rare later images of a
-    // thread (its items straddle two ranges) are stamped by that thread
-    const unsigned peers = __match_any_sync(0xffffffffu, first);
-    if (first >= 0 && __ffs(peers) - 1 == lane) stamp_image(P, acc, first, stamp);
     int32_t run = s_excl + tex;
-    int last = first;
 #pragma unroll
     for (int k = 0; k < ACT_ITEMS; ++k) {
-      if (v[k]) {
-        if ((unsigned)run < (unsigned)P.nt) list[run] = tl[k];
-        else atomicExch(st.err, 2);   // only after a look-back that gave up
-        if (im[k] != last) {
-          stamp_image(P, acc, im[k], stamp);
-          last = im[k];
-        }
-        ++run;
-      }
+      if (!v[k]) continue;
+      if ((unsigned)run < (unsigned)P.nt) list[run] = tl[k];
+      else atomicExch(st.err, 2);   // only after a look-back that gave up
+      ++run;
     }
     if (chunk == nchunks - 1 && threadIdx.x == 0) *count = s_excl + agg;
     // the first tickets are 0 .. gridDim.x - 1: when they cover every chunk, none is left
@@ -1253,7 +1253,7 @@ k_active_list(PoolView P, ScanState st, int32_t* list, int32_t* count, int bump,
   if (threadIdx.x != 0) return;
   __threadfence();
   if (atomicAdd(st.done, 1) != (int)gridDim.x - 1) return;
-  // last CTA: close the scan (tickets, tag) and apply the cycle check
+  // last CTA: close the scan (tickets, tag)
   __threadfence();
   *st.ticket = 0;
   *st.done = 0;
@@ -1262,17 +1262,13 @@ k_active_list(PoolView P, ScanState st, int32_t* list, int32_t* count, int bump,
   *st.seq = sq;
   volatile int32_t* ctl = P.ctl;
   if (nchunks == 0) *count = 0;
-  const int nact = *((volatile int32_t*)count);
   ctl[CTL_PULSE] = 0;   // the list sits in queue[0]
   ctl[CTL_DDONE] = 0;
   P.qcount[1] = 0;
-  const int cycles = ctl[CTL_CYCLES] + (count_cycle ? 1 : 0);
-  ctl[CTL_CYCLES] = cycles;
   ctl[CTL_NACT] = ctl[CTL_NACT] + 1;
   // a look-back that gave up (here or in an earlier list of this solve) reaches the host
   // with the control words
   ctl[CTL_SCANERR] = ctl[CTL_SCANERR] | *((volatile int32_t*)st.err);
-  if (nact > 0 && ctl[CTL_ERR] < 3 && cycles >= ctl[CTL_MAXCYCLES]) ctl[CTL_ERR] = 2;
   __threadfence();
 }
 
@@ -1290,8 +1286,8 @@ __global__ void k_ctl_cycle(PoolView P) {
 // and (frontier rounds) the halo distances, the heights written back, and the neighbours whose
 // edge distances dropped queued.  T: the warp's 32 x 33 words of shared memory.  Returns
 // whether the tile holds an active pixel.
-__device__ __forceinline__ int bfs_tile(const PoolView& P, int t, int lane, int first, int32_t* T,
-                                        const Worklist& out) {
+__device__ __forceinline__ int bfs_tile(const PoolView& P, int t, int lane, int first, int cap,
+                                        int32_t* T, const Worklist& out) {
   const int4 nb = P.nbr[t];
   const long long base = (long long)t * GC_TILE_PX;
   // the masks are current: the flood that precedes every global relabel of a solve (or
@@ -1315,7 +1311,7 @@ __device__ __forceinline__ int bfs_tile(const PoolView& P, int t, int lane, int 
     if ((canR >> 31) && vr < GC_HINF) sr = vr + 1;
   }
   const uint32_t fin = tile_bfs_seeded(T + lane * 33, sink, canU, canD, canL, canR, lane, top,
-                                       bot, sl, sr);
+                                       bot, sl, sr, cap);
   __syncwarp();
   int chU = 0, chD = 0, chL = 0, chR = 0;
   for (int rr = 0; rr < 32; ++rr) {
@@ -1347,7 +1343,7 @@ __device__ __forceinline__ int bfs_tile(const PoolView& P, int t, int lane, int 
 }
 
 __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
-k_bfs_round(PoolView P, int first) {
+k_bfs_round(PoolView P, int first, int cap, int live) {
   trace_mark(P, first ? TR_BFS_FIRST : TR_BFS);
   __shared__ int32_t tr[WARPS_PER_CTA][32 * 33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1355,9 +1351,7 @@ k_bfs_round(PoolView P, int first) {
   const Worklist out{P.fq[in ^ 1], P.fcount + (in ^ 1), P.mark[in ^ 1]};
   int32_t* const markin = P.mark[in];
   int done = 0;
-  // first == 2: a global relabel inside the solve loop skips images whose cut was final at
-  // the previous check (no active tile); their state no longer changes
-  const int live = first == 2 ? *((volatile int32_t*)&P.ctl[CTL_CYCLES]) + 1 : 0;
+  // first == 2: a global relabel inside the solve loop covers the images live at stamp `live`
   int n, parts, nr;
   frontier_work(P, first, in, WARPS_PER_CTA, &n, &parts, &nr);
   if ((int)blockIdx.x >= parts) return;
@@ -1382,7 +1376,7 @@ k_bfs_round(PoolView P, int first) {
       }
     }
     ++done;
-    const int act = bfs_tile(P, t, lane, first, tr[warp], out);
+    const int act = bfs_tile(P, t, lane, first, cap, tr[warp], out);
     if (lane == 0) P.tact[t] = act;
   }
   if (lane == 0 && done) {
@@ -1394,10 +1388,10 @@ k_bfs_round(PoolView P, int first) {
 
 // After a flood of the host-driven loop: an image whose flood reached no sink pixel is solved
 // (its flood is the canonical cut, its sums are final) and leaves the live set; the others go
-// on to a global relabel.  all != 0: the images that continue from a previous flow
-// (img_mode == 2; the first check of a solve); else the images live in this cycle.  The last
-// cycle of a solve is counted here.  One CTA.
-__global__ void k_flood_check(PoolView P, int all) {
+// on to a global relabel, live at stamp + 1, with their sums and sink-reached stamps cleared.
+// all != 0: the images that continue from a previous flow (img_mode == 2; the first check of
+// a solve); else the images live at `stamp`.  One CTA.
+__global__ void k_flood_check(PoolView P, int all, int stamp, ImageAcc* acc) {
   __shared__ int s_left;
   if (threadIdx.x == 0) {
     s_left = 0;
@@ -1405,14 +1399,15 @@ __global__ void k_flood_check(PoolView P, int all) {
   }
   __syncthreads();
   volatile int32_t* ctl = P.ctl;
-  const int stamp = ctl[CTL_CYCLES] + 1;
   int left = 0;
   for (int i = threadIdx.x; i < P.nimg; i += blockDim.x) {
     const bool part = all ? *((volatile int32_t*)&P.img_mode[i]) == 2
                           : *((volatile int32_t*)&P.img_live[i]) == stamp;
     if (!part) continue;
     if (*((volatile int32_t*)&P.img_hit[i]) == stamp) {
-      P.img_live[i] = stamp;
+      P.img_live[i] = stamp + 1;
+      P.img_hit[i] = 0;
+      acc[i].sumpos_e = 0;
       ++left;
     } else {
       P.img_live[i] = 0;   // solved: no later stamp equals 0
@@ -1425,7 +1420,6 @@ __global__ void k_flood_check(PoolView P, int all) {
   if (ctl[CTL_ERR] != 0) n = 0;   // a cap or a self-check ends the loops
   ctl[CTL_LEFT] = n;
   ctl[CTL_NCHECK] = ctl[CTL_NCHECK] + 1;
-  if (n == 0 && !all) ctl[CTL_CYCLES] = ctl[CTL_CYCLES] + 1;
   if (n == 0) trace_record(P, TR_END);
 }
 
@@ -1544,17 +1538,16 @@ __device__ __forceinline__ void flood_sum_flush(ImageAcc* acc, const FloodSum& f
 
 // A flood round of the host-driven loop.  mode: 0 frontier round; first rounds over the
 // selected tiles: 1 all of them, 2 those of the images live in this cycle (img_live ==
-// stamp), 3 those of the images that continue from a previous flow (img_mode == 2).
+// the flood's stamp), 3 those of the images that continue from a previous flow (img_mode == 2).
 // abort_hit: frontier rounds skip the tiles of images already stamped (their flood is redone
 // in a later cycle).
 __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
-k_flood_round(PoolView P, int mode, int abort_hit, ImageAcc* acc) {
+k_flood_round(PoolView P, int mode, int abort_hit, int stamp, ImageAcc* acc) {
   trace_mark(P, mode ? TR_FLOOD_FIRST : TR_FLOOD);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int first = mode != 0;
   const int in = frontier_round_number(P, first) & 1;
   const Worklist out{P.fq[in ^ 1], P.fcount + (in ^ 1), P.mark[in ^ 1]};
-  const int stamp = *((volatile int32_t*)&P.ctl[CTL_CYCLES]) + 1;
   int32_t* const markin = P.mark[in];
   int done = 0;
   int n, parts, nr;
@@ -1724,6 +1717,13 @@ __device__ __forceinline__ bool grid_sync(const PoolView& P, unsigned long long&
 //
 // 4 CTAs of 256 threads per SM (k_discharge's shape: registers and shared memory bound it);
 // the relabel's staging shares the discharge's shared memory.
+// Cap of the relabel's distances.  Excess moves at most pulses x iters pixels a cycle, so
+// only excess near a sink matters to a cycle; distances beyond the cap are not computed, and
+// pixels there stay inactive.  Exact distances would be the chain of tile rounds across every
+// region that has excess and one unsaturated edge left (up to 34 rounds of 14-25 us at
+// 4096^2), with all its tiles discharged.  The labels stay valid: below the cap they are
+// exact, and at or above it "not below".  The cap grows with every cycle, and at once when no
+// excess lies within it, so the schedule ends in exact relabels and terminates as they do.
 constexpr int SOLVE_WARPS = DIS_THREADS / 32;
 constexpr size_t SOLVE_BFS_SMEM = (size_t)SOLVE_WARPS * 32 * 33 * sizeof(int32_t);
 constexpr size_t SOLVE_DYN_SMEM = DIS_DYN_SMEM > SOLVE_BFS_SMEM ? DIS_DYN_SMEM : SOLVE_BFS_SMEM;
@@ -1740,6 +1740,7 @@ k_solve(PoolView P, SolveArgs A) {
   int qk = 0, fk = 0;     // steps of the worklist and of the frontier (counter slots mod 3)
   int stamp = 0, cycles = 0, err = 0;
   int nrounds_f = 0, nrounds_b = 0;
+  int cap = A.cap, hlim = GC_HINF;   // of the last relabel (none yet: trivial labels)
   int v0, v1;
   // ---- prologue: control words, image modes and flow sums
   trace_mark(P, TR_BEGIN);
@@ -1775,7 +1776,7 @@ k_solve(PoolView P, SolveArgs A) {
         Worklist out{P.queue[(qk + 1) & 1], &P.ctl[CTL_Q0 + (qk + 1) % 3], P.inq[(qk + 1) & 1]};
         if (p == A.pulses - 1) out.list = nullptr;   // the relabel makes the next list
         if (bid == 0 && tid == 0) P.ctl[CTL_Q0 + (qk + 2) % 3] = 0;
-        discharge_phase(P, A.iters, bid, nb, in, v0, out, dsm,
+        discharge_phase(P, A.iters, hlim, bid, nb, in, v0, out, dsm,
                         *reinterpret_cast<DisSmem*>(dsm + DIS_PLANES * GC_TILE_PX), &mbar, phase);
         ++qk;
         alive = grid_sync(P, target, s_bc, &P.ctl[CTL_Q0 + qk % 3], &P.ctl[CTL_ERR], v0, v1);
@@ -1841,7 +1842,7 @@ k_solve(PoolView P, SolveArgs A) {
         const Worklist act_out{P.queue[qk & 1], &P.ctl[CTL_Q0 + qk % 3], nullptr};
         n = n_sel;
         rounds = 0;
-        for (bool first = true;; first = false) {
+        for (bool first = true;;) {
           trace_mark(P, first ? TR_BFS_FIRST : TR_BFS);
           const Worklist out{P.fq[(fk + 1) & 1], &P.ctl[CTL_F0 + (fk + 1) % 3], P.mark[(fk + 1) & 1]};
           if (bid == 0 && tid == 0) P.ctl[CTL_F0 + (fk + 2) % 3] = 0;
@@ -1851,7 +1852,7 @@ k_solve(PoolView P, SolveArgs A) {
             const int t = first ? cursor.tile(i) : P.fq[fk & 1][i];
             if (first && P.img_hit[cursor.image()] != stamp) continue;
             if (!first && lane == 0) P.mark[fk & 1][t] = 0;
-            const int act = bfs_tile(P, t, lane, first, dsm + warp * (32 * 33), out);
+            const int act = bfs_tile(P, t, lane, first, cap, dsm + warp * (32 * 33), out);
             if (lane == 0) {
               // a tile becomes active once (its reached set only grows): list it then
               if (act && (first || P.tact[t] == 0)) worklist_append(P, act_out, t);
@@ -1862,16 +1863,29 @@ k_solve(PoolView P, SolveArgs A) {
           ++rounds;
           alive = grid_sync(P, target, s_bc, &P.ctl[CTL_F0 + fk % 3], &P.ctl[CTL_Q0 + qk % 3], v0, v1);
           n = v0;
-          if (!alive || n == 0) break;
+          first = false;
+          if (!alive) break;
+          if (n == 0) {
+            if (v1 > 0 || cap >= GC_HINF) break;
+            // no excess within the cap of a sink: relabel again, further out
+            cap = next_cap(cap);
+            n = n_sel;
+            first = true;
+            nrounds_b += rounds;
+            rounds = 0;
+            continue;
+          }
           if (n < 0 || n > P.nt) { alive = false; break; }
           if (rounds >= A.max_rounds) { err = 1; break; }
         }
         nrounds_b += rounds;
+        hlim = cap < GC_HINF ? cap + 1 : GC_HINF;
+        cap = next_cap(cap);   // further out with every cycle
         if (!alive || err) break;
       }
     }
     if (cyc == 0 && A.fresh) {
-      // ---- the fresh images' first list: tiles with positive excess
+      // ---- the fresh images' first list
       trace_mark(P, TR_ACTIVE_LIST);
       const Worklist act_out{P.queue[qk & 1], &P.ctl[CTL_Q0 + qk % 3], nullptr};
       const int i0 = bid * DIS_THREADS + tid;
@@ -1880,7 +1894,7 @@ k_solve(PoolView P, SolveArgs A) {
         int t = -1;
         if (b + tid < n_sel) {
           t = cursor.tile(b + tid);
-          if (P.img_mode[cursor.image()] != 1 || P.tact[t] == 0) t = -1;
+          if (P.img_mode[cursor.image()] != 1 || !fresh_tile_active(P, t)) t = -1;
         }
         const unsigned m = __ballot_sync(0xffffffffu, t >= 0);
         if (m == 0) continue;
@@ -1895,7 +1909,8 @@ k_solve(PoolView P, SolveArgs A) {
       alive = grid_sync(P, target, s_bc, &P.ctl[CTL_Q0 + qk % 3], &P.ctl[CTL_Q0 + qk % 3], v0, v1);
     }
     v0 = v1;   // the worklist's length
-    if (!alive || v0 == 0) break;
+    // (an empty first list still needs the flood: no fresh tile is near a sink)
+    if (!alive || (v0 == 0 && !(cyc == 0 && A.fresh))) break;
     if (cycles >= A.max_cycles) { err = 2; break; }
   }
 
@@ -2126,8 +2141,8 @@ int launch_masks(const PoolView& P, int grid, cudaStream_t s) {
   return ok();
 }
 
-int launch_discharge(const PoolView& P, int iters, int grid, cudaStream_t s) {
-  k_discharge<<<grid, DIS_THREADS, DIS_DYN_SMEM, s>>>(P, iters);
+int launch_discharge(const PoolView& P, int iters, int hlim, int grid, cudaStream_t s) {
+  k_discharge<<<grid, DIS_THREADS, DIS_DYN_SMEM, s>>>(P, iters, hlim);
   return ok();
 }
 
@@ -2139,19 +2154,19 @@ int launch_edge_relabel_build(const PoolView& P, int32_t* list, int32_t* count,
   return ok();
 }
 
-int launch_bfs_round(const PoolView& P, int first, int grid, cudaStream_t s) {
-  k_bfs_round<<<grid, WARPS_PER_CTA * 32, 0, s>>>(P, first);
+int launch_bfs_round(const PoolView& P, int first, int cap, int live, int grid, cudaStream_t s) {
+  k_bfs_round<<<grid, WARPS_PER_CTA * 32, 0, s>>>(P, first, cap, live);
   return ok();
 }
 
-int launch_flood_round(const PoolView& P, int mode, int abort_hit, ImageAcc* acc, int grid,
-                       cudaStream_t s) {
-  k_flood_round<<<grid, WARPS_PER_CTA * 32, 0, s>>>(P, mode, abort_hit, acc);
+int launch_flood_round(const PoolView& P, int mode, int abort_hit, int stamp, ImageAcc* acc,
+                       int grid, cudaStream_t s) {
+  k_flood_round<<<grid, WARPS_PER_CTA * 32, 0, s>>>(P, mode, abort_hit, stamp, acc);
   return ok();
 }
 
-int launch_flood_check(const PoolView& P, int all, cudaStream_t s) {
-  k_flood_check<<<1, 256, 0, s>>>(P, all);
+int launch_flood_check(const PoolView& P, int all, int stamp, ImageAcc* acc, cudaStream_t s) {
+  k_flood_check<<<1, 256, 0, s>>>(P, all, stamp, acc);
   return ok();
 }
 
@@ -2175,20 +2190,17 @@ int launch_acc_reset(ImageAcc* acc, int n, cudaStream_t s) {
   return ok();
 }
 
-int launch_ctl_begin(const PoolView& P, int max_rounds, int max_cycles, ImageAcc* acc,
-                     cudaStream_t s) {
-  k_ctl_begin<<<1, 256, 0, s>>>(P, max_rounds, max_cycles, acc);
+int launch_ctl_begin(const PoolView& P, int max_rounds, ImageAcc* acc, cudaStream_t s) {
+  k_ctl_begin<<<1, 256, 0, s>>>(P, max_rounds, acc);
   return ok();
 }
 
 int launch_active_list(const PoolView& P, const ScanState& st, int32_t* list, int32_t* count,
-                       int bump, int count_cycle, int filter, ImageAcc* acc, int grid,
-                       cudaStream_t s) {
+                       int live, int fresh, int grid, cudaStream_t s) {
   const int nch = (P.nt + ACT_CHUNK - 1) / ACT_CHUNK;   // enough for any selection
   if (nch > st.max_chunks) return GC_ERR_INVALID;
   grid = grid < nch ? grid : nch;
-  k_active_list<<<grid > 0 ? grid : 1, ACT_THREADS, 0, s>>>(P, st, list, count, bump, count_cycle,
-                                                            filter, acc);
+  k_active_list<<<grid > 0 ? grid : 1, ACT_THREADS, 0, s>>>(P, st, list, count, live, fresh);
   return ok();
 }
 
