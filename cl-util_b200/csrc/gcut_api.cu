@@ -155,8 +155,8 @@ struct Pool {
   bool use_graph = true;
   ImageAcc* h_acc = nullptr;   // pinned
   int grid_dis = 0, grid_warps = 0, grid_solve = 0, sms = 1;
-  unsigned long long* dsum = nullptr;     // device: sum of |dI|^2 (gc_upload_rgba)
-  int32_t* ntab = nullptr;                // device: n-link thresholds (gc_upload_rgba)
+  unsigned long long* dsum = nullptr;     // device: state of launch_nlinks (gc_upload_rgba)
+  int32_t* ntab = nullptr;                // device: n-link table (gc_upload_rgba)
   bool uploaded = false, solved = false, edited = false, collect = false;
   bool list_valid = false, bfs_fresh = false;
   // per image: uploaded, solved since its upload or last edit, edited since its last solve
@@ -297,8 +297,8 @@ struct Pool {
     c.take(&scan.st.ticket, 4);
     scan.st.max_chunks = chunks;
     c.take(&pts, 2 * 1024);
-    c.take(&dsum, 1);
-    c.take(&ntab, GC_NLINK_LEVELS);
+    c.take(&dsum, 2);
+    c.take(&ntab, GC_NLINK_LEVELS + 1);
     if (imgs.size() == 1) c.take(&lstage, (size_t)imgs[0].W * imgs[0].H);
   }
 
@@ -451,21 +451,16 @@ struct Pool {
 
   // Capacities from an RGBA image (n-links) and int32 t-links, all on the device with no
   // host wait.  lambda == 0: the exp weighting, whose scale comes from the mean |dI|^2 over
-  // all 4-neighbour pairs (k_dsum sums it exactly, k_nlink_table turns it into the weight
-  // thresholds); lambda > 0: the reference's weighting with that LAMBDA.
+  // all 4-neighbour pairs (k_nlinks sums it exactly and turns it into the weight thresholds);
+  // lambda > 0: the reference's weighting with that LAMBDA.
   int upload_rgba(int i, const uint32_t* rgba, const int32_t* excess, int lambda, cudaStream_t s) {
     if (i < 0 || i >= (int)imgs.size()) return fail(GC_ERR_INVALID, "image index");
     if (!rgba || !excess) return fail(GC_ERR_INVALID, "null plane");
     if (lambda < 0 || lambda > GC_NLINK_MAX_LAMBDA) return fail(GC_ERR_INVALID, "lambda out of range");
     CK(cudaSetDevice(device));
     const ImageDesc& im = imgs[i];
-    if (lambda == 0) {
-      const long long npairs = (long long)(im.H - 1) * im.W + (long long)im.H * (im.W - 1);
-      CK(cudaMemsetAsync(dsum, 0, sizeof(unsigned long long), s));
-      RK(launch_dsum(rgba, im.W, im.H, dsum, sms, s));
-      RK(launch_nlink_table(dsum, npairs, ntab, s));
-    }
-    CK(cudaMemsetAsync(acc + i, 0, sizeof(ImageAcc), s));
+    if (lambda == 0) RK(launch_nlinks(rgba, im.W, im.H, dsum, ntab, acc + i, s));
+    else CK(cudaMemsetAsync(acc + i, 0, sizeof(ImageAcc), s));
     P.ktiles = nullptr;
     RK(timed(K_UPLOAD, s, [&] {
       return launch_upload_rgba(P, im, i, rgba, excess, lambda ? nullptr : ntab, lambda, tl, acc, s);

@@ -64,16 +64,15 @@ int launch_masks(const PoolView& P, int grid, cudaStream_t s);
 // n-link table of gc_upload_rgba: weight(d) = floor(50 * exp(-beta * d) + 0.5) for d = |dI|^2
 // equals the number of entries t[k] >= d (t[k] = largest d with weight >= k + 1).
 constexpr int GC_NLINK_LEVELS = 50;
-// tab: the 50 device thresholds (exp weighting), or null for the reference's weighting
+// tab: the device table of launch_nlinks (exp weighting), or null for the reference's weighting
 // floor(lambda / (0.1 sqrt(d) + 0.05) + 0.5) (gc_upload_rgba_lambda)
 int launch_upload_rgba(const PoolView& P, const ImageDesc& im, int img, const uint32_t* rgba,
                        const int32_t* excess, const int32_t* tab, int lambda, int32_t* tl,
                        ImageAcc* acc, cudaStream_t s);
-// tab[0..50) from the |dI|^2 sum (device) and the number of 4-neighbour pairs
-int launch_nlink_table(const unsigned long long* sum, long long npairs, int32_t* tab,
-                       cudaStream_t s);
-int launch_dsum(const uint32_t* rgba, int W, int H, unsigned long long* sum, int sms,
-                cudaStream_t s);
+// The mean |dI|^2 of an image and the n-link table from it (tab: 50 thresholds and a float),
+// one launch; state: two zeroed words, zero again afterwards.  Clears *acc for the upload.
+int launch_nlinks(const uint32_t* rgba, int W, int H, unsigned long long* state, int32_t* tab,
+                  ImageAcc* acc, cudaStream_t s);
 // hlim: pixels below this height are active
 int launch_discharge(const PoolView& P, int iters, int hlim, int grid, cudaStream_t s);
 int launch_edge_relabel_build(const PoolView& P, int32_t* list, int32_t* count,

@@ -28,6 +28,7 @@
 //                  pixels over residual edges (the minimal source set).
 #include <cstdio>
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 
 #include "gcut_common.cuh"
@@ -151,152 +152,16 @@ __device__ __forceinline__ RowMasks warp_rebuild_masks(const PoolView& P, int t,
   return out;
 }
 
-// Capacity sources of the upload.  PlaneSource: row-major capacity planes (gc_upload).
-// RgbaSource: n-links built from an RGBA image and the n-link table (gc_upload_rgba).
-struct PlaneSource {
-  const int32_t *up, *down, *left, *right, *excess;
-  bool vec;   // all planes 16-byte aligned and the width a multiple of 4: int4 row loads
-  __device__ __forceinline__ void prepare(int32_t*) const {}
-  // the four pixels (x0 .. x0+3, y) at once, all inside the image (x0 + 3 < W)
-  __device__ __forceinline__ void pixel4(const ImageDesc& im, int x0, int y, int (&e)[4],
-                                         int (&cu)[4], int (&cd)[4], int (&cl)[4],
-                                         int (&cr)[4]) const {
-    const long long i = (long long)y * im.W + x0;
-    const int4 a = *reinterpret_cast<const int4*>(excess + i);
-    const int4 b = *reinterpret_cast<const int4*>(up + i);
-    const int4 c = *reinterpret_cast<const int4*>(down + i);
-    const int4 d = *reinterpret_cast<const int4*>(left + i);
-    const int4 f = *reinterpret_cast<const int4*>(right + i);
-    e[0] = a.x; e[1] = a.y; e[2] = a.z; e[3] = a.w;
-    const bool top = y == 0, bottom = y == im.H - 1;
-    cu[0] = top ? 0 : b.x; cu[1] = top ? 0 : b.y; cu[2] = top ? 0 : b.z; cu[3] = top ? 0 : b.w;
-    cd[0] = bottom ? 0 : c.x; cd[1] = bottom ? 0 : c.y; cd[2] = bottom ? 0 : c.z; cd[3] = bottom ? 0 : c.w;
-    cl[0] = x0 == 0 ? 0 : d.x; cl[1] = d.y; cl[2] = d.z; cl[3] = d.w;
-    cr[0] = f.x; cr[1] = f.y; cr[2] = f.z; cr[3] = x0 + 3 == im.W - 1 ? 0 : f.w;
-  }
-  __device__ __forceinline__ void pixel(const ImageDesc& im, const int32_t*, int x, int y, int& e,
-                                        int& cu, int& cd, int& cl, int& cr) const {
-    const long long i = (long long)y * im.W + x;
-    e = excess[i];
-    cu = y > 0 ? up[i] : 0;
-    cd = y < im.H - 1 ? down[i] : 0;
-    cl = x > 0 ? left[i] : 0;
-    cr = x < im.W - 1 ? right[i] : 0;
-  }
-};
-
-__device__ __forceinline__ int rgb_dist2(uint32_t a, uint32_t b) {
-  const int dr = (int)(a & 255u) - (int)(b & 255u);
-  const int dg = (int)((a >> 8) & 255u) - (int)((b >> 8) & 255u);
-  const int db = (int)((a >> 16) & 255u) - (int)((b >> 16) & 255u);
-  return dr * dr + dg * dg + db * db;
-}
-
-// Weight of the reference's n-link rule, rounded to an integer: floor(x + 0.5) for
-// x = lambda / (0.1 sqrt(d) + 0.05) = 20 lambda / (2 sqrt(d) + 1) (graphcut.cl:1018-1031,
-// LAMBDA and EPSILON from GraphCut.pyx:25-26,92-93), exactly.  For k >= 1,
-// floor(x + 0.5) >= k  <=>  b = 40 lambda - 2k + 1 >= 0  and  4 (2k - 1)^2 d <= b^2,
-// so the weight is the largest k satisfying that integer test (monotone in k).  A double
-// estimate of k is settled by the test itself; with lambda <= 1000 and d <= 3 * 255^2 every
-// product fits in 64 bits.
-__device__ __forceinline__ bool ref_weight_at_least(long long k, long long d, long long a40) {
-  if (k < 1) return true;
-  const long long b = a40 - 2 * k + 1, a = 2 * k - 1;
-  return b >= 0 && 4 * a * a * d <= b * b;
-}
-__device__ __forceinline__ int ref_weight(int d, int lambda) {
-  const long long a40 = 40LL * lambda;
-  const double sd = sqrt((double)d);
-  long long k = (long long)floor(((double)a40 + 1.0 + 2.0 * sd) / (4.0 * sd + 2.0));
-  if (k < 0) k = 0;
-  while (k > 0 && !ref_weight_at_least(k, d, a40)) --k;
-  while (ref_weight_at_least(k + 1, d, a40)) ++k;
-  return (int)k;
-}
-
-struct RgbaSource {
-  const uint32_t* rgba;
-  const int32_t* excess;
-  const int32_t* tab;   // exp weighting: the 50 thresholds on the device; null: reference rule
-  int lambda;           // reference weighting
-  static constexpr bool vec = false;
-  __device__ __forceinline__ void pixel4(const ImageDesc&, int, int, int (&)[4], int (&)[4],
-                                         int (&)[4], int (&)[4], int (&)[4]) const {}
-  __device__ __forceinline__ void prepare(int32_t* s_tab) const {
-    if (tab && threadIdx.x < GC_NLINK_LEVELS) s_tab[threadIdx.x] = tab[threadIdx.x];
-  }
-  // exp weighting: the number of table entries >= d (the entries do not increase)
-  __device__ __forceinline__ static int table_weight(const int32_t* s_tab, int d) {
-    int lo = 0, hi = GC_NLINK_LEVELS;
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (s_tab[mid] >= d) lo = mid + 1; else hi = mid;
-    }
-    return lo;
-  }
-  __device__ __forceinline__ int weight(const int32_t* s_tab, int d) const {
-    return tab ? table_weight(s_tab, d) : ref_weight(d, lambda);
-  }
-  __device__ __forceinline__ void pixel(const ImageDesc& im, const int32_t* s_tab, int x, int y,
-                                        int& e, int& cu, int& cd, int& cl, int& cr) const {
-    const long long i = (long long)y * im.W + x;
-    const uint32_t c = rgba[i];
-    e = excess[i];
-    cu = y > 0 ? weight(s_tab, rgb_dist2(c, rgba[i - im.W])) : 0;
-    cd = y < im.H - 1 ? weight(s_tab, rgb_dist2(c, rgba[i + im.W])) : 0;
-    cl = x > 0 ? weight(s_tab, rgb_dist2(c, rgba[i - 1])) : 0;
-    cr = x < im.W - 1 ? weight(s_tab, rgb_dist2(c, rgba[i + 1])) : 0;
-  }
-};
-
-// The exp weighting's table on the device, from the |dI|^2 sum of k_dsum: weight(d) =
-// floor(50 exp(-beta d) + 0.5) with beta = 1 / (2 mean |dI|^2) (0 when the mean is 0) does
-// not increase with d, so it is stored as t[k - 1] = the largest d in [0, 3 * 255^2] with
-// weight >= k.  Thread k - 1 locates t[k - 1] from the real root of 50 exp(-beta d) + 0.5
-// = k and settles it by evaluating the formula itself at the integers around it, in double,
-// so the table reproduces a float64 evaluation of the formula pixel by pixel.
-__global__ void k_nlink_table(const unsigned long long* __restrict__ sum, long long npairs,
-                              int32_t* __restrict__ tab) {
-  const int k = (int)threadIdx.x + 1;
-  if (k > GC_NLINK_LEVELS) return;
-  const long kMax = 3L * 255 * 255;
-  const double mean = (double)(*sum) / (double)(npairs > 1 ? npairs : 1);
-  const double beta = mean > 0 ? 1.0 / (2.0 * mean) : 0.0;
-  if (beta <= 0) { tab[k - 1] = (int32_t)kMax; return; }
-  auto w = [&](long d) { return (int)floor(50.0 * exp(-beta * (double)d) + 0.5); };
-  const double root = log(50.0 / (k - 0.5)) / beta;   // weight(d) >= k  <=>  d <= root
-  long d = root >= (double)kMax ? kMax : (root < 0 ? 0 : (long)floor(root));
-  while (d < kMax && w(d + 1) >= k) ++d;
-  while (d >= 0 && w(d) < k) --d;
-  tab[k - 1] = (int32_t)d;
-}
-
-template <class Source>
-__global__ void __launch_bounds__(DIS_THREADS)
-k_upload(PoolView P, ImageDesc im, int img, Source src, int32_t* __restrict__ tl, ImageAcc* acc) {
-  trace_mark(P, TR_UPLOAD);
-  __shared__ int32_t s_tab[GC_NLINK_LEVELS];
-  src.prepare(s_tab);
-  __syncthreads();
-  const int bt = blockIdx.x;
-  const int tx = bt % im.tw, ty = bt / im.tw;
-  const int t = im.tile0 + bt;
-  const int r = threadIdx.x >> 3, c0 = (threadIdx.x & 7) * 4;
-  const int y = ty * GC_TILE + r;
-  int e[4], h[4], cu[4], cd[4], cl[4], cr[4];
+// The state of one uploaded tile, from the values the block's threads hold (thread (r, q) holds
+// pixels (r, 4q .. 4q+3)): planes, trivial labelling, t-links, row masks, flags, and the
+// image's sums.  Every thread of the block calls it.
+__device__ __forceinline__ void store_uploaded_tile(const PoolView& P, int t, int img, int r, int c0,
+                                                    const int (&e)[4], const int (&cu)[4],
+                                                    const int (&cd)[4], const int (&cl)[4],
+                                                    const int (&cr)[4], int32_t* __restrict__ tl,
+                                                    ImageAcc* acc) {
+  int h[4], bad = 0;
   long long pos = 0;
-  int bad = 0;
-  const int xb = tx * GC_TILE + c0;
-  if (src.vec && y < im.H && xb + 3 < im.W) {
-    src.pixel4(im, xb, y, e, cu, cd, cl, cr);
-  } else {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int x = xb + j;
-      e[j] = cu[j] = cd[j] = cl[j] = cr[j] = 0;
-      if (x < im.W && y < im.H) src.pixel(im, s_tab, x, y, e[j], cu[j], cd[j], cl[j], cr[j]);
-    }
-  }
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     bad |= (cu[j] | cd[j] | cl[j] | cr[j]) < 0;
@@ -352,6 +217,271 @@ k_upload(PoolView P, ImageDesc im, int img, Source src, int32_t* __restrict__ tl
     P.img_of[t] = img;
     P.mdirty[t] = 0;     // the masks above are current
   }
+}
+
+// gc_upload: row-major capacity planes.
+struct PlaneSource {
+  const int32_t *up, *down, *left, *right, *excess;
+  bool vec;   // all planes 16-byte aligned and the width a multiple of 4: int4 row loads
+};
+
+__global__ void __launch_bounds__(DIS_THREADS)
+k_upload(PoolView P, ImageDesc im, int img, PlaneSource src, int32_t* __restrict__ tl, ImageAcc* acc) {
+  trace_mark(P, TR_UPLOAD);
+  const int bt = blockIdx.x;
+  const int tx = bt % im.tw, ty = bt / im.tw;
+  const int r = threadIdx.x >> 3, c0 = (threadIdx.x & 7) * 4;
+  const int y = ty * GC_TILE + r, x0 = tx * GC_TILE + c0;
+  int e[4], cu[4], cd[4], cl[4], cr[4];
+  const bool top = y == 0, bottom = y == im.H - 1;
+  if (src.vec && y < im.H && x0 + 3 < im.W) {
+    const long long i = (long long)y * im.W + x0;
+    const int4 a = *reinterpret_cast<const int4*>(src.excess + i);
+    const int4 b = *reinterpret_cast<const int4*>(src.up + i);
+    const int4 c = *reinterpret_cast<const int4*>(src.down + i);
+    const int4 d = *reinterpret_cast<const int4*>(src.left + i);
+    const int4 f = *reinterpret_cast<const int4*>(src.right + i);
+    e[0] = a.x; e[1] = a.y; e[2] = a.z; e[3] = a.w;
+    cu[0] = top ? 0 : b.x; cu[1] = top ? 0 : b.y; cu[2] = top ? 0 : b.z; cu[3] = top ? 0 : b.w;
+    cd[0] = bottom ? 0 : c.x; cd[1] = bottom ? 0 : c.y; cd[2] = bottom ? 0 : c.z; cd[3] = bottom ? 0 : c.w;
+    cl[0] = x0 == 0 ? 0 : d.x; cl[1] = d.y; cl[2] = d.z; cl[3] = d.w;
+    cr[0] = f.x; cr[1] = f.y; cr[2] = f.z; cr[3] = x0 + 3 == im.W - 1 ? 0 : f.w;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int x = x0 + j;
+      e[j] = cu[j] = cd[j] = cl[j] = cr[j] = 0;
+      if (x < im.W && y < im.H) {
+        const long long i = (long long)y * im.W + x;
+        e[j] = src.excess[i];
+        cu[j] = top ? 0 : src.up[i];
+        cd[j] = bottom ? 0 : src.down[i];
+        cl[j] = x > 0 ? src.left[i] : 0;
+        cr[j] = x < im.W - 1 ? src.right[i] : 0;
+      }
+    }
+  }
+  store_uploaded_tile(P, im.tile0 + bt, img, r, c0, e, cu, cd, cl, cr, tl, acc);
+}
+
+__device__ __forceinline__ int rgb_dist2(uint32_t a, uint32_t b) {
+  const int dr = (int)(a & 255u) - (int)(b & 255u);
+  const int dg = (int)((a >> 8) & 255u) - (int)((b >> 8) & 255u);
+  const int db = (int)((a >> 16) & 255u) - (int)((b >> 16) & 255u);
+  return dr * dr + dg * dg + db * db;
+}
+
+// Weight of the reference's n-link rule, rounded to an integer: floor(x + 0.5) for
+// x = lambda / (0.1 sqrt(d) + 0.05) = 20 lambda / (2 sqrt(d) + 1) (graphcut.cl:1018-1031,
+// LAMBDA and EPSILON from GraphCut.pyx:25-26,92-93), exactly.  For k >= 1,
+// floor(x + 0.5) >= k  <=>  b = 40 lambda - 2k + 1 >= 0  and  4 (2k - 1)^2 d <= b^2,
+// so the weight is the largest k satisfying that integer test (monotone in k).  A float32
+// estimate of k (its error is below 0.01 of a level at lambda <= 1000) is settled by the test
+// itself; with lambda <= 1000 and d <= 3 * 255^2 every product fits in 64 bits.
+__device__ __forceinline__ bool ref_weight_at_least(int k, int d, int a40) {
+  if (k < 1) return true;
+  const int b = a40 - 2 * k + 1, a = 2 * k - 1;
+  return b >= 0 && 4LL * ((long long)a * a) * d <= (long long)b * b;
+}
+__device__ __forceinline__ int ref_weight(int d, int lambda) {
+  const int a40 = 40 * lambda;
+  const float sd = sqrtf((float)d);
+  int k = (int)(((float)a40 + 1.0f + 2.0f * sd) / (4.0f * sd + 2.0f));
+  while (k > 0 && !ref_weight_at_least(k, d, a40)) --k;
+  while (ref_weight_at_least(k + 1, d, a40)) ++k;
+  return k;
+}
+
+// n-link weights from |dI|^2.  Exp weighting: the number of table entries >= d (the entries
+// t[0..50) do not increase).  The formula itself, in float32, gives the level to within one
+// (its error is below 1e-4 of a level), and the entries beside it settle it: two independent
+// shared-memory reads where a binary search chains six.
+struct ExpWeight {
+  float scale;   // -beta * log2(e)
+  __device__ __forceinline__ int operator()(const int32_t* s_tab, int d) const {
+    int k = (int)(50.0f * exp2f(scale * (float)d) + 0.5f);   // 0 .. 50
+    while (k > 0 && s_tab[k - 1] < d) --k;
+    while (k < GC_NLINK_LEVELS && s_tab[k] >= d) ++k;
+    return k;
+  }
+};
+struct RefWeight {
+  int lambda;
+  __device__ __forceinline__ int operator()(const int32_t*, int d) const { return ref_weight(d, lambda); }
+};
+
+// The upload from an RGBA image: the weights of an n-link are the same both ways, so a thread
+// computes those to the right of and below its four pixels and takes the other two directions
+// from its neighbours (a lane of the same warp, shared memory for the row above); the tile's
+// first row and column compute theirs from the pixels across the side.  5 weights a thread
+// (9 in the tile's first warp) where one per pixel and direction takes 16.
+//
+// Bound by the planes it writes: 28 of 36 bytes a pixel.
+struct RgbaSource {
+  const uint32_t* rgba;
+  const int32_t* excess;
+  const int32_t* tab;   // exp weighting: 50 thresholds, then the float scale; null: reference rule
+  int lambda;           // reference weighting
+  bool vec;             // both 16-byte aligned and the width a multiple of 4: int4 row loads
+};
+
+template <class Weight>
+__global__ void __launch_bounds__(DIS_THREADS)
+k_upload_rgba(PoolView P, ImageDesc im, int img, RgbaSource src, Weight weight,
+              int32_t* __restrict__ tl, ImageAcc* acc) {
+  trace_mark(P, TR_UPLOAD);
+  __shared__ int32_t s_tab[GC_NLINK_LEVELS];
+  __shared__ int4 s_down[GC_TILE][8];
+  const int tid = threadIdx.x, q = tid & 7;
+  if constexpr (std::is_same_v<Weight, ExpWeight>) {
+    if (tid < GC_NLINK_LEVELS) s_tab[tid] = src.tab[tid];
+    weight.scale = __int_as_float(src.tab[GC_NLINK_LEVELS]);
+    __syncthreads();
+  }
+  const int bt = blockIdx.x;
+  const int tx = bt % im.tw, ty = bt / im.tw;
+  const int r = tid >> 3, c0 = q * 4;
+  const int y = ty * GC_TILE + r, x0 = tx * GC_TILE + c0;
+  const bool row_in = y < im.H, below_in = y + 1 < im.H;
+  const long long i = (long long)y * im.W + x0;
+  uint32_t px[4] = {0u, 0u, 0u, 0u}, below[4] = {0u, 0u, 0u, 0u};
+  int e[4] = {0, 0, 0, 0};
+  if (src.vec && x0 + 3 < im.W) {
+    if (row_in) {
+      const uint4 a = *reinterpret_cast<const uint4*>(src.rgba + i);
+      const int4 b = *reinterpret_cast<const int4*>(src.excess + i);
+      px[0] = a.x; px[1] = a.y; px[2] = a.z; px[3] = a.w;
+      e[0] = b.x; e[1] = b.y; e[2] = b.z; e[3] = b.w;
+    }
+    if (below_in) {
+      const uint4 a = *reinterpret_cast<const uint4*>(src.rgba + i + im.W);
+      below[0] = a.x; below[1] = a.y; below[2] = a.z; below[3] = a.w;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (x0 + j >= im.W) continue;
+      if (row_in) {
+        px[j] = src.rgba[i + j];
+        e[j] = src.excess[i + j];
+      }
+      if (below_in) below[j] = src.rgba[i + im.W + j];
+    }
+  }
+  // the pixel to the right of the four, and (first column) the one to the left
+  const unsigned F = 0xffffffffu;
+  uint32_t next = __shfl_down_sync(F, px[0], 1);
+  if (q == 7 && row_in && x0 + 4 < im.W) next = src.rgba[i + 4];
+  uint32_t side = 0;   // first column: the pixel to the left
+  const bool has_left = q == 0 && row_in && x0 > 0 && x0 < im.W;
+  if (has_left) side = src.rgba[i - 1];
+  int cu[4], cd[4], cl[4], cr[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t nx = j < 3 ? px[j < 3 ? j + 1 : 3] : next;
+    cr[j] = row_in && x0 + j + 1 < im.W ? weight(s_tab, rgb_dist2(px[j], nx)) : 0;
+    cd[j] = below_in && x0 + j < im.W ? weight(s_tab, rgb_dist2(px[j], below[j])) : 0;
+  }
+  cl[0] = __shfl_up_sync(F, cr[3], 1);
+  if (q == 0) cl[0] = has_left ? weight(s_tab, rgb_dist2(px[0], side)) : 0;
+  cl[1] = cr[0]; cl[2] = cr[1]; cl[3] = cr[2];
+  s_down[r][q] = make_int4(cd[0], cd[1], cd[2], cd[3]);
+  __syncthreads();
+  if (r > 0) {
+    const int4 a = s_down[r - 1][q];
+    cu[0] = a.x; cu[1] = a.y; cu[2] = a.z; cu[3] = a.w;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      cu[j] = y > 0 && row_in && x0 + j < im.W
+                  ? weight(s_tab, rgb_dist2(px[j], src.rgba[i - im.W + j])) : 0;
+  }
+  store_uploaded_tile(P, im.tile0 + bt, img, r, c0, e, cu, cd, cl, cr, tl, acc);
+}
+
+// The mean |dI|^2 over all 4-neighbour pairs and the exp weighting's table, in one launch.
+//
+// Every pixel is read once: a thread walks down DSUM_ROWS rows of one column, with the row
+// above in a register and the pixel to the left from the lane beside it (a warp reads 128
+// bytes of a row at a time; DSUM_ROWS loads in flight).  Sums are exact: 32 bits a thread (at
+// most 2 * 3 * 255^2 * DSUM_ROWS), 64 above.  The last CTA turns the total into the table and
+// clears the total and the ticket for the next call.
+//
+// The table: weight(d) = floor(50 exp(-beta d) + 0.5) with beta = 1 / (2 mean |dI|^2) (0 when
+// the mean is 0) does not increase with d, so it is stored as t[k - 1] = the largest d in
+// [0, 3 * 255^2] with weight >= k.  Thread k - 1 locates t[k - 1] from the real root of
+// 50 exp(-beta d) + 0.5 = k and settles it by evaluating the formula itself at the integers
+// around it, in double, so the table reproduces a float64 evaluation of the formula pixel by
+// pixel.  t[50] holds -beta * log2(e) as a float (ExpWeight's estimate).
+constexpr int DSUM_ROWS = 16;
+constexpr int DSUM_THREADS = 256;
+
+__device__ __forceinline__ void nlink_table(unsigned long long sum, long long npairs, int k,
+                                            int32_t* tab) {
+  const long kMax = 3L * 255 * 255;
+  const double mean = (double)sum / (double)(npairs > 1 ? npairs : 1);
+  const double beta = mean > 0 ? 1.0 / (2.0 * mean) : 0.0;
+  if (k == 1) tab[GC_NLINK_LEVELS] = __float_as_int((float)(-beta * 1.4426950408889634));
+  if (beta <= 0) { tab[k - 1] = (int32_t)kMax; return; }
+  auto w = [&](long d) { return (int)floor(50.0 * exp(-beta * (double)d) + 0.5); };
+  const double root = log(50.0 / (k - 0.5)) / beta;   // weight(d) >= k  <=>  d <= root
+  long d = root >= (double)kMax ? kMax : (root < 0 ? 0 : (long)floor(root));
+  while (d < kMax && w(d + 1) >= k) ++d;
+  while (d >= 0 && w(d) < k) --d;
+  tab[k - 1] = (int32_t)d;
+}
+
+// state: [0] the running sum, [1] the ticket (both zero between calls)
+__global__ void __launch_bounds__(DSUM_THREADS)
+k_nlinks(const uint32_t* __restrict__ rgba, int W, int H, long long npairs,
+         unsigned long long* state, int32_t* __restrict__ tab, ImageAcc* acc) {
+  __shared__ unsigned long long part[DSUM_THREADS / 32];
+  __shared__ unsigned long long s_total;
+  __shared__ int s_last;
+  const int lane = threadIdx.x & 31;
+  const long long x = (long long)blockIdx.x * DSUM_THREADS + threadIdx.x;
+  const int y0 = blockIdx.y * DSUM_ROWS;
+  const bool in = x < W;
+  unsigned sum = 0;
+  uint32_t c[DSUM_ROWS + 1], l[DSUM_ROWS];
+#pragma unroll
+  for (int k = 0; k <= DSUM_ROWS; ++k) {   // c[0]: the row above the strip
+    const int y = y0 + k - 1;
+    c[k] = in && y >= 0 && y < H ? rgba[(long long)y * W + x] : 0u;
+  }
+#pragma unroll
+  for (int k = 0; k < DSUM_ROWS; ++k)      // lane 0: the pixel left of the warp's columns
+    l[k] = lane == 0 && in && x > 0 && y0 + k < H ? rgba[(long long)(y0 + k) * W + x - 1] : 0u;
+#pragma unroll
+  for (int k = 0; k < DSUM_ROWS; ++k) {
+    const uint32_t up = __shfl_up_sync(0xffffffffu, c[k + 1], 1);
+    const uint32_t left = lane == 0 ? l[k] : up;
+    if (!in || y0 + k >= H) continue;
+    if (y0 + k > 0) sum += (unsigned)rgb_dist2(c[k + 1], c[k]);
+    if (x > 0) sum += (unsigned)rgb_dist2(c[k + 1], left);
+  }
+  unsigned long long acc64 = sum;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) acc64 += __shfl_xor_sync(0xffffffffu, acc64, o);
+  if (lane == 0) part[threadIdx.x >> 5] = acc64;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned long long tsum = 0;
+    for (int k = 0; k < DSUM_THREADS / 32; ++k) tsum += part[k];
+    if (tsum) atomicAdd(state, tsum);
+    __threadfence();
+    const unsigned long long n = (unsigned long long)gridDim.x * gridDim.y;
+    s_last = atomicAdd(state + 1, 1ull) == n - 1;
+    if (s_last) {
+      __threadfence();
+      s_total = *((volatile unsigned long long*)state);
+      state[0] = 0;
+      state[1] = 0;
+      *acc = ImageAcc{};   // the image's sums start afresh with the upload that follows
+    }
+  }
+  __syncthreads();
+  if (s_last && threadIdx.x < GC_NLINK_LEVELS) nlink_table(s_total, npairs, threadIdx.x + 1, tab);
 }
 
 // Whether a freshly uploaded tile belongs in the first list of a solve: it holds excess, and a
@@ -2078,11 +2208,13 @@ __global__ void k_brush(PoolView P, ImageDesc im, int img, const int32_t* __rest
 // ------------------------------------------------------------------------------------
 static inline int ok() { return cudaGetLastError() == cudaSuccess ? GC_OK : GC_ERR_CUDA; }
 
+static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 int launch_upload(const PoolView& P, const ImageDesc& im, int img, const int32_t* up,
                   const int32_t* down, const int32_t* left, const int32_t* right,
                   const int32_t* excess, int32_t* tl, ImageAcc* acc, cudaStream_t s) {
-  auto a16 = [](const int32_t* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-  const bool vec = im.W % 4 == 0 && a16(up) && a16(down) && a16(left) && a16(right) && a16(excess);
+  const bool vec = im.W % 4 == 0 && aligned16(up) && aligned16(down) && aligned16(left) &&
+                   aligned16(right) && aligned16(excess);
   const PlaneSource src{up, down, left, right, excess, vec};
   k_upload<<<im.tw * im.th, DIS_THREADS, 0, s>>>(P, im, img, src, tl, acc);
   return ok();
@@ -2091,48 +2223,19 @@ int launch_upload(const PoolView& P, const ImageDesc& im, int img, const int32_t
 int launch_upload_rgba(const PoolView& P, const ImageDesc& im, int img, const uint32_t* rgba,
                        const int32_t* excess, const int32_t* tab, int lambda, int32_t* tl,
                        ImageAcc* acc, cudaStream_t s) {
-  const RgbaSource src{rgba, excess, tab, lambda};
-  k_upload<<<im.tw * im.th, DIS_THREADS, 0, s>>>(P, im, img, src, tl, acc);
+  const RgbaSource src{rgba, excess, tab, lambda, im.W % 4 == 0 && aligned16(rgba) && aligned16(excess)};
+  if (tab)
+    k_upload_rgba<<<im.tw * im.th, DIS_THREADS, 0, s>>>(P, im, img, src, ExpWeight{0.0f}, tl, acc);
+  else
+    k_upload_rgba<<<im.tw * im.th, DIS_THREADS, 0, s>>>(P, im, img, src, RefWeight{lambda}, tl, acc);
   return ok();
 }
 
-int launch_nlink_table(const unsigned long long* sum, long long npairs, int32_t* tab,
-                       cudaStream_t s) {
-  k_nlink_table<<<1, 64, 0, s>>>(sum, npairs, tab);
-  return ok();
-}
-
-// Sum over all 4-neighbour pairs of |I_i - I_j|^2 (R, G, B), exact in 64 bits: the mean the
-// n-link scale beta comes from.
-__global__ void __launch_bounds__(256) k_dsum(const uint32_t* __restrict__ rgba, int W, int H,
-                                              unsigned long long* sum) {
-  __shared__ unsigned long long part[8];
-  unsigned long long acc = 0;
-  const long long n = (long long)W * H;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(i % W);
-    const uint32_t c = rgba[i];
-    if (i >= W) acc += (unsigned)rgb_dist2(c, rgba[i - W]);
-    if (x > 0) acc += (unsigned)rgb_dist2(c, rgba[i - 1]);
-  }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned long long tsum = 0;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) tsum += part[k];
-    if (tsum) atomicAdd(sum, tsum);
-  }
-}
-
-int launch_dsum(const uint32_t* rgba, int W, int H, unsigned long long* sum, int sms,
-                cudaStream_t s) {
-  const long long n = (long long)W * H;
-  long long blocks = (n + 255) / 256;
-  if (blocks > 8LL * sms) blocks = 8LL * sms;
-  k_dsum<<<(unsigned)(blocks > 0 ? blocks : 1), 256, 0, s>>>(rgba, W, H, sum);
+int launch_nlinks(const uint32_t* rgba, int W, int H, unsigned long long* state, int32_t* tab,
+                  ImageAcc* acc, cudaStream_t s) {
+  const long long npairs = (long long)(H - 1) * W + (long long)H * (W - 1);
+  const dim3 grid((W + DSUM_THREADS - 1) / DSUM_THREADS, (H + DSUM_ROWS - 1) / DSUM_ROWS);
+  k_nlinks<<<grid, DSUM_THREADS, 0, s>>>(rgba, W, H, npairs, state, tab, acc);
   return ok();
 }
 
@@ -2305,8 +2408,8 @@ void preload_kernels() {
   if (done[dev]) return;
   cudaFuncAttributes a;
   const void* kernels[] = {
-      (const void*)k_upload<PlaneSource>, (const void*)k_upload<RgbaSource>, (const void*)k_dsum,
-      (const void*)k_nlink_table,
+      (const void*)k_upload, (const void*)k_upload_rgba<ExpWeight>,
+      (const void*)k_upload_rgba<RefWeight>, (const void*)k_nlinks,
       (const void*)k_masks, (const void*)k_discharge, (const void*)k_edge_relabel_build,
       (const void*)k_bfs_round, (const void*)k_flood_round, (const void*)k_ctl_begin,
       (const void*)k_active_list, (const void*)k_ctl_cycle, (const void*)k_flood_check,

@@ -34,10 +34,12 @@ def test_far_excess_matches_oracle(cuda, oracle, w, h, graph):
         lab = gc.cut_labels().cpu().numpy()
         assert gc.flow == f_ref
         assert np.array_equal(lab, l_ref)
-        # a warm solve: the excess moves to the other end of the first row
+        # a warm solve: the excess moves to the other end of the first row (of the column, on
+        # the grid one pixel wide: the edited pixels have to be distinct)
+        far = w - 1 if w > 1 else h - 1
         t = g.excess.copy()
-        t[0, 0], t[0, w - 1] = -30, 25
-        gc.edit_tlinks(np.array([0, w - 1]), np.array([-30, 25]))
+        t.flat[0], t.flat[far] = -30, 25
+        gc.edit_tlinks(np.array([0, far]), np.array([-30, 25]))
         f_ref, l_ref = oracle.maxflow_bk(g.up, g.down, g.left, g.right, t)
         lab = gc.cut_labels().cpu().numpy()
         assert gc.flow == f_ref
