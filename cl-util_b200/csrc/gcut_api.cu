@@ -695,13 +695,15 @@ struct Pool {
     for (int cycle = 0; n > 0 || (cycle == 0 && fresh); ++cycle) {
       if (cycle >= opts.max_cycles) return fail(GC_ERR_NOT_CONVERGED, "cycle cap reached before the cut was final");
       stats.cycles++;
-      for (int p = 0; p < opts.pulses_per_relabel; ++p) {
+      const int pulses = cycle_pulses(opts.pulses_per_relabel, cycle);
+      const int iters = cycle_iters(opts.discharge_iters, cycle);
+      for (int p = 0; p < pulses; ++p) {
         if (collect) {
           RK(read_ctl(s));
           CK(cudaMemcpy(h_count, P.qcount, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost));
           stats.tiles_discharged += h_count[h_ctl[CTL_PULSE] & 1];
         }
-        RK(timed(K_DISCHARGE, s, [&] { return launch_discharge(P, opts.discharge_iters, hlim, grid_dis, s); }));
+        RK(timed(K_DISCHARGE, s, [&] { return launch_discharge(P, iters, hlim, grid_dis, s); }));
         stats.pulses++;
       }
       ++stamp;
@@ -786,7 +788,7 @@ struct Pool {
       // the solve's steps: the prologue (with the fresh images' first list), the pulses and
       // every BFS / flood round
       stats.cycles = h_ctl[CTL_CYCLES];
-      stats.pulses = stats.cycles * opts.pulses_per_relabel;
+      stats.pulses = h_ctl[CTL_PULSE];
       stats.launches = (h_ctl[CTL_NACT] ? 0 : 1) + h_ctl[CTL_NACT] + stats.pulses +
                        stats.bfs_rounds + stats.flood_rounds;
     }

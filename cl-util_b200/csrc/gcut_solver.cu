@@ -1852,7 +1852,7 @@ __device__ __forceinline__ bool grid_sync(const PoolView& P, unsigned long long&
 // pixels there stay inactive.  Exact distances would be the chain of tile rounds across every
 // region that has excess and one unsaturated edge left (up to 34 rounds of 14-25 us at
 // 4096^2), with all its tiles discharged.  The labels stay valid: below the cap they are
-// exact, and at or above it "not below".  The cap grows with every cycle, and at once when no
+// exact, and at or above it "not below".  The cap doubles with every cycle, and at once when no
 // excess lies within it, so the schedule ends in exact relabels and terminates as they do.
 constexpr int SOLVE_WARPS = DIS_THREADS / 32;
 constexpr size_t SOLVE_BFS_SMEM = (size_t)SOLVE_WARPS * 32 * 33 * sizeof(int32_t);
@@ -1869,7 +1869,7 @@ k_solve(PoolView P, SolveArgs A) {
   unsigned phase = 0;     // of mbar
   int qk = 0, fk = 0;     // steps of the worklist and of the frontier (counter slots mod 3)
   int stamp = 0, cycles = 0, err = 0;
-  int nrounds_f = 0, nrounds_b = 0;
+  int nrounds_f = 0, nrounds_b = 0, npulses = 0;
   int cap = A.cap, hlim = GC_HINF;   // of the last relabel (none yet: trivial labels)
   int v0, v1;
   // ---- prologue: control words, image modes and flow sums
@@ -1900,15 +1900,17 @@ k_solve(PoolView P, SolveArgs A) {
     // fresh images' first list
     if (cyc > 0) {
       // ---- pulses: step qk reads counter qk, adds to qk + 1, clears qk + 2 (all mod 3)
-      for (int p = 0; p < A.pulses && alive; ++p) {
+      const int pulses = cycle_pulses(A.pulses, cycles), iters = cycle_iters(A.iters, cycles);
+      for (int p = 0; p < pulses && alive && v0 > 0; ++p) {
         trace_mark(P, TR_DISCHARGE);
         const Worklist in{P.queue[qk & 1], nullptr, P.inq[qk & 1]};
         Worklist out{P.queue[(qk + 1) & 1], &P.ctl[CTL_Q0 + (qk + 1) % 3], P.inq[(qk + 1) & 1]};
-        if (p == A.pulses - 1) out.list = nullptr;   // the relabel makes the next list
+        if (p == pulses - 1) out.list = nullptr;   // the relabel makes the next list
         if (bid == 0 && tid == 0) P.ctl[CTL_Q0 + (qk + 2) % 3] = 0;
-        discharge_phase(P, A.iters, hlim, bid, nb, in, v0, out, dsm,
+        discharge_phase(P, iters, hlim, bid, nb, in, v0, out, dsm,
                         *reinterpret_cast<DisSmem*>(dsm + DIS_PLANES * GC_TILE_PX), &mbar, phase);
         ++qk;
+        ++npulses;
         alive = grid_sync(P, target, s_bc, &P.ctl[CTL_Q0 + qk % 3], &P.ctl[CTL_ERR], v0, v1);
       }
       if (!alive) break;
@@ -2053,6 +2055,7 @@ k_solve(PoolView P, SolveArgs A) {
       ctl[CTL_FLOOD_TOTAL] = nrounds_f;
       ctl[CTL_CYCLES] = cycles;
       ctl[CTL_NACT] = A.fresh ? 1 : 0;
+      ctl[CTL_PULSE] = npulses;
       trace_record(P, TR_END);
     }
     __syncthreads();

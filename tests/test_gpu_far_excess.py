@@ -1,5 +1,5 @@
 """Solves whose excess lies far from every sink: the first list of a fresh solve is empty (no
-sink in or beside a tile with excess) and the relabel's distance cap (16, then 4 times as far
+sink in or beside a tile with excess) and the relabel's distance cap (16, then twice as far
 whenever no excess lies within it, and each cycle) has to grow, past its last finite value on
 the longest grid.  Flow and canonical cut equal the exact oracle's, for the one-launch solve
 and the host-driven loop, fresh and after an edit that moves the excess."""
