@@ -78,9 +78,10 @@ enum TileFlag { TF_POS = 1, TF_SINK = 2, TF_POS_UP = 4, TF_POS_DOWN = 8, TF_POS_
                 TF_POS_RIGHT = 32, TF_SINK_UP = 64, TF_SINK_DOWN = 128, TF_SINK_LEFT = 256,
                 TF_SINK_RIGHT = 512, TF_BAD = 1024 };
 
-// Grid barrier words: arrivals of the running k_solve (bit 63: abort) and CTAs that left it,
-// in separate 128-byte lines.  The last CTA to leave clears both for the next launch.
-enum BarSlot { BAR_ARRIVE = 0, BAR_EXIT = 16, BAR_N = 32 };
+// Grid barrier words, in separate 128-byte lines: two arrival words of the running k_solve
+// (low half: arrivals, bits 32-62: a sum over the CTAs, bit 63: abort) and the CTAs that left
+// it.  The last CTA to leave clears all for the next launch.
+enum BarSlot { BAR_ARRIVE = 0, BAR_STRIDE = 16, BAR_EXIT = 32, BAR_N = 48 };
 constexpr unsigned long long GC_BAR_ABORT = 1ull << 63;
 
 // Device-side loop control words.  In the host-driven loops the last CTA of every frontier
@@ -140,12 +141,18 @@ struct SelCursor {
   __device__ __forceinline__ int image() const { return cur.w; }
 };
 
+// A running k_solve ends at its next barrier.
+__device__ __forceinline__ void abort_solve(const PoolView& P) {
+  atomicOr(P.bar + BAR_ARRIVE, GC_BAR_ABORT);
+  atomicOr(P.bar + BAR_ARRIVE + BAR_STRIDE, GC_BAR_ABORT);
+}
+
 // A self-check found a worklist value outside the pool: keep the first one, flag the solve
 // (it stops at its next check or barrier and the host returns GC_ERR_INTERNAL).
 __device__ __forceinline__ void record_bad(const PoolView& P, int where, int value) {
   if (atomicCAS(&P.ctl[CTL_BADWHERE], 0, where) == 0) P.ctl[CTL_BAD] = value;
   atomicCAS(&P.ctl[CTL_ERR], 0, 4);
-  atomicOr(P.bar + BAR_ARRIVE, GC_BAR_ABORT);   // a running k_solve ends at its next barrier
+  abort_solve(P);
 }
 
 __device__ __forceinline__ unsigned long long global_ns() {

@@ -550,32 +550,23 @@ k_masks(PoolView P) {
 // nothing in k_solve, since the relabel rebuilds the list.
 // ------------------------------------------------------------------------------------
 struct DisSmem {
-  int32_t hs[GC_TILE_PX];   // heights
-  int32_t fu[GC_TILE_PX];   // flow pushed up by each pixel this round
-  int32_t fd[GC_TILE_PX];   // flow pushed down
-  int32_t fl[GC_TILE * 8];  // flow pushed left by the first pixel of each 4-pixel strip
-  int32_t fr[GC_TILE * 8];  // flow pushed right by the last pixel of each strip
-  int32_t hu[GC_TILE], hd[GC_TILE], hl[GC_TILE], hr[GC_TILE];  // halo heights
-  // launch-start values of the tile-edge pixels that also receive atomics from the
-  // neighbouring tiles (written back as deltas against these)
+  int32_t hs[GC_TILE_PX + 2 * GC_TILE];   // heights, with a halo row above and below
+  int32_t fu[GC_TILE_PX + GC_TILE];       // flow pushed up by each pixel this sweep, and a zero row
+  int32_t fd[GC_TILE_PX + GC_TILE];       // a zero row, and flow pushed down
   int32_t eo_top[GC_TILE], eo_bot[GC_TILE], eo_left[GC_TILE], eo_right[GC_TILE];
-  int32_t cu_top[GC_TILE], cd_bot[GC_TILE], cl_left[GC_TILE], cr_right[GC_TILE];
-  // flow leaving the tile, per edge pixel, delivered at the end of the tile
-  int32_t xu[GC_TILE], xd[GC_TILE], xl[GC_TILE], xr[GC_TILE];
 };
 
 // A worklist of tiles: list, length, and the per-tile flag that keeps a tile in it once.
-struct Worklist { int32_t *list, *count, *in; };
+// local: a shared-memory counter of the tiles this CTA appends (k_solve; null elsewhere).
+struct Worklist {
+  int32_t *list, *count, *in;
+  int* local = nullptr;
+};
 
 __device__ __forceinline__ void worklist_append(const PoolView& P, const Worklist& w, int t) {
   const int pos = atomicAdd(w.count, 1);
   if (pos < P.nt) w.list[pos] = t;   // each tile at most once, so pos < nt always holds
   else record_bad(P, 1, pos);
-}
-
-__device__ __forceinline__ void worklist_add(const PoolView& P, const Worklist& w, int t) {
-  if (*((volatile int32_t*)&w.in[t]) != 0) return;   // common case: already queued
-  if (atomicExch(&w.in[t], 1) == 0) worklist_append(P, w, t);
 }
 
 __device__ __forceinline__ int4 lds4(const int32_t* p) { return *reinterpret_cast<const int4*>(p); }
@@ -642,42 +633,71 @@ __device__ __forceinline__ void dis_prefetch(const PoolView& P, int t, int32_t* 
     bulk_g2s(buf + k * GC_TILE_PX, dis_plane(P, k) + (long long)t * GC_TILE_PX, GC_TILE_PX * 4, mbar);
 }
 
-// hlim: pixels with a smaller height are active (GC_HINF: all that can reach a sink; smaller
-// after a relabel capped at distance hlim - 1, whose heights from hlim on only mean "at least
-// hlim").  A pixel that rises to hlim stays there, inactive until the next relabel.
-//
 // Discharges the n tiles of list `in` with the CTAs 0 .. nb-1 (this is CTA `bid`); the tiles
-// active afterwards or sent flow go to list `out` (none: out.list null).  buf, S and mbar are
-// the CTA's staging buffer, exchange arrays and (initialised) mbarrier; `phase` its parity,
-// kept from call to call.  Every thread of the CTA calls it.
+// active afterwards or sent flow go to list `out` (none: out.list null).  hlim: pixels with a
+// smaller height are active (GC_HINF: all that can reach a sink; smaller after a relabel capped
+// at distance hlim - 1, whose heights from hlim on only mean "at least hlim").  A pixel that
+// rises to hlim stays there, inactive until the next relabel.  buf, S and mbar are the CTA's
+// staging buffer, exchange arrays and (initialised) mbarrier; `phase` its parity, kept from
+// call to call.  Every thread of the CTA calls it.
+//
+// What bounds it: with a few hundred tiles in a list each CTA has one, and the pulse is one
+// tile's latency; with more, instruction issue.  So the sweep has no divergent branch (a
+// pixel's four pushes and its relabel are selects and minima), the horizontal neighbours come
+// by shuffle, only vertical exchange goes through shared memory, and a tile's bookkeeping is
+// one pass at the end.  Cycles of one tile alone on its SM, against branches per direction and
+// exchange through shared memory only: about 1200 a sweep (1000 to 2650), 1700 for the
+// write-back (3000).  3 CTAs per SM (80 registers) beat 4 (64, with spills) by 5 to 10 %.
 __device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, int hlim, int bid,
-                                                int nb_ctas,
-                                                const Worklist& in, int n, const Worklist& out,
-                                                int32_t* buf, DisSmem& S, uint64_t* mbar,
-                                                unsigned& phase) {
-  __shared__ int s_sent;
-  const int tid = threadIdx.x;
+                                                int nb_ctas, const Worklist& in, int n,
+                                                const Worklist& out, int32_t* buf, DisSmem& S,
+                                                uint64_t* mbar, unsigned& phase) {
+  const unsigned F = 0xffffffffu;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int r = tid >> 3, q = tid & 7, c0 = q * 4;
-  // Bookkeeping log: each finished tile leaves (tile, neighbours, flags) here, and the CTA's
-  // threads settle up to DIS_LOG tiles at once (its list entry, and the list entries and
-  // dirty flags of the neighbours it sent flow to), so the dependent L2 round trips of that
-  // bookkeeping are paid once per flush, not once per tile.  Nothing in this launch reads
-  // what it writes: the next list, the dirty flags and act_int are read by later kernels.
-  __shared__ int s_logt[DIS_LOG], s_logf[DIS_LOG];
+  // Bookkeeping log: each tile leaves (tile, neighbours, flags) here, and the CTA's threads
+  // settle up to DIS_LOG tiles at once (its list entry, and the list entries and dirty flags
+  // of the neighbours it sent flow to), so the dependent L2 round trips of that bookkeeping
+  // are paid once per flush, not once per tile.  Nothing in this pulse reads what it writes:
+  // the next list, the dirty flags and act_int are read by later steps.  A flush comes before
+  // the write-back of its last tile: the warps it occupies wait for the list's atomics while
+  // the others store.
+  __shared__ int s_logt[DIS_LOG];
+  __shared__ unsigned s_logf[DIS_LOG];
   __shared__ int4 s_lognb[DIS_LOG];
   int nlog = 0;   // the same in every thread
   auto flush_log = [&](int cnt) {
-    for (int w = tid; w < cnt * 5; w += DIS_THREADS) {
-      const int i = w / 5, k = w - i * 5;       // k = 0: the tile; 1..4: up, down, left, right
-      const int tt = s_logt[i], f = s_logf[i];
-      const int4 nbb = s_lognb[i];
-      const int target = k == 0 ? tt : k == 1 ? nbb.x : k == 2 ? nbb.y : k == 3 ? nbb.z : nbb.w;
-      if (k == 0 || ((f >> (k - 1)) & 1)) {
-        P.touched[target] = 1;
-        mark_dirty(P, target);   // its masks are rebuilt by the next flood's first round
-        if (k == 0) P.act_int[tt] = (f >> 5) & 1;
-        if (out.list && (k != 0 || ((f >> 4) & 1))) worklist_add(P, out, target);
-        if (k == 0 && P.ktiles) atomicAdd(&P.ktiles[K_DISCHARGE], 1ull);
+    for (int b = 0; b < cnt * 5; b += DIS_THREADS) {
+      const int w = b + tid;
+      bool won = false;
+      int target = 0;
+      if (w < cnt * 5) {
+        const int i = w / 5, k = w - i * 5;       // k = 0: the tile; 1..4: up, down, left, right
+        const int tt = s_logt[i];
+        const unsigned f = s_logf[i];
+        const int4 nbb = s_lognb[i];
+        target = k == 0 ? tt : k == 1 ? nbb.x : k == 2 ? nbb.y : k == 3 ? nbb.z : nbb.w;
+        if (k == 0 || ((f >> (k - 1)) & 1)) {
+          P.touched[target] = 1;
+          mark_dirty(P, target);   // its masks are rebuilt by the next flood's first round
+          if (k == 0) P.act_int[tt] = (f >> 5) & 1;
+          if (out.list && (k != 0 || ((f >> 4) & 1))) won = atomicExch(&out.in[target], 1) == 0;
+          if (k == 0 && P.ktiles) atomicAdd(&P.ktiles[K_DISCHARGE], 1ull);
+        }
+      }
+      // one add of the list's length per warp
+      const unsigned m = __ballot_sync(F, won);
+      if (m) {
+        int pos = 0;
+        if (lane == 0) {
+          pos = atomicAdd(out.count, __popc(m));
+          if (out.local) atomicAdd(out.local, __popc(m));
+        }
+        pos = __shfl_sync(F, pos, 0) + __popc(m & ((1u << lane) - 1u));
+        if (won) {
+          if (pos < P.nt) out.list[pos] = target;   // `in` deduplicates, so pos < nt always holds
+          else record_bad(P, 1, pos);
+        }
       }
     }
   };
@@ -686,281 +706,238 @@ __device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, in
     n = 0;
   }
   // list entry li: every position below the checked count was written with a tile id of
-  // the pool (by worklist_add or the compaction) before this launch
+  // the pool (by a pulse, a relabel or a compaction) before this pulse
   auto entry = [&](int li) { return in.list[li]; };
-  const bool erow = (r == 0) || (r == 31);
+  const bool erow = r == 0 || r == 31, ecol = q == 0 || q == 7;
   const int pix = r * GC_TILE + c0;
+  const bool left = q == 0;
+  int32_t* const hs = S.hs + GC_TILE + pix;        // this thread's heights (rows -1 and 32: halo)
+  if (tid < GC_TILE) {   // no flow enters from beyond the first and last row
+    S.fu[GC_TILE_PX + tid] = 0;
+    S.fd[tid] = 0;
+  }
   bool failed = false;
-  if (tid == 0 && bid < n) dis_prefetch(P, entry(bid), buf, mbar);
+  int t = 0;
+  int4 nb = make_int4(-1, -1, -1, -1);
+  if (bid < n) {
+    t = entry(bid);
+    if (tid == 0) dis_prefetch(P, t, buf, mbar);
+    nb = P.nbr[t];
+  }
   for (int li = bid; li < n; li += nb_ctas) {
-    const int t = entry(li);
-    const int4 nb = P.nbr[t];
-    if (tid < 32) S.hu[tid] = nb.x >= 0 ? P.hgt[(long long)nb.x * GC_TILE_PX + 31 * GC_TILE + tid] : GC_HINF;
-    else if (tid < 64) S.hd[tid - 32] = nb.y >= 0 ? P.hgt[(long long)nb.y * GC_TILE_PX + (tid - 32)] : GC_HINF;
-    else if (tid < 96) S.hl[tid - 64] = nb.z >= 0 ? P.hgt[(long long)nb.z * GC_TILE_PX + (tid - 64) * GC_TILE + 31] : GC_HINF;
-    else if (tid < 128) S.hr[tid - 96] = nb.w >= 0 ? P.hgt[(long long)nb.w * GC_TILE_PX + (tid - 96) * GC_TILE] : GC_HINF;
-    else if (tid < 160) S.xu[tid - 128] = 0;
-    else if (tid < 192) S.xd[tid - 160] = 0;
-    else if (tid < 224) S.xl[tid - 192] = 0;
-    else S.xr[tid - 224] = 0;
-    if (tid == 0) { in.in[t] = 0; s_sent = 0; }
+    // halo heights, loaded while the tile's copy lands
+    int4 hv = make_int4(GC_HINF, GC_HINF, GC_HINF, GC_HINF);   // first / last row: across the side
+    int hside = GC_HINF;                                       // first / last strip: across the side
+    const int nv = r == 0 ? nb.x : nb.y, nh_ = left ? nb.z : nb.w;
+    if (erow && nv >= 0)
+      hv = *reinterpret_cast<const int4*>(P.hgt + (long long)nv * GC_TILE_PX + (r == 0 ? 31 * GC_TILE : 0) + c0);
+    if (ecol && nh_ >= 0) hside = P.hgt[(long long)nh_ * GC_TILE_PX + r * GC_TILE + (left ? 31 : 0)];
+    if (tid == 0) {
+      in.in[t] = 0;
+      s_logt[nlog] = t;
+      s_lognb[nlog] = nb;
+      s_logf[nlog] = 0;
+    }
     const bool ok = mbar_wait(mbar, phase);
     if (__syncthreads_or(!ok)) { failed = true; break; }  // block-uniform
     phase ^= 1u;
-    int e[4], h[4], cu[4], cd[4], cl[4], cr[4];
+    int e[4], h[4], cu[4], cd[4], cl[4], cr[4], hcap[4];
     {
       int4 v = lds4(buf + 0 * GC_TILE_PX + pix); e[0] = v.x; e[1] = v.y; e[2] = v.z; e[3] = v.w;
+      // launch-start excess of the pixels that also receive atomics from neighbouring tiles
+      // (written back as deltas against it)
+      if (erow) sts4((r == 0 ? S.eo_top : S.eo_bot) + c0, v.x, v.y, v.z, v.w);
+      if (ecol) (left ? S.eo_left : S.eo_right)[r] = left ? v.x : v.w;
       v = lds4(buf + 1 * GC_TILE_PX + pix); h[0] = v.x; h[1] = v.y; h[2] = v.z; h[3] = v.w;
+      sts4(hs, v.x, v.y, v.z, v.w);
       v = lds4(buf + 2 * GC_TILE_PX + pix); cu[0] = v.x; cu[1] = v.y; cu[2] = v.z; cu[3] = v.w;
       v = lds4(buf + 3 * GC_TILE_PX + pix); cd[0] = v.x; cd[1] = v.y; cd[2] = v.z; cd[3] = v.w;
       v = lds4(buf + 4 * GC_TILE_PX + pix); cl[0] = v.x; cl[1] = v.y; cl[2] = v.z; cl[3] = v.w;
       v = lds4(buf + 5 * GC_TILE_PX + pix); cr[0] = v.x; cr[1] = v.y; cr[2] = v.z; cr[3] = v.w;
     }
-    // keep the launch-start values the write-back needs (tile-edge pixels only)
-    if (r == 0) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) { S.eo_top[c0 + j] = e[j]; S.cu_top[c0 + j] = cu[j]; }
-    }
-    if (r == 31) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) { S.eo_bot[c0 + j] = e[j]; S.cd_bot[c0 + j] = cd[j]; }
-    }
-    if (q == 0) { S.eo_left[r] = e[0]; S.cl_left[r] = cl[0]; }
-    if (q == 7) { S.eo_right[r] = e[3]; S.cr_right[r] = cr[3]; }
-    // height cap of tile-edge pixels for this launch (interior: none)
-    int hcap[4];
+    if (r == 0) sts4(hs - GC_TILE, hv.x, hv.y, hv.z, hv.w);
+    if (r == 31) sts4(hs + GC_TILE, hv.x, hv.y, hv.z, hv.w);
+    // heights a pixel may reach in this pulse: tile-edge pixels 2 above their start
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int c = c0 + j;
-      const bool edge = erow || c == 0 || c == 31;
+      const bool edge = erow || (j == 0 && q == 0) || (j == 3 && q == 7);
       hcap[j] = edge ? imin(h[j] + 2, hlim) : hlim;
     }
-    sts4(S.hs + pix, h[0], h[1], h[2], h[3]);
+    int xv[4] = {0, 0, 0, 0}, xh = 0;   // flow out of the tile: across the row / column side
     __syncthreads();   // every thread has its values in registers: the buffer is free
     // prefetch this CTA's next tile into the buffer while this one is worked on
-    if (tid == 0 && li + nb_ctas < n) dis_prefetch(P, entry(li + nb_ctas), buf, mbar);
+    int tn = 0;
+    int4 nbn = make_int4(-1, -1, -1, -1);
+    if (li + nb_ctas < n) {
+      tn = entry(li + nb_ctas);
+      if (tid == 0) dis_prefetch(P, tn, buf, mbar);
+      nbn = P.nbr[tn];
+    }
 
     for (int it = 0; it < iters; ++it) {
-      // neighbour heights (fixed during the push phase)
-      int hnu[4], hnd[4], hnl[4], hnr[4];
-      if (r > 0) { const int4 v = lds4(S.hs + pix - GC_TILE); hnu[0] = v.x; hnu[1] = v.y; hnu[2] = v.z; hnu[3] = v.w; }
-      else { const int4 v = lds4(S.hu + c0); hnu[0] = v.x; hnu[1] = v.y; hnu[2] = v.z; hnu[3] = v.w; }
-      if (r < 31) { const int4 v = lds4(S.hs + pix + GC_TILE); hnd[0] = v.x; hnd[1] = v.y; hnd[2] = v.z; hnd[3] = v.w; }
-      else { const int4 v = lds4(S.hd + c0); hnd[0] = v.x; hnd[1] = v.y; hnd[2] = v.z; hnd[3] = v.w; }
-      hnl[0] = c0 > 0 ? S.hs[pix - 1] : S.hl[r];
-      hnl[1] = h[0]; hnl[2] = h[1]; hnl[3] = h[2];
-      hnr[0] = h[1]; hnr[1] = h[2]; hnr[2] = h[3];
-      hnr[3] = c0 < 28 ? S.hs[pix + 4] : S.hr[r];
-
-      // push phase.  `rem` marks pixels that still hold excess after pushing: every
-      // admissible edge of theirs is then saturated, and inflow only adds residual towards
-      // higher neighbours, so they relabel without another admissibility test.
-      int ou[4], od[4], ol[4], orr[4];
+      // neighbour heights (fixed during the sweep)
+      const int4 hup = lds4(hs - GC_TILE), hdn = lds4(hs + GC_TILE);
+      const int hnu[4] = {hup.x, hup.y, hup.z, hup.w}, hnd[4] = {hdn.x, hdn.y, hdn.z, hdn.w};
+      int hl = __shfl_up_sync(F, h[3], 1), hr = __shfl_down_sync(F, h[0], 1);
+      if (q == 0) hl = hside;
+      if (q == 7) hr = hside;
+      const int hnl[4] = {hl, h[0], h[1], h[2]}, hnr[4] = {h[1], h[2], h[3], hr};
+      // push along every admissible edge: down, up, right, left
+      int ou[4] = {0, 0, 0, 0}, od[4] = {0, 0, 0, 0}, ol[4] = {0, 0, 0, 0}, orr[4] = {0, 0, 0, 0};
       int changed = 0;
-      unsigned rem = 0;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) ou[j] = od[j] = ol[j] = orr[j] = 0;
-      const bool any_act = (e[0] > 0 && h[0] < hlim) || (e[1] > 0 && h[1] < hlim) ||
-                           (e[2] > 0 && h[2] < hlim) || (e[3] > 0 && h[3] < hlim);
-      if (__any_sync(0xffffffffu, any_act)) {
+      if (__any_sync(F, (e[0] > 0 && h[0] < hlim) || (e[1] > 0 && h[1] < hlim) ||
+                            (e[2] > 0 && h[2] < hlim) || (e[3] > 0 && h[3] < hlim))) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          int ej = e[j];
-          if (ej > 0 && h[j] < hlim) {
-            const int hm1 = h[j] - 1;
-            if (cd[j] > 0 && hnd[j] == hm1) { const int f = imin(ej, cd[j]); ej -= f; cd[j] -= f; od[j] = f; }
-            if (ej > 0 && cu[j] > 0 && hnu[j] == hm1) { const int f = imin(ej, cu[j]); ej -= f; cu[j] -= f; ou[j] = f; }
-            if (ej > 0 && cr[j] > 0 && hnr[j] == hm1) { const int f = imin(ej, cr[j]); ej -= f; cr[j] -= f; orr[j] = f; }
-            if (ej > 0 && cl[j] > 0 && hnl[j] == hm1) { const int f = imin(ej, cl[j]); ej -= f; cl[j] -= f; ol[j] = f; }
-            changed |= ej != e[j];
-            rem |= (ej > 0 ? 1u : 0u) << j;
-            e[j] = ej;
-          }
+          // the height to push to (none for an inactive pixel: no height is negative)
+          const int hm1 = e[j] > 0 && h[j] < hlim ? h[j] - 1 : -1;
+          od[j] = hnd[j] == hm1 ? imin(e[j], cd[j]) : 0;
+          e[j] -= od[j]; cd[j] -= od[j];
+          ou[j] = hnu[j] == hm1 ? imin(e[j], cu[j]) : 0;
+          e[j] -= ou[j]; cu[j] -= ou[j];
+          orr[j] = hnr[j] == hm1 ? imin(e[j], cr[j]) : 0;
+          e[j] -= orr[j]; cr[j] -= orr[j];
+          ol[j] = hnl[j] == hm1 ? imin(e[j], cl[j]) : 0;
+          e[j] -= ol[j]; cl[j] -= ol[j];
+          changed |= od[j] | ou[j] | orr[j] | ol[j];
         }
       }
       // flow leaving the tile is delivered at the end of the tile
-      if (r == 0) {
+      if (warp == 0) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) { S.xu[c0 + j] += ou[j]; ou[j] = 0; }
+        for (int j = 0; j < 4; ++j) xv[j] += r == 0 ? ou[j] : 0;
       }
-      if (r == 31) {
+      if (warp == DIS_THREADS / 32 - 1) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) { S.xd[c0 + j] += od[j]; od[j] = 0; }
+        for (int j = 0; j < 4; ++j) xv[j] += r == 31 ? od[j] : 0;
       }
-      if (q == 0) { S.xl[r] += ol[0]; ol[0] = 0; }
-      if (q == 7) { S.xr[r] += orr[3]; orr[3] = 0; }
+      xh += q == 0 ? ol[0] : q == 7 ? orr[3] : 0;
       sts4(S.fu + pix, ou[0], ou[1], ou[2], ou[3]);
-      sts4(S.fd + pix, od[0], od[1], od[2], od[3]);
-      S.fl[r * 8 + q] = ol[0];
-      S.fr[r * 8 + q] = orr[3];
+      sts4(S.fd + GC_TILE + pix, od[0], od[1], od[2], od[3]);
+      int fl = __shfl_up_sync(F, orr[3], 1), fr = __shfl_down_sync(F, ol[0], 1);
+      if (q == 0) fl = 0;
+      if (q == 7) fr = 0;
       __syncthreads();
       // gather inflow; a pixel receiving flow gains the reverse residual
       {
-        const int4 a = r < 31 ? lds4(S.fu + pix + GC_TILE) : make_int4(0, 0, 0, 0);
-        const int4 bb = r > 0 ? lds4(S.fd + pix - GC_TILE) : make_int4(0, 0, 0, 0);
-        const int fb[4] = {a.x, a.y, a.z, a.w}, fa[4] = {bb.x, bb.y, bb.z, bb.w};
-        int fromleft[4], fromright[4];
-        fromleft[0] = q > 0 ? S.fr[r * 8 + q - 1] : 0;
-        fromleft[1] = orr[0]; fromleft[2] = orr[1]; fromleft[3] = orr[2];
-        fromright[0] = ol[1]; fromright[1] = ol[2]; fromright[2] = ol[3];
-        fromright[3] = q < 7 ? S.fl[r * 8 + q + 1] : 0;
+        const int4 a = lds4(S.fu + pix + GC_TILE), b = lds4(S.fd + pix);
+        const int below[4] = {a.x, a.y, a.z, a.w}, above[4] = {b.x, b.y, b.z, b.w};
+        const int fromleft[4] = {fl, orr[0], orr[1], orr[2]};
+        const int fromright[4] = {ol[1], ol[2], ol[3], fr};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          e[j] += fb[j] + fa[j] + fromleft[j] + fromright[j];
-          cd[j] += fb[j];
-          cu[j] += fa[j];
+          e[j] += below[j] + above[j] + fromleft[j] + fromright[j];
+          cd[j] += below[j];
+          cu[j] += above[j];
           cl[j] += fromleft[j];
           cr[j] += fromright[j];
         }
       }
-      // relabel phase (Jacobi; tile-edge pixels are capped at hcap)
-      int nh[4] = {h[0], h[1], h[2], h[3]};
-      const bool any_need = (e[0] > 0 && h[0] < hcap[0]) || (e[1] > 0 && h[1] < hcap[1]) ||
-                            (e[2] > 0 && h[2] < hcap[2]) || (e[3] > 0 && h[3] < hcap[3]);
-      if (__any_sync(0xffffffffu, any_need)) {
+      // relabel (Jacobi) to one above the lowest residual neighbour m.  The labelling is valid,
+      // so h <= m + 1, with equality exactly when an admissible edge is left: the pixel then
+      // keeps its height.  So does one at its limit, and an inactive one (h >= hlim >= hcap).
+      if (__any_sync(F, e[0] > 0 || e[1] > 0 || e[2] > 0 || e[3] > 0)) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          if (e[j] > 0 && h[j] < hcap[j]) {
-            const int hm1 = h[j] - 1;
-            const bool adm = !((rem >> j) & 1u) &&
-                             ((cd[j] > 0 && hnd[j] == hm1) || (cu[j] > 0 && hnu[j] == hm1) ||
-                              (cr[j] > 0 && hnr[j] == hm1) || (cl[j] > 0 && hnl[j] == hm1));
-            if (!adm) {
-              int m = GC_HINF;
-              if (cd[j] > 0) m = imin(m, hnd[j] + 1);
-              if (cu[j] > 0) m = imin(m, hnu[j] + 1);
-              if (cr[j] > 0) m = imin(m, hnr[j] + 1);
-              if (cl[j] > 0) m = imin(m, hnl[j] + 1);
-              nh[j] = imin(m, hcap[j]);
-              changed |= nh[j] != h[j];
-            }
-          }
+          int m = GC_HINF;
+          m = cd[j] > 0 ? imin(m, hnd[j]) : m;
+          m = cu[j] > 0 ? imin(m, hnu[j]) : m;
+          m = cr[j] > 0 ? imin(m, hnr[j]) : m;
+          m = cl[j] > 0 ? imin(m, hnl[j]) : m;
+          const int up = imin(m + 1, hcap[j]);
+          const int to = e[j] > 0 && up > h[j] ? up : h[j];
+          changed |= to ^ h[j];
+          ou[j] = to;
         }
-      }
-      // every read of S.hs in this iteration happened before the flow barrier above, so the
-      // new heights can be written now; the next reads follow the barrier below
+      } else {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) h[j] = nh[j];
-      sts4(S.hs + pix, h[0], h[1], h[2], h[3]);
+        for (int j = 0; j < 4; ++j) ou[j] = h[j];
+      }
+      // every read of S.hs in this sweep happened before the flow barrier above, so the new
+      // heights can be written now; the next reads follow the barrier below
+#pragma unroll
+      for (int j = 0; j < 4; ++j) h[j] = ou[j];
+      sts4(hs, h[0], h[1], h[2], h[3]);
       if (!__syncthreads_or(changed)) break;
     }
 
-    // write back: interior values are owned by this CTA; tile-edge excess and the
-    // outward residual of edge pixels also receive atomics from neighbouring tiles, so
-    // they are written as deltas against their launch-start values.
-    const long long off = (long long)t * GC_TILE_PX + pix;
-    if (!erow && q > 0 && q < 7) {
-      *(int4*)(P.exc + off) = make_int4(e[0], e[1], e[2], e[3]);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int c = c0 + j;
-        if (erow || c == 0 || c == 31) {
-          const int e0 = r == 0 ? S.eo_top[c] : r == 31 ? S.eo_bot[c] : c == 0 ? S.eo_left[r] : S.eo_right[r];
-          if (e[j] != e0) atomicAdd(P.exc + off + j, e[j] - e0);
-        } else {
-          P.exc[off + j] = e[j];
-        }
-      }
-    }
-    *(int4*)(P.hgt + off) = make_int4(h[0], h[1], h[2], h[3]);
-    if (r == 0) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int o0 = S.cu_top[c0 + j];
-        if (cu[j] != o0) atomicAdd(P.cap[DUP] + off + j, cu[j] - o0);
-      }
-    } else {
-      *(int4*)(P.cap[DUP] + off) = make_int4(cu[0], cu[1], cu[2], cu[3]);
-    }
-    if (r == 31) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int o0 = S.cd_bot[c0 + j];
-        if (cd[j] != o0) atomicAdd(P.cap[DDOWN] + off + j, cd[j] - o0);
-      }
-    } else {
-      *(int4*)(P.cap[DDOWN] + off) = make_int4(cd[0], cd[1], cd[2], cd[3]);
-    }
-    if (q == 0) {
-      const int cl0 = S.cl_left[r];
-      if (cl[0] != cl0) atomicAdd(P.cap[DLEFT] + off, cl[0] - cl0);
-      P.cap[DLEFT][off + 1] = cl[1]; P.cap[DLEFT][off + 2] = cl[2]; P.cap[DLEFT][off + 3] = cl[3];
-    } else {
-      *(int4*)(P.cap[DLEFT] + off) = make_int4(cl[0], cl[1], cl[2], cl[3]);
-    }
-    if (q == 7) {
-      const int cr0 = S.cr_right[r];
-      if (cr[3] != cr0) atomicAdd(P.cap[DRIGHT] + off + 3, cr[3] - cr0);
-      P.cap[DRIGHT][off] = cr[0]; P.cap[DRIGHT][off + 1] = cr[1]; P.cap[DRIGHT][off + 2] = cr[2];
-    } else {
-      *(int4*)(P.cap[DRIGHT] + off) = make_int4(cr[0], cr[1], cr[2], cr[3]);
-    }
-    // deliver cross-tile flow: excess of the neighbour pixel and its reverse residual
-    int sent_u = 0, sent_d = 0, sent_l = 0, sent_r = 0;
-    if (r == 0 && nb.x >= 0) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int x = S.xu[c0 + j];
-        if (x) {
-          const long long o = (long long)nb.x * GC_TILE_PX + 31 * GC_TILE + c0 + j;
-          atomicAdd(P.exc + o, x); atomicAdd(P.cap[DDOWN] + o, x); sent_u = 1;
-        }
-      }
-    }
-    if (r == 31 && nb.y >= 0) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int x = S.xd[c0 + j];
-        if (x) {
-          const long long o = (long long)nb.y * GC_TILE_PX + c0 + j;
-          atomicAdd(P.exc + o, x); atomicAdd(P.cap[DUP] + o, x); sent_d = 1;
-        }
-      }
-    }
-    if (q == 0 && nb.z >= 0) {
-      const int x = S.xl[r];
-      if (x) {
-        const long long o = (long long)nb.z * GC_TILE_PX + r * GC_TILE + 31;
-        atomicAdd(P.exc + o, x); atomicAdd(P.cap[DRIGHT] + o, x); sent_l = 1;
-      }
-    }
-    if (q == 7 && nb.w >= 0) {
-      const int x = S.xr[r];
-      if (x) {
-        const long long o = (long long)nb.w * GC_TILE_PX + r * GC_TILE;
-        atomicAdd(P.exc + o, x); atomicAdd(P.cap[DLEFT] + o, x); sent_r = 1;
-      }
-    }
-    int act = 0, act_int = 0;
+    // bits 0-3: sent up, down, left, right; 4: active; 5: interior active
+    unsigned flags = 0;
+    if (xv[0] | xv[1] | xv[2] | xv[3]) flags |= r == 0 ? 1u : 2u;
+    if (xh) flags |= left ? 4u : 8u;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int c = c0 + j;
-      const int a = e[j] > 0 && h[j] < hlim;
-      act |= a;
-      act_int |= a && !erow && c > 0 && c < 31;
+      const bool edge = erow || (j == 0 && q == 0) || (j == 3 && q == 7);
+      if (e[j] > 0 && h[j] < hlim) flags |= edge ? 16u : 48u;
     }
-    const int sent = (sent_u ? 1 : 0) | (sent_d ? 2 : 0) | (sent_l ? 4 : 0) | (sent_r ? 8 : 0);
-    if (sent) atomicOr(&s_sent, sent);
-    // the block-wide reductions also order every read of this buffer before its reuse
-    const int any_act = __syncthreads_or(act);
-    act_int = __syncthreads_or(act_int);
-    // log the tile's bookkeeping; a full log is settled now (the barrier makes the entries
-    // visible; the next write of an entry follows several more barriers)
-    if (tid == 0) {
-      s_logt[nlog] = t;
-      s_lognb[nlog] = nb;
-      s_logf[nlog] = (s_sent & 15) | (any_act ? 16 : 0) | (act_int ? 32 : 0);
+    flags = __reduce_or_sync(F, flags);
+    if (lane == 0 && flags) atomicOr(&s_logf[nlog], flags);
+    __syncthreads();   // the log entry is complete; orders the exchange arrays' reuse, too
+    // (an entry is rewritten after a flush behind at least one more barrier, but for entry 0,
+    // which only lanes of thread 0's warp read)
+    if (++nlog == DIS_LOG || li + nb_ctas >= n) {
+      flush_log(nlog);
+      nlog = 0;
+      __syncwarp();
     }
-    if (++nlog == DIS_LOG) { __syncthreads(); flush_log(nlog); nlog = 0; }
+
+    // write back: interior values are owned by this CTA; tile-edge excess and the outward
+    // residual of edge pixels also receive atomics from neighbouring tiles, so they are
+    // written as deltas.  Flow across a side goes to the neighbour pixel's excess and its
+    // reverse residual.
+    const long long off = (long long)t * GC_TILE_PX + pix;
+    *(int4*)(P.hgt + off) = make_int4(h[0], h[1], h[2], h[3]);
+    if (r != 0) *(int4*)(P.cap[DUP] + off) = make_int4(cu[0], cu[1], cu[2], cu[3]);
+    if (r != 31) *(int4*)(P.cap[DDOWN] + off) = make_int4(cd[0], cd[1], cd[2], cd[3]);
+    if (q != 0) *(int4*)(P.cap[DLEFT] + off) = make_int4(cl[0], cl[1], cl[2], cl[3]);
+    if (q != 7) *(int4*)(P.cap[DRIGHT] + off) = make_int4(cr[0], cr[1], cr[2], cr[3]);
+    if (!erow && !ecol) *(int4*)(P.exc + off) = make_int4(e[0], e[1], e[2], e[3]);
+    if (erow) {
+      const int4 v = lds4((r == 0 ? S.eo_top : S.eo_bot) + c0);
+      const int e0[4] = {v.x, v.y, v.z, v.w};
+      int32_t* const own = (r == 0 ? P.cap[DUP] : P.cap[DDOWN]) + off;
+      const long long o = (long long)nv * GC_TILE_PX + (r == 0 ? 31 * GC_TILE : 0) + c0;
+      int32_t* const rev = (r == 0 ? P.cap[DDOWN] : P.cap[DUP]) + o;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (e[j] != e0[j]) atomicAdd(P.exc + off + j, e[j] - e0[j]);
+        if (xv[j]) {   // only where the neighbour exists: capacities out of the image are 0
+          atomicAdd(own + j, -xv[j]);
+          atomicAdd(P.exc + o + j, xv[j]);
+          atomicAdd(rev + j, xv[j]);
+        }
+      }
+    }
+    if (ecol) {
+      int32_t* const own = (left ? P.cap[DLEFT] : P.cap[DRIGHT]) + off;   // the strip's plane
+      const int s0 = left ? 1 : 0;   // its three pixels that are not on the side
+      own[s0] = left ? cl[1] : cr[0];
+      own[s0 + 1] = left ? cl[2] : cr[1];
+      own[s0 + 2] = left ? cl[3] : cr[2];
+      const int js = left ? 0 : 3;
+      if (!erow) {
+        P.exc[off + s0] = left ? e[1] : e[0];
+        P.exc[off + s0 + 1] = left ? e[2] : e[1];
+        P.exc[off + s0 + 2] = left ? e[3] : e[2];
+        const int d = left ? e[0] - S.eo_left[r] : e[3] - S.eo_right[r];
+        if (d) atomicAdd(P.exc + off + js, d);
+      }
+      if (xh) {
+        const long long o = (long long)nh_ * GC_TILE_PX + r * GC_TILE + (left ? 31 : 0);
+        atomicAdd(own + js, -xh);
+        atomicAdd(P.exc + o, xh);
+        atomicAdd((left ? P.cap[DRIGHT] : P.cap[DLEFT]) + o, xh);
+      }
+    }
+    t = tn;
+    nb = nbn;
   }
-  __syncthreads();
-  flush_log(nlog);
   if (failed) {
+    flush_log(nlog);   // the tiles done before
     // a bulk copy did not complete in time: record it, let our copy drain, stop
     if (tid == 0) {
       atomicExch(&P.ctl[CTL_ERR], 3);
-      atomicOr(P.bar + BAR_ARRIVE, GC_BAR_ABORT);
+      abort_solve(P);
       mbar_wait(mbar, phase, 5 * GC_COPY_WAIT_NS);
     }
     __syncthreads();
@@ -968,7 +945,7 @@ __device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, in
 }
 
 // One pulse of the host-driven loop or of a manual push: the worklist of the pulse parity.
-__global__ void __launch_bounds__(DIS_THREADS, 4)
+__global__ void __launch_bounds__(DIS_THREADS, 3)
 k_discharge(PoolView P, int iters, int hlim) {
   trace_mark(P, TR_DISCHARGE);
   extern __shared__ __align__(128) int32_t dsm[];
@@ -1223,6 +1200,7 @@ __device__ __forceinline__ void frontier_push(const PoolView& P, const Worklist&
     const int pos = atomicAdd(out.count, 1);
     if (pos < P.nt) out.list[pos] = t;   // the mark deduplicates, so pos < nt always holds
     else record_bad(P, 5, pos);
+    if (out.local) atomicAdd(out.local, 1);
   }
 }
 
@@ -1795,46 +1773,65 @@ __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long lon
   return v;
 }
 
-// Grid barrier: every CTA's writes before it are visible to every CTA after it, the bulk
-// copies (async proxy) that follow it included.  Then thread 0 reads the words *w0 and *w1 for
-// the whole CTA: counters that no CTA writes before the barrier after this one.  Returns false
-// (the same in every thread) when the solve was aborted.  `s` : 4 words of shared memory.
-__device__ __forceinline__ bool grid_sync(const PoolView& P, unsigned long long& target,
-                                          volatile int32_t* s, const int32_t* w0,
-                                          const int32_t* w1, int& v0, int& v1) {
-  asm volatile("fence.proxy.async;" ::: "memory");   // this thread's writes, before later copies
+// Grid barrier with a sum: every CTA's writes before it are visible to every CTA after it
+// (to its bulk copies too, with Copies set), and `total` is the grid's sum of the CTAs' counts
+// *s_push, which start at 0 again.  The count travels in the upper half of the arrival word, so
+// the loop decision needs no second trip to L2 (0.35 us).  Barriers alternate between two
+// words: no CTA reaches a word's next use before all have left this one, so what they read of
+// it is the same.  `extra` (may be null): a counter no CTA writes before the next barrier, read
+// for the whole CTA into v1 when total is 0 or `always`.  Returns false (in every thread) when
+// the solve was aborted.
+struct GridBar {
+  unsigned k = 0;            // barriers passed
+  unsigned last[2] = {0, 0}; // totals of the words' last uses
+};
+template <bool Copies>
+__device__ __forceinline__ bool grid_sync(const PoolView& P, GridBar& B, volatile int32_t* s,
+                                          int* s_push, int& total, const int32_t* extra = nullptr,
+                                          int* v1 = nullptr, bool always = false) {
+  if (Copies) asm volatile("fence.proxy.async;" ::: "memory");   // this thread's writes, before later copies
   __syncthreads();
-  target += gridDim.x;
+  unsigned long long* const word = P.bar + BAR_ARRIVE + (B.k & 1) * BAR_STRIDE;
+  const unsigned target = gridDim.x * ((B.k >> 1) + 1);
   if (threadIdx.x == 0) {
+    // CTA 0 takes the word's previous total out again: the upper half is never negative
+    const unsigned mine = (unsigned)*s_push;
+    *s_push = 0;
+    unsigned long long add = ((unsigned long long)mine << 32) + 1ull;
+    if (blockIdx.x == 0) add -= (unsigned long long)((B.k & 1) ? B.last[1] : B.last[0]) << 32;
     __threadfence();
-    atomicAdd(P.bar + BAR_ARRIVE, 1ull);
+    atomicAdd(word, add);
     bool ok = false;
-    unsigned long long t0 = 0;
+    unsigned long long t0 = 0, v = 0;
     for (unsigned i = 1; i < (1u << 31); ++i) {
-      const unsigned long long v = ld_acquire(P.bar + BAR_ARRIVE);
+      v = ld_acquire(word);
       if (v & GC_BAR_ABORT) break;
-      if (v >= target) { ok = true; break; }
+      if ((unsigned)v >= target) { ok = true; break; }
       if ((i & 1023u) == 0) {
         const unsigned long long now = global_ns();
         if (t0 == 0) t0 = now;
         else if (now - t0 > GC_BARRIER_WAIT_NS) {
           atomicCAS(&P.ctl[CTL_ERR], 0, 5);
           __threadfence();
-          atomicOr(P.bar + BAR_ARRIVE, GC_BAR_ABORT);
+          abort_solve(P);
           break;
         }
       }
     }
     __threadfence();
-    asm volatile("fence.proxy.async;" ::: "memory");
+    if (Copies) asm volatile("fence.proxy.async;" ::: "memory");
+    const int n = (int)((v >> 32) & 0x7fffffffu);
     s[0] = ok;
-    s[1] = ok ? *((const volatile int32_t*)w0) : 0;
-    s[2] = ok ? *((const volatile int32_t*)w1) : 0;
+    s[1] = n;
+    s[2] = ok && extra && (always || n == 0) ? *((const volatile int32_t*)extra) : 0;
   }
   __syncthreads();
-  v0 = s[1];
-  v1 = s[2];
-  return s[0] != 0;
+  total = s[1];
+  if (v1) *v1 = s[2];
+  if (B.k & 1) B.last[1] = (unsigned)total; else B.last[0] = (unsigned)total;
+  ++B.k;
+  // the arrivals' half must not overflow into the sum (after 2^32 arrivals: hours)
+  return s[0] != 0 && target < 0xffff0000u;
 }
 
 // The solve over the selection (see Pool::solve_images): images that continue from a previous
@@ -1858,23 +1855,25 @@ constexpr int SOLVE_WARPS = DIS_THREADS / 32;
 constexpr size_t SOLVE_BFS_SMEM = (size_t)SOLVE_WARPS * 32 * 33 * sizeof(int32_t);
 constexpr size_t SOLVE_DYN_SMEM = DIS_DYN_SMEM > SOLVE_BFS_SMEM ? DIS_DYN_SMEM : SOLVE_BFS_SMEM;
 
-__global__ void __launch_bounds__(DIS_THREADS, 4)
+__global__ void __launch_bounds__(DIS_THREADS, 3)
 k_solve(PoolView P, SolveArgs A) {
   extern __shared__ __align__(128) int32_t dsm[];
   __shared__ uint64_t mbar;
   __shared__ int32_t s_bc[4];
+  __shared__ int s_push;   // tiles this CTA has queued since the last barrier
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int bid = blockIdx.x, nb = gridDim.x;
-  unsigned long long target = 0;
+  GridBar bar;
   unsigned phase = 0;     // of mbar
   int qk = 0, fk = 0;     // steps of the worklist and of the frontier (counter slots mod 3)
   int stamp = 0, cycles = 0, err = 0;
   int nrounds_f = 0, nrounds_b = 0, npulses = 0;
   int cap = A.cap, hlim = GC_HINF;   // of the last relabel (none yet: trivial labels)
-  int v0, v1;
+  int v0, v1 = 0;
   // ---- prologue: control words, image modes and flow sums
   trace_mark(P, TR_BEGIN);
   if (tid == 0) {
+    s_push = 0;
     mbar_init(&mbar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -1893,7 +1892,7 @@ k_solve(PoolView P, SolveArgs A) {
       A.acc[img].sumpos_e = 0;   // the floods of this solve accumulate it
     }
   }
-  bool alive = grid_sync(P, target, s_bc, &P.ctl[CTL_ERR], &P.ctl[CTL_ERR], v0, v1);
+  bool alive = grid_sync<true>(P, bar, s_bc, &s_push, v0);
 
   for (int cyc = 0; alive; ++cyc) {
     // cyc 0 is the part before the first pulses: the warm images' flood and relabel, and the
@@ -1904,14 +1903,14 @@ k_solve(PoolView P, SolveArgs A) {
       for (int p = 0; p < pulses && alive && v0 > 0; ++p) {
         trace_mark(P, TR_DISCHARGE);
         const Worklist in{P.queue[qk & 1], nullptr, P.inq[qk & 1]};
-        Worklist out{P.queue[(qk + 1) & 1], &P.ctl[CTL_Q0 + (qk + 1) % 3], P.inq[(qk + 1) & 1]};
+        Worklist out{P.queue[(qk + 1) & 1], &P.ctl[CTL_Q0 + (qk + 1) % 3], P.inq[(qk + 1) & 1], &s_push};
         if (p == pulses - 1) out.list = nullptr;   // the relabel makes the next list
         if (bid == 0 && tid == 0) P.ctl[CTL_Q0 + (qk + 2) % 3] = 0;
         discharge_phase(P, iters, hlim, bid, nb, in, v0, out, dsm,
                         *reinterpret_cast<DisSmem*>(dsm + DIS_PLANES * GC_TILE_PX), &mbar, phase);
         ++qk;
         ++npulses;
-        alive = grid_sync(P, target, s_bc, &P.ctl[CTL_Q0 + qk % 3], &P.ctl[CTL_ERR], v0, v1);
+        alive = grid_sync<true>(P, bar, s_bc, &s_push, v0);
       }
       if (!alive) break;
     }
@@ -1925,7 +1924,7 @@ k_solve(PoolView P, SolveArgs A) {
       FloodSum fs;
       for (bool first = true;; first = false) {
         trace_mark(P, first ? TR_FLOOD_FIRST : TR_FLOOD);
-        const Worklist out{P.fq[(fk + 1) & 1], &P.ctl[CTL_F0 + (fk + 1) % 3], P.mark[(fk + 1) & 1]};
+        const Worklist out{P.fq[(fk + 1) & 1], &P.ctl[CTL_F0 + (fk + 1) % 3], P.mark[(fk + 1) & 1], &s_push};
         if (bid == 0 && tid == 0) P.ctl[CTL_F0 + (fk + 2) % 3] = 0;
         const int i0 = warp * nb + bid;
         SelCursor cursor(P, first ? nr : 0, i0 < n ? i0 : 0);
@@ -1954,7 +1953,7 @@ k_solve(PoolView P, SolveArgs A) {
         }
         ++fk;
         ++rounds;
-        alive = grid_sync(P, target, s_bc, &P.ctl[CTL_F0 + fk % 3], hits, v0, v1);
+        alive = grid_sync<false>(P, bar, s_bc, &s_push, v0, hits, &v1);
         n = v0;
         if (!alive || n == 0) break;
         if (n < 0 || n > P.nt) { alive = false; break; }   // (never: frontier_push counts a tile once)
@@ -1976,7 +1975,7 @@ k_solve(PoolView P, SolveArgs A) {
         rounds = 0;
         for (bool first = true;;) {
           trace_mark(P, first ? TR_BFS_FIRST : TR_BFS);
-          const Worklist out{P.fq[(fk + 1) & 1], &P.ctl[CTL_F0 + (fk + 1) % 3], P.mark[(fk + 1) & 1]};
+          const Worklist out{P.fq[(fk + 1) & 1], &P.ctl[CTL_F0 + (fk + 1) % 3], P.mark[(fk + 1) & 1], &s_push};
           if (bid == 0 && tid == 0) P.ctl[CTL_F0 + (fk + 2) % 3] = 0;
           const int i0 = warp * nb + bid;
           SelCursor cursor(P, first ? nr : 0, i0 < n ? i0 : 0);
@@ -1993,7 +1992,7 @@ k_solve(PoolView P, SolveArgs A) {
           }
           ++fk;
           ++rounds;
-          alive = grid_sync(P, target, s_bc, &P.ctl[CTL_F0 + fk % 3], &P.ctl[CTL_Q0 + qk % 3], v0, v1);
+          alive = grid_sync<true>(P, bar, s_bc, &s_push, v0, &P.ctl[CTL_Q0 + qk % 3], &v1);
           n = v0;
           first = false;
           if (!alive) break;
@@ -2038,7 +2037,7 @@ k_solve(PoolView P, SolveArgs A) {
           else record_bad(P, 1, pos);
         }
       }
-      alive = grid_sync(P, target, s_bc, &P.ctl[CTL_Q0 + qk % 3], &P.ctl[CTL_Q0 + qk % 3], v0, v1);
+      alive = grid_sync<true>(P, bar, s_bc, &s_push, v0, &P.ctl[CTL_Q0 + qk % 3], &v1, true);
     }
     v0 = v1;   // the worklist's length
     // (an empty first list still needs the flood: no fresh tile is near a sink)
@@ -2071,6 +2070,7 @@ k_solve(PoolView P, SolveArgs A) {
   if (tid == 0 && atomicAdd(P.bar + BAR_EXIT, 1ull) == (unsigned long long)nb - 1) {
     P.bar[BAR_EXIT] = 0;
     P.bar[BAR_ARRIVE] = 0;
+    P.bar[BAR_ARRIVE + BAR_STRIDE] = 0;
   }
 }
 
