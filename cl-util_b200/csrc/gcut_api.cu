@@ -267,7 +267,7 @@ struct Pool {
     c.take(&P.msink, (size_t)nt * 32);
     c.take(&P.mexc, (size_t)nt * 32);
     c.take(&P.mreach, (size_t)nt * 32);
-    int32_t** small[] = {&P.touched, &P.act_int, &P.mark[0], &P.mark[1], &P.tact, &P.tflag, &P.img_of,
+    int32_t** small[] = {&P.touched, &P.act_int, &P.mark[0], &P.mark[1], &P.tact, &P.hstate, &P.tflag, &P.img_of,
                          &P.queue[0], &P.queue[1], &P.inq[0], &P.inq[1], &P.mdirty};
     for (auto** p : small) c.take(p, nt);
     c.take(&P.qcount, 2);

@@ -46,6 +46,7 @@ struct PoolView {
   int32_t* fq[2];         // [nt] frontier lists of the BFS / flood rounds (dedup by mark[k])
   int32_t* fcount;        // [2] frontier list lengths
   int32_t* tact;          // [nt] tile has an active pixel (excess > 0, height < HINF)
+  int32_t* hstate;        // [nt] the tile's heights are 1: all 0, 2: all GC_HINF, 0: not known
   int32_t* tflag;         // [nt] where the uploaded tile has excess and sinks (TileFlag)
   int32_t* img_of;        // [nt] image index of the tile
   int32_t* mdirty;        // [nt] the tile's planes changed after its masks were written

@@ -207,6 +207,7 @@ __device__ __forceinline__ void store_uploaded_tile(const PoolView& P, int t, in
     if (tp) atomicAdd(&acc[img].sumpos_t, (unsigned long long)tp);
     if (tf & TF_BAD) atomicAdd(&acc[img].bad_caps, 1);
     P.tflag[t] = (int32_t)tf;
+    P.hstate[t] = 0;
     P.tact[t] = (tf & TF_POS) != 0;
     P.touched[t] = 0;
     P.act_int[t] = 0;
@@ -680,7 +681,10 @@ __device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, in
         if (k == 0 || ((f >> (k - 1)) & 1)) {
           P.touched[target] = 1;
           mark_dirty(P, target);   // its masks are rebuilt by the next flood's first round
-          if (k == 0) P.act_int[tt] = (f >> 5) & 1;
+          if (k == 0) {
+            P.act_int[tt] = (f >> 5) & 1;
+            P.hstate[tt] = 0;
+          }
           if (out.list && (k != 0 || ((f >> 4) & 1))) won = atomicExch(&out.in[target], 1) == 0;
           if (k == 0 && P.ktiles) atomicAdd(&P.ktiles[K_DISCHARGE], 1ull);
         }
@@ -1066,6 +1070,7 @@ k_edge_relabel_build(PoolView P, int32_t* list, int32_t* count, ScanState st) {
     if (lane == 0) {
       flag[warp * PER_WARP + k] = active;
       P.touched[t] = 0;
+      P.hstate[t] = 0;   // its heights may have changed
       if (P.ktiles) atomicAdd(&P.ktiles[K_EDGE_BUILD], 1ull);
     }
   }
@@ -1390,12 +1395,98 @@ __global__ void k_ctl_cycle(PoolView P) {
   __threadfence();
 }
 
+// ---- relabel within a small cap: distances as bit planes ----------------------------
+// With cap <= BFS_NEAR_CAP every distance fits in BFS_PLANES bits.  Lane r keeps bit b of the
+// distances of row r in plane[b], so a level costs a few logic operations instead of a store
+// per pixel, and the rows are turned into int4 stores once at the end.
+constexpr int BFS_PLANES = 7;
+constexpr int BFS_NEAR_CAP = (1 << BFS_PLANES) - 1;
+
+struct NearBfs {
+  uint32_t vis;                  // reached pixels of row `lane`
+  uint32_t plane[BFS_PLANES];    // their distances (0 where not reached)
+  // distances of row `lane`'s pixel at column c (0 or 31)
+  __device__ __forceinline__ int side(int c) const {
+    int d = 0;
+#pragma unroll
+    for (int b = 0; b < BFS_PLANES; ++b) d |= (int)((plane[b] >> c) & 1u) << b;
+    return (vis >> c) & 1u ? d : GC_HINF;
+  }
+  // distance of column `lane`'s pixel in row `row` (uniform)
+  __device__ __forceinline__ int across(int row, int lane) const {
+    int d = 0;
+#pragma unroll
+    for (int b = 0; b < BFS_PLANES; ++b)
+      d |= (int)((__shfl_sync(0xffffffffu, plane[b], row) >> lane) & 1u) << b;
+    return (__shfl_sync(0xffffffffu, vis, row) >> lane) & 1u ? d : GC_HINF;
+  }
+};
+
+// tile_bfs_seeded for cap <= BFS_NEAR_CAP.
+__device__ __forceinline__ NearBfs tile_bfs_near(uint32_t sink, uint32_t canU, uint32_t canD,
+                                                 uint32_t canL, uint32_t canR, int lane,
+                                                 bool seeded, int top, int bot, int sl, int sr,
+                                                 int cap) {
+  const unsigned FULL = 0xffffffffu;
+  NearBfs B;
+  B.vis = 0;
+#pragma unroll
+  for (int b = 0; b < BFS_PLANES; ++b) B.plane[b] = 0;
+  uint32_t Fr = 0;
+  if (lane == 0) canU = 0;     // the row above / below lies in another tile (seeds stand for it)
+  if (lane == 31) canD = 0;
+  int L = 0;
+  if (!__any_sync(FULL, sink != 0)) L = seeded ? warp_min(imin(imin(top, bot), imin(sl, sr))) : GC_HINF;
+  // a level visits a pixel or jumps to a later seed, and L rises with each
+  while (L <= cap) {
+    uint32_t N = ((Fr >> 1) & canR) | ((Fr << 1) & canL) | (__shfl_up_sync(FULL, Fr, 1) & canU) |
+                 (__shfl_down_sync(FULL, Fr, 1) & canD);
+    if (L == 0) N |= sink;
+    if (seeded) {
+      const uint32_t bt = __ballot_sync(FULL, top == L), bb = __ballot_sync(FULL, bot == L);
+      N |= (sl == L ? 1u : 0u) | (sr == L ? 0x80000000u : 0u);
+      if (lane == 0) N |= bt;
+      if (lane == 31) N |= bb;
+    }
+    N &= ~B.vis;
+    B.vis |= N;
+#pragma unroll
+    for (int b = 0; b < BFS_PLANES; ++b) B.plane[b] |= (L >> b) & 1 ? N : 0u;
+    Fr = N;
+    if (__any_sync(FULL, N != 0)) {
+      ++L;
+      continue;
+    }
+    if (!seeded) break;
+    // the frontier is empty: the next level that still has an unvisited seed
+    const uint32_t v0 = __shfl_sync(FULL, B.vis, 0), v31 = __shfl_sync(FULL, B.vis, 31);
+    int cand = GC_HINF;
+    if (top > L && !((v0 >> lane) & 1u)) cand = imin(cand, top);
+    if (bot > L && !((v31 >> lane) & 1u)) cand = imin(cand, bot);
+    if (sl > L && !(B.vis & 1u)) cand = imin(cand, sl);
+    if (sr > L && !(B.vis >> 31)) cand = imin(cand, sr);
+    L = warp_min(cand);
+  }
+  return B;
+}
+
+// The four low bits of x in the low bits of four bytes.
+__device__ __forceinline__ uint32_t spread4(uint32_t x) { return ((x & 15u) * 0x00204081u) & 0x01010101u; }
+
 // One tile of a global relabel, by one warp: the in-tile BFS seeded by the tile's sink pixels
-// and (frontier rounds) the halo distances, the heights written back, and the neighbours whose
-// edge distances dropped queued.  T: the warp's 32 x 33 words of shared memory.  Returns
-// whether the tile holds an active pixel.
+// and (frontier rounds) the halo distances, the heights written back, and the neighbours queued
+// that a changed edge distance could lower.  T: the warp's 32 x 33 words of shared memory (used
+// beyond BFS_NEAR_CAP only).  Returns whether the tile holds an active pixel (-1: nothing
+// changed since the tile's last round).
+//
+// Bound by latency and by the 4 KiB of heights a tile stores.  So: a tile whose heights are all
+// 0 or all unreached, and were so before, stores nothing (hstate; most tiles of a large image);
+// a frontier tile none of whose seeds is below its edge's distance stops after 8 loads; and a
+// neighbour is queued only if one of its edge pixels has a residual edge into a changed pixel
+// and is no sink itself (in the first round nearly every tile used to queue all four).
 __device__ __forceinline__ int bfs_tile(const PoolView& P, int t, int lane, int first, int cap,
                                         int32_t* T, const Worklist& out) {
+  const unsigned FULL = 0xffffffffu;
   const int4 nb = P.nbr[t];
   const long long base = (long long)t * GC_TILE_PX;
   // the masks are current: the flood that precedes every global relabel of a solve (or
@@ -1403,44 +1494,84 @@ __device__ __forceinline__ int bfs_tile(const PoolView& P, int t, int lane, int 
   const uint32_t* mc = P.mcan + (long long)t * 128;
   const uint32_t canU = mc[lane], canD = mc[32 + lane], canL = mc[64 + lane], canR = mc[96 + lane];
   const uint32_t sink = P.msink[(long long)t * 32 + lane];
+  const uint32_t pos = P.mexc[(long long)t * 32 + lane];
+  // edge pixels of the neighbours that a distance of this tile could lower (a word over the
+  // columns for up and down; a flag of this lane's row for left and right)
+  uint32_t wantU = 0, wantD = 0, wantL = 0, wantR = 0;
+  if (nb.x >= 0) wantU = P.mcan[(long long)nb.x * 128 + 32 + 31] & ~P.msink[(long long)nb.x * 32 + 31];
+  if (nb.y >= 0) wantD = P.mcan[(long long)nb.y * 128] & ~P.msink[(long long)nb.y * 32];
+  if (nb.z >= 0) wantL = (P.mcan[(long long)nb.z * 128 + 96 + lane] & ~P.msink[(long long)nb.z * 32 + lane]) >> 31;
+  if (nb.w >= 0) wantR = P.mcan[(long long)nb.w * 128 + 64 + lane] & ~P.msink[(long long)nb.w * 32 + lane] & 1u;
   // seeds from the neighbour tiles' heights (frontier rounds only): an edge pixel with a
   // residual edge into the neighbour starts at the neighbour's height + 1
   int top = GC_HINF, bot = GC_HINF, sl = GC_HINF, sr = GC_HINF;
+  int oT = GC_HINF, oB = GC_HINF, oL = GC_HINF, oR = GC_HINF;   // this tile's edges before
   if (!first) {
-    const uint32_t cu0 = __shfl_sync(0xffffffffu, canU, 0);
-    const uint32_t cd31 = __shfl_sync(0xffffffffu, canD, 31);
+    const uint32_t cu0 = __shfl_sync(FULL, canU, 0);
+    const uint32_t cd31 = __shfl_sync(FULL, canD, 31);
     const int vu = nb.x >= 0 ? P.hgt[(long long)nb.x * GC_TILE_PX + 31 * GC_TILE + lane] : GC_HINF;
     const int vd = nb.y >= 0 ? P.hgt[(long long)nb.y * GC_TILE_PX + lane] : GC_HINF;
     const int vl = nb.z >= 0 ? P.hgt[(long long)nb.z * GC_TILE_PX + lane * GC_TILE + 31] : GC_HINF;
     const int vr = nb.w >= 0 ? P.hgt[(long long)nb.w * GC_TILE_PX + lane * GC_TILE] : GC_HINF;
+    oT = P.hgt[base + lane];
+    oB = P.hgt[base + 31 * GC_TILE + lane];
+    oL = P.hgt[base + lane * GC_TILE];
+    oR = P.hgt[base + lane * GC_TILE + 31];
     if (((cu0 >> lane) & 1u) && vu < GC_HINF) top = vu + 1;
     if (((cd31 >> lane) & 1u) && vd < GC_HINF) bot = vd + 1;
     if ((canL & 1u) && vl < GC_HINF) sl = vl + 1;
     if ((canR >> 31) && vr < GC_HINF) sr = vr + 1;
+    const int lim = imin(cap, GC_HINF - 1);
+    if (!__any_sync(FULL, (top < oT && top <= lim) || (bot < oB && bot <= lim) ||
+                              (sl < oL && sl <= lim) || (sr < oR && sr <= lim)))
+      return -1;
   }
-  const uint32_t fin = tile_bfs_seeded(T + lane * 33, sink, canU, canD, canL, canR, lane, top,
-                                       bot, sl, sr, cap);
-  __syncwarp();
-  int chU = 0, chD = 0, chL = 0, chR = 0;
-  for (int rr = 0; rr < 32; ++rr) {
-    const int nv = T[rr * 33 + lane];
-    int* p = P.hgt + base + rr * GC_TILE + lane;
-    if (first) {
-      *p = nv;
-      const int fv = nv < GC_HINF;
-      chU |= (rr == 0) & fv; chD |= (rr == 31) & fv; chL |= (lane == 0) & fv; chR |= (lane == 31) & fv;
-    } else {
-      const int ov = *p;
-      if (nv != ov) *p = nv;
-      const int dec = nv < ov;
-      chU |= (rr == 0) & dec; chD |= (rr == 31) & dec; chL |= (lane == 0) & dec; chR |= (lane == 31) & dec;
+  uint32_t fin;
+  int nT, nB, nL, nR;   // the edges now
+  int state = 0;        // hstate: 1 all 0, 2 all unreached, 0 neither
+  if (cap <= BFS_NEAR_CAP) {
+    const NearBfs B = tile_bfs_near(sink, canU, canD, canL, canR, lane, !first, top, bot, sl, sr, cap);
+    fin = B.vis;
+    uint32_t any = 0;
+#pragma unroll
+    for (int b = 0; b < BFS_PLANES; ++b) any |= B.plane[b];
+    if (__all_sync(FULL, fin == FULL && any == 0)) state = 1;
+    else if (__all_sync(FULL, fin == 0)) state = 2;
+    nT = B.across(0, lane);
+    nB = B.across(31, lane);
+    nL = B.side(0);
+    nR = B.side(31);
+    if (state == 0 || P.hstate[t] != state) {
+      const int q = lane & 7;
+#pragma unroll 2
+      for (int k = 0; k < 8; ++k) {   // rows 4k .. 4k+3; this lane: four pixels of row 4k + lane / 8
+        const int src = 4 * k + (lane >> 3);
+        uint32_t d4 = 0;
+#pragma unroll
+        for (int b = 0; b < BFS_PLANES; ++b)
+          d4 |= spread4(__shfl_sync(FULL, B.plane[b], src) >> (4 * q)) << b;
+        const uint32_t f4 = __shfl_sync(FULL, B.vis, src) >> (4 * q);
+        const int4 v = make_int4(f4 & 1u ? (int)(d4 & 255u) : GC_HINF, f4 & 2u ? (int)((d4 >> 8) & 255u) : GC_HINF,
+                                 f4 & 4u ? (int)((d4 >> 16) & 255u) : GC_HINF, f4 & 8u ? (int)(d4 >> 24) : GC_HINF);
+        *(int4*)(P.hgt + base + src * GC_TILE + 4 * q) = v;
+      }
     }
+  } else {
+    fin = tile_bfs_seeded(T + lane * 33, sink, canU, canD, canL, canR, lane, top, bot, sl, sr, cap);
+    __syncwarp();
+    for (int rr = 0; rr < 32; ++rr) P.hgt[base + rr * GC_TILE + lane] = T[rr * 33 + lane];
+    nT = T[lane];
+    nB = T[31 * 33 + lane];
+    nL = T[lane * 33];
+    nR = T[lane * 33 + 31];
+    __syncwarp();
   }
-  __syncwarp();
-  chU = __any_sync(0xffffffffu, chU); chD = __any_sync(0xffffffffu, chD);
-  chL = __any_sync(0xffffffffu, chL); chR = __any_sync(0xffffffffu, chR);
-  const uint32_t pos = P.mexc[(long long)t * 32 + lane];
-  const int act = __any_sync(0xffffffffu, (pos & fin) != 0);
+  if (lane == 0) P.hstate[t] = state;
+  const int chU = __any_sync(FULL, nT < oT && ((wantU >> lane) & 1u));
+  const int chD = __any_sync(FULL, nB < oB && ((wantD >> lane) & 1u));
+  const int chL = __any_sync(FULL, nL < oL && wantL);
+  const int chR = __any_sync(FULL, nR < oR && wantR);
+  const int act = __any_sync(FULL, (pos & fin) != 0);
   // the neighbours to queue, one lane each (their atomics run in parallel)
   if (lane < 4) {
     const int go = lane == 0 ? chU : lane == 1 ? chD : lane == 2 ? chL : chR;
@@ -1485,7 +1616,7 @@ k_bfs_round(PoolView P, int first, int cap, int live) {
     }
     ++done;
     const int act = bfs_tile(P, t, lane, first, cap, tr[warp], out);
-    if (lane == 0) P.tact[t] = act;
+    if (lane == 0 && act >= 0) P.tact[t] = act;
   }
   if (lane == 0 && done) {
     atomicAdd(&P.rcnt[in], done);
@@ -1986,8 +2117,8 @@ k_solve(PoolView P, SolveArgs A) {
             const int act = bfs_tile(P, t, lane, first, cap, dsm + warp * (32 * 33), out);
             if (lane == 0) {
               // a tile becomes active once (its reached set only grows): list it then
-              if (act && (first || P.tact[t] == 0)) worklist_append(P, act_out, t);
-              if (first || act) P.tact[t] = act;
+              if (act > 0 && (first || P.tact[t] == 0)) worklist_append(P, act_out, t);
+              if (first || act > 0) P.tact[t] = act;
             }
           }
           ++fk;
