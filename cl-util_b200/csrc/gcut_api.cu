@@ -170,7 +170,8 @@ struct Pool {
   std::vector<int32_t> sel_key, sel_last;   // a selection; the one last copied to the device
   int32_t* trace_words = nullptr;   // device: trace on/off and entry count (P.trace_ctl when on)
   bool one_launch = false;          // the last solve ran as one launch (k_solve)
-  bool lists_stale = false;         // worklists or barrier words may be left over
+  bool lists_stale = false;         // worklists, counters, stamps or sums may be left over
+  int stamp_base = 0;               // no stamp in img_hit is above this
   gc_stats stats{};
   // profiling: event pairs around every launch, tiles processed per kernel kind
   bool prof = false;
@@ -633,14 +634,19 @@ struct Pool {
     const bool host = prof || collect || !use_graph;
     one_launch = !host;
     list_valid = false;   // the next manual push starts from a new list
-    // left by manual steps or a failed solve: worklist flags, barrier words
-    if (lists_stale) {
+    // left by manual steps, a host-driven or a failed solve: worklist flags, barrier and control
+    // words, stamps, sums
+    if (lists_stale || stamp_base > (1 << 30)) {
       CK(cudaMemsetAsync(P.inq[0], 0, sizeof(int32_t) * nt, s));
       CK(cudaMemsetAsync(P.inq[1], 0, sizeof(int32_t) * nt, s));
       CK(cudaMemsetAsync(P.bar, 0, sizeof(unsigned long long) * BAR_N, s));
+      CK(cudaMemsetAsync(P.ctl, 0, sizeof(int32_t) * CTL_N, s));
+      CK(cudaMemsetAsync(P.img_hit, 0, sizeof(int32_t) * imgs.size(), s));
+      RK(launch_acc_reset(acc, (int)imgs.size(), s));
+      stamp_base = 0;
     }
     lists_stale = true;   // until this solve succeeds
-    int r = host ? solve_host(s, warm, fresh) : solve_launch(s, warm, fresh, n, after, lmode, lbuf);
+    int r = host ? solve_host(s, warm, fresh, idx, n) : solve_launch(s, warm, fresh, idx, n, after, lmode, lbuf);
     if (r) return r;
     if (host && after) {   // the host-driven solve has finished: queue the work and wait
       RK((*after)(s));
@@ -648,7 +654,10 @@ struct Pool {
     }
     RK(finish_check(s, idx, n, /*err_in_ctl=*/true));
     one_launch = false;
-    lists_stale = host;   // the host-driven loop leaves worklist flags set
+    // a one-launch solve leaves everything clean (its results reached the host directly);
+    // the host-driven loop leaves worklist flags, stamps and sums
+    lists_stale = host || !P.host_out;
+    stamp_base += h_ctl[CTL_CYCLES] + 2;   // a flood per cycle, one before the first
     for (int k = 0; k < n; ++k) {
       img_solved[idx[k]] = 1;
       img_edited[idx[k]] = 0;
@@ -665,10 +674,10 @@ struct Pool {
   // its termination check, and for the images that are not solved a global relabel and the
   // next active-tile list.  The last flood of every image is its canonical cut, so no
   // separate flood phase follows.
-  int solve_host(cudaStream_t s, bool warm, bool fresh) {
+  int solve_host(cudaStream_t s, bool warm, bool fresh, const int* idx, int count) {
     RK(prof_begin(s));
     RK(launch_ctl_begin(P, opts.max_bfs_rounds, acc, s));
-    int n = 0, cap = kFirstCap, hlim = GC_HINF, stamp = 1;
+    int n = 0, cap = kFirstCap, hlim = kFirstLimit, stamp = 1;
     auto list_active = [&](int first) {
       RK(timed(K_COMPACT, s, [&] { return launch_active_list(P, scan.st, list, counts, stamp + 1, first, 2 * sms, s); }));
       return read_count(s, &n);
@@ -709,9 +718,17 @@ struct Pool {
       ++stamp;
       RK(flood_and_relabel(2));
     }
-    CK(cudaMemcpyAsync(h_acc, acc, sizeof(ImageAcc) * imgs.size(), cudaMemcpyDeviceToHost, s));
+    RK(copy_sums(idx, count, s));
     RK(read_ctl(s));
     RK(prof_end(s));
+    return GC_OK;
+  }
+
+  // the sums of the solved images to their places in the host mirror (the others' words on the
+  // device may have been reset since their own solves)
+  int copy_sums(const int* idx, int count, cudaStream_t s) {
+    for (int k = 0; k < count; ++k)
+      CK(cudaMemcpyAsync(h_acc + idx[k], acc + idx[k], sizeof(ImageAcc), cudaMemcpyDeviceToHost, s));
     return GC_OK;
   }
 
@@ -733,12 +750,17 @@ struct Pool {
   // (bytes / packed) of the pool's one image, into lbuf.  As many CTAs as the device holds,
   // but no more than selected tiles: a barrier among few CTAs is cheaper, and each tile still
   // has a CTA of its own.
-  int solve_launch(cudaStream_t s, bool warm, bool fresh, int ranges, const After* after,
-                   int lmode, uint8_t* lbuf) {
+  int solve_launch(cudaStream_t s, bool warm, bool fresh, const int* idx, int ranges,
+                   const After* after, int lmode, uint8_t* lbuf) {
     SolveArgs a{};
     a.acc = acc;
     a.ranges = ranges;
     a.tiles = sel_tiles;
+    const std::vector<int32_t>& sk = sel_last;   // the selection now on the device
+    a.sel0 = make_int4(sk[2], sk[3], sk[4], sk[5]);
+    a.mode0 = sk[6];
+    a.stamp0 = stamp_base;
+    a.clean = P.host_out != nullptr;
     a.warm = warm;
     a.fresh = fresh;
     a.iters = opts.discharge_iters;
@@ -752,9 +774,10 @@ struct Pool {
     P.ktiles = nullptr;
     const int grid = grid_solve < sel_tiles ? grid_solve : sel_tiles;
     if (launch_solve(P, a, grid > 0 ? grid : 1, s)) return fail(GC_ERR_CUDA, "solve launch failed");
-    if (!P.host_out)   // control words and per-image sums are adjacent on both sides: one copy
-      CK(cudaMemcpyAsync(h_ctl, P.ctl, sizeof(int32_t) * CTL_N + sizeof(ImageAcc) * imgs.size(),
-                         cudaMemcpyDeviceToHost, s));
+    if (!P.host_out) {
+      CK(cudaMemcpyAsync(h_ctl, P.ctl, sizeof(int32_t) * CTL_N, cudaMemcpyDeviceToHost, s));
+      RK(copy_sums(idx, ranges, s));
+    }
     if (after) RK((*after)(s));
     CK(cudaStreamSynchronize(s));
     return GC_OK;
@@ -819,6 +842,7 @@ struct Pool {
   int step_relabel(cudaStream_t s) {
     if (!uploaded) return fail(GC_ERR_STATE, "relabel before upload");
     solved = false;
+    lists_stale = true;
     bfs_fresh = false;
     list_valid = true;
     img_solved.assign(imgs.size(), 0);
@@ -828,6 +852,7 @@ struct Pool {
   }
   int step_start_bfs(cudaStream_t s) {
     if (!uploaded) return fail(GC_ERR_STATE, "startBfs before upload");
+    lists_stale = true;
     bool warm;
     RK(select_all(&warm, s));
     RK(launch_ctl_begin(P, opts.max_bfs_rounds, acc, s));

@@ -134,12 +134,19 @@ struct SelCursor {
     k = lo;
     cur = nr > 0 ? sel[k] : make_int4(0, 0, 0, 0);
   }
+  // with the first range at hand: a selection of one range needs no load
+  __device__ __forceinline__ SelCursor(const PoolView& P, int nranges, int i, const int4& first)
+      : SelCursor(P, nranges > 1 ? nranges : 0, i) {
+    nr = nranges;
+    if (nranges == 1) cur = first;
+  }
   // tile of selected index i (i >= the previous index asked for)
   __device__ __forceinline__ int tile(int i) {
     while (i >= cur.z + cur.y && k + 1 < nr) cur = sel[++k];
     return cur.x + (i - cur.z);
   }
   __device__ __forceinline__ int image() const { return cur.w; }
+  __device__ __forceinline__ int range() const { return k; }
 };
 
 // A running k_solve ends at its next barrier.

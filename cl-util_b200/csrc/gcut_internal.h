@@ -111,6 +111,10 @@ __device__ __host__ __forceinline__ int cycle_pulses(int pulses, int cycle) {
 __device__ __host__ __forceinline__ int cycle_iters(int iters, int cycle) {
   return cycle == 0 ? iters : iters + 3;
 }
+// Active heights before the first relabel, whose trivial labels (0 at sinks, 1 elsewhere) say
+// little: below 4, excess far from a sink stops rising after three sweeps instead of keeping
+// its warps busy.  (3: more cycles; unlimited: 512^2 3 %, 64 grids 4 % slower.)
+constexpr int kFirstLimit = 4;
 constexpr int kFirstCap = 16;
 constexpr int kLastCap = 1 << 12;   // above it: exact distances
 __device__ __host__ __forceinline__ int next_cap(int cap) {
@@ -120,6 +124,10 @@ __device__ __host__ __forceinline__ int next_cap(int cap) {
 struct SolveArgs {
   ImageAcc* acc;
   int ranges, tiles;        // the selection's size (its ranges are in P.sel)
+  int4 sel0;                // its first range
+  int mode0;                // and its mode
+  int stamp0;               // every stamp in img_hit is at most this; the floods take the next ones
+  int clean;                // leave the counters and sums at zero (the results reach the host)
   int warm, fresh;          // some selected image continues from a flow / is freshly uploaded
   int iters, pulses;        // sweeps per discharge, discharges per cycle
   int max_rounds, max_cycles;

@@ -102,9 +102,10 @@ __device__ __forceinline__ void mark_dirty(const PoolView& P, int t) { P.mdirty[
 struct RowMasks { uint32_t up, down, left, right, sink, exc; };
 
 // Rebuilds tile t's row masks and its sum of max(excess, 0) from its planes with one warp:
-// lane c reads column c of four rows at a time (one 128-byte line per row and plane), and a
+// lane c reads column c of REB_ROWS rows at a time (one 128-byte line per row and plane), and a
 // ballot over the lanes is the row's mask.  Writes the masks and the sum, clears the dirty
 // flag, and returns row `lane`'s masks to each lane and the tile's sum to every lane.
+constexpr int REB_ROWS = 8;
 __device__ __forceinline__ RowMasks warp_rebuild_masks(const PoolView& P, int t, int lane,
                                                        long long* tile_pos) {
   const unsigned F = 0xffffffffu;
@@ -112,10 +113,10 @@ __device__ __forceinline__ RowMasks warp_rebuild_masks(const PoolView& P, int t,
   RowMasks out{0u, 0u, 0u, 0u, 0u, 0u};
   long long pos = 0;
 #pragma unroll 1
-  for (int r0 = 0; r0 < GC_TILE; r0 += 4) {
-    int v[4][5];
+  for (int r0 = 0; r0 < GC_TILE; r0 += REB_ROWS) {
+    int v[REB_ROWS][5];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < REB_ROWS; ++k) {
       const long long o = base + (r0 + k) * GC_TILE;
       v[k][0] = P.exc[o];
       v[k][1] = P.cap[DUP][o];
@@ -124,7 +125,7 @@ __device__ __forceinline__ RowMasks warp_rebuild_masks(const PoolView& P, int t,
       v[k][4] = P.cap[DRIGHT][o];
     }
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < REB_ROWS; ++k) {
       const uint32_t mu = __ballot_sync(F, v[k][1] > 0), md = __ballot_sync(F, v[k][2] > 0);
       const uint32_t ml = __ballot_sync(F, v[k][3] > 0), mr = __ballot_sync(F, v[k][4] > 0);
       const uint32_t ms = __ballot_sync(F, v[k][0] < 0), me = __ballot_sync(F, v[k][0] > 0);
@@ -555,6 +556,7 @@ struct DisSmem {
   int32_t fu[GC_TILE_PX + GC_TILE];       // flow pushed up by each pixel this sweep, and a zero row
   int32_t fd[GC_TILE_PX + GC_TILE];       // a zero row, and flow pushed down
   int32_t eo_top[GC_TILE], eo_bot[GC_TILE], eo_left[GC_TILE], eo_right[GC_TILE];
+  int32_t xv_top[GC_TILE], xv_bot[GC_TILE];   // flow out of the tile across its first / last row
 };
 
 // A worklist of tiles: list, length, and the per-tile flag that keeps a tile in it once.
@@ -598,6 +600,14 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* mbar, unsigned parity) {
                : "=r"(ok) : "r"(a), "r"(parity) : "memory");
   return ok != 0;
 }
+// Asynchronous copies of a few bytes global -> shared memory by one thread (cp.async).
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* dst, const void* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // A tile copy normally lands in microseconds; a wait gives up after this long.  The bound
 // is on time, not on polls: try_wait may return at once, and a poll count then would allow
 // only milliseconds under load (a CTA that gave up early would leave while its copy is
@@ -654,7 +664,7 @@ __device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, in
                                                 const Worklist& out, int32_t* buf, DisSmem& S,
                                                 uint64_t* mbar, unsigned& phase) {
   const unsigned F = 0xffffffffu;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31;
   const int r = tid >> 3, q = tid & 7, c0 = q * 4;
   // Bookkeeping log: each tile leaves (tile, neighbours, flags) here, and the CTA's threads
   // settle up to DIS_LOG tiles at once (its list entry, and the list entries and dirty flags
@@ -720,15 +730,26 @@ __device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, in
     S.fu[GC_TILE_PX + tid] = 0;
     S.fd[tid] = 0;
   }
+  // Tile ids and neighbour ids run ahead of the tiles (thread 0, asynchronous copies into
+  // shared memory), so no warp waits for a list entry before its tile's sweeps: while tile k
+  // is worked on, the entry of tile k + 2 and the neighbours of tile k + 1 arrive.
+  __shared__ int s_id[2];            // entries of the tiles after this one, by parity
+  __shared__ __align__(16) int4 s_nb[2];   // neighbour ids by parity
   bool failed = false;
-  int t = 0;
-  int4 nb = make_int4(-1, -1, -1, -1);
+  int par = 0;
   if (bid < n) {
-    t = entry(bid);
-    if (tid == 0) dis_prefetch(P, t, buf, mbar);
-    nb = P.nbr[t];
+    if (tid == 0) {
+      const int t0 = entry(bid);
+      dis_prefetch(P, t0, buf, mbar);
+      s_id[0] = t0;
+      s_nb[0] = P.nbr[t0];
+      if (bid + nb_ctas < n) s_id[1] = entry(bid + nb_ctas);
+    }
+    __syncthreads();
   }
-  for (int li = bid; li < n; li += nb_ctas) {
+  for (int li = bid; li < n; li += nb_ctas, par ^= 1) {
+    const int t = s_id[par];
+    const int4 nb = s_nb[par];
     // halo heights, loaded while the tile's copy lands
     int4 hv = make_int4(GC_HINF, GC_HINF, GC_HINF, GC_HINF);   // first / last row: across the side
     int hside = GC_HINF;                                       // first / last strip: across the side
@@ -750,7 +771,10 @@ __device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, in
       int4 v = lds4(buf + 0 * GC_TILE_PX + pix); e[0] = v.x; e[1] = v.y; e[2] = v.z; e[3] = v.w;
       // launch-start excess of the pixels that also receive atomics from neighbouring tiles
       // (written back as deltas against it)
-      if (erow) sts4((r == 0 ? S.eo_top : S.eo_bot) + c0, v.x, v.y, v.z, v.w);
+      if (erow) {
+        sts4((r == 0 ? S.eo_top : S.eo_bot) + c0, v.x, v.y, v.z, v.w);
+        sts4((r == 0 ? S.xv_top : S.xv_bot) + c0, 0, 0, 0, 0);
+      }
       if (ecol) (left ? S.eo_left : S.eo_right)[r] = left ? v.x : v.w;
       v = lds4(buf + 1 * GC_TILE_PX + pix); h[0] = v.x; h[1] = v.y; h[2] = v.z; h[3] = v.w;
       sts4(hs, v.x, v.y, v.z, v.w);
@@ -767,15 +791,14 @@ __device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, in
       const bool edge = erow || (j == 0 && q == 0) || (j == 3 && q == 7);
       hcap[j] = edge ? imin(h[j] + 2, hlim) : hlim;
     }
-    int xv[4] = {0, 0, 0, 0}, xh = 0;   // flow out of the tile: across the row / column side
+    int xh = 0;   // flow out of the tile across the first / last column (rows: S.xv_*)
     __syncthreads();   // every thread has its values in registers: the buffer is free
     // prefetch this CTA's next tile into the buffer while this one is worked on
-    int tn = 0;
-    int4 nbn = make_int4(-1, -1, -1, -1);
-    if (li + nb_ctas < n) {
-      tn = entry(li + nb_ctas);
-      if (tid == 0) dis_prefetch(P, tn, buf, mbar);
-      nbn = P.nbr[tn];
+    if (tid == 0 && li + nb_ctas < n) {
+      const int tn = s_id[par ^ 1];
+      dis_prefetch(P, tn, buf, mbar);
+      copy_async<16>(&s_nb[par ^ 1], P.nbr + tn);
+      if (li + 2 * nb_ctas < n) copy_async<4>(&s_id[par], in.list + li + 2 * nb_ctas);
     }
 
     for (int it = 0; it < iters; ++it) {
@@ -807,13 +830,13 @@ __device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, in
         }
       }
       // flow leaving the tile is delivered at the end of the tile
-      if (warp == 0) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) xv[j] += r == 0 ? ou[j] : 0;
+      if (r == 0) {
+        const int4 x = lds4(S.xv_top + c0);
+        sts4(S.xv_top + c0, x.x + ou[0], x.y + ou[1], x.z + ou[2], x.w + ou[3]);
       }
-      if (warp == DIS_THREADS / 32 - 1) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) xv[j] += r == 31 ? od[j] : 0;
+      if (r == 31) {
+        const int4 x = lds4(S.xv_bot + c0);
+        sts4(S.xv_bot + c0, x.x + od[0], x.y + od[1], x.z + od[2], x.w + od[3]);
       }
       xh += q == 0 ? ol[0] : q == 7 ? orr[3] : 0;
       sts4(S.fu + pix, ou[0], ou[1], ou[2], ou[3]);
@@ -839,8 +862,9 @@ __device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, in
       }
       // relabel (Jacobi) to one above the lowest residual neighbour m.  The labelling is valid,
       // so h <= m + 1, with equality exactly when an admissible edge is left: the pixel then
-      // keeps its height.  So does one at its limit, and an inactive one (h >= hlim >= hcap).
-      if (__any_sync(F, e[0] > 0 || e[1] > 0 || e[2] > 0 || e[3] > 0)) {
+      // keeps its height.  So does one at its limit, and an inactive one (h >= hlim >= hcap);
+      // a warp of only such pixels skips the step.
+      if (__any_sync(F, (e[0] > 0 && h[0] < hcap[0]) || (e[1] > 0 && h[1] < hcap[1]) || (e[2] > 0 && h[2] < hcap[2]) || (e[3] > 0 && h[3] < hcap[3]))) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           int m = GC_HINF;
@@ -867,7 +891,9 @@ __device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, in
 
     // bits 0-3: sent up, down, left, right; 4: active; 5: interior active
     unsigned flags = 0;
-    if (xv[0] | xv[1] | xv[2] | xv[3]) flags |= r == 0 ? 1u : 2u;
+    int4 xo = make_int4(0, 0, 0, 0);
+    if (erow) xo = lds4((r == 0 ? S.xv_top : S.xv_bot) + c0);
+    if (xo.x | xo.y | xo.z | xo.w) flags |= r == 0 ? 1u : 2u;
     if (xh) flags |= left ? 4u : 8u;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -876,6 +902,7 @@ __device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, in
     }
     flags = __reduce_or_sync(F, flags);
     if (lane == 0 && flags) atomicOr(&s_logf[nlog], flags);
+    if (tid == 0) copy_async_wait();   // the next tile's ids
     __syncthreads();   // the log entry is complete; orders the exchange arrays' reuse, too
     // (an entry is rewritten after a flush behind at least one more barrier, but for entry 0,
     // which only lanes of thread 0's warp read)
@@ -898,7 +925,7 @@ __device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, in
     if (!erow && !ecol) *(int4*)(P.exc + off) = make_int4(e[0], e[1], e[2], e[3]);
     if (erow) {
       const int4 v = lds4((r == 0 ? S.eo_top : S.eo_bot) + c0);
-      const int e0[4] = {v.x, v.y, v.z, v.w};
+      const int e0[4] = {v.x, v.y, v.z, v.w}, xv[4] = {xo.x, xo.y, xo.z, xo.w};
       int32_t* const own = (r == 0 ? P.cap[DUP] : P.cap[DDOWN]) + off;
       const long long o = (long long)nv * GC_TILE_PX + (r == 0 ? 31 * GC_TILE : 0) + c0;
       int32_t* const rev = (r == 0 ? P.cap[DDOWN] : P.cap[DUP]) + o;
@@ -933,8 +960,6 @@ __device__ __forceinline__ void discharge_phase(const PoolView& P, int iters, in
         atomicAdd((left ? P.cap[DRIGHT] : P.cap[DLEFT]) + o, xh);
       }
     }
-    t = tn;
-    nb = nbn;
   }
   if (failed) {
     flush_log(nlog);   // the tiles done before
@@ -1687,70 +1712,99 @@ struct FloodSum {
   }
 };
 
-// One tile of a flood round, by one warp.  hits: counts the images whose sink-reached stamp
-// this flood sets (null: not counted).
-__device__ __forceinline__ void flood_tile(const PoolView& P, int t, int lane, int first, int img,
-                                           int stamp, int32_t* hits, const Worklist& out,
-                                           ImageAcc* acc, FloodSum& fs) {
-  const int4 nb = P.nbr[t];
-  uint32_t canU, canD, canL, canR, sink, R, R0;
-  long long ps = 0;
-  if (first && P.mdirty[t] != 0) {
-    // the tile changed since its masks were written (a discharge or an edit): rebuild them
-    // here, before anything reads them (every tile of an image this round covers is done
-    // in this round, so the frontier rounds and the global relabel after it see them)
-    const RowMasks m = warp_rebuild_masks(P, t, lane, &ps);
-    canU = m.up; canD = m.down; canL = m.left; canR = m.right;
-    sink = m.sink;
-    R = m.exc;
-  } else {
-    const uint32_t* mc = P.mcan + (long long)t * 128;
-    canU = mc[lane]; canD = mc[32 + lane]; canL = mc[64 + lane]; canR = mc[96 + lane];
-    sink = P.msink[(long long)t * 32 + lane];
-    if (first) {
-      R = P.mexc[(long long)t * 32 + lane];
-      ps = P.tpos[t];
-    }
-  }
-  if (first) {
-    R0 = 0;
-    if (lane == 0 && ps) fs.add(acc, img, ps);   // taken with the tile's masks
-  } else {
-    R = R0 = P.mreach[(long long)t * 32 + lane];
-    if (lane == 0 && nb.x >= 0)
-      R |= P.mreach[(long long)nb.x * 32 + 31] & P.mcan[(long long)nb.x * 128 + 32 + 31];
-    if (lane == 31 && nb.y >= 0)
-      R |= P.mreach[(long long)nb.y * 32] & P.mcan[(long long)nb.y * 128 + 0];
-    if (nb.z >= 0 && ((P.mreach[(long long)nb.z * 32 + lane] & P.mcan[(long long)nb.z * 128 + 96 + lane]) >> 31))
-      R |= 1u;
-    if (nb.w >= 0 && ((P.mreach[(long long)nb.w * 32 + lane] & P.mcan[(long long)nb.w * 128 + 64 + lane]) & 1u))
-      R |= 0x80000000u;
-  }
+// The masks a warp floods a tile with: lane = row.
+struct TileMasks { uint32_t canU, canD, canL, canR, sink, exc; };
+
+__device__ __forceinline__ TileMasks load_masks(const PoolView& P, int t, int lane) {
+  const uint32_t* mc = P.mcan + (long long)t * 128;
+  return TileMasks{mc[lane], mc[32 + lane], mc[64 + lane], mc[96 + lane],
+                   P.msink[(long long)t * 32 + lane], P.mexc[(long long)t * 32 + lane]};
+}
+
+// Everything in a row that the pixels of R reach to the right over the edges M (bit x: x to
+// x + 1): the carry of (R & M) + M runs through each run of edges from its lowest seed to the
+// pixel after its end.  (A seed inside the run flips back, but is in R.)
+__device__ __forceinline__ uint32_t fill_up_bits(uint32_t R, uint32_t M) { return R | (((R & M) + M) ^ M); }
+
+// Floods tile t from R (which it extends) inside the tile, by one warp; writes the reached set,
+// stamps the image when it meets a sink, and queues the neighbours it reaches into.  R0: the
+// reached set before (0 in a first round).  hits: counts the images whose stamp this flood
+// sets (null: not counted).
+__device__ __forceinline__ void flood_fill(const PoolView& P, int t, int4 nb, int lane, int img,
+                                           int stamp, const TileMasks& m, uint32_t R, uint32_t R0,
+                                           int32_t* hits, const Worklist& out) {
+  const unsigned FULL = 0xffffffffu;
+  const uint32_t toDown = lane == 31 ? 0u : m.canD, toUp = lane == 0 ? 0u : m.canU;
+  const uint32_t leftRev = __brev(m.canL);
+  // every step reaches at least one pixel more; rows fill at once
   for (int guard = 0; guard < GC_TILE_PX + 1; ++guard) {
-    uint32_t dn = __shfl_up_sync(0xffffffffu, R & canD, 1);   // row r-1 flows down into r
-    uint32_t up = __shfl_down_sync(0xffffffffu, R & canU, 1); // row r+1 flows up into r
+    uint32_t dn = __shfl_up_sync(FULL, R & toDown, 1);   // row r-1 flows down into r
+    uint32_t up = __shfl_down_sync(FULL, R & toUp, 1);   // row r+1 flows up into r
     if (lane == 0) dn = 0;
     if (lane == 31) up = 0;
-    const uint32_t N = R | ((R & canR) << 1) | ((R & canL) >> 1) | dn | up;
-    if (!__any_sync(0xffffffffu, N != R)) break;
+    uint32_t N = R | dn | up;
+    N = fill_up_bits(N, m.canR);
+    N = __brev(fill_up_bits(__brev(N), leftRev));
+    if (!__any_sync(FULL, N != R)) break;
     R = N;
   }
   P.mreach[(long long)t * 32 + lane] = R;
-  if (__any_sync(0xffffffffu, (R & sink) != 0) && lane == 0 &&
+  if (__any_sync(FULL, (R & m.sink) != 0) && lane == 0 &&
       *((volatile int32_t*)&P.img_hit[img]) != stamp) {
     if (!hits) P.img_hit[img] = stamp;
     else if (atomicExch(&P.img_hit[img], stamp) != stamp) atomicAdd(hits, 1);
   }
-  const uint32_t nw = first ? R : (R & ~R0);
-  const int sU = __any_sync(0xffffffffu, lane == 0 && (nw & canU));
-  const int sD = __any_sync(0xffffffffu, lane == 31 && (nw & canD));
-  const int sL = __any_sync(0xffffffffu, (nw & canL & 1u) != 0);
-  const int sR = __any_sync(0xffffffffu, ((nw & canR) >> 31) != 0);
+  const uint32_t nw = R & ~R0;
+  const int sU = __any_sync(FULL, lane == 0 && (nw & m.canU));
+  const int sD = __any_sync(FULL, lane == 31 && (nw & m.canD));
+  const int sL = __any_sync(FULL, (nw & m.canL & 1u) != 0);
+  const int sR = __any_sync(FULL, ((nw & m.canR) >> 31) != 0);
   if (lane < 4) {   // the neighbours to queue, one lane each
     const int go = lane == 0 ? sU : lane == 1 ? sD : lane == 2 ? sL : sR;
     const int nt = lane == 0 ? nb.x : lane == 1 ? nb.y : lane == 2 ? nb.z : nb.w;
     if (go && nt >= 0) frontier_push(P, out, nt);
   }
+}
+
+// One tile of a frontier round: what it had reached, and what the neighbours' reached sets
+// reach across its sides.
+__device__ __forceinline__ void flood_frontier_tile(const PoolView& P, int t, int lane, int img,
+                                                    int stamp, int32_t* hits, const Worklist& out) {
+  const int4 nb = P.nbr[t];
+  const TileMasks m = load_masks(P, t, lane);
+  const uint32_t R0 = P.mreach[(long long)t * 32 + lane];
+  uint32_t R = R0;
+  if (lane == 0 && nb.x >= 0)
+    R |= P.mreach[(long long)nb.x * 32 + 31] & P.mcan[(long long)nb.x * 128 + 32 + 31];
+  if (lane == 31 && nb.y >= 0)
+    R |= P.mreach[(long long)nb.y * 32] & P.mcan[(long long)nb.y * 128 + 0];
+  if (nb.z >= 0 && ((P.mreach[(long long)nb.z * 32 + lane] & P.mcan[(long long)nb.z * 128 + 96 + lane]) >> 31))
+    R |= 1u;
+  if (nb.w >= 0 && ((P.mreach[(long long)nb.w * 32 + lane] & P.mcan[(long long)nb.w * 128 + 64 + lane]) & 1u))
+    R |= 0x80000000u;
+  if (!__any_sync(0xffffffffu, R != R0)) return;   // nothing new comes in
+  flood_fill(P, t, nb, lane, img, stamp, m, R, R0, hits, out);
+}
+
+// One tile of a first round, by one warp; a tile that changed since its masks were written (a
+// discharge or an edit) gets them rebuilt first, before anything reads them (every tile of an
+// image a first round covers is done in it, so the frontier rounds and the global relabel
+// after it see them).
+__device__ __forceinline__ void flood_first_tile(const PoolView& P, int t, int lane, int img,
+                                                 int stamp, const Worklist& out, ImageAcc* acc,
+                                                 FloodSum& fs) {
+  const int4 nb = P.nbr[t];
+  TileMasks m;
+  long long ps = 0;
+  if (P.mdirty[t] != 0) {
+    const RowMasks rm = warp_rebuild_masks(P, t, lane, &ps);
+    m = TileMasks{rm.up, rm.down, rm.left, rm.right, rm.sink, rm.exc};
+  } else {
+    m = load_masks(P, t, lane);
+    ps = P.tpos[t];
+  }
+  if (lane == 0 && ps) fs.add(acc, img, ps);   // taken with the tile's masks
+  flood_fill(P, t, nb, lane, img, stamp, m, m.exc, 0, nullptr, out);
 }
 
 // The CTA's warps add their sums, once per image.  Every thread of the CTA calls it.
@@ -1764,14 +1818,19 @@ __device__ __forceinline__ void flood_sum_flush(ImageAcc* acc, const FloodSum& f
     s_sum[warp] = fs.sum;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int a = 0; a < WARPS; ++a) {
-      if (s_img[a] < 0) continue;
-      unsigned long long v = s_sum[a];
-      for (int b = a + 1; b < WARPS; ++b)
-        if (s_img[b] == s_img[a]) { v += s_sum[b]; s_img[b] = -1; }
-      atomicAdd(&acc[s_img[a]].sumpos_e, v);
+  if (warp == 0) {   // lane a: the sum of the warps that hold warp a's image, added by the first
+    const int mine = lane < WARPS ? s_img[lane] : -1;
+    const unsigned long long v = lane < WARPS ? s_sum[lane] : 0ull;
+    unsigned long long total = 0;
+    bool first = true;
+#pragma unroll
+    for (int b = 0; b < WARPS; ++b) {
+      const bool same = __shfl_sync(0xffffffffu, mine, b) == mine;
+      const unsigned long long x = __shfl_sync(0xffffffffu, v, b);
+      if (same) total += x;
+      if (same && b < lane) first = false;
     }
+    if (lane < WARPS && mine >= 0 && first) atomicAdd(&acc[mine].sumpos_e, total);
   }
 }
 
@@ -1807,7 +1866,8 @@ k_flood_round(PoolView P, int mode, int abort_hit, int stamp, ImageAcc* acc) {
     if (mode == 3 && P.img_mode[img] != 2) continue;
     if (mode == 0 && abort_hit && *((volatile int32_t*)&P.img_hit[img]) == stamp) continue;
     ++done;
-    flood_tile(P, t, lane, first, img, stamp, nullptr, out, acc, fs);
+    if (first) flood_first_tile(P, t, lane, img, stamp, out, acc, fs);
+    else flood_frontier_tile(P, t, lane, img, stamp, nullptr, out);
   }
   if (lane == 0 && done) {
     atomicAdd(&P.rcnt[in], done);
@@ -1887,12 +1947,11 @@ __global__ void k_labels_packed(PoolView P, ImageDesc im, uint8_t* out) {
 
 // ------------------------------------------------------------------------------------
 // The whole solve as one cooperative launch: every CTA runs the same steps (pulses, flood
-// rounds, relabel rounds), with a grid barrier after each, and the loop decisions are taken
-// by every CTA from the counters it reads behind the barrier.
+// rounds, relabel rounds), with a grid barrier after each.
 //
-// A barrier costs 1-2 us.  The CUDA graph this replaces (the same steps as kernel nodes under
-// WHILE and IF nodes) paid a kernel's launch and drain per step and 5-11 us per conditional
-// node passed.
+// A barrier costs about 2 us.  The CUDA graph this replaces (the same steps as kernel nodes
+// under WHILE and IF nodes) paid a kernel's launch and drain per step and 5-11 us per
+// conditional node passed.
 // ------------------------------------------------------------------------------------
 // A barrier wait gives up after this long (a step of the largest pool takes well under a
 // second): it raises the abort flag, and every CTA leaves at its next barrier.
@@ -1904,34 +1963,134 @@ __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long lon
   return v;
 }
 
-// Grid barrier with a sum: every CTA's writes before it are visible to every CTA after it
-// (to its bulk copies too, with Copies set), and `total` is the grid's sum of the CTAs' counts
-// *s_push, which start at 0 again.  The count travels in the upper half of the arrival word, so
-// the loop decision needs no second trip to L2 (0.35 us).  Barriers alternate between two
-// words: no CTA reaches a word's next use before all have left this one, so what they read of
-// it is the same.  `extra` (may be null): a counter no CTA writes before the next barrier, read
-// for the whole CTA into v1 when total is 0 or `always`.  Returns false (in every thread) when
-// the solve was aborted.
-struct GridBar {
-  unsigned k = 0;            // barriers passed
-  unsigned last[2] = {0, 0}; // totals of the words' last uses
+// The solve's loop state, one copy per CTA in shared memory, written by thread 0 only (inside
+// solve_barrier): the same in every CTA, because it follows from the same counters.  Kept out
+// of registers: what a step spills is reloaded from L2, since the barriers' fences empty L1.
+enum SolveStep { ST_LIST, ST_PULSE, ST_FLOOD_FIRST, ST_FLOOD, ST_BFS_FIRST, ST_BFS, ST_END };
+struct SolveState {
+  int step;
+  int cyc;                  // 0 before the first pulses (warm images' flood, first list)
+  int n;                    // tiles of the step's list
+  int pulse, pulses, iters; // of the cycle
+  int qk, fk;               // steps of the worklist and of the frontier (counter slots mod 3)
+  int stamp, prev;          // the flood's stamp, the one before it (0: none)
+  int cycles, cap, hlim;    // finished cycles; the next relabel's cap, the last one's limit
+  int rounds;               // of the flood or relabel that runs
+  int nf, nb, np;           // flood rounds, relabel rounds, pulses of the solve
+  int err;
+  int push;                 // tiles this CTA has queued since the last barrier
+  unsigned bar;             // barriers passed
+  unsigned last[2];         // sums of the barrier words' last uses
 };
-template <bool Copies>
-__device__ __forceinline__ bool grid_sync(const PoolView& P, GridBar& B, volatile int32_t* s,
-                                          int* s_push, int& total, const int32_t* extra = nullptr,
-                                          int* v1 = nullptr, bool always = false) {
-  if (Copies) asm volatile("fence.proxy.async;" ::: "memory");   // this thread's writes, before later copies
+
+__device__ __forceinline__ void begin_cycle(const SolveArgs& A, SolveState& s, int list) {
+  ++s.cyc;
+  s.n = list;
+  s.pulse = 0;
+  s.pulses = cycle_pulses(A.pulses, s.cycles);
+  s.iters = cycle_iters(A.iters, s.cycles);
+  s.step = ST_PULSE;
+}
+
+// The step after `s.step`, which the whole grid has finished; total: tiles queued in it.
+// Thread 0 only.
+__device__ __forceinline__ void next_step(const PoolView& P, const SolveArgs& A, SolveState& s, int total) {
+  int list = -1;   // >= 0: a cycle begins with a worklist of this length
+  s.n = total;
+  switch (s.step) {
+    case ST_LIST:
+      list = *((volatile int32_t*)&P.ctl[CTL_Q0 + s.qk % 3]);
+      break;
+    case ST_PULSE:
+      ++s.qk;
+      ++s.np;
+      if (++s.pulse < s.pulses && total > 0) break;
+      s.step = ST_FLOOD_FIRST;
+      s.prev = s.stamp == A.stamp0 ? 0 : s.stamp;
+      ++s.stamp;
+      break;
+    case ST_FLOOD_FIRST:
+    case ST_FLOOD: {
+      ++s.fk;
+      ++s.nf;
+      ++s.rounds;
+      if (total > 0) {
+        s.step = ST_FLOOD;
+        if (s.rounds >= A.max_rounds) s.err = 1;
+        break;
+      }
+      const int left = *((volatile int32_t*)&P.ctl[CTL_H0 + s.stamp % 3]);   // images that met a sink
+      if (s.cyc > 0) ++s.cycles;
+      if (blockIdx.x == 0) trace_record(P, TR_CHECK);
+      s.rounds = 0;
+      s.step = left > 0 ? ST_BFS_FIRST : s.cyc == 0 && A.fresh ? ST_LIST : ST_END;
+      break;
+    }
+    case ST_BFS_FIRST:
+    case ST_BFS:
+      ++s.fk;
+      ++s.nb;
+      ++s.rounds;
+      if (total > 0) {
+        s.step = ST_BFS;
+        if (s.rounds >= A.max_rounds) s.err = 1;
+        break;
+      }
+      s.rounds = 0;
+      list = *((volatile int32_t*)&P.ctl[CTL_Q0 + s.qk % 3]);
+      if (list == 0 && s.cap < GC_HINF) {   // no excess within the cap of a sink: further out
+        s.cap = next_cap(s.cap);
+        s.step = ST_BFS_FIRST;
+        list = -1;
+        break;
+      }
+      s.hlim = s.cap < GC_HINF ? s.cap + 1 : GC_HINF;
+      s.cap = next_cap(s.cap);   // further out with every cycle
+      if (s.cyc == 0 && A.fresh) {
+        s.step = ST_LIST;
+        list = -1;
+      }
+      break;
+  }
+  if (list >= 0) {
+    if (list == 0 && s.step != ST_LIST) {
+      s.step = ST_END;
+    } else if (s.cycles >= A.max_cycles) {
+      s.err = 2;
+    } else {
+      begin_cycle(A, s, list);
+      if (list == 0) {   // no fresh tile is near a sink: straight to the flood
+        s.step = ST_FLOOD_FIRST;
+        s.prev = s.stamp == A.stamp0 ? 0 : s.stamp;
+        ++s.stamp;
+      }
+    }
+  }
+  if (s.n < 0 || s.n > P.nt) {   // self-check: a list holds each tile at most once
+    record_bad(P, 6, s.n);
+    s.err = 4;
+  }
+  if (s.err) s.step = ST_END;
+}
+
+// Grid barrier and step change: every CTA's writes before it are visible to every CTA after
+// it, its bulk copies included, and `s` holds the next step.  The CTAs' counts of queued tiles
+// travel in the upper half of the arrival word, so the loop decision needs no second trip to L2
+// (0.35 us).  Barriers alternate between two words: no CTA reaches a word's next use before all
+// have left this one, so what they read of it is the same.  A solve that was aborted ends.
+__device__ __forceinline__ void solve_barrier(const PoolView& P, const SolveArgs& A, SolveState& s) {
+  // this thread's writes to the planes, before later bulk copies (a flood writes none)
+  if (s.step != ST_FLOOD_FIRST && s.step != ST_FLOOD) asm volatile("fence.proxy.async;" ::: "memory");
   __syncthreads();
-  unsigned long long* const word = P.bar + BAR_ARRIVE + (B.k & 1) * BAR_STRIDE;
-  const unsigned target = gridDim.x * ((B.k >> 1) + 1);
   if (threadIdx.x == 0) {
-    // CTA 0 takes the word's previous total out again: the upper half is never negative
-    const unsigned mine = (unsigned)*s_push;
-    *s_push = 0;
-    unsigned long long add = ((unsigned long long)mine << 32) + 1ull;
-    if (blockIdx.x == 0) add -= (unsigned long long)((B.k & 1) ? B.last[1] : B.last[0]) << 32;
+    unsigned long long* const word = P.bar + BAR_ARRIVE + (s.bar & 1) * BAR_STRIDE;
+    const unsigned target = gridDim.x * ((s.bar >> 1) + 1);
+    // CTA 0 takes the word's previous sum out again: the upper half is never negative
+    unsigned long long add = ((unsigned long long)(unsigned)s.push << 32) + 1ull;
+    if (blockIdx.x == 0) add -= (unsigned long long)s.last[s.bar & 1] << 32;
     __threadfence();
     atomicAdd(word, add);
+    s.push = 0;
     bool ok = false;
     unsigned long long t0 = 0, v = 0;
     for (unsigned i = 1; i < (1u << 31); ++i) {
@@ -1950,19 +2109,153 @@ __device__ __forceinline__ bool grid_sync(const PoolView& P, GridBar& B, volatil
       }
     }
     __threadfence();
-    if (Copies) asm volatile("fence.proxy.async;" ::: "memory");
-    const int n = (int)((v >> 32) & 0x7fffffffu);
-    s[0] = ok;
-    s[1] = n;
-    s[2] = ok && extra && (always || n == 0) ? *((const volatile int32_t*)extra) : 0;
+    asm volatile("fence.proxy.async;" ::: "memory");
+    const unsigned total = (unsigned)(v >> 32) & 0x7fffffffu;
+    s.last[s.bar & 1] = total;
+    ++s.bar;
+    // the arrivals' half must not overflow into the sum (after 2^32 arrivals: hours)
+    if (!ok || target >= 0xffff0000u) {
+      s.err = 5;
+      s.step = ST_END;
+    } else {
+      next_step(P, A, s, (int)total);
+    }
   }
   __syncthreads();
-  total = s[1];
-  if (v1) *v1 = s[2];
-  if (B.k & 1) B.last[1] = (unsigned)total; else B.last[0] = (unsigned)total;
-  ++B.k;
-  // the arrivals' half must not overflow into the sum (after 2^32 arrivals: hours)
-  return s[0] != 0 && target < 0xffff0000u;
+}
+
+constexpr int SOLVE_WARPS = DIS_THREADS / 32;
+
+// The first round of a flood in k_solve: SOLVE_WARPS tiles of the selection at a time, a warp
+// per tile.  The tiles among them that changed since their masks were written are rebuilt
+// first: up to REB_SPLIT by the whole CTA, one after another with the next one's loads in
+// flight (5 vector loads a thread and tile, one trip to L2), more by a warp each (a chain of
+// trips, but all tiles at once).  Over 48 tiles, one per CTA, the round takes 6.7 us against
+// 9.2 with a warp per tile; over 4096 tiles with three to five changed ones per CTA the whole
+// CTA took 26 us where the warps take 18.
+// sm: SOLVE_WARPS x REB_WORDS (6 x 32 words of masks, 2 x 8 half sums).
+constexpr int REB_WORDS = 6 * 32 + 2 * SOLVE_WARPS;
+constexpr int REB_SPLIT = 2;
+
+__device__ __forceinline__ void flood_first_phase(const PoolView& P, const SolveArgs& A,
+                                                  SolveState& st, uint32_t* sm) {
+  __shared__ int s_dt[2][SOLVE_WARPS];
+  const unsigned FULL = 0xffffffffu;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int bid = blockIdx.x, nb_ctas = gridDim.x, n = A.tiles;
+  const int stamp = st.stamp, prev = st.prev, cyc = st.cyc;
+  int32_t* const hits = &P.ctl[CTL_H0 + stamp % 3];
+  const Worklist out{(st.fk & 1) ? P.fq[0] : P.fq[1], &P.ctl[CTL_F0 + (st.fk + 1) % 3],
+                     (st.fk & 1) ? P.mark[0] : P.mark[1], &st.push};
+  const int i0 = warp * nb_ctas + bid;
+  SelCursor cursor(P, A.ranges, i0 < n ? i0 : 0, A.sel0);
+  FloodSum fs;
+  int par = 0;
+  for (int b = 0; b < n; b += SOLVE_WARPS * nb_ctas, par ^= 1) {   // the same for every warp
+    const int i = b + i0;
+    int t = -1, img = 0, dirty = 0;
+    int4 nb = make_int4(-1, -1, -1, -1);
+    TileMasks m{0u, 0u, 0u, 0u, 0u, 0u};
+    long long ps = 0;
+    if (i < n) {
+      t = cursor.tile(i);
+      img = cursor.image();
+      if ((unsigned)img >= (unsigned)P.nimg || (unsigned)t >= (unsigned)P.nt) {   // self-check
+        if (lane == 0) record_bad(P, 4, img);
+        t = -1;
+      } else {
+        // all loads before the first decision
+        const int hit = *((volatile int32_t*)&P.img_hit[img]);
+        const int mode = A.ranges == 1 ? A.mode0 : P.sel_mode[cursor.range()];
+        dirty = P.mdirty[t];
+        nb = P.nbr[t];
+        m = load_masks(P, t, lane);
+        ps = P.tpos[t];
+        const bool part = cyc == 0 ? mode == 2
+                                   : (hit == stamp || (prev > 0 && hit == prev) || (cyc == 1 && mode == 1));
+        if (!part) t = -1;
+      }
+    }
+    if (t < 0) dirty = 0;
+    if (lane == 0) s_dt[par][warp] = dirty ? t : -1;
+    const int ndirty = __syncthreads_count(dirty && lane == 0);
+    if (ndirty > REB_SPLIT) {
+      if (dirty) {
+        const RowMasks rm = warp_rebuild_masks(P, t, lane, &ps);
+        m = TileMasks{rm.up, rm.down, rm.left, rm.right, rm.sink, rm.exc};
+      }
+    } else if (ndirty > 0) {
+      // rebuild: thread (r, q) reads pixels (r, 4q .. 4q+3); this warp makes rows 4 warp .. + 3
+      const int dt = s_dt[par][lane & (SOLVE_WARPS - 1)];
+      unsigned todo = __ballot_sync(FULL, dt >= 0) & ((1u << SOLVE_WARPS) - 1u);
+      int4 v[5];
+      auto load = [&](int td) {
+        const long long o = (long long)td * GC_TILE_PX + tid * 4;
+        v[0] = *(const int4*)(P.cap[DUP] + o);
+        v[1] = *(const int4*)(P.cap[DDOWN] + o);
+        v[2] = *(const int4*)(P.cap[DLEFT] + o);
+        v[3] = *(const int4*)(P.cap[DRIGHT] + o);
+        v[4] = *(const int4*)(P.exc + o);
+      };
+      load(__shfl_sync(FULL, dt, __ffs(todo) - 1));
+      while (todo) {
+        const int w = __ffs(todo) - 1;
+        const int td = __shfl_sync(FULL, dt, w);
+        todo &= todo - 1;
+        uint32_t k[6];
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+          k[p] = warp_row_mask(__ballot_sync(FULL, v[p].x > 0), __ballot_sync(FULL, v[p].y > 0),
+                               __ballot_sync(FULL, v[p].z > 0), __ballot_sync(FULL, v[p].w > 0), lane & 3);
+        k[4] = warp_row_mask(__ballot_sync(FULL, v[4].x < 0), __ballot_sync(FULL, v[4].y < 0),
+                             __ballot_sync(FULL, v[4].z < 0), __ballot_sync(FULL, v[4].w < 0), lane & 3);
+        k[5] = warp_row_mask(__ballot_sync(FULL, v[4].x > 0), __ballot_sync(FULL, v[4].y > 0),
+                             __ballot_sync(FULL, v[4].z > 0), __ballot_sync(FULL, v[4].w > 0), lane & 3);
+        // sum of the positive excess, in halves that fit 32 bits over a warp's 128 pixels
+        const unsigned e0 = v[4].x > 0 ? v[4].x : 0, e1 = v[4].y > 0 ? v[4].y : 0;
+        const unsigned e2 = v[4].z > 0 ? v[4].z : 0, e3 = v[4].w > 0 ? v[4].w : 0;
+        const unsigned lo = (e0 & 0xffffu) + (e1 & 0xffffu) + (e2 & 0xffffu) + (e3 & 0xffffu);
+        const unsigned hi = (e0 >> 16) + (e1 >> 16) + (e2 >> 16) + (e3 >> 16);
+        if (todo) load(__shfl_sync(FULL, dt, __ffs(todo) - 1));   // the next tile's, in flight
+        const unsigned slo = __reduce_add_sync(FULL, lo), shi = __reduce_add_sync(FULL, hi);
+        uint32_t* const sw = sm + w * REB_WORDS;
+        if (lane < 4) {
+          const int row = 4 * warp + lane;
+          uint32_t* const mc = P.mcan + (long long)td * 128;
+#pragma unroll
+          for (int p = 0; p < 4; ++p) {
+            mc[32 * p + row] = k[p];
+            sw[32 * p + row] = k[p];
+          }
+          P.msink[(long long)td * 32 + row] = k[4];
+          P.mexc[(long long)td * 32 + row] = k[5];
+          sw[128 + row] = k[4];
+          sw[160 + row] = k[5];
+        }
+        if (lane == 0) {
+          sw[192 + 2 * warp] = slo;
+          sw[193 + 2 * warp] = shi;
+        }
+      }
+      __syncthreads();
+      if (dirty) {
+        const uint32_t* const sw = sm + warp * REB_WORDS;
+        m = TileMasks{sw[lane], sw[32 + lane], sw[64 + lane], sw[96 + lane], sw[128 + lane], sw[160 + lane]};
+        ps = 0;
+#pragma unroll
+        for (int w = 0; w < SOLVE_WARPS; ++w)
+          ps += (long long)sw[192 + 2 * w] + ((long long)sw[193 + 2 * w] << 16);
+        if (lane == 0) {
+          P.tpos[t] = ps;
+          P.mdirty[t] = 0;
+        }
+      }
+    }
+    if (t < 0) continue;
+    if (lane == 0 && ps) fs.add(A.acc, img, ps);   // taken with the tile's masks
+    flood_fill(P, t, nb, lane, img, stamp, m, m.exc, 0, hits, out);
+  }
+  flood_sum_flush<SOLVE_WARPS>(A.acc, fs);
 }
 
 // The solve over the selection (see Pool::solve_images): images that continue from a previous
@@ -1973,8 +2266,6 @@ __device__ __forceinline__ bool grid_sync(const PoolView& P, GridBar& B, volatil
 // in the solve; an image whose flood reached a sink carries that stamp in img_hit, which
 // selects it for the relabel and for the next flood.
 //
-// 4 CTAs of 256 threads per SM (k_discharge's shape: registers and shared memory bound it);
-// the relabel's staging shares the discharge's shared memory.
 // Cap of the relabel's distances.  Excess moves at most pulses x iters pixels a cycle, so
 // only excess near a sink matters to a cycle; distances beyond the cap are not computed, and
 // pixels there stay inactive.  Exact distances would be the chain of tile rounds across every
@@ -1982,181 +2273,132 @@ __device__ __forceinline__ bool grid_sync(const PoolView& P, GridBar& B, volatil
 // 4096^2), with all its tiles discharged.  The labels stay valid: below the cap they are
 // exact, and at or above it "not below".  The cap doubles with every cycle, and at once when no
 // excess lies within it, so the schedule ends in exact relabels and terminates as they do.
-constexpr int SOLVE_WARPS = DIS_THREADS / 32;
+//
+// 3 CTAs of 256 threads per SM (see discharge_phase); the relabel's and the flood's staging
+// share the discharge's shared memory.
 constexpr size_t SOLVE_BFS_SMEM = (size_t)SOLVE_WARPS * 32 * 33 * sizeof(int32_t);
 constexpr size_t SOLVE_DYN_SMEM = DIS_DYN_SMEM > SOLVE_BFS_SMEM ? DIS_DYN_SMEM : SOLVE_BFS_SMEM;
+static_assert(SOLVE_WARPS * REB_WORDS * sizeof(uint32_t) <= SOLVE_DYN_SMEM, "rebuild staging");
 
 __global__ void __launch_bounds__(DIS_THREADS, 3)
 k_solve(PoolView P, SolveArgs A) {
   extern __shared__ __align__(128) int32_t dsm[];
   __shared__ uint64_t mbar;
-  __shared__ int32_t s_bc[4];
-  __shared__ int s_push;   // tiles this CTA has queued since the last barrier
+  __shared__ SolveState st;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int bid = blockIdx.x, nb = gridDim.x;
-  GridBar bar;
   unsigned phase = 0;     // of mbar
-  int qk = 0, fk = 0;     // steps of the worklist and of the frontier (counter slots mod 3)
-  int stamp = 0, cycles = 0, err = 0;
-  int nrounds_f = 0, nrounds_b = 0, npulses = 0;
-  int cap = A.cap, hlim = GC_HINF;   // of the last relabel (none yet: trivial labels)
-  int v0, v1 = 0;
-  // ---- prologue: control words, image modes and flow sums
+  // ---- prologue: no reset and no barrier (the solve before left counters and sums at zero, and
+  // stamps of another solve equal none of this one's)
   trace_mark(P, TR_BEGIN);
   if (tid == 0) {
-    s_push = 0;
+    st = SolveState{};
+    st.cap = A.cap;
+    st.hlim = kFirstLimit;    // no relabel yet: trivial labels
+    st.stamp = A.stamp0;
+    st.step = ST_LIST;
+    if (A.warm) {
+      st.step = ST_FLOOD_FIRST;
+      ++st.stamp;
+    } else if (nb >= A.tiles) {
+      // a tile per CTA: the first list needs no step of its own.  It has one entry per CTA, and
+      // to a CTA whose tile is not active it is empty.
+      if (bid == 0) trace_record(P, TR_ACTIVE_LIST);
+      begin_cycle(A, st, 0);
+      if (bid < A.tiles) {
+        SelCursor cursor(P, A.ranges, bid, A.sel0);
+        const int t = cursor.tile(bid);
+        if (fresh_tile_active(P, t)) {
+          P.queue[0][bid] = t;
+          st.n = bid + 1;
+        }
+      }
+    }
     mbar_init(&mbar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  const int nr = A.ranges, n_sel = A.tiles;
-  if (bid == 0) {
-    for (int i = tid; i < CTL_N; i += DIS_THREADS) P.ctl[i] = 0;
-    for (int i = tid; i < P.nimg; i += DIS_THREADS) {
-      P.img_hit[i] = 0;
-      P.img_mode[i] = 0;
-    }
-    __syncthreads();
-    for (int k = tid; k < nr; k += DIS_THREADS) {
-      const int img = P.sel[k].w;
-      if ((unsigned)img >= (unsigned)P.nimg) { record_bad(P, 4, img); continue; }
-      P.img_mode[img] = P.sel_mode[k];
-      A.acc[img].sumpos_e = 0;   // the floods of this solve accumulate it
-    }
-  }
-  bool alive = grid_sync<true>(P, bar, s_bc, &s_push, v0);
+  __syncthreads();
 
-  for (int cyc = 0; alive; ++cyc) {
-    // cyc 0 is the part before the first pulses: the warm images' flood and relabel, and the
-    // fresh images' first list
-    if (cyc > 0) {
-      // ---- pulses: step qk reads counter qk, adds to qk + 1, clears qk + 2 (all mod 3)
-      const int pulses = cycle_pulses(A.pulses, cycles), iters = cycle_iters(A.iters, cycles);
-      for (int p = 0; p < pulses && alive && v0 > 0; ++p) {
-        trace_mark(P, TR_DISCHARGE);
-        const Worklist in{P.queue[qk & 1], nullptr, P.inq[qk & 1]};
-        Worklist out{P.queue[(qk + 1) & 1], &P.ctl[CTL_Q0 + (qk + 1) % 3], P.inq[(qk + 1) & 1], &s_push};
-        if (p == pulses - 1) out.list = nullptr;   // the relabel makes the next list
-        if (bid == 0 && tid == 0) P.ctl[CTL_Q0 + (qk + 2) % 3] = 0;
-        discharge_phase(P, iters, hlim, bid, nb, in, v0, out, dsm,
-                        *reinterpret_cast<DisSmem*>(dsm + DIS_PLANES * GC_TILE_PX), &mbar, phase);
-        ++qk;
-        ++npulses;
-        alive = grid_sync<true>(P, bar, s_bc, &s_push, v0);
+  for (int step = st.step; step != ST_END; step = st.step) {
+    if (step == ST_PULSE) {
+      // reads counter qk, adds to qk + 1, clears qk + 2 (all mod 3)
+      trace_mark(P, TR_DISCHARGE);
+      const int qk = st.qk;
+      const Worklist in{(qk & 1) ? P.queue[1] : P.queue[0], nullptr, (qk & 1) ? P.inq[1] : P.inq[0]};
+      Worklist out{(qk & 1) ? P.queue[0] : P.queue[1], &P.ctl[CTL_Q0 + (qk + 1) % 3],
+                   (qk & 1) ? P.inq[0] : P.inq[1], &st.push};
+      if (st.pulse == st.pulses - 1) out.list = nullptr;   // the relabel makes the next list
+      if (bid == 0 && tid == 0) P.ctl[CTL_Q0 + (qk + 2) % 3] = 0;
+      discharge_phase(P, st.iters, st.hlim, bid, nb, in, st.n, out, dsm,
+                      *reinterpret_cast<DisSmem*>(dsm + DIS_PLANES * GC_TILE_PX), &mbar, phase);
+    } else if (step == ST_FLOOD_FIRST) {
+      trace_mark(P, TR_FLOOD_FIRST);
+      if (bid == 0 && tid == 0) {
+        P.ctl[CTL_H0 + (st.stamp + 1) % 3] = 0;
+        P.ctl[CTL_F0 + (st.fk + 2) % 3] = 0;
       }
-      if (!alive) break;
-    }
-    int left = 0;
-    if (cyc > 0 || A.warm) {
-      // ---- flood, first round over the selection, then frontier rounds
-      const int prev = stamp++;
-      int32_t* const hits = &P.ctl[CTL_H0 + stamp % 3];
-      if (bid == 0 && tid == 0) P.ctl[CTL_H0 + (stamp + 1) % 3] = 0;
-      int n = n_sel, rounds = 0;
-      FloodSum fs;
-      for (bool first = true;; first = false) {
-        trace_mark(P, first ? TR_FLOOD_FIRST : TR_FLOOD);
-        const Worklist out{P.fq[(fk + 1) & 1], &P.ctl[CTL_F0 + (fk + 1) % 3], P.mark[(fk + 1) & 1], &s_push};
-        if (bid == 0 && tid == 0) P.ctl[CTL_F0 + (fk + 2) % 3] = 0;
-        const int i0 = warp * nb + bid;
-        SelCursor cursor(P, first ? nr : 0, i0 < n ? i0 : 0);
-        for (int i = i0; i < n; i += SOLVE_WARPS * nb) {
-          const int t = first ? cursor.tile(i) : P.fq[fk & 1][i];
-          if (!first && lane == 0) P.mark[fk & 1][t] = 0;
-          const int img = first ? cursor.image() : P.img_of[t];
-          if ((unsigned)img >= (unsigned)P.nimg || (unsigned)t >= (unsigned)P.nt) {   // self-check
-            if (lane == 0) record_bad(P, 4, img);
-            continue;
-          }
-          const int hit = *((volatile int32_t*)&P.img_hit[img]);
-          if (first) {
-            const int mode = P.img_mode[img];
-            const bool part = cyc == 0 ? mode == 2
-                                       : (hit == stamp || (prev > 0 && hit == prev) || (cyc == 1 && mode == 1));
-            if (!part) continue;
-          } else if (hit == stamp) {
-            continue;   // not solved: its flood is redone in a later cycle
-          }
-          flood_tile(P, t, lane, first, img, stamp, hits, out, A.acc, fs);
+      flood_first_phase(P, A, st, reinterpret_cast<uint32_t*>(dsm));
+    } else if (step == ST_FLOOD) {
+      trace_mark(P, TR_FLOOD);
+      const int fk = st.fk, stamp = st.stamp, n = st.n;
+      const Worklist out{(fk & 1) ? P.fq[0] : P.fq[1], &P.ctl[CTL_F0 + (fk + 1) % 3],
+                         (fk & 1) ? P.mark[0] : P.mark[1], &st.push};
+      const int32_t* const list = (fk & 1) ? P.fq[1] : P.fq[0];
+      int32_t* const mark = (fk & 1) ? P.mark[1] : P.mark[0];
+      if (bid == 0 && tid == 0) P.ctl[CTL_F0 + (fk + 2) % 3] = 0;
+      for (int i = warp * nb + bid; i < n; i += SOLVE_WARPS * nb) {
+        const int t = list[i];
+        const int img = P.img_of[t];
+        if (lane == 0) mark[t] = 0;
+        if ((unsigned)img >= (unsigned)P.nimg) {   // self-check
+          if (lane == 0) record_bad(P, 4, img);
+          continue;
         }
-        if (first) {
-          flood_sum_flush<SOLVE_WARPS>(A.acc, fs);
-          fs = FloodSum{};
-        }
-        ++fk;
-        ++rounds;
-        alive = grid_sync<false>(P, bar, s_bc, &s_push, v0, hits, &v1);
-        n = v0;
-        if (!alive || n == 0) break;
-        if (n < 0 || n > P.nt) { alive = false; break; }   // (never: frontier_push counts a tile once)
-        if (rounds >= A.max_rounds) { err = 1; break; }
+        // an image whose flood reached a sink is not solved: it is flooded again later
+        if (*((volatile int32_t*)&P.img_hit[img]) == stamp) continue;
+        flood_frontier_tile(P, t, lane, img, stamp, &P.ctl[CTL_H0 + stamp % 3], out);
       }
-      nrounds_f += rounds;
-      left = v1;   // images whose flood reached a sink
-      if (cyc > 0) ++cycles;
-      if (bid == 0 && tid == 0) trace_record(P, TR_CHECK);
-      if (!alive || err) break;
-      if (left == 0 && !(cyc == 0 && A.fresh)) break;   // solved
-      if (left > 0) {
-        // ---- global relabel of the images not solved; it lists their active tiles
-        if (bid == 0)   // their sums start afresh with their next flood
-          for (int i = tid; i < P.nimg; i += DIS_THREADS)
-            if (P.img_hit[i] == stamp) A.acc[i].sumpos_e = 0;
-        const Worklist act_out{P.queue[qk & 1], &P.ctl[CTL_Q0 + qk % 3], nullptr};
-        n = n_sel;
-        rounds = 0;
-        for (bool first = true;;) {
-          trace_mark(P, first ? TR_BFS_FIRST : TR_BFS);
-          const Worklist out{P.fq[(fk + 1) & 1], &P.ctl[CTL_F0 + (fk + 1) % 3], P.mark[(fk + 1) & 1], &s_push};
-          if (bid == 0 && tid == 0) P.ctl[CTL_F0 + (fk + 2) % 3] = 0;
-          const int i0 = warp * nb + bid;
-          SelCursor cursor(P, first ? nr : 0, i0 < n ? i0 : 0);
-          for (int i = i0; i < n; i += SOLVE_WARPS * nb) {
-            const int t = first ? cursor.tile(i) : P.fq[fk & 1][i];
-            if (first && P.img_hit[cursor.image()] != stamp) continue;
-            if (!first && lane == 0) P.mark[fk & 1][t] = 0;
-            const int act = bfs_tile(P, t, lane, first, cap, dsm + warp * (32 * 33), out);
-            if (lane == 0) {
-              // a tile becomes active once (its reached set only grows): list it then
-              if (act > 0 && (first || P.tact[t] == 0)) worklist_append(P, act_out, t);
-              if (first || act > 0) P.tact[t] = act;
-            }
-          }
-          ++fk;
-          ++rounds;
-          alive = grid_sync<true>(P, bar, s_bc, &s_push, v0, &P.ctl[CTL_Q0 + qk % 3], &v1);
-          n = v0;
-          first = false;
-          if (!alive) break;
-          if (n == 0) {
-            if (v1 > 0 || cap >= GC_HINF) break;
-            // no excess within the cap of a sink: relabel again, further out
-            cap = next_cap(cap);
-            n = n_sel;
-            first = true;
-            nrounds_b += rounds;
-            rounds = 0;
-            continue;
-          }
-          if (n < 0 || n > P.nt) { alive = false; break; }
-          if (rounds >= A.max_rounds) { err = 1; break; }
+    } else if (step == ST_BFS_FIRST || step == ST_BFS) {
+      // global relabel of the images not solved; it lists their active tiles
+      const int first = step == ST_BFS_FIRST;
+      trace_mark(P, first ? TR_BFS_FIRST : TR_BFS);
+      const int fk = st.fk, stamp = st.stamp, cap = st.cap, qk = st.qk;
+      const int n = first ? A.tiles : st.n;
+      if (first && bid == 0)   // their sums start afresh with their next flood
+        for (int i = tid; i < P.nimg; i += DIS_THREADS)
+          if (P.img_hit[i] == stamp) A.acc[i].sumpos_e = 0;
+      const Worklist act_out{(qk & 1) ? P.queue[1] : P.queue[0], &P.ctl[CTL_Q0 + qk % 3], nullptr};
+      const Worklist out{(fk & 1) ? P.fq[0] : P.fq[1], &P.ctl[CTL_F0 + (fk + 1) % 3],
+                         (fk & 1) ? P.mark[0] : P.mark[1], &st.push};
+      const int32_t* const list = (fk & 1) ? P.fq[1] : P.fq[0];
+      int32_t* const mark = (fk & 1) ? P.mark[1] : P.mark[0];
+      if (bid == 0 && tid == 0) P.ctl[CTL_F0 + (fk + 2) % 3] = 0;
+      const int i0 = warp * nb + bid;
+      SelCursor cursor(P, first ? A.ranges : 0, i0 < n ? i0 : 0, A.sel0);
+      for (int i = i0; i < n; i += SOLVE_WARPS * nb) {
+        const int t = first ? cursor.tile(i) : list[i];
+        if (first && P.img_hit[cursor.image()] != stamp) continue;
+        if (!first && lane == 0) mark[t] = 0;
+        const int act = bfs_tile(P, t, lane, first, cap, dsm + warp * (32 * 33), out);
+        if (lane == 0) {
+          // a tile becomes active once (its reached set only grows): list it then
+          if (act > 0 && (first || P.tact[t] == 0)) worklist_append(P, act_out, t);
+          if (first || act > 0) P.tact[t] = act;
         }
-        nrounds_b += rounds;
-        hlim = cap < GC_HINF ? cap + 1 : GC_HINF;
-        cap = next_cap(cap);   // further out with every cycle
-        if (!alive || err) break;
       }
-    }
-    if (cyc == 0 && A.fresh) {
-      // ---- the fresh images' first list
+    } else if (step == ST_LIST) {
+      // the fresh images' first list
       trace_mark(P, TR_ACTIVE_LIST);
-      const Worklist act_out{P.queue[qk & 1], &P.ctl[CTL_Q0 + qk % 3], nullptr};
+      const int qk = st.qk;
+      const Worklist act_out{(qk & 1) ? P.queue[1] : P.queue[0], &P.ctl[CTL_Q0 + qk % 3], nullptr};
       const int i0 = bid * DIS_THREADS + tid;
-      SelCursor cursor(P, nr, i0 < n_sel ? i0 : 0);
-      for (int b = bid * DIS_THREADS; b < n_sel; b += nb * DIS_THREADS) {   // CTA-uniform
+      SelCursor cursor(P, A.ranges, i0 < A.tiles ? i0 : 0, A.sel0);
+      for (int b = bid * DIS_THREADS; b < A.tiles; b += nb * DIS_THREADS) {   // CTA-uniform
         int t = -1;
-        if (b + tid < n_sel) {
+        if (b + tid < A.tiles) {
           t = cursor.tile(b + tid);
-          if (P.img_mode[cursor.image()] != 1 || !fresh_tile_active(P, t)) t = -1;
+          const int mode = A.ranges == 1 ? A.mode0 : P.sel_mode[cursor.range()];
+          if (mode != 1 || !fresh_tile_active(P, t)) t = -1;
         }
         const unsigned m = __ballot_sync(0xffffffffu, t >= 0);
         if (m == 0) continue;
@@ -2168,37 +2410,44 @@ k_solve(PoolView P, SolveArgs A) {
           else record_bad(P, 1, pos);
         }
       }
-      alive = grid_sync<true>(P, bar, s_bc, &s_push, v0, &P.ctl[CTL_Q0 + qk % 3], &v1, true);
     }
-    v0 = v1;   // the worklist's length
-    // (an empty first list still needs the flood: no fresh tile is near a sink)
-    if (!alive || (v0 == 0 && !(cyc == 0 && A.fresh))) break;
-    if (cycles >= A.max_cycles) { err = 2; break; }
+    solve_barrier(P, A, st);
   }
 
   // ---- results: control words and sums to the host, labels of a one-image handle
   if (bid == 0) {
     if (tid == 0) {
       volatile int32_t* ctl = P.ctl;
-      if (err || !alive) atomicCAS(&P.ctl[CTL_ERR], 0, err ? err : 5);
-      ctl[CTL_BFS_TOTAL] = nrounds_b;
-      ctl[CTL_FLOOD_TOTAL] = nrounds_f;
-      ctl[CTL_CYCLES] = cycles;
+      if (st.err) atomicCAS(&P.ctl[CTL_ERR], 0, st.err);
+      ctl[CTL_BFS_TOTAL] = st.nb;
+      ctl[CTL_FLOOD_TOTAL] = st.nf;
+      ctl[CTL_CYCLES] = st.cycles;
       ctl[CTL_NACT] = A.fresh ? 1 : 0;
-      ctl[CTL_PULSE] = npulses;
+      ctl[CTL_PULSE] = st.np;
       trace_record(P, TR_END);
     }
     __syncthreads();
     publish_results(P, A.acc);
+    if (A.clean) {   // the images' sums start the next solve at zero
+      __syncthreads();
+      for (int k = tid; k < A.ranges; k += DIS_THREADS) {
+        const int img = P.sel[k].w;
+        if ((unsigned)img < (unsigned)P.nimg) A.acc[img].sumpos_e = 0;
+      }
+    }
   }
-  if (A.lmode && alive && !err) {
+  if (A.lmode && !st.err) {
     trace_mark(P, TR_LABELS);
     const long long i0 = (long long)bid * DIS_THREADS + tid, step = (long long)nb * DIS_THREADS;
     if (A.lmode == 2) write_labels_packed(P, A.im, A.labels, i0, step);
     else write_labels(P, A.im, A.labels, i0, step);
   }
-  // the last CTA to leave clears the barrier for the next launch
+  // the last CTA to leave clears the counters and the barrier for the next launch
+  __syncthreads();
+  if (tid == 0) __threadfence();
   if (tid == 0 && atomicAdd(P.bar + BAR_EXIT, 1ull) == (unsigned long long)nb - 1) {
+    if (A.clean)
+      for (int k = CTL_Q0; k < CTL_H0 + 3; ++k) P.ctl[k] = 0;
     P.bar[BAR_EXIT] = 0;
     P.bar[BAR_ARRIVE] = 0;
     P.bar[BAR_ARRIVE + BAR_STRIDE] = 0;

@@ -67,3 +67,37 @@ def test_fresh_and_warm_images_far_apart(cuda, oracle, graph):
         assert pool.flow(k) == f_ref, k
         assert np.array_equal(pool.labels(k).cpu().numpy(), l_ref), k
     pool.close_pool()
+
+
+@pytest.mark.parametrize("w,h", [(32, 32), (1184, 384), (2848, 160), (1184, 385)])
+def test_one_tile_per_cta_and_more(cuda, oracle, w, h):
+    """The first pulse without a list (no more tiles than resident CTAs: up to 444 on a B200)
+    and with one: 1, 444, 445 and 481 tiles."""
+    g = synth.random_graph(w, h, w + h, cap_max=40, tlink_max=60)
+    f_ref, l_ref = oracle.maxflow_bk(*g.planes())
+    with GraphCut(w, h) as gc:
+        gc.upload_capacities(*g.planes())
+        lab = gc.cut_labels().cpu().numpy()
+        assert gc.flow == f_ref
+        assert np.array_equal(lab, l_ref)
+
+
+def test_solves_of_both_kinds_and_steps_alternate(cuda, oracle):
+    """One handle solved by one launch, by the host-driven loop (profiling on) and stepped by
+    hand in turn, fresh and warm: each solve starts from what another kind left."""
+    g = synth.make_graph(300, 200, 4)
+    f_ref, l_ref = oracle.maxflow_bk(*g.planes())
+    with GraphCut(g.width, g.height) as gc:
+        for k in range(6):
+            gc.upload_capacities(*g.planes())
+            if k % 3 == 2:
+                gc.push()
+                gc.push()
+            for prof in ((True, False), (False, True))[k % 2]:
+                gc.set_profile(prof)
+                gc.edit_tlinks(np.array([5, 77]), np.array([1000, -1000]))
+                gc.cut()
+                gc.edit_tlinks(np.array([5, 77]), g.excess.reshape(-1)[[5, 77]])
+                gc.cut()
+                assert gc.flow == f_ref, (k, prof)
+                assert np.array_equal(gc.labels().cpu().numpy(), l_ref), (k, prof)
