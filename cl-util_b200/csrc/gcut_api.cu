@@ -577,9 +577,9 @@ struct Pool {
     return GC_OK;
   }
 
-  int compact(const int32_t* flags, int32_t* clear, cudaStream_t s) {
+  int compact(const int32_t* flags, cudaStream_t s) {
     return timed(K_COMPACT, s, [&] {
-      return launch_scan(GC_SCAN_MODE_COMPACT, flags, nullptr, clear, nullptr, list, counts, nt,
+      return launch_scan(GC_SCAN_MODE_COMPACT, flags, nullptr, nullptr, list, counts, nt,
                          0, 0, 0, 0, 0, scan.st, s);
     });
   }
@@ -828,7 +828,7 @@ struct Pool {
   int step_push(cudaStream_t s) {
     if (!uploaded) return fail(GC_ERR_STATE, "push before upload");
     if (!list_valid) {
-      RK(compact(P.tact, nullptr, s));
+      RK(compact(P.tact, s));
       RK(launch_ctl_cycle(P, s));
       list_valid = true;
     }
@@ -857,7 +857,7 @@ struct Pool {
     RK(select_all(&warm, s));
     RK(launch_ctl_begin(P, opts.max_bfs_rounds, acc, s));
     RK(global_relabel(s));
-    RK(compact(P.tact, nullptr, s));
+    RK(compact(P.tact, s));
     RK(launch_ctl_cycle(P, s));
     list_valid = true;
     bfs_fresh = true;
@@ -971,23 +971,21 @@ struct gcp_handle {
 // passed as NULL selects one shared state per device.
 //
 // The device error word is sticky: a launch that gives up a look-back wait (or whose scatter
-// index is out of range) sets it and it stays set until the host reports it.  After each
-// launch the word is copied into pinned host memory on the caller's stream; the next call on
-// the state returns GC_ERR_INTERNAL once that copy has landed with a non-zero word, and
-// gc_scan_state_error reads it synchronously.
+// index is out of range) sets it and it stays set until the host reports it.  The kernel that
+// sets it writes it to pinned host memory as well, so a call needs no copy and no event of its
+// own (which took longer than the launch): the next call on the state returns GC_ERR_INTERNAL
+// once the word has arrived, and gc_scan_state_error reads the device word synchronously.
 // ------------------------------------------------------------------------------------
 struct gc_scan_state {
   int device = 0;
   ScanBuffers buf;
-  int32_t* h_err = nullptr;     // pinned mirror of the device error word
-  cudaEvent_t ev = nullptr;     // the last mirror copy
-  bool pending = false;
+  int32_t* h_err = nullptr;     // pinned copy of the device error word, written by the kernels
   std::mutex mu;                // one call at a time on a state
   ~gc_scan_state() {
     int cur = 0;
     cudaGetDevice(&cur);
     cudaSetDevice(device);
-    if (ev) { cudaEventSynchronize(ev); cudaEventDestroy(ev); }
+    if (buf.st.status) cudaDeviceSynchronize();   // the state's launches have finished
     buf.release();
     if (h_err) cudaFreeHost(h_err);
     cudaSetDevice(cur);
@@ -1007,8 +1005,10 @@ int scan_state_init(gc_scan_state* S, int device, int chunks) {
   e = cudaHostAlloc((void**)&S->h_err, sizeof(int32_t), cudaHostAllocPortable);
   if (e) { S->h_err = nullptr; cudaGetLastError(); return fail(GC_ERR_OOM, "pinned host allocation failed"); }
   *S->h_err = 0;
-  e = cudaEventCreateWithFlags(&S->ev, cudaEventDisableTiming);
-  if (e) { S->ev = nullptr; return cuda_fail(e, "event"); }
+  void* dptr = nullptr;
+  e = cudaHostGetDevicePointer(&dptr, S->h_err, 0);
+  if (e) return cuda_fail(e, "pinned host memory");
+  S->buf.st.host_err = static_cast<int32_t*>(dptr);
   return GC_OK;
 }
 
@@ -1040,27 +1040,18 @@ int resolve_scan_state(gc_scan_state* S, gc_scan_state** out) {
   return GC_OK;
 }
 
-// An error recorded by an earlier launch whose mirror copy has landed (no wait).
+// An error recorded by an earlier launch that has reached the host (no wait).
 int scan_state_take_error(gc_scan_state* S, cudaStream_t s) {
-  if (!S->pending || cudaEventQuery(S->ev) != cudaSuccess) { cudaGetLastError(); return GC_OK; }
-  S->pending = false;
-  if (*S->h_err == 0) return GC_OK;
-  const int code = *S->h_err;
-  *S->h_err = 0;
+  volatile int32_t* h = S->h_err;
+  const int code = *h;
+  if (code == 0) return GC_OK;
+  *h = 0;
   CK(cudaMemsetAsync(S->buf.st.err, 0, sizeof(int32_t), s));
   return fail(GC_ERR_INTERNAL, code == 1 ? "an earlier call on this scan state gave up a bounded look-back wait"
                                          : "an earlier call on this scan state computed an out-of-range index");
 }
 
-// After a launch: mirror the error word into pinned memory on the caller's stream.
-int scan_state_track(gc_scan_state* S, cudaStream_t s) {
-  CK(cudaMemcpyAsync(S->h_err, S->buf.st.err, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-  CK(cudaEventRecord(S->ev, s));
-  S->pending = true;
-  return GC_OK;
-}
-
-// Runs one primitive launch on a state: reports an earlier error, launches, mirrors.
+// Runs one primitive launch on a state: reports an earlier error, launches.
 template <class F>
 int with_scan_state(gc_scan_state* state, cudaStream_t s, F&& launch) {
   gc_scan_state* S = nullptr;
@@ -1069,7 +1060,7 @@ int with_scan_state(gc_scan_state* state, cudaStream_t s, F&& launch) {
   RK(scan_state_take_error(S, s));
   const int r = launch(S->buf.st);
   if (r) return r == GC_ERR_INVALID ? fail(r, "input larger than the scan state holds") : fail(r, "launch failed");
-  return scan_state_track(S, s);
+  return GC_OK;
 }
 }  // namespace
 
@@ -1501,7 +1492,6 @@ int gc_scan_state_error(gc_scan_state* state, int* err, void* stream) {
   CK(cudaMemcpyAsync(S->h_err, S->buf.st.err, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
   *err = *S->h_err;
-  S->pending = false;
   if (*err) {
     *S->h_err = 0;
     CK(cudaMemsetAsync(S->buf.st.err, 0, sizeof(int32_t), s));
@@ -1521,7 +1511,7 @@ int gc_scan_state_selftest(gc_scan_state* state, int spins, int* err, void* stre
     st.spin_limit = spins;
     const int r = launch_lookback_selftest(st, (cudaStream_t)stream);
     if (r) return fail(r, "self-test launch failed");
-    if (!err) return scan_state_track(S, (cudaStream_t)stream);   // reported like any error
+    if (!err) return GC_OK;   // reported like any error
   }
   return gc_scan_state_error(S, err, stream);
 }
@@ -1532,7 +1522,7 @@ int gc_scan_exclusive(gc_scan_state* state, const int32_t* in, int32_t* out, int
   if (n < 0 || (n > 0 && (!in || !out)) || !total) return fail(GC_ERR_INVALID, "bad argument");
   cudaStream_t s = (cudaStream_t)stream;
   return with_scan_state(state, s, [&](const ScanState& st) {
-    return launch_scan(GC_SCAN_MODE_SCAN, in, nullptr, nullptr, out, nullptr, total, n, 0, 0, 0,
+    return launch_scan(GC_SCAN_MODE_SCAN, in, nullptr, out, nullptr, total, n, 0, 0, 0,
                        0, 0, st, s);
   });
 }
@@ -1544,7 +1534,7 @@ int gc_compact(gc_scan_state* state, const int32_t* flags, int32_t* list, int32_
   if (n > 0 && flags == list) return fail(GC_ERR_INVALID, "list must not alias flags");
   cudaStream_t s = (cudaStream_t)stream;
   return with_scan_state(state, s, [&](const ScanState& st) {
-    return launch_scan(GC_SCAN_MODE_COMPACT, flags, nullptr, nullptr, nullptr, list, length, n, 0,
+    return launch_scan(GC_SCAN_MODE_COMPACT, flags, nullptr, nullptr, list, length, n, 0,
                        0, 0, 0, 0, st, s);
   });
 }
@@ -1556,7 +1546,7 @@ int gc_tiles_build(gc_scan_state* state, const int32_t* tiles, int op, int32_t o
     return fail(GC_ERR_INVALID, "bad argument");
   cudaStream_t s = (cudaStream_t)stream;
   return with_scan_state(state, s, [&](const ScanState& st) {
-    return launch_scan(GC_SCAN_MODE_FLAG, tiles, nullptr, nullptr, nullptr, list, length, n, op,
+    return launch_scan(GC_SCAN_MODE_FLAG, tiles, nullptr, nullptr, list, length, n, op,
                        operand, 0, 0, 0, st, s);
   });
 }
@@ -1570,7 +1560,7 @@ int gc_tiles_build_logical(gc_scan_state* state, const int32_t* tiles, const int
     return fail(GC_ERR_INVALID, "bad argument");
   cudaStream_t s = (cudaStream_t)stream;
   return with_scan_state(state, s, [&](const ScanState& st) {
-    return launch_scan(GC_SCAN_MODE_LOGICAL, tiles, tiles2, nullptr, nullptr, list, length, n,
+    return launch_scan(GC_SCAN_MODE_LOGICAL, tiles, tiles2, nullptr, list, length, n,
                        op1, a1, op2, a2, logical, st, s);
   });
 }
@@ -1581,7 +1571,7 @@ int gc_tiles_incorporate(int32_t* tiles, const int32_t* tiles2, int op1, int32_t
   if (n < 0 || (n > 0 && (!tiles || !tiles2)) || op1 < 0 || op1 > 4 || op2 < 0 || op2 > 4 ||
       logical < 0 || logical > 1)
     return fail(GC_ERR_INVALID, "bad argument");
-  return launch_increment_logical(tiles, tiles2, tiles, n, op1, op2, a1, a2, logical, iteration,
+  return launch_increment_logical(tiles, tiles2, n, op1, op2, a1, a2, logical, iteration,
                                   (cudaStream_t)stream);
 }
 

@@ -206,8 +206,19 @@ struct ScanState {
   uint32_t* seq;               // launch sequence tag (bumped by the last CTA)
   int32_t* err;                // set when a look-back wait gives up (sticky until read)
   int max_chunks;
+  int32_t* host_err;           // pinned copy of *err as the device sees it (null: none)
   int spin_limit;              // polls before a look-back wait gives up; 0: GC_SPIN_LIMIT
 };
+
+// Records an error on the state, in its pinned copy too (the host reads that at the next call
+// without a copy of its own).
+__device__ __forceinline__ void scan_error(const ScanState& st, int code) {
+  atomicExch(st.err, code);
+  if (st.host_err) {
+    *((volatile int32_t*)st.host_err) = code;
+    __threadfence_system();
+  }
+}
 
 enum ScanStateFlag : unsigned { SS_NONE = 0, SS_AGG = 1, SS_PREFIX = 2 };
 
@@ -224,49 +235,14 @@ __device__ __forceinline__ int spin_limit_of(const ScanState& st) {
   return st.spin_limit > 0 ? st.spin_limit : GC_SPIN_LIMIT;
 }
 
-// Called by one thread (thread 0) of the CTA owning chunk `chunk` after it knows its own
-// aggregate.  Publishes the aggregate, walks back over predecessors and returns the
-// exclusive prefix of the chunk.  Chunks are numbered by arrival ticket, so every
+// Executed by all 32 lanes of a warp of the CTA that owns chunk `chunk`, once it knows the
+// chunk's aggregate.  Publishes the aggregate (unless `published`), walks back over the
+// predecessors (each step inspects the status words of 32 of them at once) and returns the
+// exclusive prefix of the chunk to every lane.  Chunks are numbered by arrival ticket, so every
 // predecessor belongs to a CTA that is already running.
-__device__ __forceinline__ int32_t lookback_exclusive(const ScanState& st, uint32_t tag,
-                                                      int chunk, int32_t aggregate) {
-  volatile unsigned long long* status = st.status;
-  if (chunk == 0) {
-    __threadfence();
-    status[0] = ss_pack(tag, SS_PREFIX, aggregate);
-    return 0;
-  }
-  status[chunk] = ss_pack(tag, SS_AGG, aggregate);
-  __threadfence();
-  int32_t excl = 0;
-  int j = chunk - 1;
-  int spins = 0;
-  const int limit = spin_limit_of(st);
-  while (j >= 0) {
-    unsigned long long s = status[j];
-    uint32_t stag = (uint32_t)(s >> 34);
-    unsigned sst = (unsigned)((s >> 32) & 3u);
-    if (stag != (tag & 0x3fffffffu) || sst == SS_NONE) {
-      if (++spins > limit) {
-        atomicExch(st.err, 1);
-        break;
-      }
-      __nanosleep(32);
-      continue;
-    }
-    excl += (int32_t)(uint32_t)(s & 0xffffffffull);
-    if (sst == SS_PREFIX) break;
-    --j;
-  }
-  __threadfence();
-  status[chunk] = ss_pack(tag, SS_PREFIX, excl + aggregate);
-  return excl;
-}
-
-// Warp-parallel variant, executed by all 32 lanes of one warp: each step inspects the
-// status words of 32 predecessors at once.  Returns the exclusive prefix to every lane.
 __device__ __forceinline__ int32_t lookback_exclusive_warp(const ScanState& st, uint32_t tag,
-                                                           int chunk, int32_t aggregate) {
+                                                           int chunk, int32_t aggregate,
+                                                           bool published = false) {
   const int lane = threadIdx.x & 31;
   volatile unsigned long long* status = st.status;
   const uint32_t tg = tag & 0x3fffffffu;
@@ -274,7 +250,7 @@ __device__ __forceinline__ int32_t lookback_exclusive_warp(const ScanState& st, 
     if (lane == 0) { __threadfence(); status[0] = ss_pack(tag, SS_PREFIX, aggregate); }
     return 0;
   }
-  if (lane == 0) { status[chunk] = ss_pack(tag, SS_AGG, aggregate); __threadfence(); }
+  if (lane == 0 && !published) { status[chunk] = ss_pack(tag, SS_AGG, aggregate); __threadfence(); }
   __syncwarp();
   int32_t excl = 0;
   int j = chunk - 1;
@@ -308,7 +284,7 @@ __device__ __forceinline__ int32_t lookback_exclusive_warp(const ScanState& st, 
     j -= 32;
   }
   if (lane == 0) {
-    if (gave_up) atomicExch(st.err, 1);
+    if (gave_up) scan_error(st, 1);
     __threadfence();
     status[chunk] = ss_pack(tag, SS_PREFIX, excl + aggregate);
   }

@@ -20,16 +20,16 @@ enum ScanMode {
 int scan_chunks(int n);
 // Records the message returned by gc_last_error() for the calling thread; returns code.
 int set_last_error(int code, const char* msg);
-int launch_scan(int mode, const int32_t* in, const int32_t* in2, int32_t* clear,
-                int32_t* scan_out, int32_t* list_out, int32_t* total_out, int n, int op1,
+int launch_scan(int mode, const int32_t* in, const int32_t* in2, int32_t* scan_out,
+                int32_t* list_out, int32_t* total_out, int n, int op1,
                 int32_t a1, int op2, int32_t a2, int logical, const ScanState& st,
                 cudaStream_t s);
 // One warp waits on a look-back predecessor that never publishes, until st.spin_limit
 // polls run out (sets *st.err); needs st.max_chunks >= 2.
 int launch_lookback_selftest(const ScanState& st, cudaStream_t s);
-int launch_increment_logical(const int32_t* in1, const int32_t* in2, int32_t* out, int n,
-                             int op1, int op2, int32_t a1, int32_t a2, int logical,
-                             int32_t iteration, cudaStream_t s);
+int launch_increment_logical(int32_t* tiles, const int32_t* tiles2, int n, int op1, int op2,
+                             int32_t a1, int32_t a2, int logical, int32_t iteration,
+                             cudaStream_t s);
 int launch_fill(int32_t* p, int n, int32_t v, cudaStream_t s);
 int launch_tiles_view(const int32_t* tiles, int tiles_w, int tiles_h, int tile_w, int tile_h,
                       int32_t iteration, int width, int height, uint32_t* out, cudaStream_t s);

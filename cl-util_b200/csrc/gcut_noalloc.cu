@@ -81,7 +81,7 @@ extern "C" int gc_compact_noalloc(const int32_t* flags, int32_t* list, int32_t* 
   st.seq = reinterpret_cast<uint32_t*>(words + 3);
   st.status = static_cast<unsigned long long*>(base) + 2;
   st.max_chunks = kChunks;
-  const int rc = gcut::launch_scan(gcut::GC_SCAN_MODE_COMPACT, flags, nullptr, nullptr, nullptr,
+  const int rc = gcut::launch_scan(gcut::GC_SCAN_MODE_COMPACT, flags, nullptr, nullptr,
                                    list, length, n, 0, 0, 0, 0, 0, st, s);
   if (rc != GC_OK) return noalloc_fail(rc, "gc_compact_noalloc: kernel launch failed");
   return GC_OK;

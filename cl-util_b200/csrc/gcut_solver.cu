@@ -1117,7 +1117,7 @@ k_edge_relabel_build(PoolView P, int32_t* list, int32_t* count, ScanState st) {
       if (v0) list[pos++] = tb;
       if (v1) list[pos] = tb + 1;
     } else if (v) {
-      atomicExch(st.err, 2);   // only after a look-back that gave up
+      scan_error(st, 2);   // only after a look-back that gave up
     }
     if (chunk == nchunks - 1 && lane == 0) *count = excl + agg;
     if (lane == 0) scan_finish(st, nchunks);
@@ -1377,7 +1377,7 @@ k_active_list(PoolView P, ScanState st, int32_t* list, int32_t* count, int live,
     for (int k = 0; k < ACT_ITEMS; ++k) {
       if (!v[k]) continue;
       if ((unsigned)run < (unsigned)P.nt) list[run] = tl[k];
-      else atomicExch(st.err, 2);   // only after a look-back that gave up
+      else scan_error(st, 2);   // only after a look-back that gave up
       ++run;
     }
     if (chunk == nchunks - 1 && threadIdx.x == 0) *count = s_excl + agg;

@@ -337,7 +337,7 @@ const char* gc_last_error(void);
    scatter index) set the state's error word, which stays set until reported:
    - compactions (gc_compact, gc_tiles_build, gc_tiles_build_logical) then write length -1;
    - the next call on the state returns GC_ERR_INTERNAL once the word has reached the host
-     (it is copied back after every launch, on the caller's stream);
+     (the kernel that sets it writes it to pinned host memory as well);
    - gc_scan_state_error reads it synchronously. */
 typedef struct gc_scan_state gc_scan_state;
 /* A state for launches of up to max_items items on `device`.  No counterpart in the
