@@ -236,6 +236,19 @@ struct Pool {
     if (done_ev) cudaEventRecord(done_ev, s);
   }
 
+  // An edit returns before it has run (it used to wait for the copy of its points), so the next
+  // call that touches the planes waits for it on its own stream, whichever that is.
+  bool edit_pending = false;
+  int order(cudaStream_t s) {
+    if (!edit_pending) return GC_OK;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(s, &cap));
+    if (cap == cudaStreamCaptureStatusNone) CK(cudaStreamWaitEvent(s, done_ev, 0));
+    else CK(cudaEventSynchronize(done_ev));   // a capture cannot wait for an event outside it
+    edit_pending = false;
+    return GC_OK;
+  }
+
   void release() {
     if (done_ev) {
       if (!own_arena) cudaEventSynchronize(done_ev);
@@ -443,6 +456,7 @@ struct Pool {
     if (i < 0 || i >= (int)imgs.size()) return fail(GC_ERR_INVALID, "image index");
     if (!up || !down || !left || !right || !excess) return fail(GC_ERR_INVALID, "null plane");
     CK(cudaSetDevice(device));
+    RK(order(s));
     CK(cudaMemsetAsync(acc + i, 0, sizeof(ImageAcc), s));
     P.ktiles = nullptr;
     RK(timed(K_UPLOAD, s, [&] { return launch_upload(P, imgs[i], i, up, down, left, right, excess, tl, acc, s); }));
@@ -459,6 +473,7 @@ struct Pool {
     if (!rgba || !excess) return fail(GC_ERR_INVALID, "null plane");
     if (lambda < 0 || lambda > GC_NLINK_MAX_LAMBDA) return fail(GC_ERR_INVALID, "lambda out of range");
     CK(cudaSetDevice(device));
+    RK(order(s));
     const ImageDesc& im = imgs[i];
     if (lambda == 0) RK(launch_nlinks(rgba, im.W, im.H, dsum, ntab, acc + i, s));
     else CK(cudaMemsetAsync(acc + i, 0, sizeof(ImageAcc), s));
@@ -628,6 +643,7 @@ struct Pool {
       seen[i] = 1;
     }
     CK(cudaSetDevice(device));
+    RK(order(s));
     stats = gc_stats{};
     bool warm = false, fresh = false;
     RK(set_selection(idx, n, &warm, s, &fresh));
@@ -827,6 +843,7 @@ struct Pool {
   // manual stepping (gc_push / gc_relabel / gc_start_bfs / gc_is_completed)
   int step_push(cudaStream_t s) {
     if (!uploaded) return fail(GC_ERR_STATE, "push before upload");
+    RK(order(s));
     if (!list_valid) {
       RK(compact(P.tact, s));
       RK(launch_ctl_cycle(P, s));
@@ -841,6 +858,7 @@ struct Pool {
   }
   int step_relabel(cudaStream_t s) {
     if (!uploaded) return fail(GC_ERR_STATE, "relabel before upload");
+    RK(order(s));
     solved = false;
     lists_stale = true;
     bfs_fresh = false;
@@ -852,6 +870,7 @@ struct Pool {
   }
   int step_start_bfs(cudaStream_t s) {
     if (!uploaded) return fail(GC_ERR_STATE, "startBfs before upload");
+    RK(order(s));
     lists_stale = true;
     bool warm;
     RK(select_all(&warm, s));
@@ -865,6 +884,7 @@ struct Pool {
   }
   int step_is_completed(int* done, cudaStream_t s) {
     if (!bfs_fresh) return fail(GC_ERR_STATE, "isCompleted is valid right after startBfs");
+    RK(order(s));
     int n;
     RK(read_count(s, &n));
     *done = n == 0;
@@ -1308,9 +1328,33 @@ int gc_edit_tlinks(gc_handle* h, const int32_t* idx, const int32_t* value, int n
   Pool& p = h->pool;
   if (!p.uploaded) return fail(GC_ERR_STATE, "edit before upload");
   CK(cudaSetDevice(p.device));
+  RK(p.order((cudaStream_t)stream));
   RK(launch_edit(p.P, p.imgs[0], 0, idx, value, n, p.tl, p.acc, (cudaStream_t)stream));
   p.track((cudaStream_t)stream);
   p.edited_image(0);
+  return GC_OK;
+}
+
+// Rasterises an edit's polyline (brush: the reference brush's pixel set) into image img.
+// Short polylines travel in the launch; longer ones are copied, and the call waits for the copy
+// out of its own memory.
+static int pool_edit(Pool& p, int img, const int32_t* xs, const int32_t* ys, int npts, int radius,
+                     int32_t value, bool brush, cudaStream_t s) {
+  CK(cudaSetDevice(p.device));
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  CK(cudaStreamIsCapturing(s, &cap));
+  if (cap != cudaStreamCaptureStatusNone) return fail(GC_ERR_CUDA, "an edit cannot be captured");
+  RK(p.order(s));
+  std::vector<int32_t> pts(2 * (size_t)npts);
+  for (int k = 0; k < npts; ++k) { pts[2 * k] = xs[k]; pts[2 * k + 1] = ys[k]; }
+  const bool copy = !edit_points_inline(npts);
+  if (copy) CK(cudaMemcpyAsync(p.pts, pts.data(), pts.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
+  if (brush) RK(launch_brush(p.P, p.imgs[img], img, p.pts, pts.data(), npts, radius, value, p.tl, p.acc, s));
+  else RK(launch_stroke(p.P, p.imgs[img], img, p.pts, pts.data(), npts, radius, value, p.tl, p.acc, s));
+  p.track(s);
+  if (copy) CK(cudaStreamSynchronize(s));
+  else p.edit_pending = true;
+  p.edited_image(img);
   return GC_OK;
 }
 
@@ -1319,18 +1363,8 @@ int gc_edit_stroke(gc_handle* h, const int32_t* xs, const int32_t* ys, int npts,
   g_err.clear();
   if (!h || !xs || !ys || npts < 1 || npts > 1024 || radius < 0 || radius > 4096)
     return fail(GC_ERR_INVALID, "bad stroke");
-  Pool& p = h->pool;
-  if (!p.uploaded) return fail(GC_ERR_STATE, "edit before upload");
-  CK(cudaSetDevice(p.device));
-  std::vector<int32_t> pts(2 * npts);
-  for (int k = 0; k < npts; ++k) { pts[2 * k] = xs[k]; pts[2 * k + 1] = ys[k]; }
-  cudaStream_t s = (cudaStream_t)stream;
-  CK(cudaMemcpyAsync(p.pts, pts.data(), pts.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
-  RK(launch_stroke(p.P, p.imgs[0], 0, p.pts, pts.data(), npts, radius, value, p.tl, p.acc, s));
-  p.track(s);
-  CK(cudaStreamSynchronize(s));  // pts (host vector) must outlive the copy
-  p.edited_image(0);
-  return GC_OK;
+  if (!h->pool.uploaded) return fail(GC_ERR_STATE, "edit before upload");
+  return pool_edit(h->pool, 0, xs, ys, npts, radius, value, false, (cudaStream_t)stream);
 }
 
 int gc_edit_brush(gc_handle* h, const int32_t* xs, const int32_t* ys, int npts, int radius,
@@ -1338,18 +1372,8 @@ int gc_edit_brush(gc_handle* h, const int32_t* xs, const int32_t* ys, int npts, 
   g_err.clear();
   if (!h || !xs || !ys || npts < 1 || npts > 1024 || radius > 1024)
     return fail(GC_ERR_INVALID, "bad brush stroke");
-  Pool& p = h->pool;
-  if (!p.uploaded) return fail(GC_ERR_STATE, "edit before upload");
-  CK(cudaSetDevice(p.device));
-  std::vector<int32_t> pts(2 * npts);
-  for (int k = 0; k < npts; ++k) { pts[2 * k] = xs[k]; pts[2 * k + 1] = ys[k]; }
-  cudaStream_t s = (cudaStream_t)stream;
-  CK(cudaMemcpyAsync(p.pts, pts.data(), pts.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
-  RK(launch_brush(p.P, p.imgs[0], 0, p.pts, pts.data(), npts, radius, value, p.tl, p.acc, s));
-  p.track(s);
-  CK(cudaStreamSynchronize(s));  // pts (host vector) must outlive the copy
-  p.edited_image(0);
-  return GC_OK;
+  if (!h->pool.uploaded) return fail(GC_ERR_STATE, "edit before upload");
+  return pool_edit(h->pool, 0, xs, ys, npts, radius, value, true, (cudaStream_t)stream);
 }
 
 int gc_download_state(gc_handle* h, int32_t* excess, int32_t* height, int32_t* up,
@@ -1359,6 +1383,7 @@ int gc_download_state(gc_handle* h, int32_t* excess, int32_t* height, int32_t* u
   Pool& p = h->pool;
   CK(cudaSetDevice(p.device));
   cudaStream_t s = (cudaStream_t)stream;
+  RK(p.order(s));
   const int32_t* planes[6] = {p.P.exc, p.P.hgt, p.P.cap[0], p.P.cap[1], p.P.cap[2], p.P.cap[3]};
   int32_t* outs[6] = {excess, height, up, down, left, right};
   for (int k = 0; k < 6; ++k)
@@ -1746,6 +1771,7 @@ int gcp_open(gcp_handle* p, int slot, int width, int height, int tile0, void* st
     if (tile0 < a1 && a0 < tile0 + tiles) return fail(GC_ERR_INVALID, "tile range overlaps an open slot");
   }
   CK(cudaSetDevice(pool.device));
+  RK(pool.order((cudaStream_t)stream));
   pool.imgs[slot] = d;
   RK(launch_image_tiles(pool.P, d, slot, (cudaStream_t)stream));
   pool.img_up[slot] = pool.img_solved[slot] = pool.img_edited[slot] = 0;
@@ -1787,21 +1813,8 @@ static int gcp_edit(gcp_handle* p, int slot, const int32_t* xs, const int32_t* y
   if (!xs || !ys || npts < 1 || npts > 1024 || radius > (brush ? 1024 : 4096) ||
       (!brush && radius < 0))
     return fail(GC_ERR_INVALID, "bad stroke");
-  Pool& pool = p->pool;
-  if (!pool.img_up[slot]) return fail(GC_ERR_STATE, "edit before upload");
-  CK(cudaSetDevice(pool.device));
-  std::vector<int32_t> pts(2 * npts);
-  for (int k = 0; k < npts; ++k) { pts[2 * k] = xs[k]; pts[2 * k + 1] = ys[k]; }
-  cudaStream_t s = (cudaStream_t)stream;
-  CK(cudaMemcpyAsync(pool.pts, pts.data(), pts.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
-  if (brush)
-    RK(launch_brush(pool.P, pool.imgs[slot], slot, pool.pts, pts.data(), npts, radius, value, pool.tl, pool.acc, s));
-  else
-    RK(launch_stroke(pool.P, pool.imgs[slot], slot, pool.pts, pts.data(), npts, radius, value, pool.tl, pool.acc, s));
-  pool.track(s);
-  CK(cudaStreamSynchronize(s));  // pts (host vector) must outlive the copy
-  pool.edited_image(slot);
-  return GC_OK;
+  if (!p->pool.img_up[slot]) return fail(GC_ERR_STATE, "edit before upload");
+  return pool_edit(p->pool, slot, xs, ys, npts, radius, value, brush, (cudaStream_t)stream);
 }
 
 int gcp_edit_stroke(gcp_handle* p, int slot, const int32_t* xs, const int32_t* ys, int npts,

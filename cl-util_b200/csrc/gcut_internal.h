@@ -147,6 +147,8 @@ int launch_state_out(const PoolView& P, const ImageDesc& im, const int32_t* plan
                      int32_t* out, cudaStream_t s);
 int launch_edit(const PoolView& P, const ImageDesc& im, int img, const int32_t* idx,
                 const int32_t* val, int n, int32_t* tl, ImageAcc* acc, cudaStream_t s);
+// Whether an edit of npts points carries them in its launch (pts_dev is then not read).
+bool edit_points_inline(int npts);
 // pts_dev / pts_host: the same (x, y) pairs on the device and on the host (for the bounds).
 int launch_stroke(const PoolView& P, const ImageDesc& im, int img, const int32_t* pts_dev,
                   const int32_t* pts_host, int npts, int radius, int32_t value, int32_t* tl,

@@ -2463,55 +2463,104 @@ __global__ void k_state_out(ImageDesc im, const int32_t* __restrict__ plane, int
   out[i] = plane[(long long)t * GC_TILE_PX + (y & 31) * GC_TILE + (x & 31)];
 }
 
-// T-link edits: excess moves by (new - old) t-link; the running sum of max(t, 0) follows.
-__device__ __forceinline__ void apply_tlink(const PoolView& P, const ImageDesc& im, int img,
-                                            int x, int y, int32_t v, int32_t* tl, ImageAcc* acc) {
+// T-link edits: excess moves by (new - old) t-link; returns the change of the pixel's term in
+// the running sum of max(t, 0).
+__device__ __forceinline__ long long apply_tlink(const PoolView& P, const ImageDesc& im, int x, int y,
+                                                 int32_t v, int32_t* tl) {
   const int t = im.tile0 + (y >> 5) * im.tw + (x >> 5);
   const long long o = (long long)t * GC_TILE_PX + (y & 31) * GC_TILE + (x & 31);
   const int32_t old = tl[o];
-  if (old == v) return;
+  if (old == v) return 0;
   tl[o] = v;
   atomicAdd(P.exc + o, v - old);
   mark_dirty(P, t);
-  const long long dpos = (long long)(v > 0 ? v : 0) - (long long)(old > 0 ? old : 0);
-  if (dpos) atomicAdd(&acc[img].sumpos_t, (unsigned long long)dpos);
+  return (long long)(v > 0 ? v : 0) - (long long)(old > 0 ? old : 0);
+}
+
+// Adds the CTA's changes to the image's sum: one add a warp that has any (an add per pixel, all
+// to one address, was most of a stroke's 27 us).  Every thread of the warp calls it.
+__device__ __forceinline__ void add_tlink_sum(ImageAcc* acc, int img, long long dpos) {
+  if (!__any_sync(0xffffffffu, dpos != 0)) return;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) dpos += __shfl_xor_sync(0xffffffffu, dpos, o);
+  if ((threadIdx.x & 31) == 0 && dpos) atomicAdd(&acc[img].sumpos_t, (unsigned long long)dpos);
 }
 
 __global__ void k_edit(PoolView P, ImageDesc im, int img, const int32_t* __restrict__ idx,
                        const int32_t* __restrict__ val, int n, int32_t* tl, ImageAcc* acc) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int p = idx[i];
-  if (p < 0 || p >= im.W * im.H) return;
-  apply_tlink(P, im, img, p % im.W, p / im.W, val[i], tl, acc);
+  long long dpos = 0;
+  if (i < n) {
+    const int p = idx[i];
+    if (p >= 0 && p < im.W * im.H) dpos = apply_tlink(P, im, p % im.W, p / im.W, val[i], tl);
+  }
+  add_tlink_sum(acc, img, dpos);
 }
+
+// A polyline of an edit.  Up to EDIT_INLINE points travel in the launch itself, so an edit is
+// one launch and no wait; more are read from device memory.
+constexpr int EDIT_INLINE = 64;
+struct InlinePts {
+  int32_t v[2 * EDIT_INLINE];
+  __device__ __forceinline__ int32_t operator[](int i) const { return v[i]; }
+};
+struct DevicePts {
+  const int32_t* v;
+  __device__ __forceinline__ int32_t operator[](int i) const { return v[i]; }
+};
 
 // Stroke: pixels within `radius` of the polyline get t-link `value`.  Exact integer test:
 // with a = p - A, b = B - A, L = b.b, s = a.b: inside iff |p - A|^2 <= r^2 (s <= 0),
 // |p - B|^2 <= r^2 (s >= L), else |a|^2 L - s^2 <= r^2 L.
-__device__ __forceinline__ bool in_stroke(int px, int py, const int32_t* pts, int npts, int r) {
-  const long long r2 = (long long)r * r;
-  for (int k = 0; k < (npts > 1 ? npts - 1 : 1); ++k) {
-    const long long ax = pts[2 * k], ay = pts[2 * k + 1];
-    const long long bx = npts > 1 ? pts[2 * k + 2] : ax, by = npts > 1 ? pts[2 * k + 3] : ay;
-    const long long dx = px - ax, dy = py - ay, ux = bx - ax, uy = by - ay;
-    const long long L = ux * ux + uy * uy, s = dx * ux + dy * uy;
-    if (L == 0 || s <= 0) { if (dx * dx + dy * dy <= r2) return true; continue; }
-    if (s >= L) { const long long ex = px - bx, ey = py - by; if (ex * ex + ey * ey <= r2) return true; continue; }
-    if ((dx * dx + dy * dy) * L - s * s <= r2 * L) return true;
+__device__ __forceinline__ bool in_segment(int px, int py, long long ax, long long ay, long long bx,
+                                           long long by, long long r2) {
+  const long long dx = px - ax, dy = py - ay, ux = bx - ax, uy = by - ay;
+  const long long L = ux * ux + uy * uy, s = dx * ux + dy * uy;
+  if (L == 0 || s <= 0) return dx * dx + dy * dy <= r2;
+  if (s >= L) {
+    const long long ex = px - bx, ey = py - by;
+    return ex * ex + ey * ey <= r2;
   }
-  return false;
+  return (dx * dx + dy * dy) * L - s * s <= r2 * L;
 }
 
-__global__ void k_stroke(PoolView P, ImageDesc im, int img, const int32_t* __restrict__ pts,
-                         int npts, int radius, int32_t value, int x0, int y0, int bw, int bh,
-                         int32_t* tl, ImageAcc* acc) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)bw * bh) return;
-  const int x = x0 + (int)(i % bw), y = y0 + (int)(i / bw);
-  if (x < 0 || y < 0 || x >= im.W || y >= im.H) return;
-  if (!in_stroke(x, y, pts, npts, radius)) return;
-  apply_tlink(P, im, img, x, y, value, tl, acc);
+// A CTA covers 32 x 8 pixels of the polyline's bounding box.  Its warps first mark the
+// segments whose own box, widened by the radius, meets the CTA's pixels; most CTAs of a long
+// stroke's box meet none and leave.
+constexpr int STROKE_W = 32, STROKE_H = 8;
+
+template <class Pts>
+__global__ void __launch_bounds__(STROKE_W * STROKE_H)
+k_stroke(PoolView P, ImageDesc im, int img, const Pts pts, int npts, int radius, int32_t value,
+         int x0, int y0, int x1, int y1, int32_t* tl, ImageAcc* acc) {
+  __shared__ unsigned s_near[32];   // segments to test, a bit each
+  const int tid = threadIdx.x;
+  const int bx0 = x0 + (int)blockIdx.x * STROKE_W, by0 = y0 + (int)blockIdx.y * STROKE_H;
+  const int nseg = npts > 1 ? npts - 1 : 1;
+  if (tid < 32) s_near[tid] = 0;
+  __syncthreads();
+  bool any = false;
+  for (int k = tid; k < nseg; k += STROKE_W * STROKE_H) {
+    const long long ax = pts[2 * k], ay = pts[2 * k + 1];
+    const long long bx = npts > 1 ? pts[2 * k + 2] : ax, by = npts > 1 ? pts[2 * k + 3] : ay;
+    if ((ax < bx ? ax : bx) - radius < bx0 + STROKE_W && (ax > bx ? ax : bx) + radius >= bx0 &&
+        (ay < by ? ay : by) - radius < by0 + STROKE_H && (ay > by ? ay : by) + radius >= by0) {
+      atomicOr(&s_near[k >> 5], 1u << (k & 31));
+      any = true;
+    }
+  }
+  if (!__syncthreads_or(any)) return;
+  const int x = bx0 + (tid & (STROKE_W - 1)), y = by0 + tid / STROKE_W;
+  bool hit = false;
+  const long long r2 = (long long)radius * radius;
+  if (x <= x1 && y <= y1)
+    for (int w = 0; w <= (nseg - 1) >> 5 && !hit; ++w)
+      for (unsigned m = s_near[w]; m && !hit; m &= m - 1) {
+        const int k = 32 * w + __ffs(m) - 1;
+        const int32_t ax = pts[2 * k], ay = pts[2 * k + 1];
+        hit = in_segment(x, y, ax, ay, npts > 1 ? pts[2 * k + 2] : ax, npts > 1 ? pts[2 * k + 3] : ay, r2);
+      }
+  add_tlink_sum(acc, img, hit ? apply_tlink(P, im, x, y, value, tl) : 0);
 }
 
 // Reference brush (gc_edit_brush): the pixel set of Brush.points (brush.pyx:138-161), the
@@ -2535,7 +2584,8 @@ __device__ __forceinline__ bool brush_disk(int dy, int dx, int R) {
   return __dadd_rn(__dmul_rn(a, a), __dmul_rn(b, b)) < 1.0;
 }
 
-__device__ __forceinline__ bool in_brush(int px, int py, const int32_t* pts, int npts, int R,
+template <class Pts>
+__device__ __forceinline__ bool in_brush(int px, int py, const Pts& pts, int npts, int R,
                                          const int32_t* half) {
   const int nseg = npts > 1 ? npts - 1 : 1;
   for (int k = 0; k < nseg; ++k) {
@@ -2562,8 +2612,9 @@ __device__ __forceinline__ bool in_brush(int px, int py, const int32_t* pts, int
   return false;
 }
 
-__global__ void k_brush(PoolView P, ImageDesc im, int img, const int32_t* __restrict__ pts,
-                        int npts, int R, int32_t value, int x0, int y0, int bw, int bh,
+template <class Pts>
+__global__ void k_brush(PoolView P, ImageDesc im, int img, const Pts pts, int npts, int R, 
+                        int32_t value, int x0, int y0, int bw, int bh,
                         int32_t* tl, ImageAcc* acc) {
   // half[dy + R - 1] = the largest dx >= 0 with the offset (dy, dx) inside the disc (the
   // test is monotone in |dx|; dx = 0 is inside for |dy| <= R - 1)
@@ -2579,11 +2630,13 @@ __global__ void k_brush(PoolView P, ImageDesc im, int img, const int32_t* __rest
   }
   __syncthreads();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)bw * bh) return;
-  const int x = x0 + (int)(i % bw), y = y0 + (int)(i / bw);
-  if (x < 0 || y < 0 || x >= im.W || y >= im.H) return;
-  if (!in_brush(x, y, pts, npts, R, half)) return;
-  apply_tlink(P, im, img, x, y, value, tl, acc);
+  long long dpos = 0;
+  if (i < (long long)bw * bh) {
+    const int x = x0 + (int)(i % bw), y = y0 + (int)(i / bw);
+    if (x >= 0 && y >= 0 && x < im.W && y < im.H && in_brush(x, y, pts, npts, R, half))
+      dpos = apply_tlink(P, im, x, y, value, tl);
+  }
+  add_tlink_sum(acc, img, dpos);
 }
 
 // ------------------------------------------------------------------------------------
@@ -2733,6 +2786,14 @@ int launch_edit(const PoolView& P, const ImageDesc& im, int img, const int32_t* 
   return ok();
 }
 
+bool edit_points_inline(int npts) { return npts <= EDIT_INLINE; }
+
+static InlinePts inline_pts(const int32_t* pts_host, int npts) {
+  InlinePts p{};
+  for (int k = 0; k < 2 * npts; ++k) p.v[k] = pts_host[k];
+  return p;
+}
+
 int launch_stroke(const PoolView& P, const ImageDesc& im, int img, const int32_t* pts_dev,
                   const int32_t* pts_host, int npts, int radius, int32_t value, int32_t* tl,
                   ImageAcc* acc, cudaStream_t s) {
@@ -2746,11 +2807,14 @@ int launch_stroke(const PoolView& P, const ImageDesc& im, int img, const int32_t
   int x0 = xmin - radius, y0 = ymin - radius, x1 = xmax + radius, y1 = ymax + radius;
   x0 = x0 < 0 ? 0 : x0; y0 = y0 < 0 ? 0 : y0;
   x1 = x1 > im.W - 1 ? im.W - 1 : x1; y1 = y1 > im.H - 1 ? im.H - 1 : y1;
-  if (x1 < x0 || y1 < y0) return GC_OK;
-  const int bw = x1 - x0 + 1, bh = y1 - y0 + 1;
-  const long long n = (long long)bw * bh;
-  k_stroke<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P, im, img, pts_dev, npts, radius, value,
-                                                     x0, y0, bw, bh, tl, acc);
+  if (x1 < x0 || y1 < y0) return GC_OK;   // (so the grid below covers pixels of the image only)
+  const dim3 grid((x1 - x0) / STROKE_W + 1, (y1 - y0) / STROKE_H + 1);
+  if (npts <= EDIT_INLINE)
+    k_stroke<<<grid, STROKE_W * STROKE_H, 0, s>>>(P, im, img, inline_pts(pts_host, npts), npts, radius,
+                                                  value, x0, y0, x1, y1, tl, acc);
+  else
+    k_stroke<<<grid, STROKE_W * STROKE_H, 0, s>>>(P, im, img, DevicePts{pts_dev}, npts, radius, value,
+                                                  x0, y0, x1, y1, tl, acc);
   return ok();
 }
 
@@ -2773,8 +2837,13 @@ int launch_brush(const PoolView& P, const ImageDesc& im, int img, const int32_t*
   if (x1 < x0 || y1 < y0) return GC_OK;
   const int bw = (int)(x1 - x0 + 1), bh = (int)(y1 - y0 + 1);
   const long long n = (long long)bw * bh;
-  k_brush<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P, im, img, pts_dev, npts, R, value,
-                                                     (int)x0, (int)y0, bw, bh, tl, acc);
+  const unsigned grid = (unsigned)((n + 255) / 256);
+  if (npts <= EDIT_INLINE)
+    k_brush<<<grid, 256, 0, s>>>(P, im, img, inline_pts(pts_host, npts), npts, R, value, (int)x0,
+                                 (int)y0, bw, bh, tl, acc);
+  else
+    k_brush<<<grid, 256, 0, s>>>(P, im, img, DevicePts{pts_dev}, npts, R, value, (int)x0, (int)y0,
+                                 bw, bh, tl, acc);
   return ok();
 }
 
@@ -2799,8 +2868,9 @@ void preload_kernels() {
       (const void*)k_solve,
       (const void*)k_image_tiles,
       (const void*)k_acc_reset, (const void*)k_labels_out, (const void*)k_labels_packed,
-      (const void*)k_state_out, (const void*)k_edit, (const void*)k_stroke,
-      (const void*)k_brush};
+      (const void*)k_state_out, (const void*)k_edit,
+      (const void*)k_stroke<InlinePts>, (const void*)k_stroke<DevicePts>,
+      (const void*)k_brush<InlinePts>, (const void*)k_brush<DevicePts>};
   for (const void* k : kernels) cudaFuncGetAttributes(&a, k);
   preload_scan_kernels();
   cudaGetLastError();

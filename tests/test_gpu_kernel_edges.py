@@ -84,3 +84,25 @@ def test_fit_edges(cuda, oracle, n, K, full):
     np.testing.assert_allclose(g.weights, want["weights"], rtol=1e-7, atol=1e-10)
     np.testing.assert_allclose(g.means, want["means"], rtol=1e-7, atol=1e-7)
     np.testing.assert_allclose(g.log_likelihood, want["log_likelihood"], rtol=1e-10)
+
+
+@pytest.mark.parametrize("npts,radius", [(1, 0), (2, 3), (33, 2), (64, 1), (65, 5), (300, 0)])
+def test_stroke_points_in_the_launch_and_copied(cuda, npts, radius):
+    """Strokes whose points travel in the launch (up to 64) and longer ones, partly outside the
+    image, against the host rasteriser; the state is read on another stream right after."""
+    import strokes
+    w, h = 150, 90
+    rng = np.random.default_rng(npts)
+    g = synth.random_graph(w, h, 3, cap_max=5, tlink_max=9)
+    xs = rng.integers(-20, w + 20, npts).astype(np.int32)
+    ys = rng.integers(-20, h + 20, npts).astype(np.int32)
+    want = strokes.apply(g.excess, strokes.Stroke(xs, ys, radius, 77))
+    other = cuda.cuda.Stream()
+    with GraphCut(w, h) as gc:
+        gc.upload_capacities(*g.planes())
+        cuda.cuda.synchronize()
+        gc.edit_stroke(xs, ys, radius, 77)
+        with cuda.cuda.stream(other):
+            got = gc.dExcess
+            other.synchronize()
+        assert np.array_equal(got.cpu().numpy(), want)
