@@ -475,7 +475,7 @@ struct Pool {
     CK(cudaSetDevice(device));
     RK(order(s));
     const ImageDesc& im = imgs[i];
-    if (lambda == 0) RK(launch_nlinks(rgba, im.W, im.H, dsum, ntab, acc + i, s));
+    if (lambda == 0) RK(launch_nlinks(rgba, im.W, im.H, dsum, ntab, acc + i, sms, s));
     else CK(cudaMemsetAsync(acc + i, 0, sizeof(ImageAcc), s));
     P.ktiles = nullptr;
     RK(timed(K_UPLOAD, s, [&] {

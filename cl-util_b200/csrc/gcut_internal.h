@@ -72,7 +72,7 @@ int launch_upload_rgba(const PoolView& P, const ImageDesc& im, int img, const ui
 // The mean |dI|^2 of an image and the n-link table from it (tab: 50 thresholds and a float),
 // one launch; state: two zeroed words, zero again afterwards.  Clears *acc for the upload.
 int launch_nlinks(const uint32_t* rgba, int W, int H, unsigned long long* state, int32_t* tab,
-                  ImageAcc* acc, cudaStream_t s);
+                  ImageAcc* acc, int sms, cudaStream_t s);
 // hlim: pixels below this height are active
 int launch_discharge(const PoolView& P, int iters, int hlim, int grid, cudaStream_t s);
 int launch_edge_relabel_build(const PoolView& P, int32_t* list, int32_t* count,

@@ -266,11 +266,12 @@ k_upload(PoolView P, ImageDesc im, int img, PlaneSource src, int32_t* __restrict
   store_uploaded_tile(P, im.tile0 + bt, img, r, c0, e, cu, cd, cl, cr, tl, acc);
 }
 
+// |a - b|^2 of two colours whose alpha byte is 0: byte differences and their dot product, two
+// instructions.
+constexpr uint32_t RGB_MASK = 0x00ffffffu;
 __device__ __forceinline__ int rgb_dist2(uint32_t a, uint32_t b) {
-  const int dr = (int)(a & 255u) - (int)(b & 255u);
-  const int dg = (int)((a >> 8) & 255u) - (int)((b >> 8) & 255u);
-  const int db = (int)((a >> 16) & 255u) - (int)((b >> 16) & 255u);
-  return dr * dr + dg * dg + db * db;
+  const unsigned d = __vabsdiffu4(a, b);
+  return (int)__dp4a(d, d, 0u);
 }
 
 // Weight of the reference's n-link rule, rounded to an integer: floor(x + 0.5) for
@@ -295,30 +296,32 @@ __device__ __forceinline__ int ref_weight(int d, int lambda) {
 }
 
 // n-link weights from |dI|^2.  Exp weighting: the number of table entries >= d (the entries
-// t[0..50) do not increase).  The formula itself, in float32, gives the level to within one
-// (its error is below 1e-4 of a level), and the entries beside it settle it: two independent
-// shared-memory reads where a binary search chains six.
+// t[0..50) do not increase).  The formula itself in float32 gives the level to within one: its
+// error is below 1e-4 of a level, so the level is off only next to a boundary, and the entries
+// on both sides of it, one 64-bit read, settle it.  (A binary search chains six reads.)
 struct ExpWeight {
   float scale;   // -beta * log2(e)
-  __device__ __forceinline__ int operator()(const int32_t* s_tab, int d) const {
-    int k = (int)(50.0f * exp2f(scale * (float)d) + 0.5f);   // 0 .. 50
-    while (k > 0 && s_tab[k - 1] < d) --k;
-    while (k < GC_NLINK_LEVELS && s_tab[k] >= d) ++k;
-    return k;
+  __device__ __forceinline__ int operator()(const int2* s_tab, int d) const {
+    const int k = (int)(50.0f * exp2f(scale * (float)d) + 0.5f);   // 0 .. 50
+    const int2 t = s_tab[k];                                       // t[k - 1], t[k]
+    return k + (t.y >= d ? 1 : 0) - (t.x < d ? 1 : 0);
   }
 };
 struct RefWeight {
   int lambda;
-  __device__ __forceinline__ int operator()(const int32_t*, int d) const { return ref_weight(d, lambda); }
+  __device__ __forceinline__ int operator()(const int2*, int d) const { return ref_weight(d, lambda); }
 };
 
 // The upload from an RGBA image: the weights of an n-link are the same both ways, so a thread
 // computes those to the right of and below its four pixels and takes the other two directions
 // from its neighbours (a lane of the same warp, shared memory for the row above); the tile's
 // first row and column compute theirs from the pixels across the side.  5 weights a thread
-// (9 in the tile's first warp) where one per pixel and direction takes 16.
+// (9 in the tile's first warp) where one per pixel and direction takes 16.  A distance is a byte
+// difference and a byte dot product (two instructions, not eleven).
 //
-// Bound by the planes it writes: 28 of 36 bytes a pixel.
+// Bound by the planes it writes, 28 of 36 bytes a pixel (92 us at 4096x4096 and the copy rate):
+// 134 us there (166 with the distances a channel at a time and two dependent table reads a
+// weight), 1920x1080 18.8 us (23.6).  Eight CTAs an SM in place of five change nothing.
 struct RgbaSource {
   const uint32_t* rgba;
   const int32_t* excess;
@@ -332,11 +335,12 @@ __global__ void __launch_bounds__(DIS_THREADS)
 k_upload_rgba(PoolView P, ImageDesc im, int img, RgbaSource src, Weight weight,
               int32_t* __restrict__ tl, ImageAcc* acc) {
   trace_mark(P, TR_UPLOAD);
-  __shared__ int32_t s_tab[GC_NLINK_LEVELS];
+  __shared__ int2 s_tab[GC_NLINK_LEVELS + 1];   // the thresholds on both sides of a level
   __shared__ int4 s_down[GC_TILE][8];
   const int tid = threadIdx.x, q = tid & 7;
   if constexpr (std::is_same_v<Weight, ExpWeight>) {
-    if (tid < GC_NLINK_LEVELS) s_tab[tid] = src.tab[tid];
+    if (tid <= GC_NLINK_LEVELS)
+      s_tab[tid] = make_int2(tid > 0 ? src.tab[tid - 1] : 0x7fffffff, tid < GC_NLINK_LEVELS ? src.tab[tid] : -1);
     weight.scale = __int_as_float(src.tab[GC_NLINK_LEVELS]);
     __syncthreads();
   }
@@ -370,13 +374,18 @@ k_upload_rgba(PoolView P, ImageDesc im, int img, RgbaSource src, Weight weight,
       if (below_in) below[j] = src.rgba[i + im.W + j];
     }
   }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    px[j] &= RGB_MASK;
+    below[j] &= RGB_MASK;
+  }
   // the pixel to the right of the four, and (first column) the one to the left
   const unsigned F = 0xffffffffu;
   uint32_t next = __shfl_down_sync(F, px[0], 1);
-  if (q == 7 && row_in && x0 + 4 < im.W) next = src.rgba[i + 4];
+  if (q == 7 && row_in && x0 + 4 < im.W) next = src.rgba[i + 4] & RGB_MASK;
   uint32_t side = 0;   // first column: the pixel to the left
   const bool has_left = q == 0 && row_in && x0 > 0 && x0 < im.W;
-  if (has_left) side = src.rgba[i - 1];
+  if (has_left) side = src.rgba[i - 1] & RGB_MASK;
   int cu[4], cd[4], cl[4], cr[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -396,18 +405,22 @@ k_upload_rgba(PoolView P, ImageDesc im, int img, RgbaSource src, Weight weight,
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       cu[j] = y > 0 && row_in && x0 + j < im.W
-                  ? weight(s_tab, rgb_dist2(px[j], src.rgba[i - im.W + j])) : 0;
+                  ? weight(s_tab, rgb_dist2(px[j], src.rgba[i - im.W + j] & RGB_MASK)) : 0;
   }
   store_uploaded_tile(P, im.tile0 + bt, img, r, c0, e, cu, cd, cl, cr, tl, acc);
 }
 
 // The mean |dI|^2 over all 4-neighbour pairs and the exp weighting's table, in one launch.
 //
-// Every pixel is read once: a thread walks down DSUM_ROWS rows of one column, with the row
-// above in a register and the pixel to the left from the lane beside it (a warp reads 128
-// bytes of a row at a time; DSUM_ROWS loads in flight).  Sums are exact: 32 bits a thread (at
-// most 2 * 3 * 255^2 * DSUM_ROWS), 64 above.  The last CTA turns the total into the table and
-// clears the total and the ticket for the next call.
+// A thread walks down 8 rows of a strip of 4 pixels, or 4 rows of one column where the rows are
+// not 16-byte aligned (more rows take registers that loads in flight need), with the row above in registers and the pixel to the left from the
+// lane beside it, so every pixel is read once (and a strip's upper row twice), all rows' loads
+// in flight.  The CTAs are one wave that loops over the strips: at 4096x4096 the tails of eight
+// waves (64-bit reduction, ticket) were a third of the time.  Sums are exact: 32 bits a thread
+// and strip (at most 2 * PX * ROWS * 3 * 255^2), 64 above.  The last CTA turns the total into
+// the table and clears the total and the ticket for the next call.
+// Bound by memory at 4096x4096 (64 MiB: 10.6 us at the copy rate, 25 us here, 37 us with one
+// column of 16 rows a thread and a CTA a strip); at 1920x1080 6.6 us (8.5), launch and tail.
 //
 // The table: weight(d) = floor(50 exp(-beta d) + 0.5) with beta = 1 / (2 mean |dI|^2) (0 when
 // the mean is 0) does not increase with d, so it is stored as t[k - 1] = the largest d in
@@ -415,8 +428,8 @@ k_upload_rgba(PoolView P, ImageDesc im, int img, RgbaSource src, Weight weight,
 // 50 exp(-beta d) + 0.5 = k and settles it by evaluating the formula itself at the integers
 // around it, in double, so the table reproduces a float64 evaluation of the formula pixel by
 // pixel.  t[50] holds -beta * log2(e) as a float (ExpWeight's estimate).
-constexpr int DSUM_ROWS = 16;
 constexpr int DSUM_THREADS = 256;
+template <int PX> constexpr int DSUM_ROWS = PX == 4 ? 8 : 4;
 
 __device__ __forceinline__ void nlink_table(unsigned long long sum, long long npairs, int k,
                                             int32_t* tab) {
@@ -434,35 +447,51 @@ __device__ __forceinline__ void nlink_table(unsigned long long sum, long long np
 }
 
 // state: [0] the running sum, [1] the ticket (both zero between calls)
+template <int PX>
 __global__ void __launch_bounds__(DSUM_THREADS)
 k_nlinks(const uint32_t* __restrict__ rgba, int W, int H, long long npairs,
          unsigned long long* state, int32_t* __restrict__ tab, ImageAcc* acc) {
+  constexpr int ROWS = DSUM_ROWS<PX>;
   __shared__ unsigned long long part[DSUM_THREADS / 32];
   __shared__ unsigned long long s_total;
   __shared__ int s_last;
   const int lane = threadIdx.x & 31;
-  const long long x = (long long)blockIdx.x * DSUM_THREADS + threadIdx.x;
-  const int y0 = blockIdx.y * DSUM_ROWS;
-  const bool in = x < W;
-  unsigned sum = 0;
-  uint32_t c[DSUM_ROWS + 1], l[DSUM_ROWS];
+  const int cols = (W / PX + DSUM_THREADS - 1) / DSUM_THREADS, rows = (H + ROWS - 1) / ROWS;
+  unsigned long long acc64 = 0;
+  for (long long b = blockIdx.x; b < (long long)cols * rows; b += gridDim.x) {
+    const long long x = ((b % cols) * DSUM_THREADS + threadIdx.x) * PX;
+    const int y0 = (int)(b / cols) * ROWS;
+    const bool in = x < W;          // with PX == 4 the width is a multiple of 4
+    unsigned sum = 0;
+    uint32_t c[ROWS + 1][PX], l[ROWS];
 #pragma unroll
-  for (int k = 0; k <= DSUM_ROWS; ++k) {   // c[0]: the row above the strip
-    const int y = y0 + k - 1;
-    c[k] = in && y >= 0 && y < H ? rgba[(long long)y * W + x] : 0u;
+    for (int k = 0; k <= ROWS; ++k) {   // c[0]: the row above the strip
+      const int y = y0 + k - 1;
+      const bool on = in && y >= 0 && y < H;
+      const uint32_t* const p = rgba + (long long)y * W + x;
+      if constexpr (PX == 4) {
+        const uint4 v = on ? *reinterpret_cast<const uint4*>(p) : make_uint4(0u, 0u, 0u, 0u);
+        c[k][0] = v.x & RGB_MASK; c[k][1] = v.y & RGB_MASK; c[k][2] = v.z & RGB_MASK; c[k][3] = v.w & RGB_MASK;
+      } else {
+        c[k][0] = on ? *p & RGB_MASK : 0u;
+      }
+      if (k > 0)                             // lane 0: the pixel left of the warp's columns
+        l[k - 1] = lane == 0 && on && x > 0 ? p[-1] & RGB_MASK : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
+      const uint32_t beside = __shfl_up_sync(0xffffffffu, c[k + 1][PX - 1], 1);
+      if (!in || y0 + k >= H) continue;
+      const uint32_t left = lane == 0 ? l[k] : beside;
+      if (x > 0) sum += (unsigned)rgb_dist2(c[k + 1][0], left);
+#pragma unroll
+      for (int j = 0; j < PX; ++j) {
+        if (y0 + k > 0) sum += (unsigned)rgb_dist2(c[k + 1][j], c[k][j]);
+        if (j > 0) sum += (unsigned)rgb_dist2(c[k + 1][j], c[k + 1][j - 1]);
+      }
+    }
+    acc64 += sum;
   }
-#pragma unroll
-  for (int k = 0; k < DSUM_ROWS; ++k)      // lane 0: the pixel left of the warp's columns
-    l[k] = lane == 0 && in && x > 0 && y0 + k < H ? rgba[(long long)(y0 + k) * W + x - 1] : 0u;
-#pragma unroll
-  for (int k = 0; k < DSUM_ROWS; ++k) {
-    const uint32_t up = __shfl_up_sync(0xffffffffu, c[k + 1], 1);
-    const uint32_t left = lane == 0 ? l[k] : up;
-    if (!in || y0 + k >= H) continue;
-    if (y0 + k > 0) sum += (unsigned)rgb_dist2(c[k + 1], c[k]);
-    if (x > 0) sum += (unsigned)rgb_dist2(c[k + 1], left);
-  }
-  unsigned long long acc64 = sum;
 #pragma unroll
   for (int o = 16; o; o >>= 1) acc64 += __shfl_xor_sync(0xffffffffu, acc64, o);
   if (lane == 0) part[threadIdx.x >> 5] = acc64;
@@ -472,8 +501,7 @@ k_nlinks(const uint32_t* __restrict__ rgba, int W, int H, long long npairs,
     for (int k = 0; k < DSUM_THREADS / 32; ++k) tsum += part[k];
     if (tsum) atomicAdd(state, tsum);
     __threadfence();
-    const unsigned long long n = (unsigned long long)gridDim.x * gridDim.y;
-    s_last = atomicAdd(state + 1, 1ull) == n - 1;
+    s_last = atomicAdd(state + 1, 1ull) == gridDim.x - 1;
     if (s_last) {
       __threadfence();
       s_total = *((volatile unsigned long long*)state);
@@ -2668,10 +2696,15 @@ int launch_upload_rgba(const PoolView& P, const ImageDesc& im, int img, const ui
 }
 
 int launch_nlinks(const uint32_t* rgba, int W, int H, unsigned long long* state, int32_t* tab,
-                  ImageAcc* acc, cudaStream_t s) {
+                  ImageAcc* acc, int sms, cudaStream_t s) {
   const long long npairs = (long long)(H - 1) * W + (long long)H * (W - 1);
-  const dim3 grid((W + DSUM_THREADS - 1) / DSUM_THREADS, (H + DSUM_ROWS - 1) / DSUM_ROWS);
-  k_nlinks<<<grid, DSUM_THREADS, 0, s>>>(rgba, W, H, npairs, state, tab, acc);
+  const int px = W % 4 == 0 && aligned16(rgba) ? 4 : 1;   // ragged rows have no aligned strips
+  const int rows = px == 4 ? DSUM_ROWS<4> : DSUM_ROWS<1>;
+  const long long blocks = (long long)((W / px + DSUM_THREADS - 1) / DSUM_THREADS) * ((H + rows - 1) / rows);
+  const long long wave = (px == 4 ? 4LL : 8LL) * sms;   // resident CTAs: strips of 4 take the registers
+  const int grid = (int)(blocks < wave ? blocks : wave);
+  if (px == 4) k_nlinks<4><<<grid, DSUM_THREADS, 0, s>>>(rgba, W, H, npairs, state, tab, acc);
+  else k_nlinks<1><<<grid, DSUM_THREADS, 0, s>>>(rgba, W, H, npairs, state, tab, acc);
   return ok();
 }
 
@@ -2861,7 +2894,7 @@ void preload_kernels() {
   cudaFuncAttributes a;
   const void* kernels[] = {
       (const void*)k_upload, (const void*)k_upload_rgba<ExpWeight>,
-      (const void*)k_upload_rgba<RefWeight>, (const void*)k_nlinks,
+      (const void*)k_upload_rgba<RefWeight>, (const void*)k_nlinks<1>, (const void*)k_nlinks<4>,
       (const void*)k_masks, (const void*)k_discharge, (const void*)k_edge_relabel_build,
       (const void*)k_bfs_round, (const void*)k_flood_round, (const void*)k_ctl_begin,
       (const void*)k_active_list, (const void*)k_ctl_cycle, (const void*)k_flood_check,

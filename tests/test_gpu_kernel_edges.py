@@ -73,6 +73,21 @@ def test_rgba_upload_edges(cuda, oracle, w, h, lamda, offset):
             assert np.array_equal(getattr(gc, name).cpu().numpy(), want), name
 
 
+@pytest.mark.parametrize("w,h", [(4, 4801), (3, 4763), (1028, 9), (257, 5)])
+def test_rgba_table_strips(cuda, w, h):
+    """More strips than one wave of CTAs, and columns past a CTA's, in both strip widths; the
+    alpha byte takes no part."""
+    rng = np.random.default_rng(w)
+    img = rng.integers(0, 256, (h, w, 3)).astype(np.uint8)
+    alpha = rng.integers(0, 256, (h, w, 1)).astype(np.uint8)
+    excess = np.zeros((h, w), np.int32)
+    up, down, left, right = synth.planes_from_weights(*synth.nlinks(img), excess)
+    with GraphCut(w, h) as gc:
+        gc.upload_image(np.concatenate([img, alpha], -1), excess)
+        for name, want in (("dUp", up), ("dDown", down), ("dLeft", left), ("dRight", right)):
+            assert np.array_equal(getattr(gc, name).cpu().numpy(), want), name
+
+
 @pytest.mark.parametrize("n,K,full", [(31, 2, False), (33, 5, True), (10240, 4, False),
                                       (10241, 4, True), (20481, 7, False)])
 def test_fit_edges(cuda, oracle, n, K, full):
