@@ -65,6 +65,21 @@ def test_pitched_image_clamp_and_scale(cuda, oracle):
             assert (np.abs(want) == 1000).mean() > 0.5   # saturation is exercised
 
 
+@pytest.mark.parametrize("w,h", [(32767, 3), (32768, 3), (255, 386), (129, 765)])
+@pytest.mark.parametrize("kf,kb", [(1, 2), (4, 3), (2, 7)])
+def test_around_the_small_image_limit(cuda, oracle, kf, kb, w, h):
+    """Images just below and above 98304 pixels, whole and with a row pitch, with a ragged last
+    block."""
+    torch = cuda
+    rng = np.random.default_rng(w + kf)
+    base = rng.integers(0, 2 ** 32, (h, w + 5), dtype=np.uint64).astype(np.uint32)
+    fg, bg = _random_model(rng, kf, True), _random_model(rng, kb, False)
+    dev = torch.from_numpy(base.view(np.int32)).cuda()
+    want, v = oracle.tlinks_gmm(base[:, 3:3 + w], fg, bg)
+    for img in (dev[:, 3:3 + w], dev[:, 3:3 + w].contiguous()):
+        _assert_parity(tlinks(img, fg, bg).cpu().numpy(), want, v)
+
+
 def test_empty_image(cuda):
     torch = cuda
     m = Mixture([1.0], [[0, 0, 0]], [[1, 1, 1]])
