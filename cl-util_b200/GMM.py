@@ -25,6 +25,7 @@ from _gcut import GcGmmFitResult, check, lib, ptr, stream_handle
 MIN_COVAR = 1e-3     # GMM.pyx:10, passed to gmm.cl as -D MIN_COVAR (GMM.pyx:66-71)
 INIT_COVAR = 30.0    # GMM.pyx:9, passed as -D INIT_COVAR
 TOLERANCE = 0.01     # GMM.pyx:329
+_RESULT = np.dtype(GcGmmFitResult)
 
 
 class GMM:
@@ -81,23 +82,20 @@ class GMM:
                                    int(self.full_covariance), ptr(self._result),
                                    stream_handle(stream)))
             host = self._result.cpu().numpy()
-        r = GcGmmFitResult.from_buffer_copy(host.tobytes())
+        r = host.view(_RESULT)[0]
         K = self.n_components
-        self.weights = np.array(r.weights[:K])
-        self.means = np.array([list(r.means[k]) for k in range(K)])
-        tri = np.array([list(r.covars[k]) for k in range(K)])
-        full = np.empty((K, 3, 3))
-        for k in range(K):
-            s00, s10, s11, s20, s21, s22 = tri[k]
-            full[k] = [[s00, s10, s20], [s10, s11, s21], [s20, s21, s22]]
-        self.covars = full if self.full_covariance else np.stack([np.diag(m) for m in full])
-        self.iterations = int(r.iterations)
-        self.has_converged = bool(r.converged)
-        self.log_likelihood = float(r.log_likelihood)
+        self.weights = r["weights"][:K].copy()
+        self.means = r["means"][:K].copy()
+        tri = r["covars"][:K]   # lower triangles
+        self.covars = np.ascontiguousarray(
+            tri[:, [0, 1, 3, 1, 2, 4, 3, 4, 5]].reshape(K, 3, 3)
+            if self.full_covariance else tri[:, [0, 2, 5]])
+        self.iterations = int(r["iterations"])
+        self.has_converged = bool(r["converged"])
+        self.log_likelihood = float(r["log_likelihood"])
         # the model's evaluation form as the device computed it ([K, 10] rows of gc_gauss)
-        self.device_components = np.array(
-            [[r.components[k].c, *r.components[k].mean, *r.components[k].li] for k in range(K)])
-        if r.status:
+        self.device_components = r["components"][:K].view(np.float64).reshape(K, 10).copy()
+        if r["status"]:
             raise _gcut.GCError(_gcut.GC_ERR_NOT_CONVERGED,
                                 "gc_gmm_fit: a covariance stopped being positive definite "
                                 f"after {self.iterations} iterations")

@@ -18,6 +18,7 @@ The reference's stepping methods keep their names: ``push``, ``relabel``, ``star
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 
 import numpy as np
@@ -33,26 +34,31 @@ def _as_i32_device(a, device):
     if isinstance(a, torch.Tensor):
         if a.dtype != torch.int32:
             raise TypeError("capacity planes must be int32")
+        if a.device == device and a.is_contiguous():
+            return a
         return a.to(device).contiguous()
     return torch.from_numpy(np.ascontiguousarray(a, dtype=np.int32)).to(device)
+
+
+_NO_CONTEXT = contextlib.nullcontext()
 
 
 def _device_guard(device):
     """torch.cuda.device(device), or nothing when `device` is already current: the library
     selects the device itself, and the guard only restores the caller's afterwards."""
-    import contextlib
     import torch
     if torch.cuda.current_device() == device.index:
-        return contextlib.nullcontext()
+        return _NO_CONTEXT
     return torch.cuda.device(device)
 
 
 def _on(stream):
     """Makes `stream` torch's current stream (no-op for None), so that torch copies made for
     a call are ordered before the library's kernels on that stream."""
-    import contextlib
+    if stream is None:
+        return _NO_CONTEXT
     import torch
-    return contextlib.nullcontext() if stream is None else torch.cuda.stream(stream)
+    return torch.cuda.stream(stream)
 
 
 def _as_rgba32(img):
@@ -147,13 +153,18 @@ class GraphCut:
         is copied to the device first.  Resets the residual graph."""
         import torch
         planes = (up, down, left, right, excess)
+        shape = (self.height, self.width)
+        on_gpu = in_place = True
         for p in planes:
-            if tuple(p.shape) != (self.height, self.width):
-                raise ValueError(f"plane shape {tuple(p.shape)} != {(self.height, self.width)}")
-        if all(isinstance(p, torch.Tensor) and p.is_cuda for p in planes):
-            if all(p.dtype == torch.int32 and p.device == self.device and p.is_contiguous()
-                   for p in planes):
-                dev = planes      # read in place: no conversion to order before the kernel
+            if tuple(p.shape) != shape:
+                raise ValueError(f"plane shape {tuple(p.shape)} != {shape}")
+            if not (isinstance(p, torch.Tensor) and p.is_cuda):
+                on_gpu = False
+            elif in_place:
+                in_place = p.dtype is torch.int32 and p.device == self.device and p.is_contiguous()
+        if on_gpu:
+            if in_place:
+                dev = planes      # no conversion to order before the kernel
             else:
                 with _on(stream):   # conversions are ordered before the upload kernel
                     dev = [_as_i32_device(p, self.device) for p in planes]
@@ -340,7 +351,7 @@ class GraphCut:
         ys = np.ascontiguousarray(ys, dtype=np.int32)
         if xs.shape != ys.shape or xs.ndim != 1:
             raise ValueError("xs and ys must be 1-D arrays of the same length")
-        check(lib().gc_edit_stroke(self._h, ptr(xs), ptr(ys), int(xs.shape[0]), int(radius),
+        check(lib().gc_edit_stroke(self._h, xs.ctypes.data, ys.ctypes.data, int(xs.shape[0]), int(radius),
                                    int(value), stream_handle(stream)))
         self._solved = False
 
@@ -352,7 +363,7 @@ class GraphCut:
         ys = np.ascontiguousarray(ys, dtype=np.int32)
         if xs.shape != ys.shape or xs.ndim != 1:
             raise ValueError("xs and ys must be 1-D arrays of the same length")
-        check(lib().gc_edit_brush(self._h, ptr(xs), ptr(ys), int(xs.shape[0]), int(radius),
+        check(lib().gc_edit_brush(self._h, xs.ctypes.data, ys.ctypes.data, int(xs.shape[0]), int(radius),
                                   int(value), stream_handle(stream)))
         self._solved = False
 

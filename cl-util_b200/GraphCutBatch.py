@@ -68,7 +68,9 @@ class GraphCutBatch:
             if tuple(p.shape) != (h, w):
                 raise ValueError(f"plane shape {tuple(p.shape)} != {(h, w)}")
             t = p if isinstance(p, torch.Tensor) else torch.from_numpy(np.ascontiguousarray(p, dtype=np.int32))
-            dev.append(t.to(self.device, dtype=torch.int32).contiguous())
+            if not (t.dtype is torch.int32 and t.device == self.device and t.is_contiguous()):
+                t = t.to(self.device, dtype=torch.int32).contiguous()
+            dev.append(t)
         check(lib().gcb_upload(self._h, int(i), *[ptr(d) for d in dev], stream_handle(stream)))
         self._keep[i] = dev
 

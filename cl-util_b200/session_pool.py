@@ -175,7 +175,7 @@ class SessionPool:
         ys = np.ascontiguousarray(ys, dtype=np.int32)
         if xs.shape != ys.shape or xs.ndim != 1:
             raise ValueError("xs and ys must be 1-D arrays of the same length")
-        check(fn(self._h, int(slot), ptr(xs), ptr(ys), int(xs.shape[0]), int(radius),
+        check(fn(self._h, int(slot), xs.ctypes.data, ys.ctypes.data, int(xs.shape[0]), int(radius),
                  int(value), stream_handle(stream)))
 
     def edit_stroke(self, slot, xs, ys, radius: int, value: int, stream=None):
