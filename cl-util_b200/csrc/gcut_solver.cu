@@ -1250,10 +1250,9 @@ __device__ __forceinline__ void frontier_work(const PoolView& P, int first, int 
   *participants = need < 1 ? 1 : (need < (int)gridDim.x ? need : (int)gridDim.x);
 }
 
-// Queue tile t for the next round (once).  Within a round the next round's marks only go
-// from 0 to 1, so a set mark read with a plain load needs no atomic.
+// Queue tile t for the next round (once).  No look at the mark first: a round is a chain of L2
+// trips, and the exchange answers as soon as a load would.
 __device__ __forceinline__ void frontier_push(const PoolView& P, const Worklist& out, int t) {
-  if (*((volatile int32_t*)&out.in[t]) != 0) return;
   if (atomicExch(&out.in[t], 1) == 0) {
     const int pos = atomicAdd(out.count, 1);
     if (pos < P.nt) out.list[pos] = t;   // the mark deduplicates, so pos < nt always holds
@@ -1448,78 +1447,100 @@ __global__ void k_ctl_cycle(PoolView P) {
   __threadfence();
 }
 
-// ---- relabel within a small cap: distances as bit planes ----------------------------
-// With cap <= BFS_NEAR_CAP every distance fits in BFS_PLANES bits.  Lane r keeps bit b of the
-// distances of row r in plane[b], so a level costs a few logic operations instead of a store
-// per pixel, and the rows are turned into int4 stores once at the end.
-constexpr int BFS_PLANES = 7;
-constexpr int BFS_NEAR_CAP = (1 << BFS_PLANES) - 1;
+// ---- distances as bit planes --------------------------------------------------------
+// The distances of a tile above its lowest seed (`base`) mostly fit in BFS_PLANES bits.  Lane r
+// keeps bit b of those of row r in plane[b], so a level costs a few logic operations instead of
+// a store per pixel, and the rows are turned into int4 stores once at the end.  Tiles with a
+// seed further out than BFS_RANGE above their lowest fall back on tile_bfs_seeded.
+constexpr int BFS_PLANES = 8;
+constexpr int BFS_RANGE = (1 << BFS_PLANES) - 1;
+constexpr int BFS_GROUP = 2;   // levels a vote
 
-struct NearBfs {
+struct PlaneBfs {
+  int base;                      // lowest level
   uint32_t vis;                  // reached pixels of row `lane`
-  uint32_t plane[BFS_PLANES];    // their distances (0 where not reached)
+  uint32_t plane[BFS_PLANES];    // their distances above base (0 where not reached)
+  bool whole;                    // false: levels beyond base + BFS_RANGE are missing
   // distances of row `lane`'s pixel at column c (0 or 31)
   __device__ __forceinline__ int side(int c) const {
-    int d = 0;
+    int d = base;
 #pragma unroll
-    for (int b = 0; b < BFS_PLANES; ++b) d |= (int)((plane[b] >> c) & 1u) << b;
+    for (int b = 0; b < BFS_PLANES; ++b) d += (int)((plane[b] >> c) & 1u) << b;
     return (vis >> c) & 1u ? d : GC_HINF;
   }
   // distance of column `lane`'s pixel in row `row` (uniform)
   __device__ __forceinline__ int across(int row, int lane) const {
-    int d = 0;
+    int d = base;
 #pragma unroll
     for (int b = 0; b < BFS_PLANES; ++b)
-      d |= (int)((__shfl_sync(0xffffffffu, plane[b], row) >> lane) & 1u) << b;
+      d += (int)((__shfl_sync(0xffffffffu, plane[b], row) >> lane) & 1u) << b;
     return (__shfl_sync(0xffffffffu, vis, row) >> lane) & 1u ? d : GC_HINF;
   }
 };
 
-// tile_bfs_seeded for cap <= BFS_NEAR_CAP.
-__device__ __forceinline__ NearBfs tile_bfs_near(uint32_t sink, uint32_t canU, uint32_t canD,
-                                                 uint32_t canL, uint32_t canR, int lane,
-                                                 bool seeded, int top, int bot, int sl, int sr,
-                                                 int cap) {
+// tile_bfs_seeded on bit planes.  A level is a chain of a shuffle and three logic operations
+// (40 cycles); the vote on an empty frontier would double it, so BFS_GROUP levels share one (a
+// level without a frontier or a seed visits nothing).  A frontier round of a few tiles takes 11 us
+// at a cap of 64 and 15 us without one (13 with a vote a level, 22 with a store per pixel); of
+// that 7 us are its chain of L2 trips and the barrier.  (4 levels a vote: the same, more spills;
+// 7 planes: the same up to 127, slower beyond.)
+__device__ __forceinline__ PlaneBfs tile_bfs_planes(uint32_t sink, uint32_t canU, uint32_t canD,
+                                                    uint32_t canL, uint32_t canR, int lane,
+                                                    bool seeded, int top, int bot, int sl, int sr,
+                                                    int cap) {
   const unsigned FULL = 0xffffffffu;
-  NearBfs B;
+  PlaneBfs B;
   B.vis = 0;
+  B.whole = true;
 #pragma unroll
   for (int b = 0; b < BFS_PLANES; ++b) B.plane[b] = 0;
-  uint32_t Fr = 0;
+  uint32_t Fr = 0, over = 0;
   if (lane == 0) canU = 0;     // the row above / below lies in another tile (seeds stand for it)
   if (lane == 31) canD = 0;
   int L = 0;
   if (!__any_sync(FULL, sink != 0)) L = seeded ? warp_min(imin(imin(top, bot), imin(sl, sr))) : GC_HINF;
-  // a level visits a pixel or jumps to a later seed, and L rises with each
-  while (L <= cap) {
-    uint32_t N = ((Fr >> 1) & canR) | ((Fr << 1) & canL) | (__shfl_up_sync(FULL, Fr, 1) & canU) |
-                 (__shfl_down_sync(FULL, Fr, 1) & canD);
-    if (L == 0) N |= sink;
-    if (seeded) {
-      const uint32_t bt = __ballot_sync(FULL, top == L), bb = __ballot_sync(FULL, bot == L);
-      N |= (sl == L ? 1u : 0u) | (sr == L ? 0x80000000u : 0u);
-      if (lane == 0) N |= bt;
-      if (lane == 31) N |= bb;
-    }
-    N &= ~B.vis;
-    B.vis |= N;
+  B.base = L;
+  const int lim = imin(cap, GC_HINF - 1);
+  const int last = L <= lim - BFS_RANGE ? L + BFS_RANGE : lim;
+  // L rises by BFS_GROUP or jumps to a later seed
+  while (L <= last) {
 #pragma unroll
-    for (int b = 0; b < BFS_PLANES; ++b) B.plane[b] |= (L >> b) & 1 ? N : 0u;
-    Fr = N;
-    if (__any_sync(FULL, N != 0)) {
-      ++L;
-      continue;
+    for (int k = 0; k < BFS_GROUP; ++k, ++L) {
+      uint32_t N = ((Fr >> 1) & canR) | ((Fr << 1) & canL) | (__shfl_up_sync(FULL, Fr, 1) & canU) |
+                   (__shfl_down_sync(FULL, Fr, 1) & canD);
+      if (k == 0 && L == 0) N |= sink;
+      if (seeded) {
+        const uint32_t bt = __ballot_sync(FULL, top == L), bb = __ballot_sync(FULL, bot == L);
+        N |= (sl == L ? 1u : 0u) | (sr == L ? 0x80000000u : 0u);
+        if (lane == 0) N |= bt;
+        if (lane == 31) N |= bb;
+      }
+      N &= ~B.vis;
+      if (L > last) {   // too far out to hold
+        over |= N;
+        N = 0;
+      }
+      B.vis |= N;
+      const int d = L - B.base;
+#pragma unroll
+      for (int b = 0; b < BFS_PLANES; ++b) B.plane[b] |= (d >> b) & 1 ? N : 0u;
+      Fr = N;
     }
-    if (!seeded) break;
+    if (__any_sync(FULL, Fr != 0)) continue;
+    if (L > last + 1 && __any_sync(FULL, over != 0)) break;
+    if (!seeded) return B;
     // the frontier is empty: the next level that still has an unvisited seed
     const uint32_t v0 = __shfl_sync(FULL, B.vis, 0), v31 = __shfl_sync(FULL, B.vis, 31);
     int cand = GC_HINF;
-    if (top > L && !((v0 >> lane) & 1u)) cand = imin(cand, top);
-    if (bot > L && !((v31 >> lane) & 1u)) cand = imin(cand, bot);
-    if (sl > L && !(B.vis & 1u)) cand = imin(cand, sl);
-    if (sr > L && !(B.vis >> 31)) cand = imin(cand, sr);
+    if (!((v0 >> lane) & 1u)) cand = imin(cand, top);
+    if (!((v31 >> lane) & 1u)) cand = imin(cand, bot);
+    if (!(B.vis & 1u)) cand = imin(cand, sl);
+    if (!(B.vis >> 31)) cand = imin(cand, sr);
     L = warp_min(cand);
+    if (L > lim) return B;
   }
+  // something lies beyond `last`: beyond the cap, or only beyond the planes' range
+  B.whole = last == lim;
   return B;
 }
 
@@ -1529,7 +1550,7 @@ __device__ __forceinline__ uint32_t spread4(uint32_t x) { return ((x & 15u) * 0x
 // One tile of a global relabel, by one warp: the in-tile BFS seeded by the tile's sink pixels
 // and (frontier rounds) the halo distances, the heights written back, and the neighbours queued
 // that a changed edge distance could lower.  T: the warp's 32 x 33 words of shared memory (used
-// beyond BFS_NEAR_CAP only).  Returns whether the tile holds an active pixel (-1: nothing
+// where distances span more than BFS_RANGE only).  Returns whether the tile holds an active pixel (-1: nothing
 // changed since the tile's last round).
 //
 // Bound by latency and by the 4 KiB of heights a tile stores.  So: a tile whose heights are all
@@ -1579,16 +1600,15 @@ __device__ __forceinline__ int bfs_tile(const PoolView& P, int t, int lane, int 
                               (sl < oL && sl <= lim) || (sr < oR && sr <= lim)))
       return -1;
   }
-  uint32_t fin;
   int nT, nB, nL, nR;   // the edges now
   int state = 0;        // hstate: 1 all 0, 2 all unreached, 0 neither
-  if (cap <= BFS_NEAR_CAP) {
-    const NearBfs B = tile_bfs_near(sink, canU, canD, canL, canR, lane, !first, top, bot, sl, sr, cap);
-    fin = B.vis;
+  const PlaneBfs B = tile_bfs_planes(sink, canU, canD, canL, canR, lane, !first, top, bot, sl, sr, cap);
+  uint32_t fin = B.vis;
+  if (B.whole) {
     uint32_t any = 0;
 #pragma unroll
     for (int b = 0; b < BFS_PLANES; ++b) any |= B.plane[b];
-    if (__all_sync(FULL, fin == FULL && any == 0)) state = 1;
+    if (B.base == 0 && __all_sync(FULL, fin == FULL && any == 0)) state = 1;
     else if (__all_sync(FULL, fin == 0)) state = 2;
     nT = B.across(0, lane);
     nB = B.across(31, lane);
@@ -1604,8 +1624,10 @@ __device__ __forceinline__ int bfs_tile(const PoolView& P, int t, int lane, int 
         for (int b = 0; b < BFS_PLANES; ++b)
           d4 |= spread4(__shfl_sync(FULL, B.plane[b], src) >> (4 * q)) << b;
         const uint32_t f4 = __shfl_sync(FULL, B.vis, src) >> (4 * q);
-        const int4 v = make_int4(f4 & 1u ? (int)(d4 & 255u) : GC_HINF, f4 & 2u ? (int)((d4 >> 8) & 255u) : GC_HINF,
-                                 f4 & 4u ? (int)((d4 >> 16) & 255u) : GC_HINF, f4 & 8u ? (int)(d4 >> 24) : GC_HINF);
+        const int4 v = make_int4(f4 & 1u ? B.base + (int)(d4 & 255u) : GC_HINF,
+                                 f4 & 2u ? B.base + (int)((d4 >> 8) & 255u) : GC_HINF,
+                                 f4 & 4u ? B.base + (int)((d4 >> 16) & 255u) : GC_HINF,
+                                 f4 & 8u ? B.base + (int)(d4 >> 24) : GC_HINF);
         *(int4*)(P.hgt + base + src * GC_TILE + 4 * q) = v;
       }
     }

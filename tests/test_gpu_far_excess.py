@@ -1,5 +1,5 @@
 """Solves whose excess lies far from every sink: the first list of a fresh solve is empty (no
-sink in or beside a tile with excess) and the relabel's distance cap (16, then twice as far
+sink in or beside a tile with excess) and the relabel's distance cap (8, then twice as far
 whenever no excess lies within it, and each cycle) has to grow, past its last finite value on
 the longest grid.  Flow and canonical cut equal the exact oracle's, for the one-launch solve
 and the host-driven loop, fresh and after an edit that moves the excess."""
@@ -101,3 +101,30 @@ def test_solves_of_both_kinds_and_steps_alternate(cuda, oracle):
                 gc.cut()
                 assert gc.flow == f_ref, (k, prof)
                 assert np.array_equal(gc.labels().cpu().numpy(), l_ref), (k, prof)
+
+
+@pytest.mark.parametrize("graph", [True, False])
+@pytest.mark.parametrize("w,h", [(8, 32), (9, 31), (32, 32), (70, 40)])
+def test_snake_distances(cuda, oracle, w, h, graph):
+    """Residual edges along one winding path only: distances inside a tile of 255, 256 and more,
+    and tiles entered again and again at far distances.  A global relabel gives the distance
+    along the path; the solve equals the oracle's."""
+    path = [(y, x) for y in range(h) for x in (range(w) if y % 2 == 0 else range(w - 1, -1, -1))]
+    planes = [np.zeros((h, w), np.int32) for _ in range(5)]
+    up, down, left, right, excess = planes
+    for (y0, x0), (y1, x1) in zip(path, path[1:]):
+        a, b = {(1, 0): (down, up), (0, 1): (right, left), (0, -1): (left, right)}[y1 - y0, x1 - x0]
+        a[y0, x0] = b[y1, x1] = 7
+    excess[path[-1]] = 30      # the far end; the sink is the first corner
+    excess[0, 0] = -20
+    with GraphCut(w, h, use_graph=graph) as gc:
+        gc.upload_capacities(*planes)
+        gc.startBfs()
+        want = np.zeros((h, w), np.int64)
+        for d, p in enumerate(path):
+            want[p] = d
+        assert np.array_equal(gc.dHeight.cpu().numpy(), want)
+        gc.upload_capacities(*planes)
+        f_ref, l_ref = oracle.maxflow_bk(*planes)
+        assert np.array_equal(gc.cut_labels().cpu().numpy(), l_ref)
+        assert gc.flow == f_ref
