@@ -1,10 +1,9 @@
 // C ABI of libgcut.so: tile pools, the solve loop and the data-parallel primitives.
 //
-// The host loop mirrors GraphCut.cut (GraphCut.pyx:348-418) at a coarser grain: where the
-// reference enqueues ~30 kernels and blocks on ~5 device->host reads per push iteration,
-// a cycle here is `pulses_per_relabel` x {discharge, edge-relabel + list rebuild} and one
-// exact global relabel, all enqueued without a host wait; the host reads one int (the
-// active-tile count) per cycle and one per few BFS rounds.
+// A solve replaces GraphCut.cut (GraphCut.pyx:348-418), which enqueues ~30 kernels and blocks
+// on ~5 device->host reads per push iteration: here it is one launch (k_solve) and one host
+// wait.  solve_host runs the same steps as separate launches decided by the host, for
+// profiling and stats collection.
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -243,8 +242,15 @@ struct Pool {
     if (!edit_pending) return GC_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(s, &cap));
-    if (cap == cudaStreamCaptureStatusNone) CK(cudaStreamWaitEvent(s, done_ev, 0));
-    else CK(cudaEventSynchronize(done_ev));   // a capture cannot wait for an event outside it
+    if (cap == cudaStreamCaptureStatusNone) {
+      CK(cudaStreamWaitEvent(s, done_ev, 0));
+    } else {   // a capture cannot wait for an event outside it: the host does
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      CK(cudaThreadExchangeStreamCaptureMode(&mode));
+      const cudaError_t e = cudaEventSynchronize(done_ev);
+      CK(cudaThreadExchangeStreamCaptureMode(&mode));
+      CK(e);
+    }
     edit_pending = false;
     return GC_OK;
   }
@@ -561,8 +567,7 @@ struct Pool {
     return set_selection(all.data(), (int)all.size(), any_warm, s);
   }
 
-  // exact BFS distances to the sink pixels (global relabel); sets tact.  h: condition
-  // handle when captured into a graph (0: host-driven rounds)
+  // exact BFS distances to the sink pixels (global relabel); sets tact
   int global_relabel(cudaStream_t s, int first = 1) {
     RK(timed(K_MASKS, s, [&] { return launch_masks(P, grid_warps, s); }));
     RK(timed(K_BFS_FIRST, s, [&] { return launch_bfs_round(P, first, GC_HINF, 0, grid_warps, s); }));

@@ -121,3 +121,23 @@ def test_stroke_points_in_the_launch_and_copied(cuda, npts, radius):
             got = gc.dExcess
             other.synchronize()
         assert np.array_equal(got.cpu().numpy(), want)
+
+
+def test_upload_captured_after_an_edit(cuda, oracle):
+    """A stroke is still on its way when the next upload is captured into a CUDA graph: the
+    capture holds the upload alone, and its replay gives the cold solve."""
+    torch = cuda
+    g = synth.make_graph(130, 70, 5)
+    planes = [torch.from_numpy(p).cuda() for p in g.planes()]
+    f_ref, l_ref = oracle.maxflow_bk(*g.planes())
+    with GraphCut(g.width, g.height) as gc:
+        gc.upload_capacities(*planes)
+        gc.cut()
+        graph = torch.cuda.CUDAGraph()
+        gc.edit_stroke([3, 100], [5, 60], 4, 500)
+        with torch.cuda.graph(graph):
+            gc.upload_capacities(*planes)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(gc.cut_labels().cpu().numpy(), l_ref)
+        assert gc.flow == f_ref
