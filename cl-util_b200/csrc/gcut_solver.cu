@@ -6,6 +6,10 @@
 // relabels the whole image with a Jacobi pass (:538-577) and computes the global relabel
 // with init_bfs/bfs_intratile/bfs_intertile (:582-1016) over compacted tile lists.  Here:
 //
+//  * k_solve       a whole solve in one cooperative launch: the steps below with grid barriers
+//                  between them, the loops decided on the device.  The kernels named here run
+//                  the same steps as launches of their own, for the manual stepping calls and
+//                  the host-driven loop.
 //  * k_discharge   one CTA of 256 threads per listed tile (persistent over the device-side
 //                  list): the tile's excess, height and four residual planes arrive in shared
 //                  memory by bulk copy (the next tile's copy overlaps this tile's work), with
@@ -20,10 +24,10 @@
 //                  active-tile list with the single-pass decoupled look-back compaction in
 //                  the same launch (IncrementalTileList.build + StreamCompact + PrefixSum);
 //                  the manual relabel step (GraphCut.relabel) only.
-//  * k_bfs_round   exact global relabel: per tile, one warp runs a bit-parallel multi-source
-//                  BFS (32-bit row masks of residual edges, lane = row) seeded by sink
-//                  pixels and by the halo distances, and marks neighbours whose edge
-//                  distances changed; the marked tiles form the next frontier.
+//  * k_bfs_round   global relabel, exact up to a distance cap: per tile, one warp runs a
+//                  bit-parallel multi-source BFS (32-bit row masks of residual edges, lane =
+//                  row) seeded by sink pixels and by the halo distances, and queues neighbours
+//                  whose edge distances could drop for the next round.
 //  * k_flood_round canonical cut: the same tile rounds flood the set reachable from excess
 //                  pixels over residual edges (the minimal source set).
 #include <cstdio>
@@ -47,22 +51,31 @@ __device__ __forceinline__ int imin(int a, int b) { return a < b ? a : b; }
 // isolated (all zero).  Heights start at 0 for sink pixels and 1 otherwise (a valid
 // labelling).  Replaces init_gc + load_tiles (graphcut.cl:63-112, 1033-1132).
 // ------------------------------------------------------------------------------------
-// Spreads bits 0..7 of x to bit positions 0, 4, ..., 28.
-__device__ __forceinline__ uint32_t spread8(uint32_t x) {
-  x &= 0xffu;
-  x = (x | (x << 12)) & 0x000F000Fu;
-  x = (x | (x << 6)) & 0x03030303u;
-  x = (x | (x << 3)) & 0x11111111u;
-  return x;
-}
-
-// Row mask of row (lane & 3) of this warp's four rows, from the ballots of the four pixels
-// each thread holds (thread (g, q) of the warp holds pixels 4q..4q+3 of row g).
-__device__ __forceinline__ uint32_t warp_row_mask(uint32_t b0, uint32_t b1, uint32_t b2, uint32_t b3,
-                                                  int ri) {
-  const int sh = 8 * ri;
-  return spread8(b0 >> sh) | (spread8(b1 >> sh) << 1) | (spread8(b2 >> sh) << 2) |
-         (spread8(b3 >> sh) << 3);
+// Row masks of four rows from a warp whose thread (g, q) holds pixels 4q..4q+3 of row g: thread
+// (g, k) returns mask k of row g (0-3: residual edge up / down / left / right, 4: sink, 5:
+// positive excess; 6, 7: nothing).  Each thread packs its four pixels of every mask as nibble k
+// of a word, and the eight threads of a row transpose their 8 x 8 nibbles: three shuffles.  (A
+// ballot per mask and pixel, its bits then spread, took 300 instructions a thread for 70, and
+// kept the ALU pipe of the uploads 68 % busy: 2048x2048 planes 35.5 us, now 32.2.)
+__device__ __forceinline__ uint32_t row_masks(const int (&e)[4], const int (&cu)[4], const int (&cd)[4],
+                                              const int (&cl)[4], const int (&cr)[4], int lane) {
+  uint32_t w = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    w |= cu[j] > 0 ? 1u << j : 0u;
+    w |= cd[j] > 0 ? 0x10u << j : 0u;
+    w |= cl[j] > 0 ? 0x100u << j : 0u;
+    w |= cr[j] > 0 ? 0x1000u << j : 0u;
+    w |= e[j] < 0 ? 0x10000u << j : 0u;
+    w |= e[j] > 0 ? 0x100000u << j : 0u;
+  }
+  const unsigned F = 0xffffffffu;
+  // halves, bytes, nibbles with the thread 4, 2, 1 further
+  w = __byte_perm(w, __shfl_xor_sync(F, w, 4), lane & 4 ? 0x3276 : 0x5410);
+  w = __byte_perm(w, __shfl_xor_sync(F, w, 2), lane & 2 ? 0x3715 : 0x6240);
+  const uint32_t o = __shfl_xor_sync(F, w, 1);
+  const uint32_t keep = lane & 1 ? 0xf0f0f0f0u : 0x0f0f0f0fu;
+  return (w & keep) | (__funnelshift_l(o, o, lane & 1 ? 28 : 4) & ~keep);
 }
 
 // Row masks of tile t (residual edge up / down / left / right, sink, positive excess) from
@@ -71,27 +84,10 @@ __device__ __forceinline__ uint32_t warp_row_mask(uint32_t b0, uint32_t b1, uint
 __device__ __forceinline__ void write_tile_masks(const PoolView& P, int t, const int (&e)[4],
                                                  const int (&cu)[4], const int (&cd)[4],
                                                  const int (&cl)[4], const int (&cr)[4]) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const unsigned F = 0xffffffffu;
-  uint32_t m[6];
-  const int* planes4[4] = {cu, cd, cl, cr};
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int* v = planes4[k];
-    m[k] = warp_row_mask(__ballot_sync(F, v[0] > 0), __ballot_sync(F, v[1] > 0),
-                         __ballot_sync(F, v[2] > 0), __ballot_sync(F, v[3] > 0), lane & 3);
-  }
-  m[4] = warp_row_mask(__ballot_sync(F, e[0] < 0), __ballot_sync(F, e[1] < 0),
-                       __ballot_sync(F, e[2] < 0), __ballot_sync(F, e[3] < 0), lane & 3);
-  m[5] = warp_row_mask(__ballot_sync(F, e[0] > 0), __ballot_sync(F, e[1] > 0),
-                       __ballot_sync(F, e[2] > 0), __ballot_sync(F, e[3] > 0), lane & 3);
-  if (lane < 4) {
-    const int row = 4 * w + lane;
-    uint32_t* mc = P.mcan + (long long)t * 128;
-    mc[row] = m[0]; mc[32 + row] = m[1]; mc[64 + row] = m[2]; mc[96 + row] = m[3];
-    P.msink[(long long)t * 32 + row] = m[4];
-    P.mexc[(long long)t * 32 + row] = m[5];
-  }
+  const int lane = threadIdx.x & 31, k = lane & 7;
+  const uint32_t m = row_masks(e, cu, cd, cl, cr, lane);
+  uint32_t* const dst = k < 4 ? P.mcan + (long long)t * 128 + 32 * k : (k == 4 ? P.msink : P.mexc) + (long long)t * 32;
+  if (k < 6) dst[threadIdx.x >> 3] = m;
 }
 
 // Tile t's planes changed after its masks were written: the first flood round that covers
@@ -320,8 +316,8 @@ struct RefWeight {
 // difference and a byte dot product (two instructions, not eleven).
 //
 // Bound by the planes it writes, 28 of 36 bytes a pixel (92 us at 4096x4096 and the copy rate):
-// 134 us there (166 with the distances a channel at a time and two dependent table reads a
-// weight), 1920x1080 18.8 us (23.6).  Eight CTAs an SM in place of five change nothing.
+// 121 us there (166 with the distances a channel at a time, two dependent table reads a weight
+// and a ballot per mask and pixel), 1920x1080 16.5 us (23.6).  Eight CTAs an SM in place of five change nothing.
 struct RgbaSource {
   const uint32_t* rgba;
   const int32_t* excess;
@@ -1999,9 +1995,12 @@ __global__ void k_labels_packed(PoolView P, ImageDesc im, uint8_t* out) {
 // The whole solve as one cooperative launch: every CTA runs the same steps (pulses, flood
 // rounds, relabel rounds), with a grid barrier after each.
 //
-// A barrier costs about 2 us.  The CUDA graph this replaces (the same steps as kernel nodes
-// under WHILE and IF nodes) paid a kernel's launch and drain per step and 5-11 us per
-// conditional node passed.
+// Bound by latency: a step of a few tiles is its barrier (1.5 us), a chain of L2 trips and one
+// tile's work, and a solve is 5 to 30 such steps (hundreds on the hardest grids); the pulses of
+// large grids are bound by the ALU pipe (integer minima and selects run at half rate).  As a
+// CUDA graph (the same steps as kernel nodes under WHILE and IF nodes) each step paid a launch
+// and a drain, and 5-11 us per conditional node: 256x192 98-169 us from upload to labels against
+// 35-71 now, 2048x2048 300-690 against 145-230, strokes at 4096x4096 210-650 against 112-123.
 // ------------------------------------------------------------------------------------
 // A barrier wait gives up after this long (a step of the largest pool takes well under a
 // second): it raises the abort flag, and every CTA leaves at its next barrier.
@@ -2252,15 +2251,9 @@ __device__ __forceinline__ void flood_first_phase(const PoolView& P, const Solve
         const int w = __ffs(todo) - 1;
         const int td = __shfl_sync(FULL, dt, w);
         todo &= todo - 1;
-        uint32_t k[6];
-#pragma unroll
-        for (int p = 0; p < 4; ++p)
-          k[p] = warp_row_mask(__ballot_sync(FULL, v[p].x > 0), __ballot_sync(FULL, v[p].y > 0),
-                               __ballot_sync(FULL, v[p].z > 0), __ballot_sync(FULL, v[p].w > 0), lane & 3);
-        k[4] = warp_row_mask(__ballot_sync(FULL, v[4].x < 0), __ballot_sync(FULL, v[4].y < 0),
-                             __ballot_sync(FULL, v[4].z < 0), __ballot_sync(FULL, v[4].w < 0), lane & 3);
-        k[5] = warp_row_mask(__ballot_sync(FULL, v[4].x > 0), __ballot_sync(FULL, v[4].y > 0),
-                             __ballot_sync(FULL, v[4].z > 0), __ballot_sync(FULL, v[4].w > 0), lane & 3);
+        const uint32_t mk = row_masks({v[4].x, v[4].y, v[4].z, v[4].w}, {v[0].x, v[0].y, v[0].z, v[0].w},
+                                      {v[1].x, v[1].y, v[1].z, v[1].w}, {v[2].x, v[2].y, v[2].z, v[2].w},
+                                      {v[3].x, v[3].y, v[3].z, v[3].w}, lane);
         // sum of the positive excess, in halves that fit 32 bits over a warp's 128 pixels
         const unsigned e0 = v[4].x > 0 ? v[4].x : 0, e1 = v[4].y > 0 ? v[4].y : 0;
         const unsigned e2 = v[4].z > 0 ? v[4].z : 0, e3 = v[4].w > 0 ? v[4].w : 0;
@@ -2269,18 +2262,10 @@ __device__ __forceinline__ void flood_first_phase(const PoolView& P, const Solve
         if (todo) load(__shfl_sync(FULL, dt, __ffs(todo) - 1));   // the next tile's, in flight
         const unsigned slo = __reduce_add_sync(FULL, lo), shi = __reduce_add_sync(FULL, hi);
         uint32_t* const sw = sm + w * REB_WORDS;
-        if (lane < 4) {
-          const int row = 4 * warp + lane;
-          uint32_t* const mc = P.mcan + (long long)td * 128;
-#pragma unroll
-          for (int p = 0; p < 4; ++p) {
-            mc[32 * p + row] = k[p];
-            sw[32 * p + row] = k[p];
-          }
-          P.msink[(long long)td * 32 + row] = k[4];
-          P.mexc[(long long)td * 32 + row] = k[5];
-          sw[128 + row] = k[4];
-          sw[160 + row] = k[5];
+        const int k = lane & 7, row = tid >> 3;
+        if (k < 6) {
+          (k < 4 ? P.mcan + (long long)td * 128 + 32 * k : (k == 4 ? P.msink : P.mexc) + (long long)td * 32)[row] = mk;
+          sw[32 * k + row] = mk;
         }
         if (lane == 0) {
           sw[192 + 2 * warp] = slo;
