@@ -158,12 +158,14 @@ __device__ __forceinline__ void store_uploaded_tile(const PoolView& P, int t, in
                                                     const int (&cr)[4], int32_t* __restrict__ tl,
                                                     ImageAcc* acc) {
   int h[4], bad = 0;
-  long long pos = 0;
+  unsigned lo = 0, hi = 0;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     bad |= (cu[j] | cd[j] | cl[j] | cr[j]) < 0;
     h[j] = e[j] < 0 ? 0 : 1;
-    pos += e[j] > 0 ? e[j] : 0;
+    const unsigned p = e[j] > 0 ? e[j] : 0;
+    lo += p & 0xffffu;   // halves that fit 32 bits over a warp's 128 pixels
+    hi += p >> 16;
   }
   const bool p4 = e[0] > 0 || e[1] > 0 || e[2] > 0 || e[3] > 0;
   const bool s4 = e[0] < 0 || e[1] < 0 || e[2] < 0 || e[3] < 0;
@@ -184,8 +186,9 @@ __device__ __forceinline__ void store_uploaded_tile(const PoolView& P, int t, in
   if (threadIdx.x < 32) P.mreach[(long long)t * 32 + threadIdx.x] = 0u;   // no flood yet
   __shared__ long long wpos[DIS_THREADS / 32];
   __shared__ unsigned wflag[DIS_THREADS / 32];
-#pragma unroll
-  for (int o = 16; o; o >>= 1) pos += __shfl_xor_sync(0xffffffffu, pos, o);
+  lo = __reduce_add_sync(0xffffffffu, lo);
+  hi = __reduce_add_sync(0xffffffffu, hi);
+  const long long pos = (long long)hi * 65536 + lo;
   tf = __reduce_or_sync(0xffffffffu, tf);
   if ((threadIdx.x & 31) == 0) {
     wpos[threadIdx.x >> 5] = pos;
@@ -316,7 +319,7 @@ struct RefWeight {
 // difference and a byte dot product (two instructions, not eleven).
 //
 // Bound by the planes it writes, 28 of 36 bytes a pixel (92 us at 4096x4096 and the copy rate):
-// 121 us there (166 with the distances a channel at a time, two dependent table reads a weight
+// 119 us there (166 with the distances a channel at a time, two dependent table reads a weight
 // and a ballot per mask and pixel), 1920x1080 16.5 us (23.6).  Eight CTAs an SM in place of five change nothing.
 struct RgbaSource {
   const uint32_t* rgba;
