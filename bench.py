@@ -94,7 +94,7 @@ def parse():
                          "ncu summaries of those two kernels are made from")
     ap.add_argument("--host-driven", action="store_true",
                     help="solve loops decided by the host (use_graph=0); ncu does not profile "
-                         "kernels inside conditional CUDA-graph nodes, so profiling runs use this")
+                         "the steps of the one-launch solve apart, so profiling runs use this")
     return ap.parse_args()
 
 
@@ -367,7 +367,7 @@ def main():
         f_ref, l_ref = O.maxflow_bk(*g.planes())
         parity = bool(flow == f_ref and np.array_equal(lab, l_ref))
 
-        # timed region: one CUDA-graph launch per solve (profiling off)
+        # timed region: one launch per solve (profiling off)
         step_ms = []
         launches = 0
         clocks = ClockSampler(local)
@@ -383,22 +383,20 @@ def main():
                 ev1.record(stream)
                 ev1.synchronize()
                 step_ms.append(ev0.elapsed_time(ev1))
-                # + the upload and the solve graph's labels: the node after the first cycle
-                # writes them when that cycle ends the solve, else it returns at once and the
-                # node after the solve loop writes them
-                st = gc.stats()
-                launches += st["launches"] + 1 + (1 if st["cycles"] <= 1 else 2)
+                # the upload and the solve, which writes the labels itself; the host-driven
+                # loop launches every step, and the labels
+                launches += 2 if not args.host_driven else gc.stats()["launches"] + 2
         torch.cuda.synchronize()
         barrier()
         total_ms = reduce_max(sum(step_ms), torch.device("cuda", local))
         mpix_all = world * args.steps * W * H / 1e6
         value = mpix_all / (total_ms / 1000)
 
-        # the graph-mode timeline from the device-side trace (kernel start stamps inside the
-        # CUDA graph, which host profilers do not list): one solve, outside the timed region
+        # the timeline from the device-side trace (start stamps of the steps inside the one
+        # launch, which host profilers do not list): one solve, outside the timed region
         import _gcut
         gc.set_trace(True, stream=stream)
-        step()   # switching the trace on rebuilds the solve graph: not part of the timeline
+        step()   # a first traced step, not part of the timeline
         flush.fill_(1)
         stream.synchronize()
         gc.set_trace(True, stream=stream)   # a fresh trace
@@ -556,10 +554,16 @@ def main():
             e2e_models["gmm_fit"] = time_gmm_fit(g, stream, rank == 0 and world == 1
                                                  and not args.no_cpu_baseline)
 
-    # roofline of the dominant kernel (largest summed event time)
+    # roofline of the step's largest part: the upload by its span in the trace, a kind of solve
+    # step by its event time as a kernel of its own (the host-driven loop's rounds that find
+    # nothing to do would count there, so the choice is the trace's)
     peak, peak_kind = measured_peak()
-    dom = max(prof_tot.items(), key=lambda kv: kv[1]["ms"])
-    dname, d = dom
+    spans = {k: v for k, v in timeline.items() if k in ALGO_BYTES_PER_TILE}
+    dname = max(spans, key=lambda k: spans[k][1]) if spans else "discharge"
+    d = prof_tot.get(dname)
+    if not d or not d["launches"]:
+        n_dom, us_dom = spans.get(dname, [1, 0.0])
+        d = {"launches": n_dom, "ms": us_dom / 1000, "tiles": n_dom * ((W + 31) // 32) * ((H + 31) // 32)}
     algo_bytes = d["tiles"] * ALGO_BYTES_PER_TILE.get(dname, 0)
     if dname == "compact":
         algo_bytes = d["launches"] * ((W // 32) * (H // 32)) * 8
@@ -586,7 +590,7 @@ def main():
                                    "t-links x100, 50*exp(-beta*dI^2) n-links), seed 1+rank",
                        "l2": "flushed between steps (256 MiB write, outside the timed region)",
                        "parallelism": f"replicas x{world}",
-                       "loop": "host-driven" if args.host_driven else "one CUDA graph per solve",
+                       "loop": "host-driven" if args.host_driven else "one cooperative launch per solve",
                        "step": "GraphCut.upload_capacities from device planes, then "
                                "GraphCut.cut_labels (gc_solve_labels: the solve and the labels "
                                "into device memory, one host wait)",
@@ -601,8 +605,8 @@ def main():
             "gpu_launches": launches,
             "ms_per_step_host_driven": sum(prof_ms) / len(prof_ms),
             "graph_timeline_us": {"kernels": timeline, "upload_start_to_labels_start": timeline_total,
-                                  "how": "device-side trace of one graph solve: per kernel kind "
-                                         "[launches, us from its start to the next kernel's start]"},
+                                  "how": "device-side trace of one solve: per step kind "
+                                         "[steps, us from its start to the next step's start]"},
             "roofline": {"bound": "hbm", "kernel": dname, "achieved": achieved, "peak": peak,
                          "peak_kind": peak_kind, "unit": "GB/s",
                          "frac": achieved / peak if peak else None, "traffic": traffic,
@@ -692,7 +696,7 @@ def _percentile(xs, p):
 
 def run_batch(args):
     """Config 2: `--batch` (64) independent grids, sides drawn from {256, 384, ..., 1536},
-    solved together in one tile pool (one CUDA-graph launch per solve over a shared tile
+    solved together in one tile pool (one launch per solve over a shared tile
     worklist), against the same grids solved one at a time by the single-grid solver.
     Under torchrun each rank takes its LPT share of the grids (by pixel count); the job's
     time is the slowest rank's."""
@@ -782,7 +786,7 @@ def run_batch(args):
         "data": "synthetic",
         "config": {"workload": f"{len(all_shapes)} independent grids, sides uniform in "
                                "{256,384,...,1536}, built as the synthetic generator, seeds "
-                               "10000+i; one tile pool per rank, one CUDA-graph solve",
+                               "10000+i; one tile pool per rank, one launch a solve",
                    "total_mpix": mpix, "l2": "flushed between steps",
                    "parallelism": f"LPT split of the grids over {world} rank(s)"},
         "single_solver_one_at_a_time": {"value": mpix / (ms_single / 1000), "unit": UNIT,
@@ -1020,8 +1024,8 @@ def run_serving(args):
     dev_planes = [[torch.from_numpy(p).cuda() for p in g.planes()] for g in graphs]
     trace = poisson_trace(np.random.default_rng(6), args.rate, args.duration, len(graphs))
     budget = 64 << 30
-    # warm-up: an untimed trace of another seed (up to 15 s): the driver's first few hundred
-    # CUDA-graph instantiations in a process are slow, which is start-up, not serving
+    # warm-up: an untimed trace of another seed (up to 15 s): the first launches and pinned
+    # allocations of a process are start-up, not serving
     warm = poisson_trace(np.random.default_rng(7), args.rate, min(args.duration, 15.0),
                          len(graphs))
     run_trace(graphs, host_planes, warm, "batching", budget, seed=8)

@@ -86,7 +86,7 @@ enum BarSlot { BAR_ARRIVE = 0, BAR_STRIDE = 16, BAR_EXIT = 32, BAR_N = 48 };
 constexpr unsigned long long GC_BAR_ABORT = 1ull << 63;
 
 // Device-side loop control words.  In the host-driven loops the last CTA of every frontier
-// round advances the round parity; k_solve keeps its loop state in registers and uses the
+// round advances the round parity; k_solve keeps its loop state in shared memory and uses the
 // rotating counters (CTL_Q0.., CTL_F0.., CTL_H0..) and the totals.
 enum CtlSlot {
   CTL_RND = 0,        // frontier round number (its parity selects the mark buffer)

@@ -6,7 +6,7 @@ one of two servers with the same request / result interface:
 
 * ``BatchingServer``: continuous batching.  Every session lives in one session pool
   (session_pool.SessionPool, gcp_* in include/gcut.h); each tick of its worker takes every
-  request ready at that moment and solves them all in one launch of the pool's CUDA graph,
+  request ready at that moment and solves them all in one launch over the pool,
   so requests of different sizes overlap on the device and none waits for a graph build;
 * ``GraphCutServer``: the plain one-at-a-time solver, one GraphCut handle per session,
   described below.
@@ -522,8 +522,7 @@ class BatchingServer:
     images and applies the strokes, solves all of them together (gcp_solve), and reads every
     flow and bit-packed cut back.  Requests that arrive meanwhile join the next tick, so the
     solves of different sizes overlap on the device inside one launch instead of on
-    concurrent streams, and no request waits for a CUDA-graph construction: the pool's graph
-    is built at start-up.  Results do not depend on the mix: each session's flow value and
+    concurrent streams.  Results do not depend on the mix: each session's flow value and
     canonical cut are unique for its graph.
 
     Same request / result interface as GraphCutServer (submit, drain, close, results,
@@ -583,7 +582,7 @@ class BatchingServer:
         return lo
 
     def _warm_up(self):
-        """Builds the pool's CUDA graphs before the first request: a fresh solve and a warm
+        """Runs every kernel of a request once before the first one: a fresh solve and a warm
         one of a small image."""
         torch = self.torch
         t0 = self.pool.alloc_tiles(64, 64)

@@ -1,12 +1,12 @@
 """SessionPool: many resident graphs in one tile pool, any subset solved by one launch.
 
 The serving loop keeps every session's residual graph on the device between requests.
-With one solver handle per session, concurrent requests need concurrent streams and every
-new image size a CUDA-graph construction of its own.  A session pool (gcp_* in
+With one solver handle per session, concurrent requests need concurrent streams and a
+launch each.  A session pool (gcp_* in
 include/gcut.h) holds all sessions in one arena instead: a session opens on a slot with a
 range of the pool's tiles, and a solve takes a list of slots, so the requests that are
 ready at one moment (new images of different sizes, brush strokes on resident sessions) are
-solved together by one launch of the pool's CUDA graph, built once for the pool.
+solved together by one launch.
 
     pool = SessionPool(max_tiles=65536, max_sessions=256)
     t0 = pool.alloc_tiles(w, h)             # a range of tiles (None when full)

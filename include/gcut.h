@@ -60,17 +60,18 @@ typedef struct gc_opts {
                               heights 0 (sink pixels) / 1 (others) */
   int max_cycles;          /* cap on global-relabel cycles; exceeded -> GC_ERR_NOT_CONVERGED */
   int max_bfs_rounds;      /* cap on tile rounds of one BFS / flood fill */
-  int use_graph;           /* 1: the solve is one CUDA-graph launch whose loops are WHILE nodes
-                              decided on the device (one host wait per solve); 0: the host
-                              drives the loops (used when profiling is on) */
+  int use_graph;           /* 1: the solve is one launch of a persistent cooperative kernel
+                              that decides its loops on the device (one host wait per solve);
+                              0: the host drives the loops (used when profiling is on) */
 } gc_opts;
 
 typedef struct gc_stats {
   int64_t cycles;          /* global-relabel cycles of the last solve */
-  int64_t pulses;          /* discharge launches */
+  int64_t pulses;          /* discharge pulses */
   int64_t bfs_rounds;      /* tile rounds over all global relabels */
   int64_t flood_rounds;    /* tile rounds of the canonical-cut flood fill */
-  int64_t launches;        /* kernels launched by the last solve */
+  int64_t launches;        /* steps of the last solve: kernels launched by the host-driven
+                              loop, steps between grid barriers of the one-launch solve */
   int64_t tiles_discharged;/* sum over pulses of the active-list length (host-visible
                               only when stats collection is on) */
 } gc_stats;
@@ -217,7 +218,7 @@ int gc_gmm_fit(const uint32_t* samples, int n, int n_components, int max_iterati
 
 /* Max-flow to the final cut.  Replaces GraphCut.cut (GraphCut.pyx:348-418); warm-starts
    from the current residual graph when called again after gc_edit_tlinks.  Blocks the
-   calling host thread until the solve is done (one wait for the solve's CUDA graph; the
+   calling host thread until the solve is done (one wait for its one launch; the
    host-driven path of gc_set_profile / gc_set_collect_stats reads the loop counters between
    launches). */
 int gc_solve(gc_handle* h, void* stream);
@@ -301,20 +302,17 @@ int gc_set_profile(gc_handle* h, int on);
 int gc_get_profile(const gc_handle* h, gc_kernel_prof* out, int n);
 const char* gc_kernel_name(int kind);
 
-/* Device-side trace of the solves, for looking inside a CUDA-graph solve (whose kernels a
-   host profiler does not list): while on, the first thread of every solver kernel appends
-   (start time in ns of the GPU's global timer, kind) to a buffer of GC_TRACE_MAX entries in
-   the handle's memory; the difference of consecutive start times is a kernel's duration
-   including its launch.  Kinds: 0 solve start, 1 active-tile list, 2 discharge, 3 mask
+/* Device-side trace of the solves, for looking inside a one-launch solve (whose steps a host
+   profiler does not list): while on, the first thread of every solver kernel, and of every
+   step of the one-launch solve, appends (start time in ns of the GPU's global timer, kind) to
+   a buffer of GC_TRACE_MAX entries in the handle's memory; the difference of consecutive start
+   times is a step's duration including its launch or barrier.  Kinds: 0 solve start, 1 active-tile list, 2 discharge, 3 mask
    rebuild, 4 flood first round, 5 flood round, 6 flood check, 7 BFS first round, 8 BFS
    round, 9 upload, 10 labels, 11 solve end.  gc_set_trace turns it on or off and empties
    the buffer; gc_get_trace copies up to max_entries entries (two uint64 each) and sets *n
    to the number written since (it may exceed the buffer).  Both synchronise `stream`.
-   The kernels take the trace as an argument, so an untraced solve pays nothing for it;
-   switching it on or off therefore rebuilds the solve's CUDA graph at the next solve (one
-   graph instantiation; calling gc_set_trace again with the same state only empties the
-   buffer).  No counterpart in the reference (its host loop timed kernels with OpenCL
-   events). */
+   The kernels take the trace as an argument, so an untraced solve pays nothing for it.  No
+   counterpart in the reference (its host loop timed kernels with OpenCL events). */
 #define GC_TRACE_MAX 2048
 int gc_set_trace(gc_handle* h, int on, void* stream);
 int gc_get_trace(gc_handle* h, uint64_t* entries, int max_entries, int* n, void* stream);
@@ -451,9 +449,7 @@ int gcb_get_trace(gcb_handle* b, uint64_t* entries, int max_entries, int* n, voi
    A pool of max_tiles 32x32 tiles and max_sessions image slots in one arena.  An image
    (a serving session) opens on a slot with a caller-chosen range of tiles, keeps its
    residual graph there between requests, and any set of slots is solved together by one
-   launch of the pool's CUDA graph; the other slots keep their state and results.  The graph
-   is built on the pool's first solves (one for solves of fresh uploads only, one when some
-   slot continues from a previous flow), so requests never wait for a graph construction.
+   launch; the other slots keep their state and results.
    No counterpart in the reference (one GraphCut object per image, GraphCut.pyx:80-154).
    One caller thread and one stream per pool at a time. */
 typedef struct gcp_handle gcp_handle;
@@ -479,7 +475,7 @@ int gcp_edit_stroke(gcp_handle* p, int slot, const int32_t* xs, const int32_t* y
                     int radius, int32_t value, void* stream);
 int gcp_edit_brush(gcp_handle* p, int slot, const int32_t* xs, const int32_t* ys, int npts,
                    int radius, int32_t value, void* stream);
-/* Solves the n listed slots (distinct, open, uploaded) together: one graph launch; a slot
+/* Solves the n listed slots (distinct, open, uploaded) together: one launch; a slot
    uploaded since its last solve starts fresh, an edited or solved one warm-starts from its
    previous flow.  Blocks the calling thread until the solve is done. */
 int gcp_solve(gcp_handle* p, const int* slots, int n, void* stream);
