@@ -99,14 +99,12 @@ enum CtlSlot {
   CTL_ERR = 7,        // 1: round cap, 2: cycle cap, 3: copy wait gave up, 4: self-check,
                       // 5: grid-barrier wait gave up
   CTL_MAXROUNDS = 8,
-  CTL_MAXCYCLES = 9,
   CTL_PULSE = 10,     // discharge launches since the last list rebuild (parity = worklist)
   CTL_DDONE = 11,     // CTAs finished in the current discharge launch
   CTL_BAD = 12,       // first out-of-range worklist value seen by a self-check
   CTL_BADWHERE = 13,  // 1: worklist append, 2: worklist length, 3: list length, 4: image id
                       // (or tile) of the selection, 5: frontier append, 6: frontier length,
                       // 9: selection size
-  CTL_RESERVED = 14,
   CTL_NCHECK = 15,    // flood checks run (k_flood_check launches)
   CTL_NACT = 16,      // active-list rebuilds run (k_active_list launches)
   CTL_LEFT = 17,      // images still running after the last flood check
