@@ -16,9 +16,10 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "gcut_schedule.h"
+
 #define GC_TILE 32
 #define GC_TILE_PX 1024
-#define GC_HINF 0x3fffffff
 
 namespace gcut {
 
@@ -84,38 +85,6 @@ enum TileFlag { TF_POS = 1, TF_SINK = 2, TF_POS_UP = 4, TF_POS_DOWN = 8, TF_POS_
 // it.  The last CTA to leave clears all for the next launch.
 enum BarSlot { BAR_ARRIVE = 0, BAR_STRIDE = 16, BAR_EXIT = 32, BAR_N = 48 };
 constexpr unsigned long long GC_BAR_ABORT = 1ull << 63;
-
-// Device-side loop control words.  In the host-driven loops the last CTA of every frontier
-// round advances the round parity; k_solve keeps its loop state in shared memory and uses the
-// rotating counters (CTL_Q0.., CTL_F0.., CTL_H0..) and the totals.
-enum CtlSlot {
-  CTL_RND = 0,        // frontier round number (its parity selects the mark buffer)
-  CTL_DONE = 1,       // CTAs finished in the current round
-  CTL_LASTCNT = 2,    // tiles processed by the last finished round
-  CTL_ROUNDS = 3,     // rounds of the current frontier loop
-  CTL_BFS_TOTAL = 4,  // BFS rounds of the solve
-  CTL_FLOOD_TOTAL = 5,
-  CTL_CYCLES = 6,     // global-relabel cycles of the solve
-  CTL_ERR = 7,        // 1: round cap, 2: cycle cap, 3: copy wait gave up, 4: self-check,
-                      // 5: grid-barrier wait gave up
-  CTL_MAXROUNDS = 8,
-  CTL_PULSE = 10,     // discharge launches since the last list rebuild (parity = worklist)
-  CTL_DDONE = 11,     // CTAs finished in the current discharge launch
-  CTL_BAD = 12,       // first out-of-range worklist value seen by a self-check
-  CTL_BADWHERE = 13,  // 1: worklist append, 2: worklist length, 3: list length, 4: image id
-                      // (or tile) of the selection, 5: frontier append, 6: frontier length,
-                      // 9: selection size
-  CTL_NCHECK = 15,    // flood checks run (k_flood_check launches)
-  CTL_NACT = 16,      // active-list rebuilds run (k_active_list launches)
-  CTL_LEFT = 17,      // images still running after the last flood check
-  CTL_SCANERR = 18,   // the scan state's error word, as the last active list saw it
-  // k_solve's counters, three of each: a step reads one (filled by the step before), adds to
-  // the next and clears the third, so one grid barrier per step orders all three uses
-  CTL_Q0 = 20,        // worklist lengths
-  CTL_F0 = 24,        // frontier lengths
-  CTL_H0 = 28,        // images whose flood reached a sink
-  CTL_N = 64          // the control words fill 256 bytes; the per-image sums follow them
-};
 
 // Walks consecutive selected indices: the tile of index i, with the range found once by a
 // binary search over the ranges' first indices and then followed range by range.

@@ -92,50 +92,13 @@ int launch_ctl_begin(const PoolView& P, int max_rounds, ImageAcc* acc, cudaStrea
 // take part by fresh_tile_active; grid: most CTAs, which loop over the selection's chunks
 int launch_active_list(const PoolView& P, const ScanState& st, int32_t* list, int32_t* count,
                        int live, int fresh, int grid, cudaStream_t s);
-// The schedule of a solve: pulses and sweeps of cycle `cycle` (0, 1, ...) from the handle's
-// options, and the relabel's distance cap (its first value, and the next after `cap`).
-//
-// A cycle costs a flood and a relabel over the images left (60 us at 2048^2) besides its
-// pulses (10 us each on a few hundred tiles).  Most solves end after one or two cycles, which
-// the options' own schedule suits; the excess left after that has to travel far, and then more
-// work between relabels pays: twice the sweeps from the second cycle, twice the pulses with
-// each from the third.  Mean over 12 seeds against the fixed schedule 3 x 2 (and its worst
-// seed), one B200: 2048^2 1740 -> 515 us (13133 -> 3216), 512^2 424 -> 241, 803x607 under the
-// lamda rule 690 -> 317, 4096^2 image 1108 -> 974.
-__device__ __host__ __forceinline__ int cycle_pulses(int pulses, int cycle) {
-  const int most = pulses > 16 ? pulses : 16;
-  const int shift = cycle < 2 ? 0 : cycle - 1 < 4 ? cycle - 1 : 4;
-  const long long p = (long long)pulses << shift;
-  return p < most ? (int)p : most;
-}
-__device__ __host__ __forceinline__ int cycle_iters(int iters, int cycle) {
-  return cycle == 0 ? iters : iters + 3;
-}
-// Active heights before the first relabel, whose trivial labels (0 at sinks, 1 elsewhere) say
-// little: below 4, excess far from a sink stops rising after three sweeps instead of keeping
-// its warps busy.  (3: more cycles; unlimited: 512^2 3 %, 64 grids 4 % slower.)
-constexpr int kFirstLimit = 4;
-// The first relabel reaches 8 pixels around the sinks: what is further out gets its distances
-// with a later cap, if it is still active then.  (Mean us over 12 seeds, caps 4 / 8 / 10: 64 grids
-// 5025 / 4613 / 4844, 1920x1080 models 290 / 264 / 272, 4096^2 image 727 / 686 / 682; over 9 seeds,
-// caps 16 / 8: models 287 / 273, 12 sessions 516 / 491, strokes at 4096^2 145 / 140.)
-constexpr int kFirstCap = 8;
-constexpr int kLastCap = 1 << 12;   // above it: exact distances
-__device__ __host__ __forceinline__ int next_cap(int cap) {
-  return cap >= kLastCap ? GC_HINF : cap * 2;
-}
 // The whole solve as one cooperative launch of `grid` CTAs (at most occupancy_solve()).
-struct SolveArgs {
+struct SolveArgs : SolvePlan {
   ImageAcc* acc;
   int ranges, tiles;        // the selection's size (its ranges are in P.sel)
   int4 sel0;                // its first range
   int mode0;                // and its mode
-  int stamp0;               // every stamp in img_hit is at most this; the floods take the next ones
   int clean;                // leave the counters and sums at zero (the results reach the host)
-  int warm, fresh;          // some selected image continues from a flow / is freshly uploaded
-  int iters, pulses;        // sweeps per discharge, discharges per cycle
-  int max_rounds, max_cycles;
-  int cap;                  // distance cap of the first relabel
   int lmode;                // 0 no labels; image im's labels: 1 a byte per pixel, 2 packed
   uint8_t* labels;
   ImageDesc im;

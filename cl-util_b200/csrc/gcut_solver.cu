@@ -2015,116 +2015,6 @@ __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long lon
   return v;
 }
 
-// The solve's loop state, one copy per CTA in shared memory, written by thread 0 only (inside
-// solve_barrier): the same in every CTA, because it follows from the same counters.  Kept out
-// of registers: what a step spills is reloaded from L2, since the barriers' fences empty L1.
-enum SolveStep { ST_LIST, ST_PULSE, ST_FLOOD_FIRST, ST_FLOOD, ST_BFS_FIRST, ST_BFS, ST_END };
-struct SolveState {
-  int step;
-  int cyc;                  // 0 before the first pulses (warm images' flood, first list)
-  int n;                    // tiles of the step's list
-  int pulse, pulses, iters; // of the cycle
-  int qk, fk;               // steps of the worklist and of the frontier (counter slots mod 3)
-  int stamp, prev;          // the flood's stamp, the one before it (0: none)
-  int cycles, cap, hlim;    // finished cycles; the next relabel's cap, the last one's limit
-  int rounds;               // of the flood or relabel that runs
-  int nf, nb, np;           // flood rounds, relabel rounds, pulses of the solve
-  int err;
-  int push;                 // tiles this CTA has queued since the last barrier
-  unsigned bar;             // barriers passed
-  unsigned last[2];         // sums of the barrier words' last uses
-};
-
-__device__ __forceinline__ void begin_cycle(const SolveArgs& A, SolveState& s, int list) {
-  ++s.cyc;
-  s.n = list;
-  s.pulse = 0;
-  s.pulses = cycle_pulses(A.pulses, s.cycles);
-  s.iters = cycle_iters(A.iters, s.cycles);
-  s.step = ST_PULSE;
-}
-
-// The step after `s.step`, which the whole grid has finished; total: tiles queued in it.
-// Thread 0 only.
-__device__ __forceinline__ void next_step(const PoolView& P, const SolveArgs& A, SolveState& s, int total) {
-  int list = -1;   // >= 0: a cycle begins with a worklist of this length
-  s.n = total;
-  switch (s.step) {
-    case ST_LIST:
-      list = *((volatile int32_t*)&P.ctl[CTL_Q0 + s.qk % 3]);
-      break;
-    case ST_PULSE:
-      ++s.qk;
-      ++s.np;
-      if (++s.pulse < s.pulses && total > 0) break;
-      s.step = ST_FLOOD_FIRST;
-      s.prev = s.stamp == A.stamp0 ? 0 : s.stamp;
-      ++s.stamp;
-      break;
-    case ST_FLOOD_FIRST:
-    case ST_FLOOD: {
-      ++s.fk;
-      ++s.nf;
-      ++s.rounds;
-      if (total > 0) {
-        s.step = ST_FLOOD;
-        if (s.rounds >= A.max_rounds) s.err = 1;
-        break;
-      }
-      const int left = *((volatile int32_t*)&P.ctl[CTL_H0 + s.stamp % 3]);   // images that met a sink
-      if (s.cyc > 0) ++s.cycles;
-      if (blockIdx.x == 0) trace_record(P, TR_CHECK);
-      s.rounds = 0;
-      s.step = left > 0 ? ST_BFS_FIRST : s.cyc == 0 && A.fresh ? ST_LIST : ST_END;
-      break;
-    }
-    case ST_BFS_FIRST:
-    case ST_BFS:
-      ++s.fk;
-      ++s.nb;
-      ++s.rounds;
-      if (total > 0) {
-        s.step = ST_BFS;
-        if (s.rounds >= A.max_rounds) s.err = 1;
-        break;
-      }
-      s.rounds = 0;
-      list = *((volatile int32_t*)&P.ctl[CTL_Q0 + s.qk % 3]);
-      if (list == 0 && s.cap < GC_HINF) {   // no excess within the cap of a sink: further out
-        s.cap = next_cap(s.cap);
-        s.step = ST_BFS_FIRST;
-        list = -1;
-        break;
-      }
-      s.hlim = s.cap < GC_HINF ? s.cap + 1 : GC_HINF;
-      s.cap = next_cap(s.cap);   // further out with every cycle
-      if (s.cyc == 0 && A.fresh) {
-        s.step = ST_LIST;
-        list = -1;
-      }
-      break;
-  }
-  if (list >= 0) {
-    if (list == 0 && s.step != ST_LIST) {
-      s.step = ST_END;
-    } else if (s.cycles >= A.max_cycles) {
-      s.err = 2;
-    } else {
-      begin_cycle(A, s, list);
-      if (list == 0) {   // no fresh tile is near a sink: straight to the flood
-        s.step = ST_FLOOD_FIRST;
-        s.prev = s.stamp == A.stamp0 ? 0 : s.stamp;
-        ++s.stamp;
-      }
-    }
-  }
-  if (s.n < 0 || s.n > P.nt) {   // self-check: a list holds each tile at most once
-    record_bad(P, 6, s.n);
-    s.err = 4;
-  }
-  if (s.err) s.step = ST_END;
-}
-
 // Grid barrier and step change: every CTA's writes before it are visible to every CTA after
 // it, its bulk copies included, and `s` holds the next step.  The CTAs' counts of queued tiles
 // travel in the upper half of the arrival word, so the loop decision needs no second trip to L2
@@ -2170,7 +2060,10 @@ __device__ __forceinline__ void solve_barrier(const PoolView& P, const SolveArgs
       s.err = 5;
       s.step = ST_END;
     } else {
-      next_step(P, A, s, (int)total);
+      const int was = s.step;
+      next_step(P.ctl, P.nt, A, s, (int)total);
+      if (blockIdx.x == 0 && total == 0 && (was == ST_FLOOD_FIRST || was == ST_FLOOD)) trace_record(P, TR_CHECK);
+      if (s.err == 4) record_bad(P, 6, (int)total);
     }
   }
   __syncthreads();
@@ -2359,14 +2252,13 @@ k_solve(PoolView P, SolveArgs A) {
 
   for (int step = st.step; step != ST_END; step = st.step) {
     if (step == ST_PULSE) {
-      // reads counter qk, adds to qk + 1, clears qk + 2 (all mod 3)
       trace_mark(P, TR_DISCHARGE);
       const int qk = st.qk;
       const Worklist in{(qk & 1) ? P.queue[1] : P.queue[0], nullptr, (qk & 1) ? P.inq[1] : P.inq[0]};
-      Worklist out{(qk & 1) ? P.queue[0] : P.queue[1], &P.ctl[CTL_Q0 + (qk + 1) % 3],
+      Worklist out{(qk & 1) ? P.queue[0] : P.queue[1], &P.ctl[list_slot(st)],
                    (qk & 1) ? P.inq[0] : P.inq[1], &st.push};
       if (st.pulse == st.pulses - 1) out.list = nullptr;   // the relabel makes the next list
-      if (bid == 0 && tid == 0) P.ctl[CTL_Q0 + (qk + 2) % 3] = 0;
+      if (bid == 0 && tid == 0) P.ctl[list_slot_cleared(st)] = 0;
       discharge_phase(P, st.iters, st.hlim, bid, nb, in, st.n, out, dsm,
                       *reinterpret_cast<DisSmem*>(dsm + DIS_PLANES * GC_TILE_PX), &mbar, phase);
     } else if (step == ST_FLOOD_FIRST) {
@@ -2405,7 +2297,7 @@ k_solve(PoolView P, SolveArgs A) {
       if (first && bid == 0)   // their sums start afresh with their next flood
         for (int i = tid; i < P.nimg; i += DIS_THREADS)
           if (P.img_hit[i] == stamp) A.acc[i].sumpos_e = 0;
-      const Worklist act_out{(qk & 1) ? P.queue[1] : P.queue[0], &P.ctl[CTL_Q0 + qk % 3], nullptr};
+      const Worklist act_out{(qk & 1) ? P.queue[1] : P.queue[0], &P.ctl[list_slot(st)], nullptr};
       const Worklist out{(fk & 1) ? P.fq[0] : P.fq[1], &P.ctl[CTL_F0 + (fk + 1) % 3],
                          (fk & 1) ? P.mark[0] : P.mark[1], &st.push};
       const int32_t* const list = (fk & 1) ? P.fq[1] : P.fq[0];
@@ -2428,7 +2320,7 @@ k_solve(PoolView P, SolveArgs A) {
       // the fresh images' first list
       trace_mark(P, TR_ACTIVE_LIST);
       const int qk = st.qk;
-      const Worklist act_out{(qk & 1) ? P.queue[1] : P.queue[0], &P.ctl[CTL_Q0 + qk % 3], nullptr};
+      const Worklist act_out{(qk & 1) ? P.queue[1] : P.queue[0], &P.ctl[list_slot(st)], nullptr};
       const int i0 = bid * DIS_THREADS + tid;
       SelCursor cursor(P, A.ranges, i0 < A.tiles ? i0 : 0, A.sel0);
       for (int b = bid * DIS_THREADS; b < A.tiles; b += nb * DIS_THREADS) {   // CTA-uniform
