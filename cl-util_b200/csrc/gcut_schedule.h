@@ -39,7 +39,8 @@ enum CtlSlot {
   CTL_LEFT = 17,      // images still running after the last flood check
   CTL_SCANERR = 18,   // the scan state's error word, as the last active list saw it
   // k_solve's counters, three of each: a step reads one (filled by the step before), adds to
-  // the next and clears the third, so one grid barrier per step orders all three uses
+  // the next and clears the third, so one grid barrier per step orders all three uses (the
+  // worklists': list_slot)
   CTL_Q0 = 20,        // worklist lengths
   CTL_F0 = 24,        // frontier lengths
   CTL_H0 = 28,        // images whose flood reached a sink
@@ -93,7 +94,7 @@ struct SolveState {
   int cyc;                  // 0 before the first pulses (warm images' flood, first list)
   int n;                    // tiles of the step's list
   int pulse, pulses, iters; // of the cycle
-  int qk, fk;               // steps of the worklist and of the frontier (counter slots mod 3)
+  int qk, fk;               // worklists and frontier steps so far (counter slots mod 3)
   int stamp, prev;          // the flood's stamp, the one before it (0: none)
   int cycles, cap, hlim;    // finished cycles; the next relabel's cap, the last one's limit
   int rounds;               // of the flood or relabel that runs
@@ -105,10 +106,14 @@ struct SolveState {
 };
 
 // Worklist counter that a step adds the tiles it lists to (a pulse: the next worklist's), and
-// the one that it clears for a later step (-1: none).  next_step reads the former of a list or
-// relabel after the barrier, where other CTAs may be in the next step already.
+// the one that it clears for a later step (-1: none).  next_step reads a list's or relabel's
+// counter after the barrier, when other CTAs may be in the next step already: so a relabel that
+// starts over because it listed nothing counts in the next slot, and a slot is cleared a step
+// before it is counted in and not in the step after its reading.
 GC_HD int list_slot(const SolveState& s) { return CTL_Q0 + (s.step == ST_PULSE ? s.qk + 1 : s.qk) % 3; }
-GC_HD int list_slot_cleared(const SolveState& s) { return s.step == ST_PULSE ? CTL_Q0 + (s.qk + 2) % 3 : -1; }
+GC_HD int list_slot_cleared(const SolveState& s) {
+  return s.step == ST_PULSE ? CTL_Q0 + (s.qk + 2) % 3 : s.step == ST_BFS_FIRST ? CTL_Q0 + (s.qk + 1) % 3 : -1;
+}
 
 GC_HD void begin_cycle(const SolvePlan& A, SolveState& s, int list) {
   ++s.cyc;
@@ -166,6 +171,7 @@ GC_HD void next_step(const volatile int32_t* ctl, int nt, const SolvePlan& A, So
       list = ctl[list_slot(s)];
       if (list == 0 && s.cap < GC_HINF) {   // no excess within the cap of a sink: further out
         s.cap = next_cap(s.cap);
+        ++s.qk;   // this list's counter may still be read; the list is empty
         s.step = ST_BFS_FIRST;
         list = -1;
         break;

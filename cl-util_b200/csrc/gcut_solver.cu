@@ -2251,6 +2251,7 @@ k_solve(PoolView P, SolveArgs A) {
   __syncthreads();
 
   for (int step = st.step; step != ST_END; step = st.step) {
+    if (bid == 0 && tid == 0 && list_slot_cleared(st) >= 0) P.ctl[list_slot_cleared(st)] = 0;
     if (step == ST_PULSE) {
       trace_mark(P, TR_DISCHARGE);
       const int qk = st.qk;
@@ -2258,7 +2259,6 @@ k_solve(PoolView P, SolveArgs A) {
       Worklist out{(qk & 1) ? P.queue[0] : P.queue[1], &P.ctl[list_slot(st)],
                    (qk & 1) ? P.inq[0] : P.inq[1], &st.push};
       if (st.pulse == st.pulses - 1) out.list = nullptr;   // the relabel makes the next list
-      if (bid == 0 && tid == 0) P.ctl[list_slot_cleared(st)] = 0;
       discharge_phase(P, st.iters, st.hlim, bid, nb, in, st.n, out, dsm,
                       *reinterpret_cast<DisSmem*>(dsm + DIS_PLANES * GC_TILE_PX), &mbar, phase);
     } else if (step == ST_FLOOD_FIRST) {

@@ -1,0 +1,84 @@
+// Steps the decisions of a one-launch solve (csrc/gcut_schedule.h) for two CTAs, one of which
+// is always a whole step ahead: it has decided the next step and done that step's counting
+// before the other reads the counters of the step both have finished.  The steps' outcomes are
+// random.  Prints the first disagreement and returns 1, else returns 0.
+#include <cstdio>
+#include <cstring>
+#include <random>
+
+#include "gcut_schedule.h"
+
+using namespace gcut;
+
+namespace {
+
+bool same(const SolveState& a, const SolveState& b) {
+  return a.step == b.step && a.cyc == b.cyc && a.n == b.n && a.pulse == b.pulse && a.pulses == b.pulses &&
+         a.iters == b.iters && a.qk == b.qk && a.fk == b.fk && a.stamp == b.stamp && a.prev == b.prev &&
+         a.cycles == b.cycles && a.cap == b.cap && a.hlim == b.hlim && a.rounds == b.rounds && a.err == b.err;
+}
+
+bool makes_list(int step) { return step == ST_LIST || step == ST_BFS_FIRST || step == ST_BFS; }
+bool floods(int step) { return step == ST_FLOOD_FIRST || step == ST_FLOOD; }
+
+int run(unsigned seed, bool ahead_is_cta0) {
+  std::mt19937 rng(seed);
+  auto pick = [&](int n) { return (int)(rng() % (unsigned)n); };
+  SolvePlan plan{};
+  plan.stamp0 = pick(4);
+  plan.warm = pick(2);
+  plan.fresh = plan.warm ? pick(2) : 1;
+  plan.iters = 3;
+  plan.pulses = 1 + pick(3);
+  plan.max_rounds = plan.max_cycles = 1000;
+  plan.cap = kFirstCap;
+  SolveState ahead{};
+  ahead.cap = plan.cap;
+  ahead.hlim = kFirstLimit;
+  ahead.stamp = plan.stamp0 + plan.warm;
+  ahead.step = plan.warm ? ST_FLOOD_FIRST : ST_LIST;
+  SolveState behind = ahead;
+  int32_t ctl[CTL_N] = {};
+  int listed = 0;       // tiles of the worklist in the making
+  int last_total = 0;   // tiles queued in the step both have finished
+  for (int k = 0; k < 300 && ahead.step != ST_END; ++k) {
+    const int step = ahead.step;
+    const bool last_pulse = step == ST_PULSE && ahead.pulse == ahead.pulses - 1;   // queues nothing
+    const int total = step == ST_LIST || last_pulse || pick(3) ? 0 : 1 + pick(5);
+    const int tiles = makes_list(step) && pick(3) == 0 ? 1 + pick(5) : 0;
+    const int hits = floods(step) && pick(2);
+    if (step == ST_BFS_FIRST) listed = 0;
+    // the step counts from zero (a list that follows a relabel: from what that listed)
+    const int from = floods(step) ? ctl[CTL_H0 + ahead.stamp % 3] : ctl[list_slot(ahead)];
+    if ((step == ST_FLOOD_FIRST || step == ST_PULSE) ? from != 0 : makes_list(step) && from != listed)
+      return std::printf("seed %u: step %d counts from %d\n", seed, step, from), 1;
+    auto clear = [&](const SolveState& s) {
+      if (list_slot_cleared(s) >= 0) ctl[list_slot_cleared(s)] = 0;
+      if (s.step == ST_FLOOD_FIRST) ctl[CTL_H0 + (s.stamp + 1) % 3] = 0;
+    };
+    if (ahead_is_cta0) clear(ahead);
+    if (floods(step)) ctl[CTL_H0 + ahead.stamp % 3] += hits;
+    else ctl[list_slot(ahead)] += step == ST_PULSE ? total : tiles;
+    listed = step == ST_PULSE ? 0 : listed + tiles;
+    // the other CTA leaves the barrier of the step before only now
+    if (k > 0) next_step(ctl, 1000, plan, behind, last_total);
+    if (!same(ahead, behind))
+      return std::printf("seed %u: one CTA at step %d with a list of %d, another at step %d with %d\n", seed,
+                         ahead.step, ahead.n, behind.step, behind.n), 1;
+    if (!ahead_is_cta0) clear(behind);
+    next_step(ctl, 1000, plan, ahead, total);
+    last_total = total;
+    if (makes_list(step) && ahead.step == ST_PULSE && ahead.n != listed)
+      return std::printf("seed %u: a list of %d for %d tiles\n", seed, ahead.n, listed), 1;
+  }
+  return 0;
+}
+
+}  // namespace
+
+int main() {
+  for (unsigned seed = 0; seed < 20000; ++seed)
+    for (int cta0 = 0; cta0 < 2; ++cta0)
+      if (run(seed, cta0)) return 1;
+  return 0;
+}
