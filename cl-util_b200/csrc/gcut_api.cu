@@ -235,23 +235,26 @@ struct Pool {
     if (done_ev) cudaEventRecord(done_ev, s);
   }
 
-  // An edit returns before it has run (it used to wait for the copy of its points), so the next
-  // call that touches the planes waits for it on its own stream, whichever that is.
+  // An edit returns before it has run.  It has an event of its own, which no other call records
+  // (track moves done_ev to whatever stream a call came on), and every call that touches the
+  // planes waits for it on its own stream, whichever that is, until a solve has waited for one
+  // of them on the host.
+  cudaEvent_t edit_ev = nullptr;
   bool edit_pending = false;
   int order(cudaStream_t s) {
     if (!edit_pending) return GC_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(s, &cap));
     if (cap == cudaStreamCaptureStatusNone) {
-      CK(cudaStreamWaitEvent(s, done_ev, 0));
+      CK(cudaStreamWaitEvent(s, edit_ev, 0));
     } else {   // a capture cannot wait for an event outside it: the host does
       cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
       CK(cudaThreadExchangeStreamCaptureMode(&mode));
-      const cudaError_t e = cudaEventSynchronize(done_ev);
+      const cudaError_t e = cudaEventSynchronize(edit_ev);
       CK(cudaThreadExchangeStreamCaptureMode(&mode));
       CK(e);
+      edit_pending = false;
     }
-    edit_pending = false;
     return GC_OK;
   }
 
@@ -260,6 +263,11 @@ struct Pool {
       if (!own_arena) cudaEventSynchronize(done_ev);
       cudaEventDestroy(done_ev);
       done_ev = nullptr;
+    }
+    if (edit_ev) {
+      if (!own_arena) cudaEventSynchronize(edit_ev);
+      cudaEventDestroy(edit_ev);
+      edit_ev = nullptr;
     }
     if (stage) cudaFree(stage);   // host-upload staging, allocated on first use
     if (arena && own_arena) cudaFree(arena);
@@ -398,6 +406,8 @@ struct Pool {
     }
     e = cudaEventCreateWithFlags(&done_ev, cudaEventDisableTiming);
     if (e) { done_ev = nullptr; release(); return cuda_fail(e, "event"); }
+    e = cudaEventCreateWithFlags(&edit_ev, cudaEventDisableTiming);
+    if (e) { edit_ev = nullptr; release(); return cuda_fail(e, "event"); }
     Carve place{arena, 0};
     layout(place);
     // tracing starts off: the kernels see a null trace_ctl and skip the mark without a load
@@ -669,6 +679,7 @@ struct Pool {
     lists_stale = true;   // until this solve succeeds
     int r = host ? solve_host(s, warm, fresh, idx, n) : solve_launch(s, warm, fresh, idx, n, after, lmode, lbuf);
     if (r) return r;
+    edit_pending = false;   // the solve followed the edits, and the host has waited for it
     if (host && after) {   // the host-driven solve has finished: queue the work and wait
       RK((*after)(s));
       CK(cudaStreamSynchronize(s));
@@ -1357,9 +1368,14 @@ static int pool_edit(Pool& p, int img, const int32_t* xs, const int32_t* ys, int
   if (brush) RK(launch_brush(p.P, p.imgs[img], img, p.pts, pts.data(), npts, radius, value, p.tl, p.acc, s));
   else RK(launch_stroke(p.P, p.imgs[img], img, p.pts, pts.data(), npts, radius, value, p.tl, p.acc, s));
   p.track(s);
-  if (copy) CK(cudaStreamSynchronize(s));
-  else p.edit_pending = true;
   p.edited_image(img);
+  if (copy) {
+    CK(cudaStreamSynchronize(s));
+    p.edit_pending = false;
+  } else {
+    CK(cudaEventRecord(p.edit_ev, s));
+    p.edit_pending = true;
+  }
   return GC_OK;
 }
 

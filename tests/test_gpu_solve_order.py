@@ -37,3 +37,65 @@ def test_relabels_that_start_over(cuda, oracle, nearest):
             lab = gc.cut_labels()
             assert gc.flow == f_ref, k
             assert np.array_equal(lab.cpu().numpy(), l_ref), k
+
+
+def test_solve_after_an_edit_on_another_stream(cuda, oracle):
+    """A stroke on slot 0 waits behind other work on its stream; the labels of slot 1 are read on
+    a second stream, and slot 0 is solved on a third: the solve has the stroke in it."""
+    import strokes
+    import synth
+    from session_pool import SessionPool, tiles_of
+    graphs = [synth.make_graph(300, 200, 1), synth.make_graph(130, 70, 2)]
+    stroke = strokes.Stroke(np.array([40, 200], np.int32), np.array([30, 150], np.int32), 9, 900)
+    pool = SessionPool(sum(tiles_of(g.width, g.height) for g in graphs), 2)
+    a, b, c = (cuda.cuda.Stream() for _ in range(3))
+    for k, g in enumerate(graphs):
+        pool.open(k, g.width, g.height, pool.alloc_tiles(g.width, g.height))
+        pool.upload_capacities(k, *g.planes())
+    pool.solve([0, 1])
+    with cuda.cuda.stream(a):
+        cuda.cuda._sleep(20_000_000)   # about 10 ms
+    pool.edit_stroke(0, stroke.xs, stroke.ys, stroke.radius, stroke.value, stream=a)
+    with cuda.cuda.stream(b):
+        lab1 = pool.labels(1, stream=b)
+    b.synchronize()
+    assert np.array_equal(lab1.cpu().numpy(), oracle.maxflow_bk(*graphs[1].planes())[1])
+    pool.solve([0], stream=c)
+    g = graphs[0]
+    f_ref, l_ref = oracle.maxflow_bk(g.up, g.down, g.left, g.right, strokes.apply(g.excess, stroke))
+    assert pool.flow(0) == f_ref
+    assert np.array_equal(pool.labels(0).cpu().numpy(), l_ref)
+    cuda.cuda.synchronize()
+    pool.close_pool()
+
+
+@pytest.mark.parametrize("destroy", [False, True])
+def test_an_edit_behind_a_refused_call(cuda, oracle, destroy):
+    """A stroke waits behind other work on its stream; labels are refused on another stream (the
+    edit is not solved yet); then a cut on a third stream, or the end of a handle in caller-owned
+    memory, comes after the stroke."""
+    import _gcut
+    import strokes
+    import synth
+    g = synth.make_graph(130, 70, 3)
+    stroke = strokes.Stroke(np.array([20, 100], np.int32), np.array([10, 60], np.int32), 5, -700)
+    arena = cuda.zeros(GraphCut.arena_bytes(g.width, g.height) // 4 + 64, dtype=cuda.int32, device="cuda")
+    arena = arena[(-arena.data_ptr() % 256) // 4:]
+    a, b, c = (cuda.cuda.Stream() for _ in range(3))
+    gc = GraphCut(g.width, g.height, arena=arena)
+    gc.upload_capacities(*g.planes())
+    gc.cut()
+    with cuda.cuda.stream(a):
+        cuda.cuda._sleep(20_000_000)
+    gc.edit_stroke(stroke.xs, stroke.ys, stroke.radius, stroke.value, stream=a)
+    with pytest.raises(_gcut.GCError):
+        gc.labels(stream=b)
+    if destroy:
+        gc.close()
+        assert a.query()
+        return
+    gc.cut(stream=c)
+    f_ref, l_ref = oracle.maxflow_bk(g.up, g.down, g.left, g.right, strokes.apply(g.excess, stroke))
+    assert gc.flow == f_ref
+    assert np.array_equal(gc.labels().cpu().numpy(), l_ref)
+    gc.close()
