@@ -665,6 +665,8 @@ struct Pool {
     const bool host = prof || collect || !use_graph;
     one_launch = !host;
     list_valid = false;   // the next manual push starts from a new list
+    const bool bfs = bfs_fresh;
+    bfs_fresh = false;    // a solve that fails leaves no distances to go by
     // left by manual steps, a host-driven or a failed solve: worklist flags, barrier and control
     // words, stamps, sums
     if (lists_stale || stamp_base > (1 << 30)) {
@@ -690,6 +692,7 @@ struct Pool {
     // the host-driven loop leaves worklist flags, stamps and sums
     lists_stale = host || !P.host_out;
     stamp_base += h_ctl[CTL_CYCLES] + 2;   // a flood per cycle, one before the first
+    bfs_fresh = bfs;      // (see step_is_completed)
     for (int k = 0; k < n; ++k) {
       img_solved[idx[k]] = 1;
       img_edited[idx[k]] = 0;
@@ -901,10 +904,17 @@ struct Pool {
   int step_is_completed(int* done, cudaStream_t s) {
     if (!bfs_fresh) return fail(GC_ERR_STATE, "isCompleted is valid right after startBfs");
     RK(order(s));
+    bool cut = true;   // solved since startBfs, or before it: the cut and the sums are there
+    for (const uint8_t v : img_solved) cut = cut && v;
+    if (cut) {
+      *done = 1;
+      return GC_OK;
+    }
     int n;
     RK(read_count(s, &n));
     *done = n == 0;
     if (*done) {
+      lists_stale = true;   // the flood leaves its sums and stamps
       RK(launch_acc_reset(acc, (int)imgs.size(), s));
       RK(launch_flood_round(P, 1, 0, 1, acc, grid_warps, s));
       RK(frontier_rounds(s, /*flood=*/true, 0, 0, 1));

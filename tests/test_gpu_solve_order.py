@@ -99,3 +99,31 @@ def test_an_edit_behind_a_refused_call(cuda, oracle, destroy):
     assert gc.flow == f_ref
     assert np.array_equal(gc.labels().cpu().numpy(), l_ref)
     gc.close()
+
+
+@pytest.mark.parametrize("graph", [True, False])
+def test_is_completed_after_a_cut(cuda, oracle, graph):
+    """isCompleted once more after startBfs and a cut, fresh and warm: the cut is complete, and the
+    next cut's flow is not short of what that call summed.  After a cut that failed there are no
+    distances to go by, and isCompleted is refused."""
+    import _gcut
+    import synth
+    g = synth.make_graph(200, 130, 6)
+    f_ref, l_ref = oracle.maxflow_bk(*g.planes())
+    with GraphCut(g.width, g.height, use_graph=graph) as gc:
+        gc.upload_capacities(*g.planes())
+        for k in range(3):
+            gc.startBfs()
+            gc.cut()
+            assert gc.isCompleted() and gc.isCompleted(), k
+            assert gc.flow == f_ref, k
+            gc.cut()
+            assert gc.flow == f_ref, k
+            assert np.array_equal(gc.labels().cpu().numpy(), l_ref), k
+    with GraphCut(200, 32, use_graph=graph, max_cycles=1) as gc:
+        gc.upload_capacities(*corridors(200, 32, 150, 1))
+        gc.startBfs()
+        with pytest.raises(_gcut.GCError):
+            gc.cut()      # the excess is too far from the sinks for the first cycle
+        with pytest.raises(_gcut.GCError):
+            gc.isCompleted()
