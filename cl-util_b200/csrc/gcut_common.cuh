@@ -80,11 +80,9 @@ enum TileFlag { TF_POS = 1, TF_SINK = 2, TF_POS_UP = 4, TF_POS_DOWN = 8, TF_POS_
                 TF_POS_RIGHT = 32, TF_SINK_UP = 64, TF_SINK_DOWN = 128, TF_SINK_LEFT = 256,
                 TF_SINK_RIGHT = 512, TF_BAD = 1024 };
 
-// Grid barrier words, in separate 128-byte lines: two arrival words of the running k_solve
-// (low half: arrivals, bits 32-62: a sum over the CTAs, bit 63: abort) and the CTAs that left
-// it.  The last CTA to leave clears all for the next launch.
+// Grid barrier words, in separate 128-byte lines: two arrival words of the running k_solve (see
+// bar_arrivals) and the CTAs that left it.  The last CTA to leave clears all for the next launch.
 enum BarSlot { BAR_ARRIVE = 0, BAR_STRIDE = 16, BAR_EXIT = 32, BAR_N = 48 };
-constexpr unsigned long long GC_BAR_ABORT = 1ull << 63;
 
 // Walks consecutive selected indices: the tile of index i, with the range found once by a
 // binary search over the ranges' first indices and then followed range by range.

@@ -101,9 +101,37 @@ struct SolveState {
   int nf, nb, np;           // flood rounds, relabel rounds, pulses of the solve
   int err;
   int push;                 // tiles this CTA has queued since the last barrier
-  unsigned bar;             // barriers passed
-  unsigned last[2];         // sums of the barrier words' last uses
+  unsigned long long bar;   // barriers passed
+  unsigned last[2];         // sum halves that the barrier words' last uses left
 };
+
+// A grid barrier word: the low half counts arrivals, bits 32-62 hold a sum over the CTAs (tiles
+// queued since the last barrier), bit 63 ends the solve.  Barriers alternate between two words,
+// and no CTA reaches a word's next use before all have left this one, so a use is over exactly
+// when the low half stands at the arrivals of all uses so far, modulo 2^32: no number of
+// barriers is too many.  When the low half wraps, its carry adds one to the sum of that use.
+constexpr unsigned long long GC_BAR_ABORT = 1ull << 63;
+GC_HD unsigned long long bar_arrivals(const SolveState& s, unsigned ctas) {   // before this use
+  return (s.bar >> 1) * ctas;
+}
+// What a CTA adds; CTA 0 takes out what the word's last use left in the sum half, which so never
+// falls below zero.
+GC_HD unsigned long long bar_add(const SolveState& s, bool cta0) {
+  const unsigned long long add = ((unsigned long long)(unsigned)s.push << 32) + 1ull;
+  return cta0 ? add - ((unsigned long long)s.last[s.bar & 1] << 32) : add;
+}
+GC_HD bool bar_full(const SolveState& s, unsigned ctas, unsigned long long word) {
+  return (unsigned)word == (unsigned)(bar_arrivals(s, ctas) + ctas);
+}
+// The sum of a use that is over; passes the barrier.
+GC_HD unsigned bar_pass(SolveState& s, unsigned ctas, unsigned long long word) {
+  const unsigned long long before = bar_arrivals(s, ctas);
+  const unsigned sum = (unsigned)(word >> 32) & 0x7fffffffu;
+  s.push = 0;
+  s.last[s.bar & 1] = sum;
+  ++s.bar;
+  return sum - (unsigned)(((before + ctas) >> 32) - (before >> 32));
+}
 
 // Worklist counter that a step adds the tiles it lists to (a pulse: the next worklist's), and
 // the one that it clears for a later step (-1: none).  next_step reads a list's or relabel's

@@ -2017,28 +2017,22 @@ __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long lon
 
 // Grid barrier and step change: every CTA's writes before it are visible to every CTA after
 // it, its bulk copies included, and `s` holds the next step.  The CTAs' counts of queued tiles
-// travel in the upper half of the arrival word, so the loop decision needs no second trip to L2
-// (0.35 us).  Barriers alternate between two words: no CTA reaches a word's next use before all
-// have left this one, so what they read of it is the same.  A solve that was aborted ends.
+// travel in the arrival word, so the loop decision needs no second trip to L2 (0.35 us).  What
+// the CTAs read of a full word is the same.  A solve that was aborted ends.
 __device__ __forceinline__ void solve_barrier(const PoolView& P, const SolveArgs& A, SolveState& s) {
   // this thread's writes to the planes, before later bulk copies (a flood writes none)
   if (s.step != ST_FLOOD_FIRST && s.step != ST_FLOOD) asm volatile("fence.proxy.async;" ::: "memory");
   __syncthreads();
   if (threadIdx.x == 0) {
-    unsigned long long* const word = P.bar + BAR_ARRIVE + (s.bar & 1) * BAR_STRIDE;
-    const unsigned target = gridDim.x * ((s.bar >> 1) + 1);
-    // CTA 0 takes the word's previous sum out again: the upper half is never negative
-    unsigned long long add = ((unsigned long long)(unsigned)s.push << 32) + 1ull;
-    if (blockIdx.x == 0) add -= (unsigned long long)s.last[s.bar & 1] << 32;
+    unsigned long long* const word = P.bar + BAR_ARRIVE + (int)(s.bar & 1) * BAR_STRIDE;
     __threadfence();
-    atomicAdd(word, add);
-    s.push = 0;
+    atomicAdd(word, bar_add(s, blockIdx.x == 0));
     bool ok = false;
     unsigned long long t0 = 0, v = 0;
     for (unsigned i = 1; i < (1u << 31); ++i) {
       v = ld_acquire(word);
       if (v & GC_BAR_ABORT) break;
-      if ((unsigned)v >= target) { ok = true; break; }
+      if (bar_full(s, gridDim.x, v)) { ok = true; break; }
       if ((i & 1023u) == 0) {
         const unsigned long long now = global_ns();
         if (t0 == 0) t0 = now;
@@ -2052,18 +2046,14 @@ __device__ __forceinline__ void solve_barrier(const PoolView& P, const SolveArgs
     }
     __threadfence();
     asm volatile("fence.proxy.async;" ::: "memory");
-    const unsigned total = (unsigned)(v >> 32) & 0x7fffffffu;
-    s.last[s.bar & 1] = total;
-    ++s.bar;
-    // the arrivals' half must not overflow into the sum (after 2^32 arrivals: hours)
-    if (!ok || target >= 0xffff0000u) {
+    if (!ok) {
       s.err = 5;
       s.step = ST_END;
     } else {
-      const int was = s.step;
-      next_step(P.ctl, P.nt, A, s, (int)total);
+      const int total = (int)bar_pass(s, gridDim.x, v), was = s.step;
+      next_step(P.ctl, P.nt, A, s, total);
       if (blockIdx.x == 0 && total == 0 && (was == ST_FLOOD_FIRST || was == ST_FLOOD)) trace_record(P, TR_CHECK);
-      if (s.err == 4) record_bad(P, 6, (int)total);
+      if (s.err == 4) record_bad(P, 6, total);
     }
   }
   __syncthreads();

@@ -1,7 +1,8 @@
 // Steps the decisions of a one-launch solve (csrc/gcut_schedule.h) for two CTAs, one of which
 // is always a whole step ahead: it has decided the next step and done that step's counting
 // before the other reads the counters of the step both have finished.  The steps' outcomes are
-// random.  Prints the first disagreement and returns 1, else returns 0.
+// random.  Then grid barriers around the wrap of their arrival counts.  Prints the first
+// disagreement and returns 1, else returns 0.
 #include <cstdio>
 #include <cstring>
 #include <random>
@@ -74,9 +75,38 @@ int run(unsigned seed, bool ahead_is_cta0) {
   return 0;
 }
 
+// Barriers of `ctas` CTAs whose words start `left` uses before their arrivals reach a multiple of
+// 2^32: every use is over at its last arrival only, and its sum is what the CTAs queued.
+int barriers(unsigned ctas, unsigned left, unsigned seed) {
+  std::mt19937 rng(seed);
+  SolveState s{};
+  const unsigned long long uses = (1ull << 32) / ctas - left;
+  s.bar = 2 * uses;
+  unsigned long long word[2] = {(uses * ctas) & 0xffffffffull, (uses * ctas) & 0xffffffffull};
+  for (int k = 0; k < 40; ++k) {
+    unsigned long long& w = word[s.bar & 1];
+    unsigned want = 0;
+    const unsigned zero = rng() % ctas;   // CTA 0 comes at any time among the others
+    for (unsigned c = 0; c < ctas; ++c) {
+      if (bar_full(s, ctas, w)) return std::printf("%u CTAs: over after %u\n", ctas, c), 1;
+      s.push = rng() % 3 ? 0 : rng() % 1000;
+      want += s.push;
+      w += bar_add(s, c == zero);
+      if (w & GC_BAR_ABORT) return std::printf("%u CTAs: aborted\n", ctas), 1;
+    }
+    if (!bar_full(s, ctas, w)) return std::printf("%u CTAs: not over\n", ctas), 1;
+    const unsigned got = bar_pass(s, ctas, w);
+    if (got != want) return std::printf("%u CTAs: a sum of %u, not %u\n", ctas, got, want), 1;
+  }
+  return 0;
+}
+
 }  // namespace
 
 int main() {
+  for (unsigned ctas : {1u, 2u, 3u, 128u, 443u, 444u})
+    for (unsigned left = 0; left < 8; ++left)
+      if (barriers(ctas, left, 8 * ctas + left)) return 1;
   for (unsigned seed = 0; seed < 20000; ++seed)
     for (int cta0 = 0; cta0 < 2; ++cta0)
       if (run(seed, cta0)) return 1;
