@@ -170,6 +170,7 @@ struct Pool {
   int32_t* trace_words = nullptr;   // device: trace on/off and entry count (P.trace_ctl when on)
   bool one_launch = false;          // the last solve ran as one launch (k_solve)
   bool lists_stale = false;         // worklists, counters, stamps or sums may be left over
+  bool marks_stale = false;         // frontier marks may be left over (see begin_rounds)
   int stamp_base = 0;               // no stamp in img_hit is above this
   gc_stats stats{};
   // profiling: event pairs around every launch, tiles processed per kernel kind
@@ -584,6 +585,16 @@ struct Pool {
     return frontier_rounds(s, /*flood=*/false, GC_HINF);
   }
 
+  // Before a call's first frontier round.  A loop of rounds that ran to its end has cleared every
+  // tile's mark; one that did not (the round cap, an aborted solve) leaves those of the tiles it
+  // queued last, which no later round would queue again.
+  int begin_rounds(cudaStream_t s) {
+    if (marks_stale)
+      for (int k = 0; k < 2; ++k) CK(cudaMemsetAsync(P.mark[k], 0, sizeof(int32_t) * nt, s));
+    marks_stale = true;   // until the call has succeeded
+    return GC_OK;
+  }
+
   // host-driven rounds over the marked tiles until a round finds none; the host reads
   // the control words once per batch of rounds
   int frontier_rounds(cudaStream_t s, bool flood, int cap, int abort_hit = 0, int stamp = 0) {
@@ -668,7 +679,7 @@ struct Pool {
     const bool bfs = bfs_fresh;
     bfs_fresh = false;    // a solve that fails leaves no distances to go by
     // left by manual steps, a host-driven or a failed solve: worklist flags, barrier and control
-    // words, stamps, sums
+    // words, stamps, sums (frontier marks: begin_rounds)
     if (lists_stale || stamp_base > (1 << 30)) {
       CK(cudaMemsetAsync(P.inq[0], 0, sizeof(int32_t) * nt, s));
       CK(cudaMemsetAsync(P.inq[1], 0, sizeof(int32_t) * nt, s));
@@ -679,6 +690,7 @@ struct Pool {
       stamp_base = 0;
     }
     lists_stale = true;   // until this solve succeeds
+    RK(begin_rounds(s));
     int r = host ? solve_host(s, warm, fresh, idx, n) : solve_launch(s, warm, fresh, idx, n, after, lmode, lbuf);
     if (r) return r;
     edit_pending = false;   // the solve followed the edits, and the host has waited for it
@@ -687,6 +699,7 @@ struct Pool {
       CK(cudaStreamSynchronize(s));
     }
     RK(finish_check(s, idx, n, /*err_in_ctl=*/true));
+    marks_stale = false;
     one_launch = false;
     // a one-launch solve leaves everything clean (its results reached the host directly);
     // the host-driven loop leaves worklist flags, stamps and sums
@@ -894,7 +907,9 @@ struct Pool {
     bool warm;
     RK(select_all(&warm, s));
     RK(launch_ctl_begin(P, opts.max_bfs_rounds, acc, s));
+    RK(begin_rounds(s));
     RK(global_relabel(s));
+    marks_stale = false;
     RK(compact(P.tact, s));
     RK(launch_ctl_cycle(P, s));
     list_valid = true;
@@ -916,8 +931,10 @@ struct Pool {
     if (*done) {
       lists_stale = true;   // the flood leaves its sums and stamps
       RK(launch_acc_reset(acc, (int)imgs.size(), s));
+      RK(begin_rounds(s));
       RK(launch_flood_round(P, 1, 0, 1, acc, grid_warps, s));
       RK(frontier_rounds(s, /*flood=*/true, 0, 0, 1));
+      marks_stale = false;
       CK(cudaMemcpyAsync(h_acc, acc, sizeof(ImageAcc) * imgs.size(), cudaMemcpyDeviceToHost, s));
       RK(read_ctl(s));
       RK(finish_check(s));

@@ -127,3 +127,30 @@ def test_is_completed_after_a_cut(cuda, oracle, graph):
             gc.cut()      # the excess is too far from the sinks for the first cycle
         with pytest.raises(_gcut.GCError):
             gc.isCompleted()
+
+
+@pytest.mark.parametrize("graph,first,left_over", [(True, "cut", 13), (False, "cut", 9),
+                                                   (True, "startBfs", 16), (False, "startBfs", 16)])
+def test_solve_after_one_that_ran_out_of_rounds(cuda, oracle, graph, first, left_over):
+    """A row of 24 tiles whose cut or startBfs needs more rounds than allowed fails with a tile
+    still queued for the next round (the host-driven rounds run on to the end of their batch).  The
+    t-links then change so that excess and sink are in the tiles beside that one: the next cut,
+    whose flood has to queue it, is the oracle's."""
+    import _gcut
+    w, h = 32 * 24, 32
+    up, down, left, right, excess = (np.zeros((h, w), np.int32) for _ in range(5))
+    left[16, 1:] = 5   # none to the right, where the floods would go on to the end of the row
+    far = [32 * 22 + 4, 32 * 3 + 20]
+    excess[16, far] = 7, -6
+    with GraphCut(w, h, use_graph=graph, max_bfs_rounds=9) as gc:
+        gc.upload_capacities(up, down, left, right, excess)
+        with pytest.raises(_gcut.GCError):
+            getattr(gc, first)()
+        idx = 16 * w + np.array([*far, 32 * (left_over + 1) + 4, 32 * (left_over - 1) + 20])
+        val = np.array([0, 0, 7, -6])
+        gc.edit_tlinks(idx, val)
+        excess.flat[idx] = val
+        f_ref, l_ref = oracle.maxflow_bk(up, down, left, right, excess)
+        lab = gc.cut_labels()
+        assert gc.flow == f_ref == 5
+        assert np.array_equal(lab.cpu().numpy(), l_ref)
