@@ -725,7 +725,7 @@ struct Pool {
   int solve_host(cudaStream_t s, bool warm, bool fresh, const int* idx, int count) {
     RK(prof_begin(s));
     RK(launch_ctl_begin(P, opts.max_bfs_rounds, acc, s));
-    int n = 0, cap = kFirstCap, hlim = kFirstLimit, stamp = 1;
+    int n = 0, cap = first_cap(opts.initial_relabel), hlim = kFirstLimit, stamp = 1;
     auto list_active = [&](int first) {
       RK(timed(K_COMPACT, s, [&] { return launch_active_list(P, scan.st, list, counts, stamp + 1, first, 2 * sms, s); }));
       return read_count(s, &n);
@@ -742,7 +742,7 @@ struct Pool {
         RK(list_active(0));
         hlim = cap < GC_HINF ? cap + 1 : GC_HINF;
         const bool last = cap >= GC_HINF;
-        cap = next_cap(cap);
+        cap = cap_after(cap, mode == 3 && opts.initial_relabel);
         if (n > 0 || last) break;
       }
       return GC_OK;
@@ -815,7 +815,7 @@ struct Pool {
     a.pulses = opts.pulses_per_relabel;
     a.max_rounds = opts.max_bfs_rounds;
     a.max_cycles = opts.max_cycles;
-    a.cap = kFirstCap;
+    a.cap = first_cap(opts.initial_relabel);
     a.lmode = lmode;
     a.labels = lbuf;
     a.im = imgs[0];

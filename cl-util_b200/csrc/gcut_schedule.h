@@ -75,6 +75,9 @@ constexpr int kFirstLimit = 4;
 constexpr int kFirstCap = 8;
 constexpr int kLastCap = 1 << 12;   // above it: exact distances
 GC_HD int next_cap(int cap) { return cap >= kLastCap ? GC_HINF : cap * 2; }
+// initial_relabel: the relabel before the first pulses is exact, and the caps start after it.
+GC_HD int first_cap(int initial_relabel) { return initial_relabel ? GC_HINF : kFirstCap; }
+GC_HD int cap_after(int cap, bool initial) { return initial && cap >= GC_HINF ? kFirstCap : next_cap(cap); }
 
 // What the decisions of a one-launch solve depend on.
 struct SolvePlan {
@@ -82,7 +85,7 @@ struct SolvePlan {
   int warm, fresh;          // some selected image continues from a flow / is freshly uploaded
   int iters, pulses;        // sweeps per discharge, discharges per cycle
   int max_rounds, max_cycles;
-  int cap;                  // distance cap of the first relabel
+  int cap;                  // distance cap of the first relabel (first_cap)
 };
 
 // The solve's loop state, one copy per CTA in shared memory, written by thread 0 only (inside
@@ -205,7 +208,7 @@ GC_HD void next_step(const volatile int32_t* ctl, int nt, const SolvePlan& A, So
         break;
       }
       s.hlim = s.cap < GC_HINF ? s.cap + 1 : GC_HINF;
-      s.cap = next_cap(s.cap);   // further out with every cycle
+      s.cap = cap_after(s.cap, s.cyc == 0 && A.cap >= GC_HINF);   // further out with every cycle
       if (s.cyc == 0 && A.fresh) {
         s.step = ST_LIST;
         list = -1;

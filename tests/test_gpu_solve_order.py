@@ -154,3 +154,19 @@ def test_solve_after_one_that_ran_out_of_rounds(cuda, oracle, graph, first, left
         lab = gc.cut_labels()
         assert gc.flow == f_ref == 5
         assert np.array_equal(lab.cpu().numpy(), l_ref)
+
+
+@pytest.mark.parametrize("graph", [True, False])
+def test_initial_relabel_is_exact(cuda, oracle, graph):
+    """initial_relabel: one global relabel, without a distance cap, before the first pulse, also
+    where all excess is further from the sinks than any first cap."""
+    planes = corridors(600, 64, 300, 2)
+    f_ref, l_ref = oracle.maxflow_bk(*planes)
+    with GraphCut(600, 64, use_graph=graph, initial_relabel=True) as gc:
+        gc.upload_capacities(*planes)
+        gc.set_trace(True)
+        lab = gc.cut_labels()
+        kinds = [k for k, _ in gc.trace()]
+        assert gc.flow == f_ref
+        assert np.array_equal(lab.cpu().numpy(), l_ref)
+        assert kinds[:kinds.index("discharge")].count("bfs_first") == 1
