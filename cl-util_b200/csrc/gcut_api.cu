@@ -240,15 +240,20 @@ struct Pool {
   // (track moves done_ev to whatever stream a call came on), and every call that touches the
   // planes waits for it on its own stream, whichever that is, until a solve has waited for one
   // of them on the host.
+  // A call captured into a CUDA graph runs whenever that graph is launched, and cannot wait for
+  // an edit made since: so once a call was captured, edits return only when they have run.
   cudaEvent_t edit_ev = nullptr;
   bool edit_pending = false;
+  bool captured = false;
   int order(cudaStream_t s) {
-    if (!edit_pending) return GC_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(s, &cap));
     if (cap == cudaStreamCaptureStatusNone) {
-      CK(cudaStreamWaitEvent(s, edit_ev, 0));
-    } else {   // a capture cannot wait for an event outside it: the host does
+      if (edit_pending) CK(cudaStreamWaitEvent(s, edit_ev, 0));
+      return GC_OK;
+    }
+    captured = true;
+    if (edit_pending) {   // a capture cannot wait for an event outside it: the host does
       cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
       CK(cudaThreadExchangeStreamCaptureMode(&mode));
       const cudaError_t e = cudaEventSynchronize(edit_ev);
@@ -1380,7 +1385,7 @@ int gc_edit_tlinks(gc_handle* h, const int32_t* idx, const int32_t* value, int n
 
 // Rasterises an edit's polyline (brush: the reference brush's pixel set) into image img.
 // Short polylines travel in the launch; longer ones are copied, and the call waits for the copy
-// out of its own memory.
+// out of its own memory (and see order).
 static int pool_edit(Pool& p, int img, const int32_t* xs, const int32_t* ys, int npts, int radius,
                      int32_t value, bool brush, cudaStream_t s) {
   CK(cudaSetDevice(p.device));
@@ -1396,7 +1401,7 @@ static int pool_edit(Pool& p, int img, const int32_t* xs, const int32_t* ys, int
   else RK(launch_stroke(p.P, p.imgs[img], img, p.pts, pts.data(), npts, radius, value, p.tl, p.acc, s));
   p.track(s);
   p.edited_image(img);
-  if (copy) {
+  if (copy || p.captured) {
     CK(cudaStreamSynchronize(s));
     p.edit_pending = false;
   } else {

@@ -170,3 +170,28 @@ def test_initial_relabel_is_exact(cuda, oracle, graph):
         assert gc.flow == f_ref
         assert np.array_equal(lab.cpu().numpy(), l_ref)
         assert kinds[:kinds.index("discharge")].count("bfs_first") == 1
+
+
+def test_replay_of_an_upload_after_an_edit(cuda, oracle):
+    """An upload captured into a CUDA graph is launched on another stream after a stroke that was
+    held back on its own: the upload comes last, and the cut is the uploaded graph's."""
+    import synth
+    g = synth.make_graph(130, 70, 8)
+    planes = [cuda.from_numpy(p).cuda() for p in g.planes()]
+    f_ref, l_ref = oracle.maxflow_bk(*g.planes())
+    a, b = cuda.cuda.Stream(), cuda.cuda.Stream()
+    with GraphCut(g.width, g.height) as gc:
+        gc.upload_capacities(*planes)
+        gc.cut()
+        graph = cuda.cuda.CUDAGraph()
+        with cuda.cuda.graph(graph):
+            gc.upload_capacities(*planes)
+        for _ in range(2):
+            with cuda.cuda.stream(a):
+                cuda.cuda._sleep(20_000_000)
+            gc.edit_stroke([3, 100], [5, 60], 4, 500, stream=a)
+            with cuda.cuda.stream(b):
+                graph.replay()
+            cuda.cuda.synchronize()
+            assert np.array_equal(gc.cut_labels().cpu().numpy(), l_ref)
+            assert gc.flow == f_ref
