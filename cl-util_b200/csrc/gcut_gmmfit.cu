@@ -176,7 +176,9 @@ k_gmm_fit(const uint32_t* __restrict__ samples, int n, int K, int max_iter, doub
     double d1[2] = {0.0, 0.0}, d2[2] = {0.0, 0.0}, lsum = 0.0;
     for (int i0 = rank * kThreads + warp * 32; i0 < n; i0 += stride) {   // warp-uniform
       const int i = i0 + lane;
-      const uint32_t px = i < n ? samples[i] : 0u;
+      // lanes past the end repeat the last sample and count 0 times: 0 times the responsibilities
+      // of any other colour need not be 0, where no component is within reach of it
+      const uint32_t px = samples[i < n ? i : n - 1];
       const double x0 = (double)(px & 0xFFu), x1 = (double)((px >> 8) & 0xFFu),
                    x2 = (double)((px >> 16) & 0xFFu);
       double e[KMAX];
