@@ -174,11 +174,12 @@ k_gmm_fit(const uint32_t* __restrict__ samples, int n, int K, int max_iter, doub
     const int buf = t & 1;
     // E-step (em1): responsibilities and their moment sums
     double d1[2] = {0.0, 0.0}, d2[2] = {0.0, 0.0}, lsum = 0.0;
-    for (int i0 = rank * kThreads + warp * 32; i0 < n; i0 += stride) {   // warp-uniform
-      const int i = i0 + lane;
+    // (unsigned: the index passes n, which may be near 2^31, by up to a stride)
+    for (unsigned i0 = rank * kThreads + warp * 32; i0 < (unsigned)n; i0 += stride) {   // warp-uniform
+      const unsigned i = i0 + lane;
       // lanes past the end repeat the last sample and count 0 times: 0 times the responsibilities
       // of any other colour need not be 0, where no component is within reach of it
-      const uint32_t px = samples[i < n ? i : n - 1];
+      const uint32_t px = samples[i < (unsigned)n ? i : (unsigned)n - 1];
       const double x0 = (double)(px & 0xFFu), x1 = (double)((px >> 8) & 0xFFu),
                    x2 = (double)((px >> 16) & 0xFFu);
       double e[KMAX];
@@ -202,8 +203,8 @@ k_gmm_fit(const uint32_t* __restrict__ samples, int n, int K, int max_iter, doub
           e[k] = exp(e[k] - m);
           s += e[k];
         }
-      if (i < n) lsum += m + log(s);
-      const double inv = i < n ? 1.0 / s : 0.0;
+      if (i < (unsigned)n) lsum += m + log(s);
+      const double inv = i < (unsigned)n ? 1.0 / s : 0.0;
       __syncwarp();   // the last step's reads of the rows
 #pragma unroll
       for (int k = 0; k < KMAX; ++k)
