@@ -126,6 +126,15 @@ GC_HD unsigned long long bar_add(const SolveState& s, bool cta0) {
 GC_HD bool bar_full(const SolveState& s, unsigned ctas, unsigned long long word) {
   return (unsigned)word == (unsigned)(bar_arrivals(s, ctas) + ctas);
 }
+// How long a CTA waits for the others, in ns: 5 s, far beyond any step's passes over the largest
+// pool, and 4 us a sweep of the tiles a CTA may have in a pulse (a sweep takes 0.5 to 2 us; how
+// many there are is the caller's option, without a limit).
+GC_HD unsigned long long bar_wait_ns(const SolveState& s, unsigned ctas) {
+  if (s.step != ST_PULSE) return 5000000000ull;
+  const unsigned long long sweeps = ((unsigned)s.n / ctas + 1ull) * (unsigned)s.iters;
+  const unsigned long long most = 1ull << 50;
+  return 5000000000ull + 4000ull * (sweeps < most ? sweeps : most);
+}
 // The sum of a use that is over; passes the barrier.
 GC_HD unsigned bar_pass(SolveState& s, unsigned ctas, unsigned long long word) {
   const unsigned long long before = bar_arrivals(s, ctas);

@@ -2005,10 +2005,6 @@ __global__ void k_labels_packed(PoolView P, ImageDesc im, uint8_t* out) {
 // and a drain, and 5-11 us per conditional node: 256x192 98-169 us from upload to labels against
 // 35-71 now, 2048x2048 300-690 against 145-230, strokes at 4096x4096 210-650 against 112-123.
 // ------------------------------------------------------------------------------------
-// A barrier wait gives up after this long (a step of the largest pool takes well under a
-// second): it raises the abort flag, and every CTA leaves at its next barrier.
-constexpr unsigned long long GC_BARRIER_WAIT_NS = 5000000000ull;
-
 __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p) {
   unsigned long long v;
   asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
@@ -2018,7 +2014,8 @@ __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long lon
 // Grid barrier and step change: every CTA's writes before it are visible to every CTA after
 // it, its bulk copies included, and `s` holds the next step.  The CTAs' counts of queued tiles
 // travel in the arrival word, so the loop decision needs no second trip to L2 (0.35 us).  What
-// the CTAs read of a full word is the same.  A solve that was aborted ends.
+// the CTAs read of a full word is the same.  A wait gives up after bar_wait_ns: it raises the
+// abort flag, and every CTA leaves at its next barrier.  A solve that was aborted ends.
 __device__ __forceinline__ void solve_barrier(const PoolView& P, const SolveArgs& A, SolveState& s) {
   // this thread's writes to the planes, before later bulk copies (a flood writes none)
   if (s.step != ST_FLOOD_FIRST && s.step != ST_FLOOD) asm volatile("fence.proxy.async;" ::: "memory");
@@ -2036,7 +2033,7 @@ __device__ __forceinline__ void solve_barrier(const PoolView& P, const SolveArgs
       if ((i & 1023u) == 0) {
         const unsigned long long now = global_ns();
         if (t0 == 0) t0 = now;
-        else if (now - t0 > GC_BARRIER_WAIT_NS) {
+        else if (now - t0 > bar_wait_ns(s, gridDim.x)) {
           atomicCAS(&P.ctl[CTL_ERR], 0, 5);
           __threadfence();
           abort_solve(P);

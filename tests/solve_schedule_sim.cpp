@@ -101,9 +101,27 @@ int barriers(unsigned ctas, unsigned left, unsigned seed) {
   return 0;
 }
 
+// A barrier waits longer than a pulse can take: 2 us a sweep, all sweeps of all a CTA's tiles.
+int waits() {
+  for (const int iters : {1, 1000, 10000000, 2147483647})
+    for (const int n : {1, 444, 445, 1 << 26})
+      for (const unsigned ctas : {1u, 444u}) {
+        SolveState s{};
+        s.step = ST_PULSE;
+        s.n = n;
+        s.iters = iters;
+        const double takes = 2e3 * iters * ((n + ctas - 1) / ctas);
+        const unsigned long long ns = bar_wait_ns(s, ctas);
+        if ((double)ns < (takes < 4e18 ? takes : 4e18))
+          return std::printf("%d tiles, %u CTAs, %d sweeps: %llu ns\n", n, ctas, iters, ns), 1;
+      }
+  return 0;
+}
+
 }  // namespace
 
 int main() {
+  if (waits()) return 1;
   for (unsigned ctas : {1u, 2u, 3u, 128u, 443u, 444u})
     for (unsigned left = 0; left < 8; ++left)
       if (barriers(ctas, left, 8 * ctas + left)) return 1;
