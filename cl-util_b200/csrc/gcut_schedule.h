@@ -63,7 +63,9 @@ GC_HD int cycle_pulses(int pulses, int cycle) {
   const long long p = (long long)pulses << shift;
   return p < most ? (int)p : most;
 }
-GC_HD int cycle_iters(int iters, int cycle) { return cycle == 0 ? iters : iters + 3; }
+GC_HD int cycle_iters(int iters, int cycle) {
+  return cycle == 0 || iters > 0x7fffffff - 3 ? iters : iters + 3;   // (any positive count is an option)
+}
 // Active heights before the first relabel, whose trivial labels (0 at sinks, 1 elsewhere) say
 // little: below 4, excess far from a sink stops rising after three sweeps instead of keeping
 // its warps busy.  (3: more cycles; unlimited: 512^2 3 %, 64 grids 4 % slower.)

@@ -118,10 +118,21 @@ int waits() {
   return 0;
 }
 
+// Any positive option gives positive counts in every cycle, none below the first cycle's.
+int counts() {
+  for (const int k : {1, 3, 17, 2147483644, 2147483645, 2147483647})
+    for (int cycle = 0; cycle < 40; ++cycle) {
+      const volatile int sweeps = cycle_iters(k, cycle), pulses = cycle_pulses(k, cycle);
+      if (sweeps < k || pulses < k)
+        return std::printf("%d: %d sweeps, %d pulses in cycle %d\n", k, sweeps, pulses, cycle), 1;
+    }
+  return 0;
+}
+
 }  // namespace
 
 int main() {
-  if (waits()) return 1;
+  if (waits() || counts()) return 1;
   for (unsigned ctas : {1u, 2u, 3u, 128u, 443u, 444u})
     for (unsigned left = 0; left < 8; ++left)
       if (barriers(ctas, left, 8 * ctas + left)) return 1;
