@@ -318,7 +318,6 @@ struct Pool {
       P.sel_mode = reinterpret_cast<int32_t*>(P.sel + imgs.size());
     }
     c.take(&P.tpos, nt);
-    c.take(&P.rcnt, 2);
     c.take(&P.ctl, CTL_N);
     c.take(&acc, imgs.size());
     c.take(&ktiles, GC_NKERN);

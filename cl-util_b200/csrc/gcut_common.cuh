@@ -39,7 +39,6 @@ struct PoolView {
   int32_t* touched;       // [nt] tile was discharged or received cross-tile flow
   int32_t* act_int;       // [nt] tile has an active interior pixel after its discharge
   int32_t* mark[2];       // [nt] BFS / flood-fill frontier marks, alternating by round
-  int32_t* rcnt;          // [2] tiles processed by the current / next frontier round
   int32_t* ctl;           // [CTL_N] device-side loop control (see CtlSlot)
   int32_t* queue[2];      // [nt] active-tile worklists, alternating by pulse
   int32_t* qcount;        // [2] worklist lengths

@@ -50,15 +50,10 @@ struct ImageAcc {
 };
 
 // Solver kernels (gcut_solver.cu).
-struct Launch {
-  int grid_discharge;   // persistent CTAs for the discharge kernel
-  int grid_warps;       // CTAs (4 warps each) for the per-tile warp kernels
-};
-
 int launch_upload(const PoolView& P, const ImageDesc& im, int img, const int32_t* up,
                   const int32_t* down, const int32_t* left, const int32_t* right,
                   const int32_t* excess, int32_t* tl, ImageAcc* acc, cudaStream_t s);
-// reads the worklist queue[ctl[CTL_PULSE] & 1], builds the other one
+// rebuilds the row masks of the selected tiles whose planes changed since they were written
 int launch_masks(const PoolView& P, int grid, cudaStream_t s);
 
 // n-link table of gc_upload_rgba: weight(d) = floor(50 * exp(-beta * d) + 0.5) for d = |dI|^2
@@ -73,7 +68,8 @@ int launch_upload_rgba(const PoolView& P, const ImageDesc& im, int img, const ui
 // one launch; state: two zeroed words, zero again afterwards.  Clears *acc for the upload.
 int launch_nlinks(const uint32_t* rgba, int W, int H, unsigned long long* state, int32_t* tab,
                   ImageAcc* acc, int sms, cudaStream_t s);
-// hlim: pixels below this height are active
+// reads the worklist queue[ctl[CTL_PULSE] & 1], builds the other one; hlim: pixels below this
+// height are active
 int launch_discharge(const PoolView& P, int iters, int hlim, int grid, cudaStream_t s);
 int launch_edge_relabel_build(const PoolView& P, int32_t* list, int32_t* count,
                               const ScanState& st, cudaStream_t s);

@@ -20,7 +20,7 @@ namespace gcut {
 enum CtlSlot {
   CTL_RND = 0,        // frontier round number (its parity selects the mark buffer)
   CTL_DONE = 1,       // CTAs finished in the current round
-  CTL_LASTCNT = 2,    // tiles processed by the last finished round
+  CTL_LASTCNT = 2,    // tiles the last finished round queued for the next
   CTL_ROUNDS = 3,     // rounds of the current frontier loop
   CTL_BFS_TOTAL = 4,  // BFS rounds of the solve
   CTL_FLOOD_TOTAL = 5,
@@ -53,7 +53,7 @@ enum CtlSlot {
 // A cycle costs a flood and a relabel over the images left (60 us at 2048^2) besides its
 // pulses (10 us each on a few hundred tiles).  Most solves end after one or two cycles, which
 // the options' own schedule suits; the excess left after that has to travel far, and then more
-// work between relabels pays: twice the sweeps from the second cycle, twice the pulses with
+// work between relabels pays: three more sweeps from the second cycle, twice the pulses with
 // each from the third.  Mean over 12 seeds against the fixed schedule 3 x 2 (and its worst
 // seed), one B200: 2048^2 1740 -> 515 us (13133 -> 3216), 512^2 424 -> 241, 803x607 under the
 // lamda rule 690 -> 317, 4096^2 image 1108 -> 974.

@@ -1270,7 +1270,6 @@ __device__ __forceinline__ void frontier_round_end(const PoolView& P, int first,
   __threadfence();
   volatile int32_t* ctl = P.ctl;
   const int out = in ^ 1;
-  P.rcnt[in] = 0;
   const int next = *((volatile int32_t*)&P.fcount[out]);
   P.fcount[in] = 0;   // this round's list is consumed
   ctl[CTL_LASTCNT] = next;
@@ -1309,8 +1308,6 @@ __global__ void k_ctl_begin(PoolView P, int max_rounds, ImageAcc* acc) {
   }
   if (threadIdx.x == 0) {
     P.ctl[CTL_MAXROUNDS] = max_rounds;
-    P.rcnt[0] = 0;
-    P.rcnt[1] = 0;
     P.fcount[0] = 0;
     P.fcount[1] = 0;
   }
@@ -1692,10 +1689,8 @@ k_bfs_round(PoolView P, int first, int cap, int live) {
     const int act = bfs_tile(P, t, lane, first, cap, tr[warp], out);
     if (lane == 0 && act >= 0) P.tact[t] = act;
   }
-  if (lane == 0 && done) {
-    atomicAdd(&P.rcnt[in], done);
-    if (P.ktiles) atomicAdd(&P.ktiles[first ? K_BFS_FIRST : K_BFS], (unsigned long long)done);
-  }
+  if (lane == 0 && done && P.ktiles)
+    atomicAdd(&P.ktiles[first ? K_BFS_FIRST : K_BFS], (unsigned long long)done);
   frontier_round_end(P, first, in, CTL_BFS_TOTAL, parts);
 }
 
@@ -1918,10 +1913,8 @@ k_flood_round(PoolView P, int mode, int abort_hit, int stamp, ImageAcc* acc) {
     if (first) flood_first_tile(P, t, lane, img, stamp, out, acc, fs);
     else flood_frontier_tile(P, t, lane, img, stamp, nullptr, out);
   }
-  if (lane == 0 && done) {
-    atomicAdd(&P.rcnt[in], done);
-    if (P.ktiles) atomicAdd(&P.ktiles[first ? K_FLOOD_FIRST : K_FLOOD], (unsigned long long)done);
-  }
+  if (lane == 0 && done && P.ktiles)
+    atomicAdd(&P.ktiles[first ? K_FLOOD_FIRST : K_FLOOD], (unsigned long long)done);
   if (first) flood_sum_flush<WARPS_PER_CTA>(acc, fs);
   frontier_round_end(P, first, in, CTL_FLOOD_TOTAL, parts);
 }
