@@ -237,8 +237,8 @@ class GraphCut:
 
     def cut_labels(self, out=None, packed=False, stream=None):
         """cut() and labels() (or labels_packed() with packed=True) in one call with one host
-        wait: the labels kernel follows the solve on the stream (gc_solve_labels).  Returns
-        the label tensor."""
+        wait: the solve's launch writes them as its last step (gc_solve_labels).  Returns the
+        label tensor."""
         import torch
         if out is None:
             shape = (self.height, (self.width + 7) // 8) if packed else (self.height, self.width)

@@ -61,8 +61,11 @@ typedef struct gc_opts {
   int max_cycles;          /* cap on global-relabel cycles; exceeded -> GC_ERR_NOT_CONVERGED */
   int max_bfs_rounds;      /* cap on tile rounds of one BFS / flood fill */
   int use_graph;           /* 1: the solve is one launch of a persistent cooperative kernel
-                              that decides its loops on the device (one host wait per solve);
-                              0: the host drives the loops (used when profiling is on) */
+                              that decides its loops on the device (one host wait per solve).
+                              From a few hundred tiles on its blocks fill the device until it
+                              ends, so other kernels, the solves of other handles among them,
+                              wait for it or hold it back; 0: the host drives the loops, a
+                              launch a step (used when profiling is on) */
 } gc_opts;
 
 typedef struct gc_stats {
@@ -95,7 +98,7 @@ int gc_arena_bytes(int width, int height, int64_t* bytes);
    alone allocates its staging on first use).  A server that sub-allocates one HBM region
    between sessions uses this to keep cudaMalloc / cudaFree, which synchronise the device,
    off its request path.  gc_destroy waits for the work of the handle's last call (on that
-   call's stream), after which the caller may reuse the memory.  No counterpart in the
+   call's stream) and for its last edit, after which the caller may reuse the memory.  No counterpart in the
    reference (GraphCut.__init__ allocates its buffers, GraphCut.pyx:117-154). */
 int gc_create_in(int width, int height, const gc_opts* opts, void* arena, int64_t bytes,
                  gc_handle** out);
@@ -225,9 +228,8 @@ int gc_solve(gc_handle* h, void* stream);
 
 /* gc_solve, then the canonical labels into the DEVICE buffer `labels` (packed != 0: the
    bit-packed rows of gc_labels_packed, else one byte per pixel as gc_labels), with one host
-   wait for both: the labels kernel is queued behind the solve on `stream` instead of after
-   the host has seen the solve finish.  On an error return the buffer's content is
-   unspecified. */
+   wait for both: the solve's launch writes them as its last step (the host-driven loop queues
+   the labels kernel behind itself).  On an error return the buffer's content is unspecified. */
 int gc_solve_labels(gc_handle* h, uint8_t* labels, int packed, void* stream);
 
 /* Manual stepping, mirroring the reference methods a caller can drive one at a time (the
@@ -237,8 +239,8 @@ int gc_solve_labels(gc_handle* h, uint8_t* labels, int packed, void* stream);
    rebuild (GraphCut.relabel, GraphCut.pyx:224-240); gc_start_bfs = exact global relabel
    and the active-tile list from it (GraphCut.startBfs, GraphCut.pyx:187-222);
    gc_is_completed = 1 when no pixel with excess > 0 can reach a sink pixel, valid right
-   after gc_start_bfs (GraphCut.isCompleted, GraphCut.pyx:328-346); it also computes the
-   canonical cut and the flow when it returns 1. */
+   after gc_start_bfs (GraphCut.isCompleted, GraphCut.pyx:328-346) and after solves that
+   succeeded since then; it also computes the canonical cut and the flow when it returns 1. */
 int gc_push(gc_handle* h, void* stream);
 int gc_relabel(gc_handle* h, void* stream);
 int gc_start_bfs(gc_handle* h, void* stream);
@@ -264,7 +266,11 @@ int gc_labels_packed_host(gc_handle* h, uint8_t* bits, void* stream);
    the previous flow.  Indices must be distinct within one call. */
 int gc_edit_tlinks(gc_handle* h, const int32_t* idx, const int32_t* value, int n, void* stream);
 /* Stroke edit: every pixel within `radius` of the polyline (xs[i], ys[i]), i < npts (host
-   arrays, integer pixel centres) gets t-link `value`.  Rasterised on the device. */
+   arrays, integer pixel centres) gets t-link `value`.  Rasterised on the device.  With up to 64
+   points the call returns before the edit has run; every later call on the handle, from any
+   stream, and gc_destroy come after it.  A CUDA graph that holds a captured call of the handle
+   (an upload, say) runs outside this order, so once a call was captured, edits return only when
+   they have run.  An edit itself cannot be captured (GC_ERR_CUDA). */
 int gc_edit_stroke(gc_handle* h, const int32_t* xs, const int32_t* ys, int npts, int radius,
                    int32_t value, void* stream);
 
